@@ -110,18 +110,21 @@ __device__ __forceinline__ void keccak_f1600(uint64_t (&a)[25]) {
 }
 
 // Keccak-f[1600] spread over a warp: lane t < 25 holds lane t = x + 5y of
-// the state, the other lanes carry copies that nothing reads.  A round is
-// ten 64-bit shuffles (theta's column sums, the two neighbour columns,
-// pi's lane permutation, chi's two row neighbours) around a handful of
-// integer ops per lane, so one permutation's latency is a few shuffle
-// round trips per round instead of one thread's whole serial chain: the
-// form for nodes whose many blocks would otherwise set a level's time.
+// the state, the other lanes carry copies that nothing reads.  One
+// permutation's latency is a few shuffle round trips per round instead of
+// one thread's whole serial chain: the form for nodes whose serial blocks
+// would otherwise set a level's time.  A round is three dependent shuffle
+// steps -- the four other words of the column, the two neighbour columns'
+// parities, and chi's three words fetched straight from the lanes pi takes
+// them from (chi after a separate pi step is a fourth round trip) -- nine
+// 64-bit shuffles around ~20 integer ops per lane.
 struct CoopLanes {
-  uint32_t col[5];   // theta: the lanes of this lane's column
+  uint32_t col[4];   // theta: the other lanes of this lane's column
   uint32_t cm1, cp1; // lanes holding column x - 1 and x + 1
-  uint32_t rot;      // rho offset of this lane
-  uint32_t src;      // pi: the lane whose rotated word lands here
-  uint32_t chi1, chi2;
+  uint32_t rot;      // rho offset of this lane, mod 32
+  bool swap;         // rho offset of 32 or more
+  uint32_t src[3];   // pi then chi: the lanes whose rotated words land at x, x + 1, x + 2 of this row
+  uint32_t iota;     // all ones in lane 0
 };
 
 __device__ __forceinline__ CoopLanes coop_lanes(int lane) {
@@ -132,46 +135,42 @@ __device__ __forceinline__ CoopLanes coop_lanes(int lane) {
   const uint32_t x = t % 5u, y = t / 5u;
   CoopLanes c;
 #pragma unroll
-  for (int k = 0; k < 5; ++k) c.col[k] = x + 5u * (uint32_t)k;
+  for (uint32_t k = 0; k < 4; ++k) c.col[k] = x + 5u * ((y + k + 1u) % 5u);
   c.cm1 = (x + 4u) % 5u;
   c.cp1 = (x + 1u) % 5u;
-  c.rot = kRho[t];
-  // pi: B[x'][y'] = A[x][y] with x' = y, y' = (2x + 3y) mod 5; here (x', y')
-  // = (x, y), so the source has y_s = x and x_s = 3 (y - 3x) mod 5
-  const uint32_t xs = (3u * (y + 15u - 3u * x)) % 5u, ys = x;
-  c.src = xs + 5u * ys;
-  c.chi1 = (x + 1u) % 5u + 5u * y;
-  c.chi2 = (x + 2u) % 5u + 5u * y;
-  return c;
-}
-
-__device__ __forceinline__ uint64_t rotl64_var(uint64_t v, uint32_t r) {
-  uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
-  if (r & 32u) {
-    const uint32_t t = lo;
-    lo = hi;
-    hi = t;
+  c.rot = kRho[t] & 31u;
+  c.swap = (kRho[t] & 32u) != 0u;
+  // pi: B[x'][y'] = A[x][y] with x' = y, y' = (2x + 3y) mod 5, so the word at
+  // (x', y') comes from y_s = x' and x_s = 3 (y' - 3x') mod 5
+#pragma unroll
+  for (uint32_t k = 0; k < 3; ++k) {
+    const uint32_t xk = (x + k) % 5u;
+    c.src[k] = (3u * (y + 15u - 3u * xk)) % 5u + 5u * xk;
   }
-  const uint32_t s = r & 31u;
-  const uint32_t nh = __funnelshift_l(lo, hi, s), nl = __funnelshift_l(hi, lo, s);
-  return ((uint64_t)nh << 32) | nl;
+  c.iota = lane == 0 ? 0xffffffffu : 0u;
+  return c;
 }
 
 // All 32 lanes call it together; returns this lane's state word after the
 // permutation.
-__device__ __forceinline__ uint64_t keccak_f1600_warp(uint64_t a, const CoopLanes &c, int lane) {
+__device__ __forceinline__ uint64_t keccak_f1600_warp(uint64_t a, const CoopLanes &c) {
   constexpr unsigned kAll = 0xffffffffu;
-#pragma unroll 1
+#pragma unroll 4
   for (int r = 0; r < 24; ++r) {
-    const uint64_t cs = __shfl_sync(kAll, a, c.col[0]) ^ __shfl_sync(kAll, a, c.col[1]) ^
-                        __shfl_sync(kAll, a, c.col[2]) ^ __shfl_sync(kAll, a, c.col[3]) ^
-                        __shfl_sync(kAll, a, c.col[4]);
+    const uint64_t cs = a ^ __shfl_sync(kAll, a, c.col[0]) ^ __shfl_sync(kAll, a, c.col[1]) ^
+                        __shfl_sync(kAll, a, c.col[2]) ^ __shfl_sync(kAll, a, c.col[3]);
     const uint64_t dm = __shfl_sync(kAll, cs, c.cm1), dp = __shfl_sync(kAll, cs, c.cp1);
     a ^= dm ^ rotl64(dp, 1);
-    const uint64_t b = __shfl_sync(kAll, rotl64_var(a, c.rot), c.src);
-    const uint64_t b1 = __shfl_sync(kAll, b, c.chi1), b2 = __shfl_sync(kAll, b, c.chi2);
-    a = b ^ (~b1 & b2);
-    if (lane == 0) a ^= kKeccakRC[r];
+    const uint32_t alo = (uint32_t)a, ahi = (uint32_t)(a >> 32);
+    const uint32_t lo = c.swap ? ahi : alo, hi = c.swap ? alo : ahi;
+    const uint32_t rh = __funnelshift_l(lo, hi, c.rot), rl = __funnelshift_l(hi, lo, c.rot);
+    const uint32_t l0 = __shfl_sync(kAll, rl, c.src[0]), l1 = __shfl_sync(kAll, rl, c.src[1]),
+                   l2 = __shfl_sync(kAll, rl, c.src[2]);
+    const uint32_t h0 = __shfl_sync(kAll, rh, c.src[0]), h1 = __shfl_sync(kAll, rh, c.src[1]),
+                   h2 = __shfl_sync(kAll, rh, c.src[2]);
+    const uint32_t nl = (l0 ^ (~l1 & l2)) ^ ((uint32_t)kKeccakRC[r] & c.iota);
+    const uint32_t nh = (h0 ^ (~h1 & h2)) ^ ((uint32_t)(kKeccakRC[r] >> 32) & c.iota);
+    a = ((uint64_t)nh << 32) | nl;
   }
   return a;
 }

@@ -1463,24 +1463,124 @@ __device__ __forceinline__ void hash_node(const TrieView &tv, uint32_t ref, uint
   }
 }
 
-// Message buffer of one warp for hash_full_warp (8 Keccak blocks).
+// Message buffer of one warp for the warp-cooperative hashing (8 Keccak blocks).
 constexpr int kWarpMsgBytes = 8 * 136;
+
+// Up to 32 bytes of a message item, in four little-endian words.
+struct Bytes32 {
+  uint64_t w[4];
+};
+
+// One lane's item of a message: at most 9 prefix bytes (pre, the header of a
+// string or a list; kept as 8 + the length) and a body that is in registers
+// when it has at most 32 bytes (a node's hash, a short value), else in memory.
+struct WarpItem {
+  uint64_t pre = 0;
+  uint32_t pren = 0, blen = 0;
+  Bytes32 body{};
+  const uint8_t *far = nullptr;  // body of more than 32 bytes
+};
+
+// The item a branch (or a short node) writes for child `r`: child_item with
+// the bytes of hashes and short values already loaded, every load of a lane
+// issued before the first is used.
+template <bool kCoh>
+__device__ __forceinline__ WarpItem warp_child_item(const TrieView &tv, uint32_t r) {
+  WarpItem it;
+  const uint32_t kind = ref_kind(r), idx = ref_idx(r);
+  if (kind == KIND_NULL) {
+    it.pre = 0x80;
+    it.pren = 1;
+    return it;
+  }
+  if (kind == KIND_VALUE) {
+    const unsigned long long vid = ldn<kCoh>(tv.value_vid + idx);
+    const ValueRec rc = load_rec(tv, vid);
+    const uint8_t *v = tv.vals + rc.off;
+    it.blen = rc.len;
+    if (rc.len > 32) {
+      it.far = v;
+    } else {
+#pragma unroll
+      for (uint32_t w = 0; w < 4; ++w)
+        if (8 * w < rc.len) it.body.w[w] = ld8<kCoh>(v + 8 * w);
+    }
+  } else {
+    const bool full = kind == KIND_FULL;
+    const ulonglong2 *h = reinterpret_cast<const ulonglong2 *>((full ? tv.full_hash : tv.short_hash) + (size_t)idx * 32);
+    const ulonglong2 a = __ldcg(h), b = __ldcg(h + 1);
+    it.blen = __ldcg((full ? tv.full_hlen : tv.short_hlen) + idx);
+    it.body = Bytes32{{a.x, a.y, b.x, b.y}};
+    if (tv.geth_mode && it.blen < 32) return it;  // go-ethereum embeds small nodes
+  }
+  if (it.blen == 1 && (uint8_t)it.body.w[0] < 0x80) return it;  // single byte is its own encoding
+  rlp_head(it.blen, 0x80, 0xb7, it.pre, it.pren);
+  return it;
+}
+
+// Bytes [0, n) of v at message position p, clipped to the window [lo, hi).
+__device__ __forceinline__ void put_prefix(uint8_t *msg, uint32_t lo, uint32_t hi, uint64_t v, uint32_t n, uint32_t p) {
+  for (uint32_t q = 0; q < n; ++q)
+    if (p + q >= lo && p + q < hi) msg[p + q - lo] = (uint8_t)(v >> (8 * q));
+}
+
+// A body held in registers (at most 32 bytes) at position p, clipped.
+__device__ __forceinline__ void put_body32(uint8_t *msg, uint32_t lo, uint32_t hi, const Bytes32 &b, uint32_t n,
+                                           uint32_t p) {
+  if (p + n <= lo || p >= hi) return;
+  if (p >= lo && p + n <= hi) {
+    uint8_t *m = msg + (p - lo);
+#pragma unroll
+    for (uint32_t j = 0; j < 32; ++j)
+      if (j < n) m[j] = (uint8_t)(b.w[j >> 3] >> (8 * (j & 7)));
+  } else {  // across a window's edge (behind a long value)
+#pragma unroll
+    for (uint32_t w = 0; w < 4; ++w) put_prefix(msg, lo, hi, b.w[w], n > 8 * w ? min(8u, n - 8 * w) : 0u, p + 8 * w);
+  }
+}
+
+// The warp copies a long body (n bytes at src, message position p), clipped:
+// whole aligned 8-byte words of the window where it covers them (unaligned
+// loads, all lanes' in flight together), single bytes at the two ends.
+template <bool kCoh>
+__device__ __forceinline__ void put_far(uint8_t *msg, uint32_t lo, uint32_t hi, const uint8_t *src, uint32_t n,
+                                        uint32_t p, int lane) {
+  const uint32_t a = max(p, lo) - lo, z = min(p + n, hi) - lo;  // window range
+  if (p + n <= lo || p >= hi) return;
+  const uint8_t *s0 = src + ((int64_t)lo - (int64_t)p);  // byte of window offset 0 (read only inside [a, z))
+  const uint32_t wa = (a + 7) & ~7u, wz = z & ~7u;
+  if (wa >= wz) {
+    for (uint32_t j = a + lane; j < z; j += 32) msg[j] = ldn<kCoh>(s0 + j);
+    return;
+  }
+  uint64_t *m64 = reinterpret_cast<uint64_t *>(msg);
+  for (uint32_t j = wa + 8u * lane; j < wz; j += 256) m64[j >> 3] = ld8<kCoh>(s0 + j);
+  if (a + lane < wa) msg[a + lane] = ldn<kCoh>(s0 + a + lane);
+  if (wz + lane < z) msg[wz + lane] = ldn<kCoh>(s0 + wz + lane);
+}
 
 // Warp-cooperative encode + hash of branch node idx, for levels with few
 // nodes or for branches of many blocks, where one thread's serial chain is
-// the latency: the message is built window by window (kWarpMsgBytes, 8
-// blocks) in the warp's shared buffer, every lane copying a share of each
-// item's bytes (lane k < 17 holds child k's item, the header goes first),
-// and absorbed with the warp-spread permutation.  All 32 lanes call it with
-// the same idx.
+// the latency.  Lane k < 17 loads child k's item; a scan gives every item its
+// place, and the message is built window by window (kWarpMsgBytes, 8 blocks)
+// in the warp's shared buffer -- every lane its own item's bytes at once,
+// long values by all lanes -- and absorbed with the warp-spread permutation.
+// All 32 lanes call it with the same idx.
+// Bound by latency: one chain of dependent loads (node, children, hashes),
+// then the serial permutations.  Building item after item (one L2 round trip
+// each) took a 16-child branch 15-17 us per level of a 1M-key trie; this
+// form takes 10-11.
 template <bool kCoh>
 __device__ __forceinline__ void hash_full_warp(const TrieView &tv, uint32_t idx, uint8_t *msg, const CoopLanes &cl) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  if (ldn<kCoh>(tv.full_dead + idx)) return;  // unlinked by a delete: nothing to hash
-  EncItem it{0, 0, 0, nullptr, 0};
-  if (lane < 17) it = child_item<kCoh>(tv, ldn<kCoh>(tv.full_child + (size_t)idx * 17 + lane));
-  const uint32_t sz = lane < 17 ? it.pren + it.blen : 0u;
+  const uint32_t r = lane < 17 ? ldn<kCoh>(tv.full_child + (size_t)idx * 17 + lane) : 0u;
+  const bool dead = ldn<kCoh>(tv.full_dead + idx) != 0;
+  const bool force = tv.geth_mode && ldn<kCoh>(tv.full_depth + idx) == 0;
+  if (dead) return;  // unlinked by a delete: nothing to hash
+  WarpItem it;
+  if (lane < 17) it = warp_child_item<kCoh>(tv, r);
+  const uint32_t sz = it.pren + it.blen;
   uint32_t incl = sz;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -1492,11 +1592,10 @@ __device__ __forceinline__ void hash_full_warp(const TrieView &tv, uint32_t idx,
   uint32_t hn;
   rlp_head(payload, 0xc0, 0xf7, hdr, hn);
   const uint32_t total = payload + hn;
-  const bool force = tv.geth_mode && ldn<kCoh>(tv.full_depth + idx) == 0;
   const bool raw = total < 32 && !force;
   const uint32_t nblk = raw ? 1u : (total + 1 + 135) / 136;
-  const uint32_t padded = nblk * 136;
   const uint32_t my_off = hn + incl - sz;  // message offset of this lane's item
+  const unsigned far = __ballot_sync(kAll, it.far != nullptr);
   uint64_t *m64 = reinterpret_cast<uint64_t *>(msg);
   uint64_t a = 0;  // this lane's word of the state
   for (uint32_t b0 = 0; b0 < nblk; b0 += kWarpMsgBytes / 136) {
@@ -1504,33 +1603,26 @@ __device__ __forceinline__ void hash_full_warp(const TrieView &tv, uint32_t idx,
     const uint32_t lo = b0 * 136, hi = lo + wb * 136;
     for (uint32_t w = lane; w < wb * 17; w += 32) m64[w] = 0;
     __syncwarp();
-    if (lane == 0)
-      for (uint32_t q = 0; q < hn; ++q)
-        if (q >= lo && q < hi) msg[q - lo] = (uint8_t)(hdr >> (8 * q));
-    // items in order; the lanes share each item's bytes that fall in the window
-    for (int k = 0; k < 17; ++k) {
-      const uint32_t p = __shfl_sync(kAll, my_off, k);
-      const uint32_t pren = __shfl_sync(kAll, it.pren, k);
-      const uint32_t blen = __shfl_sync(kAll, it.blen, k);
-      const uint64_t pre = __shfl_sync(kAll, it.pre, k);
-      const uint8_t *body = reinterpret_cast<const uint8_t *>(
-          __shfl_sync(kAll, reinterpret_cast<unsigned long long>(it.body), k));
-      const uint32_t n = pren + blen;
-      if (p >= hi || p + n <= lo) continue;
-      const uint32_t j0 = lo > p ? lo - p : 0u, j1 = min(n, hi - p);
-      for (uint32_t j = j0 + (uint32_t)lane; j < j1; j += 32)
-        msg[p + j - lo] = j < pren ? (uint8_t)(pre >> (8 * j)) : ldn<kCoh>(body + (j - pren));
+    if (lane == 31) put_prefix(msg, lo, hi, hdr, hn, 0);
+    put_prefix(msg, lo, hi, it.pre, it.pren, my_off);
+    if (!it.far) put_body32(msg, lo, hi, it.body, it.blen, my_off + it.pren);
+    for (unsigned m = far; m; m &= m - 1) {
+      const int k = __ffs(m) - 1;
+      const uint8_t *src = reinterpret_cast<const uint8_t *>(
+          __shfl_sync(kAll, reinterpret_cast<unsigned long long>(it.far), k));
+      const uint32_t n = __shfl_sync(kAll, it.blen, k), p = __shfl_sync(kAll, my_off + it.pren, k);
+      put_far<kCoh>(msg, lo, hi, src, n, p, lane);
     }
     __syncwarp();
     if (raw) break;  // under 32 bytes: the window holds the whole encoding
     if (lane == 0) {  // Keccak padding (pad byte 0x01 ... last byte |= 0x80)
       if (total >= lo && total < hi) msg[total - lo] ^= 0x01;
-      if (padded - 1 >= lo && padded - 1 < hi) msg[padded - 1 - lo] ^= 0x80;
+      if (hi == nblk * 136) msg[wb * 136 - 1] ^= 0x80;
     }
     __syncwarp();
     for (uint32_t bb = 0; bb < wb; ++bb) {
       if (lane < 17) a ^= m64[bb * 17 + lane];
-      a = keccak_f1600_warp(a, cl, lane);
+      a = keccak_f1600_warp(a, cl);
     }
     __syncwarp();  // the next window reuses the buffer
   }
