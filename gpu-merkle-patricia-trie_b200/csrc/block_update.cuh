@@ -226,7 +226,7 @@ __device__ __forceinline__ void write_root(const TrieView &tv, uint32_t tr, uint
 }
 
 __global__ void __launch_bounds__(256, 2) k_block(TrieView tv0, DirtyList dl, BlockBufs bb, uint32_t retry_limit) {
-  extern __shared__ uint64_t smem[];  // 17 message words per thread; histogram
+  extern __shared__ __align__(16) uint32_t smem[];  // kStageWords message words per thread; histogram
   BlockDesc *D = bb.desc;
   const int n = D->n, n0 = D->n0, n_out = D->n_out;
   const uint64_t vid_base = D->vid_base;
@@ -243,13 +243,13 @@ __global__ void __launch_bounds__(256, 2) k_block(TrieView tv0, DirtyList dl, Bl
   const int gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const int t_spread = lane * W + gw;
   // this warp's message buffer for hash_full_warp, after the staging words
-  uint8_t *wmsg = reinterpret_cast<uint8_t *>(smem + 17 * blockDim.x) + (threadIdx.x >> 5) * kWarpMsgBytes;
+  uint8_t *wmsg = reinterpret_cast<uint8_t *>(smem + kStageWords * blockDim.x) + (threadIdx.x >> 5) * kWarpMsgBytes;
   // staging outcome: every CTA reads the same words, so all leave together
   if (D->bad || D->noncontig || D->stream_terms != D->key_terms) {
     if (t == 0) atomicOr(&D->status, 2u);
     return;
   }
-  uint32_t *hist = reinterpret_cast<uint32_t *>(smem);
+  uint32_t *hist = smem;
   for (int s = 0; s < 2; ++s) {
     const int i0 = s ? n0 : 0, i1 = s ? n : n0;
     tv.gen = D->gen + (uint32_t)s;

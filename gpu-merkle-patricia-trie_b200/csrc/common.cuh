@@ -20,6 +20,7 @@ __host__ __device__ __forceinline__ uint32_t ref_idx(uint32_t r) { return r & 0x
 __host__ __device__ __forceinline__ uint32_t make_ref(uint32_t k, uint32_t i) { return (k << 30) | i; }
 
 constexpr uint32_t kMaxNodes = 0x3FFFFFFFu;  // per node kind
+constexpr uint32_t kNoNode = 0xFFFFFFFFu;    // no node index
 constexpr int kMaxKeyNibbles = 1024;          // longest accepted hex key
 constexpr uint16_t kLcpInf = 0xFFFF;
 
@@ -74,6 +75,7 @@ struct TrieView {
   uint8_t *full_hash;     // [cap_full * 32]
   uint8_t *full_hlen;
   uint8_t *full_dead;     // 1: unlinked by a delete (no longer in any trie)
+  uint32_t *full_ext;     // the extension last seen above it (see ext_above), kNoNode before any
   // short nodes
   uint64_t *short_key;    // nibble offset into the key arena
   uint32_t *short_klen;

@@ -177,18 +177,18 @@ __device__ __forceinline__ uint64_t keccak_f1600_warp(uint64_t a, const CoopLane
 
 // Streaming sponge.  Message bytes are pushed in little-endian runs of <= 8
 // bytes; whole 64-bit words go to this thread's 17-word staging block in
-// shared memory (word w at stage[w * stride]), which absorb() folds into the
-// register state.  Callers absorb when full() after a push (a push emits at
+// shared memory (a column of 32-bit halves: half h at stage[h * stride]),
+// which absorb() folds into the register state.  Callers absorb when full() after a push (a push emits at
 // most one word), so the permutation has a single call site.
 struct Sponge {
   uint64_t a[25];
   uint64_t acc;      // partial word
   uint32_t accn;     // bytes in acc (0..7)
   uint32_t w;        // words staged in this block (0..17)
-  uint64_t *stage;
+  uint32_t *stage;
   uint32_t stride;
 
-  __device__ __forceinline__ void reset(uint64_t *st, uint32_t strd) {
+  __device__ __forceinline__ void reset(uint32_t *st, uint32_t strd) {
 #pragma unroll
     for (int i = 0; i < 25; ++i) a[i] = 0;
     acc = 0;
@@ -198,8 +198,15 @@ struct Sponge {
     stride = strd;
   }
   __device__ __forceinline__ bool full() const { return w == 17; }
+  __device__ __forceinline__ void put(uint32_t i, uint64_t word) {
+    stage[2 * i * stride] = (uint32_t)word;
+    stage[(2 * i + 1) * stride] = (uint32_t)(word >> 32);
+  }
+  __device__ __forceinline__ uint64_t word(uint32_t i) const {
+    return ((uint64_t)stage[(2 * i + 1) * stride] << 32) | stage[2 * i * stride];
+  }
   __device__ __forceinline__ void emit(uint64_t word) {
-    stage[w * stride] = word;
+    put(w, word);
     ++w;
   }
   // push n (1..8) bytes held little-endian in v; bytes >= n of v are zero
@@ -226,16 +233,16 @@ struct Sponge {
   }
   // Keccak padding of the final block (pad byte 0x01, last byte |= 0x80)
   __device__ __forceinline__ void pad() {
-    stage[w * stride] = acc | (0x01ull << (8 * accn));
-    for (uint32_t j = w + 1; j < 17; ++j) stage[j * stride] = 0;
-    stage[16 * stride] ^= 0x8000000000000000ull;
+    put(w, acc | (0x01ull << (8 * accn)));
+    for (uint32_t j = w + 1; j < 17; ++j) put(j, 0);
+    stage[33 * stride] ^= 0x80000000u;
     w = 17;
     acc = 0;
     accn = 0;
   }
   __device__ __forceinline__ void absorb() {
 #pragma unroll
-    for (int i = 0; i < 17; ++i) a[i] ^= stage[i * stride];
+    for (int i = 0; i < 17; ++i) a[i] ^= word(i);
     keccak_f1600(a);
     w = 0;
   }

@@ -12,7 +12,7 @@ namespace gmpt {
 
 __global__ void __launch_bounds__(128) k_keccak256_batch(const uint8_t *data, const int64_t *offs, int n,
                                                          uint8_t *out) {
-  extern __shared__ uint64_t stage_all[];
+  extern __shared__ uint32_t stage_all[];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int64_t s = offs[2 * i], e = offs[2 * i + 1];

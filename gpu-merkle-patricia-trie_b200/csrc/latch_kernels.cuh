@@ -128,6 +128,7 @@ __device__ __noinline__ void latch_from(TrieView tv, DirtyList dl, uint32_t *sp,
     tv.full_epoch[br] = gen;
     tv.full_hlen[br] = 0;
     tv.full_dead[br] = 0;
+    tv.full_ext[br] = kNoNode;
     // the old node's remainder
     uint32_t rest = schild;
     bool use_left = sl - mm - 1 > 0;

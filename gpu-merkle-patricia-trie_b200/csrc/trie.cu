@@ -27,11 +27,13 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kHashThreads = kHashLevelThreads;
-// k_hash_level_wide (132 registers: three CTAs per SM) for launches that
+// k_hash_level_wide (167 registers: three CTAs per SM) for launches that
 // cannot place more than three CTAs on each of B200's 148 SMs anyway
 constexpr unsigned kWideGrid = 3 * 148;
 // branch hash class (blocks - 1) from which a branch is hashed by a warp
 constexpr uint32_t kWarpMinClass = 4;
+// up to this many leaves are hashed a warp each
+constexpr uint32_t kWarpLeafMax = 2048;
 constexpr uint32_t kMaxDepths = kMaxKeyNibbles + 2;  // nibble depths a dirty node can have
 // LockNU batches of at least this many keys drop repeated keys first
 constexpr int kDedupMinKeys = 1 << 16;
@@ -102,7 +104,8 @@ Trie::Trie(int device, int geth_mode, int max_tries, bool unified)
 Trie::~Trie() {
   cudaSetDevice(dev_);
   if (st_) cudaStreamSynchronize(st_);
-  void *ptrs[] = {tv_.full_child, tv_.full_epoch, tv_.full_depth, tv_.full_hash, tv_.full_hlen, tv_.full_dead, fl_refs_,
+  void *ptrs[] = {tv_.full_child, tv_.full_epoch, tv_.full_depth, tv_.full_hash, tv_.full_hlen, tv_.full_dead, tv_.full_ext,
+                  fl_refs_,
                   tv_.short_key, tv_.short_klen, tv_.short_child, tv_.short_epoch, tv_.short_depth,
                   tv_.short_dead, tv_.short_hash, tv_.short_hlen, tv_.short_claim, tv_.short_pseudo,
                   tv_.value_vid, tv_.rec, tv_.rec_hp, (void *)tv_.keys, (void *)tv_.vals,
@@ -117,7 +120,7 @@ Trie::~Trie() {
                         &ws_.sb_len, &ws_.sb_ref, &ws_.sb_d0, &ws_.sb_slot, &ws_.sb_code, &ws_.lcp,
                         &ws_.act2, &ws_.aseg, &ws_.aseg2, &ws_.kflags, &ws_.knib, &ws_.bins, &ws_.cursor,
                         &ws_.sorted_dirty, &ws_.g_keys, &ws_.g_idx, &ws_.g_hp, &ws_.g_len, &ws_.g_tid,
-                        &ws_.tid, &ws_.dd_hash, &ws_.dd_pos, &ws_.dd_sel, &ws_.dd_slot, &ws_.raw, &ws_.dirty_cls, &ws_.rw_flags,
+                        &ws_.tid, &ws_.dd_hash, &ws_.dd_pos, &ws_.dd_sel, &ws_.dd_slot, &ws_.raw, &ws_.dirty_bin, &ws_.rw_flags,
                         &ws_.rw_a, &ws_.rw_b, &ws_.rw_c, &ws_.rw_d, &ws_.rw_e, &ws_.rw_wpos, &ws_.rw_hp,
                         &ws_.rw_len, &ws_.rw_tot, &ws_.rw_kept, &ws_.rw_koff, &ws_.rw_klen, &ws_.rw_tid,
                         &ws_.del_hslot, &ws_.del_hext, &ws_.del_stamp,
@@ -222,6 +225,7 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
     if (e == cudaSuccess) e = grow_array(tv_.full_hash, o * 32, nc * 32, st_, managed_, dev_);
     if (e == cudaSuccess) e = grow_array(tv_.full_hlen, o, nc, st_, managed_, dev_);
     if (e == cudaSuccess) e = grow_array(tv_.full_dead, o, nc, st_, managed_, dev_);
+    if (e == cudaSuccess) e = grow_array(tv_.full_ext, o, nc, st_, managed_, dev_);
     if (e != cudaSuccess) return check_cuda(e, "grow branch pool");
     cap_full_ = (uint32_t)nc;
   }
@@ -292,7 +296,7 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
   tv_.cap_full = cap_full_;
   tv_.cap_short = cap_short_;
   tv_.cap_value = cap_value_;
-  stats_.device_bytes = (uint64_t)cap_full_ * (68 + 4 + 2 + 32 + 1 + 1) + (uint64_t)cap_short_ * (8 + 4 + 4 + 4 + 2 + 1 + 32 + 1 + 8) +
+  stats_.device_bytes = (uint64_t)cap_full_ * (68 + 4 + 2 + 32 + 1 + 1 + 4) + (uint64_t)cap_short_ * (8 + 4 + 4 + 4 + 2 + 1 + 32 + 1 + 8) +
                         (uint64_t)cap_value_ * 8 + cap_rec_ * 24 + cap_keys_ + cap_vals_ + cap_dirty_ * 6;
   return OK;
 }
@@ -380,6 +384,7 @@ int Trie::stage(const BatchIn &b, uint64_t &key_base, uint64_t &vid_base, uint64
   if (e != cudaSuccess) return check_cuda(e, "stage");
   *maxlen = (uint32_t)(h_small_[0] & 0xFFFFFFFFu);
   max_key_nibbles_ = std::max(max_key_nibbles_, *maxlen);
+  depth_bound_ = std::max(depth_bound_, *maxlen);
   max_value_len_ = std::max(max_value_len_, (uint32_t)(h_small_[0] >> 32));
   if (b.raw_keys) {
     // nothing to check beyond k_raw_lens (errors come back with the counters)
@@ -935,22 +940,25 @@ int Trie::put_2phase(const BatchIn &b) {
   return OK;
 }
 
-// Counting sort of the nd dirty nodes by (depth, kind, hash class) into
-// ws_.sorted_dirty; off[b] .. off[b + 1] is bin b (dirty_bin).
+// Nibble depths a node of this trie can have (0 .. the longest key staged).
+uint32_t Trie::dirty_depths() const { return std::min<uint32_t>(depth_bound_ + 1u, kMaxDepths); }
+
+// Counting sort of the nd dirty nodes into ws_.sorted_dirty; off[b] ..
+// off[b + 1] is bin b (dirty_bin).
 int Trie::bucket_dirty(uint32_t nd, uint32_t **sorted_out, std::vector<uint32_t> &off) {
   cudaError_t e = cudaSuccess;
-  const uint32_t nbins = level_bin(kMaxDepths);
+  const uint32_t nbins = level_bin(dirty_depths());
   uint32_t *bins = wsp<uint32_t>(ws_.bins, nbins, e);
   uint32_t *cursor = wsp<uint32_t>(ws_.cursor, nbins, e);
   uint32_t *sorted = wsp<uint32_t>(ws_.sorted_dirty, nd, e);
-  uint8_t *cls = wsp<uint8_t>(ws_.dirty_cls, nd, e);
+  uint16_t *bin_of = wsp<uint16_t>(ws_.dirty_bin, nd, e);
   if (e == cudaSuccess) e = cudaMemsetAsync(bins, 0, sizeof(uint32_t) * nbins, st_);
   if (e != cudaSuccess) return check_cuda(e, "hash alloc");
   // a leaf can take two or more Keccak blocks: order leaves by block count
   const int leaf_classes = (uint64_t)max_value_len_ + max_key_nibbles_ / 2 + 8 > 135 ? 1 : 0;
   int grid = std::min<int>(blocks_for(nd), 148 * 4);
   count_launch(), k_dirty_hist<<<grid, kThreads, sizeof(uint32_t) * nbins, st_>>>(
-                      tv_, dirty_ref_, dirty_depth_, (int)nd, bins, (int)nbins, leaf_classes, cls);
+                      tv_, dirty_ref_, dirty_depth_, (int)nd, bins, (int)nbins, leaf_classes, bin_of);
   std::vector<uint32_t> hb(nbins);
   off.assign((size_t)nbins + 1, 0);
   if ((e = cudaMemcpyAsync(hb.data(), bins, sizeof(uint32_t) * nbins, cudaMemcpyDeviceToHost, st_)) !=
@@ -962,7 +970,7 @@ int Trie::bucket_dirty(uint32_t nd, uint32_t **sorted_out, std::vector<uint32_t>
       cudaSuccess)
     return check_cuda(e, "hash cursor");
   count_launch(), k_dirty_scatter<<<std::min<unsigned>(blocks_for(nd), 148 * 8), kThreads, 0, st_>>>(
-                      dirty_ref_, dirty_depth_, cls, (int)nd, cursor, sorted, ctr_);
+                      dirty_ref_, bin_of, (int)nd, cursor, sorted, ctr_);
   *sorted_out = sorted;
   return OK;
 }
@@ -982,7 +990,7 @@ int Trie::bucket_and_hash() {
   std::vector<uint32_t> off;
   int rc = bucket_dirty(nd, &sorted, off);
   if (rc) return rc;
-  size_t smem = sizeof(uint64_t) * 17 * kHashThreads;
+  size_t smem = sizeof(uint32_t) * kStageWords * kHashThreads;
   int levels = 0;
   if ((e = cudaMemsetAsync(&ctr_->hashed, 0, 4, st_)) != cudaSuccess ||
       (e = cudaMemsetAsync(&ctr_->enc_bytes, 0, 16, st_)) != cudaSuccess)
@@ -1005,32 +1013,39 @@ int Trie::bucket_and_hash() {
     else
       count_launch(), k_hash_level<<<grid, kHashThreads, smem, st_>>>(tv_, refs, (int)cnt);
   };
+  auto warps = [&](const uint32_t *refs, uint32_t cnt) {
+    count_launch(), k_hash_warp<<<(cnt + 3) / 4, 128, smem_warp, st_>>>(tv_, refs, (int)cnt);
+  };
   // every leaf first (one launch), then the levels deepest first
   if (off[kLeafClasses] > 0) {
     ++levels;
-    level(sorted, off[kLeafClasses]);
+    if (off[kLeafClasses] <= kWarpLeafMax)
+      warps(sorted, off[kLeafClasses]);
+    else
+      level(sorted, off[kLeafClasses]);
   }
-  for (int d = (int)kMaxDepths - 1; d >= 0; --d) {
-    uint32_t a = off[level_bin(d)], m = off[level_bin(d) + 1], z = off[level_bin(d + 1)];
-    if (z == a) continue;
+  for (int d = (int)dirty_depths() - 1; d >= 0; --d) {
+    // branches [a, m), the extensions above them [m, z)
+    const uint32_t a = off[level_bin(d)], m = off[level_bin(d) + kHashClasses], z = off[level_bin(d + 1)];
+    if (m == a) continue;  // (an extension is listed with its branch's level)
     ++levels;
-    // branches of kWarpMinClass + 1 blocks or more: the level's first branch
-    // bins (longest first)
-    const uint32_t ml = off[level_bin(d) + 1 + (kHashClasses - kWarpMinClass)];
-    if (z - m > 0 && z - m <= (uint32_t)opt_warp_full_max_) {
-      // few branches: short nodes thread-wise, branches one warp each
-      if (m > a) level(sorted + a, m - a);
-      count_launch(), k_hash_full_warp<<<(z - m + 3) / 4, 128, smem_warp, st_>>>(tv_, sorted + m, (int)(z - m));
-    } else if (ml > m && ml - m <= (uint32_t)opt_warp_full_max_) {
+    // branches of kWarpMinClass + 1 blocks or more: the level's first bins
+    // (longest first)
+    const uint32_t ml = off[level_bin(d) + (kHashClasses - kWarpMinClass)];
+    if (m - a <= (uint32_t)opt_warp_full_max_) {
+      warps(sorted + a, m - a);  // few branches: one warp each, with its extension
+      continue;
+    }
+    if (ml > a && ml - a <= (uint32_t)opt_warp_full_max_) {
       // a few branches of many blocks (a key ending at a branch puts its
       // value, up to kilobytes, in slot 16) would set the level's time as
       // one thread's serial chain: one warp each, the rest thread-wise
-      count_launch(), k_hash_full_warp<<<(ml - m + 3) / 4, 128, smem_warp, st_>>>(tv_, sorted + m, (int)(ml - m));
-      if (m > a) level(sorted + a, m - a);
-      level(sorted + ml, z - ml);
+      warps(sorted + a, ml - a);
+      level(sorted + ml, m - ml);
     } else {
-      level(sorted + a, z - a);
+      level(sorted + a, m - a);
     }
+    if (z > m) level(sorted + m, z - m);
   }
   if (timing_) {
     cudaEventRecord(kz, st_);
@@ -1234,7 +1249,7 @@ int Trie::reset() {
   if (e != cudaSuccess) return check_cuda(e, "reset");
   n_full_ = n_short_ = n_value_ = 0;
   n_rec_ = key_used_ = val_used_ = 0;
-  max_key_nibbles_ = max_value_len_ = 0;
+  max_key_nibbles_ = max_value_len_ = depth_bound_ = 0;
   fl_n_ = 0;
   empty_ = true;
   ++gen_;
@@ -1699,7 +1714,7 @@ namespace gmpt {
 namespace {
 
 constexpr int kBlockThreads = 256;
-constexpr size_t kBlockSmem = sizeof(uint64_t) * 17 * kBlockThreads + (kBlockThreads / 32) * kWarpMsgBytes;
+constexpr size_t kBlockSmem = sizeof(uint32_t) * kStageWords * kBlockThreads + (kBlockThreads / 32) * kWarpMsgBytes;
 
 // everything a captured graph has baked in
 struct BlockSig {
@@ -1717,6 +1732,7 @@ int Trie::block_launch(bool launch) {
   cudaError_t e = cudaSuccess;
   int sms = 0, occ = 0;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockSmem)) != cudaSuccess ||
       (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_block, kBlockThreads, kBlockSmem)) != cudaSuccess)
     return check_cuda(e, "block occupancy");
   const int max_grid = occ * sms;
@@ -1902,6 +1918,7 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   gen_ += 2;
   tv_.gen = gen_;
   if (n > 0) empty_ = false;
+  if (n > 0) depth_bound_ = kMaxKeyNibbles;  // the launch does not report its longest key
   stats_.key_bytes = key_used_;
   stats_.value_bytes = val_used_;
   stats_.n_records = n_rec_;
@@ -2184,8 +2201,8 @@ int Trie::del(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool devi
   uint32_t *sorted = nullptr;
   std::vector<uint32_t> off;
   if ((rc = bucket_dirty(nd, &sorted, off))) return rc;
-  for (int d = (int)kMaxDepths - 1; d >= 0; --d) {
-    const uint32_t a = off[level_bin(d) + 1], z = off[level_bin(d + 1)];  // branches at depth d
+  for (int d = (int)dirty_depths() - 1; d >= 0; --d) {
+    const uint32_t a = off[level_bin(d)], z = off[level_bin(d) + kHashClasses];  // branches at depth d
     if (z == a) continue;
     const int cnt = (int)(z - a);
     // room for this level's new keys and short nodes, then collapse

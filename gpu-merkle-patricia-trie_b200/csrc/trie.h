@@ -199,6 +199,8 @@ class Trie {
   // longest key (nibbles) and value (bytes) staged since the last reset:
   // whether the hash pass orders leaves by Keccak block count
   uint32_t max_key_nibbles_ = 0, max_value_len_ = 0;
+  uint32_t depth_bound_ = 0;   // no node is deeper: the longest key of any put since the last reset
+  uint32_t dirty_depths() const;
   uint32_t *roots_ = nullptr;  // [n_tries_] root words
   uint32_t n_tries_ = 1;
   Counters *ctr_ = nullptr;
@@ -258,7 +260,7 @@ class Trie {
     DevBlock tid;                                               // trie ids of the batch
     DevBlock dd_hash, dd_pos, dd_sel, dd_slot;                  // LockNU batch dedup
     DevBlock raw;                                               // raw key bytes of the batch
-    DevBlock dirty_cls;                                         // hash class of each dirty node
+    DevBlock dirty_bin;                                         // hash bin of each dirty node
     DevBlock rw_flags, rw_a, rw_b, rw_c, rw_d, rw_e, rw_wpos;   // mixed read/write resolution
     DevBlock rw_hp, rw_len, rw_tot, rw_kept, rw_koff, rw_klen, rw_tid;
     DevBlock del_hslot, del_hext, del_stamp;                    // deletes: how each path branch is linked

@@ -74,6 +74,7 @@ __device__ __forceinline__ uint32_t new_full(const TrieView &tv, DirtyList d, ui
   tv.full_epoch[f] = gen;
   tv.full_hlen[f] = 0;
   tv.full_dead[f] = 0;
+  tv.full_ext[f] = kNoNode;
   dirty_push(tv.ctr, d, make_ref(KIND_FULL, f), depth);
   return f;
 }
@@ -900,8 +901,9 @@ __global__ void k_level_scatter(const uint32_t *act, const uint32_t *aseg, const
 }
 
 // ---------------------------------------------------------------------------
-// PhaseHC: dirty leaves first, then the other nodes bucketed by (nibble
-// depth, kind), deepest first
+// PhaseHC: dirty nodes with nothing dirty below them first, then the branches
+// by nibble depth, deepest first; an extension is hashed by the task of the
+// branch below it
 
 // Keccak blocks a dirty branch's encoding is expected to take, minus one,
 // capped at kHashClasses - 1: children counted as 33-byte references, and a
@@ -959,52 +961,75 @@ __device__ __forceinline__ uint32_t hash_class(const TrieView &tv, uint32_t r) {
 // about half of the lanes idle with values of up to kilobytes (1 to 31
 // blocks), and hashing leaves level by level made deep tries a chain of
 // small launches, each as long as its slowest leaf.
+//
+// An extension over a dirty branch has one input, that branch's hash, so it
+// belongs to the branch's level, not to one of its own: in a level hashed a
+// warp per branch the warp goes on to it (full_ext names it), in a level
+// hashed a thread per node it is listed behind the level's branches.  Keys
+// whose branches sit below one-nibble extensions (ASCII digits, words) would
+// otherwise take two levels per character: a 16K-key update of a 1M-key trie
+// ran 21 launches, now 12.  An extension over a clean branch (what a split or
+// a delete leaves above an untouched subtree) has no dirty input and goes
+// with the leaves.
 constexpr uint32_t kLeafClasses = 32;
-// bins: the kLeafClasses leaf bins, then per nibble depth one bin of
-// extensions and kHashClasses bins of branches; a level is one contiguous
-// range of the sorted dirty list
-constexpr uint32_t kBinsPerDepth = 1 + kHashClasses;
-constexpr uint32_t kLeafBit = 0x80;  // class byte of a leaf
+// bins: the kLeafClasses leaf bins, one bin of dead short nodes (LockNU's
+// splits leave many), then per nibble depth kHashClasses bins of branches,
+// longest first, and one of the extensions right above those branches; a
+// level is one contiguous range of the sorted dirty list
+constexpr uint32_t kDeadBin = kLeafClasses;
+constexpr uint32_t kBinsPerDepth = kHashClasses + 1;
 
-__host__ __device__ __forceinline__ uint32_t level_bin(uint32_t depth) { return kLeafClasses + depth * kBinsPerDepth; }
+__host__ __device__ __forceinline__ uint32_t level_bin(uint32_t depth) { return kLeafClasses + 1u + depth * kBinsPerDepth; }
 
-// class byte of a dirty node: kLeafBit | block class for a leaf, the hash
-// class for a branch, 0 for an extension or a dead short node (LockNU's
-// splits leave many: among the leaves they would idle lanes of the warps
-// that hash live leaves of the same block count)
-__device__ __forceinline__ uint32_t dirty_class(const TrieView &tv, uint32_t r, bool leaf_classes) {
-  const uint32_t idx = ref_idx(r);
-  if (ref_kind(r) == KIND_FULL) return full_class(tv, idx);
-  if (tv.short_dead[idx]) return 0u;
-  const uint32_t ch = tv.short_child[idx];
-  if (ref_kind(ch) != KIND_VALUE) return 0u;
-  if (!leaf_classes) return kLeafBit;
-  const uint32_t bytes = tv.short_klen[idx] / 2u + 8u + load_rec(tv, tv.value_vid[ref_idx(ch)]).len;
-  return kLeafBit | min(bytes / 136u, kLeafClasses - 1u);
+// The extension above branch f that f's task hashes, or kNoNode.  full_ext
+// may be left from an earlier pass; an extension still in the trie whose
+// child is f is f's parent, and is dirty whenever f is.
+__device__ __forceinline__ uint32_t ext_above(const TrieView &tv, uint32_t f) {
+  const uint32_t e = __ldcg(tv.full_ext + f);
+  if (e == kNoNode) return kNoNode;
+  return (__ldcg(tv.short_child + e) == make_ref(KIND_FULL, f) && !__ldcg(tv.short_dead + e)) ? e : kNoNode;
 }
 
-// bin of a dirty node from its depth, kind and class byte; inside a launch
-// the classes run longest first, so the CTAs of the slowest nodes start in
-// the first wave instead of forming the last one
-__device__ __forceinline__ uint32_t dirty_bin(uint32_t depth, uint32_t r, uint32_t cls) {
-  if (cls & kLeafBit) return kLeafClasses - 1u - (cls & ~kLeafBit);
-  return level_bin(depth) + (ref_kind(r) == KIND_FULL ? kHashClasses - cls : 0u);
+// Bin of a dirty node at nibble depth `depth`.  Inside a launch the classes
+// run longest first, so the CTAs of the slowest nodes start in the first wave
+// instead of forming the last one.  Records the extension above a dirty
+// branch in full_ext.
+__device__ __forceinline__ uint32_t dirty_bin(const TrieView &tv, uint32_t r, uint32_t depth, bool leaf_classes) {
+  const uint32_t idx = ref_idx(r);
+  if (ref_kind(r) == KIND_FULL) return level_bin(depth) + kHashClasses - 1u - full_class(tv, idx);
+  if (tv.short_dead[idx]) return kDeadBin;
+  const uint32_t ch = tv.short_child[idx];
+  if (ref_kind(ch) == KIND_FULL && tv.full_epoch[ref_idx(ch)] == tv.gen) {
+    tv.full_ext[ref_idx(ch)] = idx;
+    return level_bin(depth + tv.short_klen[idx]) + kHashClasses;
+  }
+  if (!leaf_classes) return kLeafClasses - 1u;
+  uint32_t bytes = tv.short_klen[idx] / 2u + 8u;
+  bytes += ref_kind(ch) == KIND_VALUE ? load_rec(tv, tv.value_vid[ref_idx(ch)]).len : 33u;
+  return kLeafClasses - 1u - min(bytes / 136u, kLeafClasses - 1u);
 }
 
 // Histogram of the dirty list over the bins (nbins of them, covering every
 // depth a node can have).  Leaves are classed by block count only when
 // `leaf_classes` is set (a batch held values long enough for a leaf to take
-// two or more Keccak blocks).
+// two or more Keccak blocks).  Counts are aggregated per warp: one shared
+// atomic per distinct bin, not one per node (a load's millions of leaves
+// share one bin and would queue on its address).
 __global__ void k_dirty_hist(TrieView tv, const uint32_t *ref, const uint16_t *depth, int n, uint32_t *bins,
-                             int nbins, int leaf_classes, uint8_t *cls) {
+                             int nbins, int leaf_classes, uint16_t *bin_of) {
   extern __shared__ uint32_t h[];
   for (int b = threadIdx.x; b < nbins; b += blockDim.x) h[b] = 0;
   __syncthreads();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t r = ref[i];
-    const uint32_t c = dirty_class(tv, r, leaf_classes != 0);
-    cls[i] = (uint8_t)c;
-    atomicAdd(&h[dirty_bin(depth[i], r, c)], 1u);
+  const int lane = threadIdx.x & 31;
+  for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += gridDim.x * blockDim.x) {
+    const int i = i0 + lane;
+    uint32_t b = 0xFFFFFFFFu;
+    if (i < n) {
+      b = min(dirty_bin(tv, ref[i], depth[i], leaf_classes != 0), (uint32_t)nbins - 1u);
+      bin_of[i] = (uint16_t)b;
+    }
+    const unsigned peers = __match_any_sync(0xffffffffu, b);
+    if (i < n && lane == __ffs(peers) - 1) atomicAdd(&h[b], (uint32_t)__popc(peers));
   }
   __syncthreads();
   for (int b = threadIdx.x; b < nbins; b += blockDim.x)
@@ -1015,8 +1040,8 @@ __global__ void k_dirty_hist(TrieView tv, const uint32_t *ref, const uint16_t *d
 // are aggregated per warp (match_any) and then per CTA in a shared table of
 // the bins the pass touches, so a hot bin (a level of millions of leaves)
 // takes one global atomic per CTA pass instead of one per warp.
-__global__ void __launch_bounds__(256) k_dirty_scatter(const uint32_t *ref, const uint16_t *depth, const uint8_t *cls,
-                                                       int n, uint32_t *cursor, uint32_t *out, Counters *ctr) {
+__global__ void __launch_bounds__(256) k_dirty_scatter(const uint32_t *ref, const uint16_t *bin_of, int n,
+                                                       uint32_t *cursor, uint32_t *out, Counters *ctr) {
   constexpr uint32_t kEmpty = 0xFFFFFFFFu;
   __shared__ uint32_t tbin[256], tcnt[256], tbase[256];
   const int lane = threadIdx.x & 31;
@@ -1027,7 +1052,7 @@ __global__ void __launch_bounds__(256) k_dirty_scatter(const uint32_t *ref, cons
     const int i = c0 + threadIdx.x;
     const bool ok = i < n;
     const uint32_t r = ok ? ref[i] : 0u;
-    const uint32_t b = ok ? dirty_bin(depth[i], r, cls[i]) : kEmpty;
+    const uint32_t b = ok ? bin_of[i] : kEmpty;
     const unsigned peers = __match_any_sync(0xffffffffu, b);
     const int leader = __ffs(peers) - 1;
     uint32_t slot = 0, off = 0, claimed = 0;
@@ -1204,14 +1229,105 @@ __device__ __forceinline__ void prefetch_l1(const void *p) {
   asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
-// OR the low n bytes of v into the message at byte position p (the staged
-// block is zeroed first); a chunk may straddle two 8-byte words.
-__device__ __forceinline__ void or_bytes(uint64_t *st, uint32_t S, uint64_t v, uint32_t n, uint32_t p) {
-  if (n == 0) return;
-  const uint32_t q = p >> 3, r = p & 7;
-  st[q * S] |= v << (8 * r);
-  if (r != 0 && r + n > 8) st[(q + 1) * S] |= v >> (64 - 8 * r);
+// One thread's message, written front to back as 32-bit words: word w goes
+// to st[w * stride], each once.  Bytes pending for the next word are the top
+// `pb` bytes of `prev`, so a whole source word costs one funnel shift and one
+// store whatever the byte position is.
+struct WordWriter {
+  uint32_t *st;
+  uint32_t stride;
+  uint32_t w = 0, pb = 0, prev = 0;
+  __device__ __forceinline__ WordWriter(uint32_t *s, uint32_t n) : st(s), stride(n) {}
+  __device__ __forceinline__ void word(uint32_t v) {
+    st[w * stride] = __funnelshift_l(prev, v, 8 * pb);
+    ++w;
+    prev = v;
+  }
+  // the low n (0..4) bytes of v
+  __device__ __forceinline__ void bytes(uint32_t v, uint32_t n) {
+    const uint32_t t = __funnelshift_l(prev, v, 8 * pb);  // pending bytes, then v
+    const uint32_t have = pb + n;
+    if (have >= 4) {
+      st[w * stride] = t;
+      ++w;
+      pb = have - 4;
+      prev = v << (8 * (4 - n));  // n >= 1 here: its last bytes on top
+    } else {
+      pb = have;
+      prev = have ? t << (8 * (4 - have)) : 0u;
+    }
+  }
+  // the low n (0..8) bytes of v
+  __device__ __forceinline__ void bytes8(uint64_t v, uint32_t n) {
+    bytes((uint32_t)v, min(n, 4u));
+    if (n > 4) bytes((uint32_t)(v >> 32), n - 4);
+  }
+};
+
+// n bytes at src (any alignment) appended to the message.
+template <bool kCoh>
+__device__ __forceinline__ void write_body(WordWriter &o, const uint8_t *src, uint32_t n) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
+  const uint2 *q = reinterpret_cast<const uint2 *>(a & ~uintptr_t(7));
+  const uint32_t sh = 8 * (a & 3);
+  const bool up = (a & 4) != 0;
+  const uint32_t skew = a & 7;
+  // aligned 8-byte words covering the bytes: the last one is read only if
+  // the bytes reach into it
+  auto ld = [&](uint32_t j) -> uint2 {
+    if (8 * j >= n + skew) return make_uint2(0u, 0u);
+    if constexpr (kCoh)
+      return q[j];
+    else
+      return __ldg(q + j);
+  };
+  uint2 c = ld(0);
+  uint32_t o8 = 0;
+  for (; o8 + 8 <= n; o8 += 8) {
+    const uint2 d = ld(o8 / 8 + 1);
+    const uint32_t x0 = up ? c.y : c.x, x1 = up ? d.x : c.y, x2 = up ? d.y : d.x;
+    o.word(__funnelshift_r(x0, x1, sh));
+    o.word(__funnelshift_r(x1, x2, sh));
+    c = d;
+  }
+  if (o8 < n) {
+    const uint2 d = ld(o8 / 8 + 1);
+    const uint32_t x0 = up ? c.y : c.x, x1 = up ? d.x : c.y, x2 = up ? d.y : d.x;
+    uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
+    const uint32_t r = n - o8;
+    if (r < 4) lo &= (1u << (8 * r)) - 1u;
+    hi = r > 4 ? hi & ((1u << (8 * (r - 4))) - 1u) : 0u;  // r <= 7
+    o.bytes8(((uint64_t)hi << 32) | lo, r);
+  }
 }
+
+// Four bytes from eight nibble bytes (first nibble of a byte is its high half).
+__device__ __forceinline__ uint32_t pack_pairs4(uint32_t x, uint32_t y) {
+  return __byte_perm((x << 4) | (x >> 8), (y << 4) | (y >> 8), 0x6420);
+}
+
+// n bytes packed from 2n nibbles at src appended to the message.
+__device__ __forceinline__ void write_nibbles(WordWriter &o, const uint8_t *src, uint32_t n) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
+  const uint2 *q = reinterpret_cast<const uint2 *>(a & ~uintptr_t(7));
+  const uint32_t sh = 8 * (a & 3);
+  const bool up = (a & 4) != 0;
+  uint2 c = __ldg(q);
+  for (uint32_t j = 0; 4 * j < n; ++j) {
+    const uint2 d = __ldg(q + j + 1);  // the nibble arena ends in 64 spare bytes
+    const uint32_t x0 = up ? c.y : c.x, x1 = up ? d.x : c.y, x2 = up ? d.y : d.x;
+    const uint32_t v = pack_pairs4(__funnelshift_r(x0, x1, sh), __funnelshift_r(x1, x2, sh));
+    if (4 * j + 4 <= n)
+      o.word(v);
+    else
+      o.bytes(v & ((1u << (8 * (n - 4 * j))) - 1u), n - 4 * j);
+    c = d;
+  }
+}
+
+// Staging words (32-bit) per thread: a block, and what one branch child (gap
+// bytes, tag and hash) can run past its end.
+constexpr uint32_t kStageWords = 34 + 14;
 
 // Start the loads of a child item's bytes early (hash line, or the first
 // lines of a value) so the encoder's streaming reads hit L1.
@@ -1223,10 +1339,15 @@ __device__ __forceinline__ void prefetch_child(const TrieView &tv, uint32_t r) {
     prefetch_l1(tv.short_hash + (size_t)idx * 32);
 }
 
-// Encode + hash one dirty node; `stage` is this thread's 17-word message
-// block in shared memory (word w at stage[w * stride]).
+// Encode + hash one dirty node; `stage` is this thread's column of the
+// message block in shared memory (kStageWords 32-bit words, word w at
+// stage[w * stride]).
+//
+// Bound by the integer pipe (one permutation per 136 bytes), so the encoders
+// around it are kept to few instructions per byte: whole words through one
+// funnel shift, a branch child's hash in two 16-byte loads.
 template <bool kCoh>
-__device__ __forceinline__ void hash_node(const TrieView &tv, uint32_t ref, uint64_t *stage, uint32_t stride) {
+__device__ __forceinline__ void hash_node(const TrieView &tv, uint32_t ref, uint32_t *stage, uint32_t stride) {
   uint32_t kind = ref_kind(ref), idx = ref_idx(ref);
   bool full = kind == KIND_FULL;
   // nodes a split or a delete unlinked are not hashed
@@ -1289,88 +1410,76 @@ __device__ __forceinline__ void hash_node(const TrieView &tv, uint32_t ref, uint
   sp.reset(stage, stride);
   if (!full && total <= 135) {
     // One-block short node (every leaf with a value up to ~100 bytes, every
-    // extension): place each segment's 8-byte chunks into the zeroed block
-    // with shared-memory OR, pad, and permute once.
-    uint64_t *st = sp.stage;
-    const uint32_t S = sp.stride;
+    // extension): header, key, child, padding, permuted once.
+    WordWriter o(stage, stride);
+    o.bytes((uint32_t)hdr, hn);  // at most two bytes here
+    o.bytes8(it1.pre, it1.pren);
+    write_nibbles(o, it1.body, it1.blen);
+    o.bytes((uint32_t)it2.pre, it2.pren);
+    write_body<kCoh>(o, it2.body, it2.blen);
+    if (raw) {
+      const uint32_t z = total == 0 ? 0u : (uint32_t)total;
+      o.bytes(0u, 4);  // flush the pending bytes
+      for (uint32_t w = o.w; w < 8; ++w) stage[w * stride] = 0;
+      uint64_t keep[4];
 #pragma unroll
-    for (int w = 0; w < 17; ++w) st[w * S] = 0;
-    uint32_t p = 0;
-    or_bytes(st, S, hdr, hn, p);
-    p += hn;
-    or_bytes(st, S, it1.pre, it1.pren, p);
-    p += it1.pren;
-    for (uint32_t o = 0; o < it1.blen; o += 8) {
-      uint32_t nb = min(8u, it1.blen - o);
-      or_bytes(st, S, pack_pairs8(it1.body + 2 * o) & low_bytes_mask(nb), nb, p + o);
-    }
-    p += it1.blen;
-    or_bytes(st, S, it2.pre, it2.pren, p);
-    p += it2.pren;
-    for (uint32_t o = 0; o < it2.blen; o += 8) {
-      uint32_t nb = min(8u, it2.blen - o);
-      or_bytes(st, S, ld8<kCoh>(it2.body + o) & low_bytes_mask(nb), nb, p + o);
-    }
-    p += it2.blen;
-    if (!raw) {
-      or_bytes(st, S, 0x01, 1, p);
-      st[16 * S] |= 0x8000000000000000ull;
+      for (int w = 0; w < 4; ++w) {
+        keep[w] = sp.word(w);
+        const int left = (int)z - 8 * w;
+        keep[w] = left >= 8 ? keep[w] : (left <= 0 ? 0ull : (keep[w] & ((1ull << (8 * left)) - 1)));
+      }
 #pragma unroll
-      for (int w = 0; w < 17; ++w) sp.a[w] = st[w * S];
-      keccak_f1600(sp.a);
+      for (int w = 0; w < 4; ++w) sp.a[w] = keep[w];
+    } else {
+      o.bytes(0x01u, 1);
+      o.bytes(0u, 3);  // at least the pending bytes; position 135 is inside the block
+      for (uint32_t w = o.w; w < 34; ++w) stage[w * stride] = 0;
+      stage[33 * stride] |= 0x80000000u;
+      sp.absorb();
     }
   } else if (regular) {
-  // regular branch: pending message bytes (little-endian), next slot, words
-  // left of the current child's hash
-  uint64_t buf = hdr;
-  uint32_t nb = hn, slot = 0, hj = 8;
-  const uint32_t *hw = nullptr;
-  bool last = false;
-  while (true) {
-    {  // one block: 0x80 per empty slot, 0xa0 + 32 hash bytes per child, then
-       // the Keccak padding (rlp.cuh:132-155, node.cuh:46-112)
-      uint64_t *st = sp.stage;
-      const uint32_t S = sp.stride;
-      for (int w = 0; w < 17; ++w) {
-        uint64_t word = 0;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          while (nb < 4) {
-            if (hj < 8) {
-              buf |= (uint64_t)ldn<kCoh>(hw + hj) << (8 * nb);
-              nb += 4;
-              ++hj;
-            } else if (slot < 17) {
-              if ((present >> slot) & 1u) {
-                const uint32_t r = ldn<kCoh>(chp + slot);
-                hw = reinterpret_cast<const uint32_t *>(
-                    (ref_kind(r) == KIND_FULL ? tv.full_hash : tv.short_hash) + (size_t)ref_idx(r) * 32);
-                buf |= 0xa0ull << (8 * nb);
-                hj = 0;
-              } else {
-                buf |= 0x80ull << (8 * nb);
-              }
-              nb += 1;
-              ++slot;
-            } else if (!last) {
-              buf |= 0x01ull << (8 * nb);  // Keccak padding starts here
-              nb += 1;
-              last = true;
-            } else {
-              nb = 4;  // zeros to the end of the block
-            }
-          }
-          word |= (buf & 0xFFFFFFFFull) << (32 * half);
-          buf >>= 32;
-          nb -= 4;
+    // 0x80 per empty slot, 0xa0 + 32 hash bytes per child, then the Keccak
+    // padding (rlp.cuh:132-155, node.cuh:46-112).  A child at a time: its
+    // hash in two 16-byte loads, eight funnel-shifted words out.  A block is
+    // permuted when full; what the last child wrote past it moves to the front.
+    WordWriter o(stage, stride);
+    o.bytes((uint32_t)hdr, hn);
+    uint32_t left = present;
+    int prev = -1;
+    bool done = false;
+    while (true) {
+      while (o.w < 34 && !done) {
+        const int k = left ? __ffs(left) - 1 : 17;  // next child, or the end
+        left &= left - 1;
+        uint32_t gap = (uint32_t)(k - prev - 1);
+        prev = k;
+        if (k < 17) {
+          const uint32_t r = ldn<kCoh>(chp + k);
+          const uint4 *h = reinterpret_cast<const uint4 *>(
+              (ref_kind(r) == KIND_FULL ? tv.full_hash : tv.short_hash) + (size_t)ref_idx(r) * 32);
+          const uint4 x = ldn<kCoh>(h), y = ldn<kCoh>(h + 1);
+          for (; gap >= 4; gap -= 4) o.word(0x80808080u);
+          // gap (0..3) empty slots, then the child's tag
+          o.bytes((0x80808080u & ((1u << (8 * gap)) - 1u)) | (0xa0u << (8 * gap)), gap + 1);
+          o.word(x.x), o.word(x.y), o.word(x.z), o.word(x.w);
+          o.word(y.x), o.word(y.y), o.word(y.z), o.word(y.w);
+        } else {
+          for (; gap >= 4; gap -= 4) o.word(0x80808080u);
+          o.bytes((0x80808080u & ((1u << (8 * gap)) - 1u)) | (0x01u << (8 * gap)), gap + 1);
+          o.bytes(0u, o.pb ? 4 - o.pb : 0u);  // whole words from here on
+          done = true;
         }
-        st[w * S] = word;
       }
-      if (last) st[16 * S] |= 0x8000000000000000ull;
+      const bool last = done && o.w <= 34;
+      if (last) {
+        for (uint32_t w = o.w; w < 34; ++w) stage[w * stride] = 0;
+        stage[33 * stride] |= 0x80000000u;
+      }
+      sp.absorb();
+      if (last) break;
+      for (uint32_t w = 34; w < o.w; ++w) stage[(w - 34) * stride] = stage[w * stride];
+      o.w -= 34;
     }
-    sp.absorb();
-    if (last) break;
-  }
   } else {
   // pass 2: stream
   int item = 0;
@@ -1446,21 +1555,17 @@ __device__ __forceinline__ void hash_node(const TrieView &tv, uint32_t ref, uint
   }
   uint8_t *hout = (full ? tv.full_hash : tv.short_hash) + (size_t)idx * 32;
   uint64_t *o = reinterpret_cast<uint64_t *>(hout);
-  if (raw) {
+  if (raw && full) {  // a short node's is in sp.a already
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      uint64_t v = sp.stage[w * sp.stride];
+      uint64_t v = sp.word(w);
       int keep = (int)total - 8 * w;
-      o[w] = keep >= 8 ? v : (keep <= 0 ? 0ull : (v & ((1ull << (8 * keep)) - 1)));
+      sp.a[w] = keep >= 8 ? v : (keep <= 0 ? 0ull : (v & ((1ull << (8 * keep)) - 1)));
     }
-    (full ? tv.full_hlen : tv.short_hlen)[idx] = (uint8_t)total;
-  } else {
-    o[0] = sp.a[0];
-    o[1] = sp.a[1];
-    o[2] = sp.a[2];
-    o[3] = sp.a[3];
-    (full ? tv.full_hlen : tv.short_hlen)[idx] = 32;
   }
+  reinterpret_cast<ulonglong2 *>(o)[0] = make_ulonglong2(sp.a[0], sp.a[1]);
+  reinterpret_cast<ulonglong2 *>(o)[1] = make_ulonglong2(sp.a[2], sp.a[3]);
+  (full ? tv.full_hlen : tv.short_hlen)[idx] = raw ? (uint8_t)total : 32;
 }
 
 // Message buffer of one warp for the warp-cooperative hashing (8 Keccak blocks).
@@ -1480,6 +1585,14 @@ struct WarpItem {
   Bytes32 body{};
   const uint8_t *far = nullptr;  // body of more than 32 bytes
 };
+
+// Header of a child node's item once its hash (or encoding below 32 bytes) is
+// in the body.
+__device__ __forceinline__ void node_head(const TrieView &tv, WarpItem &it) {
+  if (tv.geth_mode && it.blen < 32) return;                         // go-ethereum embeds small nodes
+  if (it.blen == 1 && (uint8_t)it.body.w[0] < 0x80) return;         // single byte is its own encoding
+  rlp_head(it.blen, 0x80, 0xb7, it.pre, it.pren);
+}
 
 // The item a branch (or a short node) writes for child `r`: child_item with
 // the bytes of hashes and short values already loaded, every load of a lane
@@ -1511,7 +1624,8 @@ __device__ __forceinline__ WarpItem warp_child_item(const TrieView &tv, uint32_t
     const ulonglong2 a = __ldcg(h), b = __ldcg(h + 1);
     it.blen = __ldcg((full ? tv.full_hlen : tv.short_hlen) + idx);
     it.body = Bytes32{{a.x, a.y, b.x, b.y}};
-    if (tv.geth_mode && it.blen < 32) return it;  // go-ethereum embeds small nodes
+    node_head(tv, it);
+    return it;
   }
   if (it.blen == 1 && (uint8_t)it.body.w[0] < 0x80) return it;  // single byte is its own encoding
   rlp_head(it.blen, 0x80, 0xb7, it.pre, it.pren);
@@ -1559,13 +1673,113 @@ __device__ __forceinline__ void put_far(uint8_t *msg, uint32_t lo, uint32_t hi, 
   if (wz + lane < z) msg[wz + lane] = ldn<kCoh>(s0 + wz + lane);
 }
 
-// Warp-cooperative encode + hash of branch node idx, for levels with few
-// nodes or for branches of many blocks, where one thread's serial chain is
-// the latency.  Lane k < 17 loads child k's item; a scan gives every item its
-// place, and the message is built window by window (kWarpMsgBytes, 8 blocks)
-// in the warp's shared buffer -- every lane its own item's bytes at once,
-// long values by all lanes -- and absorbed with the warp-spread permutation.
-// All 32 lanes call it with the same idx.
+// Zero the blocks [b0, b0 + wb) of a message in the warp's window.
+__device__ __forceinline__ void window_clear(uint64_t *m64, uint32_t wb, int lane) {
+  for (uint32_t w = lane; w < wb * 17; w += 32) m64[w] = 0;
+  __syncwarp();
+}
+
+// Pad the window [lo, lo + 136 wb) of a `total`-byte message of nblk blocks
+// and absorb it into the warp-spread state.
+__device__ __forceinline__ uint64_t window_absorb(uint64_t a, uint8_t *msg, uint32_t lo, uint32_t wb, uint32_t total,
+                                                  uint32_t nblk, const CoopLanes &cl, int lane) {
+  const uint64_t *m64 = reinterpret_cast<const uint64_t *>(msg);
+  if (lane == 0) {  // Keccak padding (pad byte 0x01 ... last byte |= 0x80)
+    if (total >= lo && total < lo + wb * 136) msg[total - lo] ^= 0x01;
+    if (lo + wb * 136 == nblk * 136) msg[wb * 136 - 1] ^= 0x80;
+  }
+  __syncwarp();
+  for (uint32_t bb = 0; bb < wb; ++bb) {
+    if (lane < 17) a ^= m64[bb * 17 + lane];
+    a = keccak_f1600_warp(a, cl);
+  }
+  __syncwarp();  // the next window reuses the buffer
+  return a;
+}
+
+// Store a node's 32-byte hash (a: the warp-spread state) or, below 32 bytes,
+// its encoding (the zero-padded window); returns lane l's word of it for
+// l < 4.
+__device__ __forceinline__ uint64_t store_hash(const TrieView &tv, uint64_t *o, uint8_t *hlen, bool raw, uint64_t a,
+                                               const uint64_t *m64, uint32_t total, uint32_t nblk, int lane) {
+  const uint64_t v = raw ? m64[lane & 3] : a;
+  if (lane < 4) o[lane] = v;
+  if (lane == 0) *hlen = raw ? (uint8_t)total : 32;
+  if (lane == 0 && tv.account) {
+    atomicAdd(&tv.ctr->enc_bytes, (unsigned long long)total);
+    atomicAdd(&tv.ctr->keccak_blocks, (unsigned long long)(raw ? 0u : nblk));
+    atomicAdd(&tv.ctr->hashed, 1u);
+  }
+  __syncwarp();
+  return v;
+}
+
+// Warp-cooperative encode + hash of short node idx (a leaf, or an extension).
+// known: the child's hash (hw: lane l < 4 holds word l, hl bytes) comes from
+// the caller, which has just computed it.  All 32 lanes call it alike.
+template <bool kCoh>
+__device__ __forceinline__ void hash_short_warp(const TrieView &tv, uint32_t idx, uint8_t *msg, const CoopLanes &cl,
+                                                bool known, uint64_t hw, uint32_t hl) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint64_t ko = ldn<kCoh>(tv.short_key + idx);
+  const uint32_t klen = ldn<kCoh>(tv.short_klen + idx);
+  const uint32_t child = ldn<kCoh>(tv.short_child + idx);
+  const bool dead = ldn<kCoh>(tv.short_dead + idx) != 0;
+  const bool force = tv.geth_mode && ldn<kCoh>(tv.short_depth + idx) == 0;
+  if (dead) return;  // unlinked by a split or a delete
+  const EncItem key = compact_item(tv, ko, klen);
+  WarpItem it;
+  if (known) {
+    it.blen = hl;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) it.body.w[w] = __shfl_sync(kAll, hw, w);
+    node_head(tv, it);
+  } else {
+    it = warp_child_item<kCoh>(tv, child);
+  }
+  const uint32_t payload = key.pren + key.blen + it.pren + it.blen;
+  uint64_t hdr;
+  uint32_t hn;
+  rlp_head(payload, 0xc0, 0xf7, hdr, hn);
+  const uint32_t total = payload + hn;
+  const bool raw = total < 32 && !force;
+  const uint32_t nblk = raw ? 1u : (total + 1 + 135) / 136;
+  const uint32_t pk = hn + key.pren, pc = pk + key.blen;  // key body, child item
+  uint64_t *m64 = reinterpret_cast<uint64_t *>(msg);
+  uint64_t a = 0;
+  for (uint32_t b0 = 0; b0 < nblk; b0 += kWarpMsgBytes / 136) {
+    const uint32_t wb = min((uint32_t)(kWarpMsgBytes / 136), nblk - b0);
+    const uint32_t lo = b0 * 136, hi = lo + wb * 136;
+    window_clear(m64, wb, lane);
+    if (lane == 31) put_prefix(msg, lo, hi, hdr, hn, 0);
+    if (lane == 30) put_prefix(msg, lo, hi, key.pre, key.pren, hn);
+    if (lane == 29) put_prefix(msg, lo, hi, it.pre, it.pren, pc);
+    for (uint32_t j = lane; j < key.blen; j += 32)
+      if (pk + j >= lo && pk + j < hi) msg[pk + j - lo] = (uint8_t)((key.body[2 * j] << 4) | key.body[2 * j + 1]);
+    if (it.far) {
+      put_far<kCoh>(msg, lo, hi, it.far, it.blen, pc + it.pren, lane);
+    } else {
+      const uint32_t q = pc + it.pren + lane;
+      const uint64_t w = lane < 16 ? (lane < 8 ? it.body.w[0] : it.body.w[1])
+                                   : (lane < 24 ? it.body.w[2] : it.body.w[3]);
+      if ((uint32_t)lane < it.blen && q >= lo && q < hi) msg[q - lo] = (uint8_t)(w >> (8 * (lane & 7)));
+    }
+    __syncwarp();
+    if (raw) break;  // under 32 bytes: the window holds the whole encoding
+    a = window_absorb(a, msg, lo, wb, total, nblk, cl, lane);
+  }
+  store_hash(tv, reinterpret_cast<uint64_t *>(tv.short_hash + (size_t)idx * 32), tv.short_hlen + idx, raw, a, m64,
+             total, nblk, lane);
+}
+
+// Warp-cooperative encode + hash of branch node idx and of the extension
+// above it, for levels with few nodes or for branches of many blocks, where
+// one thread's serial chain is the latency.  Lane k < 17 loads child k's
+// item; a scan gives every item its place, and the message is built window
+// by window (kWarpMsgBytes, 8 blocks) in the warp's shared buffer -- every
+// lane its own item's bytes at once, long values by all lanes -- and absorbed
+// with the warp-spread permutation.  All 32 lanes call it with the same idx.
 // Bound by latency: one chain of dependent loads (node, children, hashes),
 // then the serial permutations.  Building item after item (one L2 round trip
 // each) took a 16-child branch 15-17 us per level of a 1M-key trie; this
@@ -1601,8 +1815,7 @@ __device__ __forceinline__ void hash_full_warp(const TrieView &tv, uint32_t idx,
   for (uint32_t b0 = 0; b0 < nblk; b0 += kWarpMsgBytes / 136) {
     const uint32_t wb = min((uint32_t)(kWarpMsgBytes / 136), nblk - b0);
     const uint32_t lo = b0 * 136, hi = lo + wb * 136;
-    for (uint32_t w = lane; w < wb * 17; w += 32) m64[w] = 0;
-    __syncwarp();
+    window_clear(m64, wb, lane);
     if (lane == 31) put_prefix(msg, lo, hi, hdr, hn, 0);
     put_prefix(msg, lo, hi, it.pre, it.pren, my_off);
     if (!it.far) put_body32(msg, lo, hi, it.body, it.blen, my_off + it.pren);
@@ -1615,42 +1828,29 @@ __device__ __forceinline__ void hash_full_warp(const TrieView &tv, uint32_t idx,
     }
     __syncwarp();
     if (raw) break;  // under 32 bytes: the window holds the whole encoding
-    if (lane == 0) {  // Keccak padding (pad byte 0x01 ... last byte |= 0x80)
-      if (total >= lo && total < hi) msg[total - lo] ^= 0x01;
-      if (hi == nblk * 136) msg[wb * 136 - 1] ^= 0x80;
-    }
-    __syncwarp();
-    for (uint32_t bb = 0; bb < wb; ++bb) {
-      if (lane < 17) a ^= m64[bb * 17 + lane];
-      a = keccak_f1600_warp(a, cl);
-    }
-    __syncwarp();  // the next window reuses the buffer
+    a = window_absorb(a, msg, lo, wb, total, nblk, cl, lane);
   }
-  uint64_t *o = reinterpret_cast<uint64_t *>(tv.full_hash + (size_t)idx * 32);
-  if (raw) {
-    if (lane < 4) o[lane] = m64[lane];  // zero beyond total
-    if (lane == 0) tv.full_hlen[idx] = (uint8_t)total;
-  } else {
-    if (lane < 4) o[lane] = a;
-    if (lane == 0) tv.full_hlen[idx] = 32;
+  const uint64_t hw = store_hash(tv, reinterpret_cast<uint64_t *>(tv.full_hash + (size_t)idx * 32), tv.full_hlen + idx,
+                                 raw, a, m64, total, nblk, lane);
+  if constexpr (!kCoh) {
+    const uint32_t e = ext_above(tv, idx);
+    if (e != kNoNode) hash_short_warp<kCoh>(tv, e, msg, cl, true, hw, raw ? total : 32u);
   }
-  if (lane == 0 && tv.account) {
-    atomicAdd(&tv.ctr->enc_bytes, (unsigned long long)total);
-    atomicAdd(&tv.ctr->keccak_blocks, (unsigned long long)(raw ? 0u : nblk));
-    atomicAdd(&tv.ctr->hashed, 1u);
-  }
-  __syncwarp();
 }
 
-// Branch nodes one warp each (a level's branches when it has few, or its
-// branches of many blocks): 4 warps per CTA.
-__global__ void __launch_bounds__(128) k_hash_full_warp(TrieView tv, const uint32_t *refs, int count) {
+// A warp per node (4 per CTA): a level's branches when it has few, or its
+// branches of many blocks, each with the extension above it; or a few leaves.
+__global__ void __launch_bounds__(128) k_hash_warp(TrieView tv, const uint32_t *refs, int count) {
   extern __shared__ uint64_t msg_all[];  // one message window per warp
   const int j = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (j >= count) return;  // whole warps leave together
   uint8_t *msg = reinterpret_cast<uint8_t *>(msg_all) + (threadIdx.x >> 5) * kWarpMsgBytes;
   const CoopLanes cl = coop_lanes(threadIdx.x & 31);
-  hash_full_warp<false>(tv, ref_idx(refs[j]), msg, cl);
+  const uint32_t r = refs[j];
+  if (ref_kind(r) == KIND_FULL)
+    hash_full_warp<false>(tv, ref_idx(r), msg, cl);
+  else
+    hash_short_warp<false>(tv, ref_idx(r), msg, cl, false, 0, 0);
 }
 
 // Six 128-thread CTAs per SM (at most 85 registers): the permutation keeps
@@ -1666,7 +1866,7 @@ constexpr int kHashLevelThreads = 128;  // k_hash_level's block size (the partit
 #define GMPT_HASH_CTAS 6
 #endif
 __device__ __forceinline__ void hash_level_cta(const TrieView &tv, const uint32_t *refs, int count) {
-  extern __shared__ uint64_t stage_all[];
+  extern __shared__ uint32_t stage_all[];
   __shared__ uint32_t s_ref[kHashLevelThreads];
   __shared__ uint32_t s_cnt[kCtaClasses][kHashLevelThreads / 32];  // [class][warp]
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
