@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(256, 2) k_block(TrieView tv0, DirtyList dl, Bl
       ++levels;
       // short nodes [a, m) from warp 0 up, full nodes [m, z) from warp W-1 down
       for (uint32_t j = (uint32_t)t_spread; j < m - a; j += (uint32_t)T)
-        hash_node<true>(tv, __ldcg(bb.sorted + a + j), smem + threadIdx.x, blockDim.x);
+        hash_node<true, false>(tv, ref_idx(__ldcg(bb.sorted + a + j)), smem + threadIdx.x, blockDim.x);
       if (z - m <= (uint32_t)(kWarpFullPerWarp * W)) {
         // few branches: a warp per node (latency)
         for (uint32_t j = (uint32_t)(W - 1 - gw); j < z - m; j += (uint32_t)W) {
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(256, 2) k_block(TrieView tv0, DirtyList dl, Bl
       } else {
         const uint32_t t_rev = (uint32_t)(lane * W + (W - 1 - gw));
         for (uint32_t j = t_rev; j < z - m; j += (uint32_t)T)
-          hash_node<true>(tv, __ldcg(bb.sorted + m + j), smem + threadIdx.x, blockDim.x);
+          hash_node<true, true>(tv, ref_idx(__ldcg(bb.sorted + m + j)), smem + threadIdx.x, blockDim.x);
       }
       if (!grid_barrier(D, tv.ctr)) return;
     }

@@ -48,7 +48,8 @@ struct Counters {
   uint32_t n_full, n_short, n_value, pad0;
   uint32_t n_dirty, n_items, n_groups, error;
   uint64_t key_used, val_used;
-  uint32_t n_pseudo, retries_max, hashed, pad2;
+  uint32_t n_pseudo, retries_max, hashed;
+  uint32_t raw_nodes;  // 1: some node's encoding was below 32 bytes since the last reset
   unsigned long long enc_bytes, keccak_blocks;  // last hash pass
   // staging checks of the last batch
   unsigned long long stream_terms;  // bytes == 16 in the key stream

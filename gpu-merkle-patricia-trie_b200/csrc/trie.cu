@@ -1006,12 +1006,11 @@ int Trie::bucket_and_hash() {
   // a launch of at most kWideGrid CTAs cannot fill the SMs at the
   // throughput form's occupancy: it runs the wide form (more registers per
   // thread, no spills, shorter serial chains)
-  auto level = [&](const uint32_t *refs, uint32_t cnt) {
+  auto level = [&](bool full, const uint32_t *refs, uint32_t cnt) {
     const unsigned grid = blocks_for(cnt, kHashThreads);
-    if (grid <= kWideGrid)
-      count_launch(), k_hash_level_wide<<<grid, kHashThreads, smem, st_>>>(tv_, refs, (int)cnt);
-    else
-      count_launch(), k_hash_level<<<grid, kHashThreads, smem, st_>>>(tv_, refs, (int)cnt);
+    auto kern = grid <= kWideGrid ? (full ? k_hash_level_wide<true> : k_hash_level_wide<false>)
+                                  : (full ? k_hash_level<true> : k_hash_level<false>);
+    count_launch(), kern<<<grid, kHashThreads, smem, st_>>>(tv_, refs, (int)cnt);
   };
   auto warps = [&](const uint32_t *refs, uint32_t cnt) {
     count_launch(), k_hash_warp<<<(cnt + 3) / 4, 128, smem_warp, st_>>>(tv_, refs, (int)cnt);
@@ -1022,7 +1021,7 @@ int Trie::bucket_and_hash() {
     if (off[kLeafClasses] <= kWarpLeafMax)
       warps(sorted, off[kLeafClasses]);
     else
-      level(sorted, off[kLeafClasses]);
+      level(false, sorted, off[kLeafClasses]);
   }
   for (int d = (int)dirty_depths() - 1; d >= 0; --d) {
     // branches [a, m), the extensions above them [m, z)
@@ -1041,11 +1040,11 @@ int Trie::bucket_and_hash() {
       // value, up to kilobytes, in slot 16) would set the level's time as
       // one thread's serial chain: one warp each, the rest thread-wise
       warps(sorted + a, ml - a);
-      level(sorted + ml, m - ml);
+      level(true, sorted + ml, m - ml);
     } else {
-      level(sorted + a, m - a);
+      level(true, sorted + a, m - a);
     }
-    if (z > m) level(sorted + m, z - m);
+    if (z > m) level(false, sorted + m, z - m);
   }
   if (timing_) {
     cudaEventRecord(kz, st_);

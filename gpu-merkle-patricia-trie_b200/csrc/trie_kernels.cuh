@@ -902,15 +902,15 @@ __global__ void k_level_scatter(const uint32_t *act, const uint32_t *aseg, const
 
 // ---------------------------------------------------------------------------
 // PhaseHC: dirty nodes with nothing dirty below them first, then the branches
-// by nibble depth, deepest first; an extension is hashed by the task of the
-// branch below it
+// by nibble depth, deepest first; an extension over a dirty branch is hashed
+// in that branch's level
 
 // Keccak blocks a dirty branch's encoding is expected to take, minus one,
 // capped at kHashClasses - 1: children counted as 33-byte references, and a
 // value in slot 16 (a key that ends at the branch) by its length, which can
-// be kilobytes.  Branches of a level are binned by it, and k_hash_level
-// orders each CTA's nodes by block class, so the lanes of a warp need the
-// same number of permutations and none idles through another's extra ones.
+// be kilobytes.  Branches of a level are binned by it, so the lanes of a warp
+// need the same number of permutations and none idles through another's extra
+// ones.
 constexpr uint32_t kHashClasses = 8;
 
 __device__ __forceinline__ uint32_t full_bytes(const TrieView &tv, uint32_t idx) {
@@ -926,30 +926,6 @@ __device__ __forceinline__ uint32_t full_bytes(const TrieView &tv, uint32_t idx)
 
 __device__ __forceinline__ uint32_t full_class(const TrieView &tv, uint32_t idx) {
   return min(full_bytes(tv, idx) / 136u, kHashClasses - 1u);
-}
-
-// Finer classes for the order inside one hashing CTA (leaves with values of
-// up to kilobytes take 1 to 31 blocks): 1, 2, 3, 4, 5-6, 7-10, 11-18, 19+
-// blocks.
-constexpr uint32_t kCtaClasses = 8;
-
-__device__ __forceinline__ uint32_t blocks_class(uint32_t blocks_minus_1) {
-  const uint32_t b = blocks_minus_1;
-  return b < 4u ? b : (b < 6u ? 4u : (b < 10u ? 5u : (b < 18u ? 6u : 7u)));
-}
-
-__device__ __forceinline__ uint32_t hash_class(const TrieView &tv, uint32_t r) {
-  const uint32_t kind = ref_kind(r), idx = ref_idx(r);
-  uint32_t bytes;
-  if (kind == KIND_FULL) {
-    return blocks_class(full_bytes(tv, idx) / 136u);
-  } else {
-    if (tv.short_dead[idx]) return 0u;
-    const uint32_t ch = tv.short_child[idx];
-    bytes = tv.short_klen[idx] / 2u + 8u;
-    bytes += ref_kind(ch) == KIND_VALUE ? load_rec(tv, tv.value_vid[ref_idx(ch)]).len : 33u;
-  }
-  return blocks_class(bytes / 136u);
 }
 
 // Leaves (short nodes over a value) depend on nothing below them, so every
@@ -1264,64 +1240,83 @@ struct WordWriter {
   }
 };
 
-// n bytes at src (any alignment) appended to the message.
+// Four aligned 8-byte words covering bytes from `src` on, and the funnel that
+// takes unaligned 32-bit words out of them.  Loading four at a time keeps a
+// gather's L2 round trips to one per 32 bytes.
+struct SrcWords {
+  const uint2 *q;
+  uint32_t sh, skew;
+  bool up;
+  __device__ __forceinline__ explicit SrcWords(const uint8_t *src) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(src);
+    q = reinterpret_cast<const uint2 *>(a & ~uintptr_t(7));
+    skew = (uint32_t)(a & 7);
+    sh = 8 * (skew & 3);
+    up = (skew & 4) != 0;
+  }
+  // unaligned 32-bit words 0 and 1 from aligned words c, d
+  __device__ __forceinline__ uint2 pair(uint2 c, uint2 d) const {
+    const uint32_t x0 = up ? c.y : c.x, x1 = up ? d.x : c.y, x2 = up ? d.y : d.x;
+    return make_uint2(__funnelshift_r(x0, x1, sh), __funnelshift_r(x1, x2, sh));
+  }
+};
+
+// n bytes at src (any alignment) appended to the message.  An aligned word is
+// read only if the n bytes reach into it.
 template <bool kCoh>
 __device__ __forceinline__ void write_body(WordWriter &o, const uint8_t *src, uint32_t n) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-  const uint2 *q = reinterpret_cast<const uint2 *>(a & ~uintptr_t(7));
-  const uint32_t sh = 8 * (a & 3);
-  const bool up = (a & 4) != 0;
-  const uint32_t skew = a & 7;
-  // aligned 8-byte words covering the bytes: the last one is read only if
-  // the bytes reach into it
+  const SrcWords s(src);
+  const uint32_t words = (n + s.skew + 7) / 8;
   auto ld = [&](uint32_t j) -> uint2 {
-    if (8 * j >= n + skew) return make_uint2(0u, 0u);
+    if (j >= words) return make_uint2(0u, 0u);
     if constexpr (kCoh)
-      return q[j];
+      return s.q[j];
     else
-      return __ldg(q + j);
+      return __ldg(s.q + j);
   };
   uint2 c = ld(0);
-  uint32_t o8 = 0;
-  for (; o8 + 8 <= n; o8 += 8) {
-    const uint2 d = ld(o8 / 8 + 1);
-    const uint32_t x0 = up ? c.y : c.x, x1 = up ? d.x : c.y, x2 = up ? d.y : d.x;
-    o.word(__funnelshift_r(x0, x1, sh));
-    o.word(__funnelshift_r(x1, x2, sh));
-    c = d;
-  }
-  if (o8 < n) {
-    const uint2 d = ld(o8 / 8 + 1);
-    const uint32_t x0 = up ? c.y : c.x, x1 = up ? d.x : c.y, x2 = up ? d.y : d.x;
-    uint32_t lo = __funnelshift_r(x0, x1, sh), hi = __funnelshift_r(x1, x2, sh);
-    const uint32_t r = n - o8;
-    if (r < 4) lo &= (1u << (8 * r)) - 1u;
-    hi = r > 4 ? hi & ((1u << (8 * (r - 4))) - 1u) : 0u;  // r <= 7
-    o.bytes8(((uint64_t)hi << 32) | lo, r);
+  for (uint32_t j = 0; 8 * j < n; j += 4) {
+    const uint2 d[4] = {ld(j + 1), ld(j + 2), ld(j + 3), ld(j + 4)};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t at = 8 * (j + k);
+      const uint2 v = s.pair(c, d[k]);
+      c = d[k];
+      if (at + 8 <= n) {
+        o.word(v.x);
+        o.word(v.y);
+      } else if (at < n) {
+        const uint32_t r = n - at;  // 1..7
+        o.bytes(v.x, min(r, 4u));
+        if (r > 4) o.bytes(v.y, r - 4);
+      }
+    }
   }
 }
 
 // Four bytes from eight nibble bytes (first nibble of a byte is its high half).
-__device__ __forceinline__ uint32_t pack_pairs4(uint32_t x, uint32_t y) {
-  return __byte_perm((x << 4) | (x >> 8), (y << 4) | (y >> 8), 0x6420);
+__device__ __forceinline__ uint32_t pack_pairs4(uint2 v) {
+  return __byte_perm((v.x << 4) | (v.x >> 8), (v.y << 4) | (v.y >> 8), 0x6420);
 }
 
 // n bytes packed from 2n nibbles at src appended to the message.
 __device__ __forceinline__ void write_nibbles(WordWriter &o, const uint8_t *src, uint32_t n) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-  const uint2 *q = reinterpret_cast<const uint2 *>(a & ~uintptr_t(7));
-  const uint32_t sh = 8 * (a & 3);
-  const bool up = (a & 4) != 0;
-  uint2 c = __ldg(q);
-  for (uint32_t j = 0; 4 * j < n; ++j) {
-    const uint2 d = __ldg(q + j + 1);  // the nibble arena ends in 64 spare bytes
-    const uint32_t x0 = up ? c.y : c.x, x1 = up ? d.x : c.y, x2 = up ? d.y : d.x;
-    const uint32_t v = pack_pairs4(__funnelshift_r(x0, x1, sh), __funnelshift_r(x1, x2, sh));
-    if (4 * j + 4 <= n)
-      o.word(v);
-    else
-      o.bytes(v & ((1u << (8 * (n - 4 * j))) - 1u), n - 4 * j);
-    c = d;
+  const SrcWords s(src);
+  const uint32_t words = (2 * n + s.skew + 7) / 8;
+  auto ld = [&](uint32_t j) { return j < words ? __ldg(s.q + j) : make_uint2(0u, 0u); };
+  uint2 c = ld(0);
+  for (uint32_t j = 0; 4 * j < n; j += 4) {
+    const uint2 d[4] = {ld(j + 1), ld(j + 2), ld(j + 3), ld(j + 4)};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t at = 4 * (j + k);
+      const uint32_t v = pack_pairs4(s.pair(c, d[k]));
+      c = d[k];
+      if (at + 4 <= n)
+        o.word(v);
+      else if (at < n)
+        o.bytes(v, n - at);
+    }
   }
 }
 
@@ -1329,76 +1324,79 @@ __device__ __forceinline__ void write_nibbles(WordWriter &o, const uint8_t *src,
 // bytes, tag and hash) can run past its end.
 constexpr uint32_t kStageWords = 34 + 14;
 
-// Start the loads of a child item's bytes early (hash line, or the first
-// lines of a value) so the encoder's streaming reads hit L1.
-__device__ __forceinline__ void prefetch_child(const TrieView &tv, uint32_t r) {
-  uint32_t kind = ref_kind(r), idx = ref_idx(r);
-  if (kind == KIND_FULL)
-    prefetch_l1(tv.full_hash + (size_t)idx * 32);
-  else if (kind == KIND_SHORT)
-    prefetch_l1(tv.short_hash + (size_t)idx * 32);
-}
-
 // Encode + hash one dirty node; `stage` is this thread's column of the
 // message block in shared memory (kStageWords 32-bit words, word w at
 // stage[w * stride]).
 //
 // Bound by the integer pipe (one permutation per 136 bytes), so the encoders
 // around it are kept to few instructions per byte: whole words through one
-// funnel shift, a branch child's hash in two 16-byte loads.
-template <bool kCoh>
-__device__ __forceinline__ void hash_node(const TrieView &tv, uint32_t ref, uint32_t *stage, uint32_t stride) {
-  uint32_t kind = ref_kind(ref), idx = ref_idx(ref);
-  bool full = kind == KIND_FULL;
-  // nodes a split or a delete unlinked are not hashed
-  if (ldn<kCoh>((full ? tv.full_dead : tv.short_dead) + idx)) return;
+// funnel shift, a branch child's hash in two 16-byte loads.  16M-key YCSB
+// load: 16.7M one-block leaves 6.08 -> 5.12 ms (3.26 G permutations/s, 0.81
+// of the register-only rate; random value gathers are the rest), 5.1M
+// branches of two or three children 1.96 -> 1.56 ms, their extensions 1.28 ms
+// (0.97 of it).
+template <bool kCoh, bool full>
+__device__ __forceinline__ void hash_node(const TrieView &tv, uint32_t idx, uint32_t *stage, uint32_t stride) {
+  const bool dead = ldn<kCoh>((full ? tv.full_dead : tv.short_dead) + idx) != 0;
+  // a short node's fields, loaded together
+  uint64_t skey = 0;
+  uint32_t sklen = 0, schild = 0;
+  if (!full) {
+    skey = ldn<kCoh>(tv.short_key + idx);
+    sklen = ldn<kCoh>(tv.short_klen + idx);
+    schild = ldn<kCoh>(tv.short_child + idx);
+  }
+  if (dead) return;  // unlinked by a split or a delete
   // depth 0 holds exactly the roots of the forest's tries; go-ethereum
   // hashes a root whatever its size
   bool force = tv.geth_mode && (full ? ldn<kCoh>(tv.full_depth + idx) : ldn<kCoh>(tv.short_depth + idx)) == 0;
   int nitems = full ? 18 : 3;
-  // pass 1: payload size (all child loads issued together, sources prefetched)
+  // pass 1: payload size (all child loads issued together)
   uint64_t payload = 0;
   EncItem it1{0, 0, 0, nullptr, 0}, it2{0, 0, 0, nullptr, 0};  // short: key, child
   const uint32_t *chp = tv.full_child + (size_t)idx * 17;
   // branch whose children are all hashed nodes (32-byte references) and whose
-  // value slot is empty: its encoding is regular and is generated word by word
+  // value slot is empty: its encoding is regular and is generated child by
+  // child.  While no node of the tries has had an encoding below 32 bytes
+  // (raw_nodes) the children's lengths need no look: a gather of one byte per
+  // child, which costs a sector each.
   uint32_t present = 0;
   bool regular = full;
   if (full) {
     uint32_t ch[17];
 #pragma unroll
     for (int k = 0; k < 17; ++k) ch[k] = ldn<kCoh>(chp + k);
-#pragma unroll
-    for (int k = 0; k < 17; ++k) prefetch_child(tv, ch[k]);
+    const bool any_raw = __ldcg(&tv.ctr->raw_nodes) != 0;
 #pragma unroll
     for (int k = 0; k < 17; ++k) {
-      EncItem it = child_item<kCoh>(tv, ch[k]);
-      payload += it.pren + it.blen;
       const uint32_t kd = ref_kind(ch[k]);
-      if (kd == KIND_VALUE) {  // a key ending here: its value (up to kilobytes) closes the encoding
-        prefetch_l1(it.body);
-        if (it.blen > 120) prefetch_l1(it.body + 128);
-      }
-      if (kd != KIND_NULL) {
-        present |= 1u << k;
-        regular = regular && k < 16 && kd != KIND_VALUE && it.blen == 32 && it.pren == 1;
+      present |= (kd != KIND_NULL ? 1u : 0u) << k;
+      regular = regular && kd != KIND_VALUE;
+    }
+    regular = regular && present < (1u << 16);
+    payload = 17u + 32u * __popc(present);
+    if (any_raw || !regular) {
+      payload = 0;
+#pragma unroll
+      for (int k = 0; k < 17; ++k) {
+        const EncItem it = child_item<kCoh>(tv, ch[k]);
+        payload += it.pren + it.blen;
+        const uint32_t kd = ref_kind(ch[k]);
+        if (kd == KIND_VALUE) {  // a key ending here: its value (up to kilobytes) closes the encoding
+          prefetch_l1(it.body);
+          if (it.blen > 120) prefetch_l1(it.body + 128);
+        }
+        if (kd != KIND_NULL) regular = regular && it.blen == 32 && it.pren == 1;
       }
     }
   } else {
-    uint32_t child = ldn<kCoh>(tv.short_child + idx);
-    const uint8_t *kp = tv.keys + ldn<kCoh>(tv.short_key + idx);
-    prefetch_l1(kp);
-    if (ref_kind(child) == KIND_VALUE) {
-      unsigned long long vid = tv.value_vid[ref_idx(child)];
-      const ValueRec rc = load_rec(tv, vid);
-      const uint8_t *vp = tv.vals + rc.off;
-      prefetch_l1(vp);
-      if (rc.len > 120) prefetch_l1(vp + 128);
-    } else {
-      prefetch_child(tv, child);
+    prefetch_l1(tv.keys + skey);
+    it2 = child_item<kCoh>(tv, schild);
+    if (ref_kind(schild) == KIND_VALUE) {
+      prefetch_l1(it2.body);
+      if (it2.blen > 120) prefetch_l1(it2.body + 128);
     }
-    it1 = node_item<kCoh>(tv, false, idx, 1, 0);
-    it2 = node_item<kCoh>(tv, false, idx, 2, 0);
+    it1 = compact_item(tv, skey, sklen);
     payload = it1.pren + it1.blen + it2.pren + it2.blen;
   }
   uint64_t hdr;
@@ -1566,6 +1564,7 @@ __device__ __forceinline__ void hash_node(const TrieView &tv, uint32_t ref, uint
   reinterpret_cast<ulonglong2 *>(o)[0] = make_ulonglong2(sp.a[0], sp.a[1]);
   reinterpret_cast<ulonglong2 *>(o)[1] = make_ulonglong2(sp.a[2], sp.a[3]);
   (full ? tv.full_hlen : tv.short_hlen)[idx] = raw ? (uint8_t)total : 32;
+  if (raw) tv.ctr->raw_nodes = 1;
 }
 
 // Message buffer of one warp for the warp-cooperative hashing (8 Keccak blocks).
@@ -1705,6 +1704,7 @@ __device__ __forceinline__ uint64_t store_hash(const TrieView &tv, uint64_t *o, 
   const uint64_t v = raw ? m64[lane & 3] : a;
   if (lane < 4) o[lane] = v;
   if (lane == 0) *hlen = raw ? (uint8_t)total : 32;
+  if (lane == 0 && raw) tv.ctr->raw_nodes = 1;
   if (lane == 0 && tv.account) {
     atomicAdd(&tv.ctr->enc_bytes, (unsigned long long)total);
     atomicAdd(&tv.ctr->keccak_blocks, (unsigned long long)(raw ? 0u : nblk));
@@ -1853,59 +1853,40 @@ __global__ void __launch_bounds__(128) k_hash_warp(TrieView tv, const uint32_t *
     hash_short_warp<false>(tv, ref_idx(r), msg, cl, false, 0, 0);
 }
 
-// Six 128-thread CTAs per SM (at most 85 registers): the permutation keeps
-// its 25 lanes in registers; a few encoder temporaries spill, and the extra
-// resident warps hide more of the child / record gathers (measured faster
-// than five CTAs at 96 registers without spills).
-// One level, thread per node; the CTA's 128 nodes are first reordered by
-// hash class (stable counting partition from warp ballots), so warps hold
-// nodes of one Keccak block count.
-constexpr int kHashLevelThreads = 128;  // k_hash_level's block size (the partition assumes it)
+// Thread per node of one launch's list, which the bins order by Keccak block
+// count, so the lanes of a warp permute together.  (Ordering each CTA's nodes
+// again before encoding cost a barrier behind four dependent gathers: leaf
+// launch of a 1M-key load 0.76 of the integer pipe.)
+constexpr int kHashLevelThreads = 128;
 
 #ifndef GMPT_HASH_CTAS
 #define GMPT_HASH_CTAS 6
 #endif
-__device__ __forceinline__ void hash_level_cta(const TrieView &tv, const uint32_t *refs, int count) {
+template <bool kFull>
+__device__ __forceinline__ void hash_level_thread(const TrieView &tv, const uint32_t *refs, int count) {
   extern __shared__ uint32_t stage_all[];
-  __shared__ uint32_t s_ref[kHashLevelThreads];
-  __shared__ uint32_t s_cnt[kCtaClasses][kHashLevelThreads / 32];  // [class][warp]
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool valid = t < count;
-  const uint32_t r = valid ? refs[t] : 0u;
-  const uint32_t c = valid ? hash_class(tv, r) : kCtaClasses;
-  uint32_t mine = 0;
-#pragma unroll
-  for (uint32_t v = 0; v < kCtaClasses; ++v) {
-    const unsigned b = __ballot_sync(0xffffffffu, c == v);
-    if (lane == 0) s_cnt[v][warp] = (uint32_t)__popc(b);
-    if (c == v) mine = (uint32_t)__popc(b & ((1u << lane) - 1u));
-  }
-  __syncthreads();
-  if (valid) {
-    uint32_t pos = mine;
-    for (uint32_t v = 0; v < kCtaClasses; ++v)
-      for (int w = 0; w < kHashLevelThreads / 32; ++w)
-        if (v < c || (v == c && w < warp)) pos += s_cnt[v][w];
-    s_ref[pos] = r;
-  }
-  __syncthreads();
-  if (!valid) return;  // the valid nodes fill s_ref[0 .. valid count)
-  hash_node<false>(tv, s_ref[threadIdx.x], stage_all + threadIdx.x, blockDim.x);
+  if (t < count) hash_node<false, kFull>(tv, ref_idx(refs[t]), stage_all + threadIdx.x, blockDim.x);
 }
 
+// Six 128-thread CTAs per SM (at most 85 registers): the permutation keeps
+// its 25 lanes in registers; a few encoder temporaries spill, and the extra
+// resident warps hide more of the child / record gathers (measured faster
+// than five CTAs at 96 registers without spills).
 // The level kernel at the register budget of six resident CTAs per SM (the
 // throughput form), and with the whole register file open to one CTA per
 // SM: a level too small to fill the SMs is as long as the serial Keccak
 // chain of its longest node, which the wider form schedules with more
 // permutation state in flight.
+template <bool kFull>
 __global__ void __launch_bounds__(kHashLevelThreads, GMPT_HASH_CTAS) k_hash_level(TrieView tv, const uint32_t *refs,
                                                                                  int count) {
-  hash_level_cta(tv, refs, count);
+  hash_level_thread<kFull>(tv, refs, count);
 }
 
+template <bool kFull>
 __global__ void __launch_bounds__(kHashLevelThreads, 1) k_hash_level_wide(TrieView tv, const uint32_t *refs, int count) {
-  hash_level_cta(tv, refs, count);
+  hash_level_thread<kFull>(tv, refs, count);
 }
 
 // ---------------------------------------------------------------------------
