@@ -14,22 +14,19 @@
 //                    [stage 1 only] patch: value bytes of key i at
 //                      patch_off[i] := root of trie patch_trie[i]
 //                    LockNU insert of the stage's keys into their tries
-//                    bucket the dirty nodes by (nibble depth, kind)
-//                    hash them deepest level first
+//                    hash what they made dirty (hash_grid: leaves, then
+//                    every branch once its children are done)
 //                  with a grid barrier between phases, then the roots asked
 //                  for are written out.
 // Both launches plus the descriptor / counter copies are captured once as a
 // CUDA graph and replayed per block; sizes come from the device-side
 // descriptor, so the graph is rebuilt only when a buffer or pool moves.
 #pragma once
+#include "grid_hash.cuh"
 #include "latch_kernels.cuh"
 #include "trie_kernels.cuh"
 
 namespace gmpt {
-
-constexpr int kDepthBins = 2 * (kMaxKeyNibbles + 2);  // (depth, kind) buckets
-constexpr int kBlockMaxTs = 64;
-constexpr int kWarpFullPerWarp = 4;  // warp-per-branch hashing up to 4 branches per warp
 
 struct BlockDesc {
   // set by the host for every launch; copying it in also zeroes the fields
@@ -38,15 +35,12 @@ struct BlockDesc {
   int64_t kbytes, vbytes;          // stream lengths
   uint64_t key_base, val_base, vid_base;
   uint32_t gen, pad1;              // dirty generation of stage 0 (stage 1: gen + 1)
-  uint64_t barrier_ns;             // longest grid-barrier wait before giving up
-  uint32_t bar_count, bar_gen;     // grid barrier
+  uint32_t warp_max, pad2;         // hash_grid's warp_max
+  GridCtl ctl;                     // barrier_ns set, the rest zero
   // filled by k_block_stage
   uint32_t stream_terms, key_terms, noncontig, bad;  // bad: BLOCK_BAD_* bits
   // filled by k_block
-  uint32_t levels[2], dirty[2], maxbin[2];
-  uint32_t status;                 // 1: a barrier gave up; 2: stopped on bad input
-  uint32_t n_ts;                   // phase timeline of CTA 0 (globaltimer, ns)
-  uint64_t ts[kBlockMaxTs];
+  uint32_t levels[2], dirty[2];    // hash waves and dirty nodes of each stage
 };
 
 enum : uint32_t { BLOCK_BAD_KEY = 1, BLOCK_BAD_TRIE = 2, BLOCK_BAD_PATCH = 4, BLOCK_BAD_VALUE = 8 };
@@ -63,74 +57,20 @@ struct BlockBufs {
   uint8_t *out;            // [n_out * 33] root bytes + length
   uint64_t *koff;          // [n] staged key offsets
   uint32_t *klen;          // [n]
-  uint32_t *bins;          // [2 stages][2][kDepthBins + 1]: counts, offsets
-  uint32_t *cursor;        // [kDepthBins]
-  uint32_t *sorted;        // dirty refs bucketed by (depth, kind)
+  uint32_t *ready;         // branches whose dirty children are hashed
   BlockDesc *desc;
 };
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// A barrier wait longer than BlockDesc::barrier_ns (2 s unless the trie's
-// "block_barrier_ns" option says otherwise) gives up: the CTA raises
-// ERR_BARRIER and leaves the kernel, and so does every CTA at its next
-// barrier.
-
-// Grid-wide barrier of a cooperative launch (all CTAs co-resident).
-// Returns false when this CTA must stop.
-__device__ bool grid_barrier(BlockDesc *D, Counters *ctr) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    volatile uint32_t *vgen = &D->bar_gen;
-    const uint32_t g = *vgen;
-    __threadfence();
-    const uint32_t arrived = atomicAdd(&D->bar_count, 1u);
-    if (arrived == gridDim.x - 1) {
-      atomicExch(&D->bar_count, 0u);
-      __threadfence();
-      atomicAdd(&D->bar_gen, 1u);
-    } else {
-      const uint64_t t0 = global_ns();
-      const uint64_t limit = D->barrier_ns;
-      uint32_t spins = 0;
-      while (*vgen == g) {
-        __nanosleep(64);
-        if ((++spins & 63) == 0 && global_ns() - t0 > limit) {
-          ok = 0;
-          break;
-        }
-      }
-    }
-    if (!ok) {
-      set_error(ctr, ERR_BARRIER);
-      atomicOr(&D->status, 1u);
-    } else if (*reinterpret_cast<volatile uint32_t *>(&D->status) & 1u) {
-      ok = 0;  // another CTA gave up earlier
-    }
-    __threadfence();
-    s_ok = ok;
-    if (blockIdx.x == 0 && D->n_ts < kBlockMaxTs) D->ts[D->n_ts++] = global_ns();
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
 
 // Copy the streams into the arenas (8-byte words; the last partial word is
 // masked and 64 zero bytes follow each stream), validate keys and pairs, and
 // build the value records.  Grid-stride; every thread runs to the end.
-__global__ void __launch_bounds__(256) k_block_stage(TrieView tv, BlockBufs bb) {
+__global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, BlockBufs bb) {
   BlockDesc *D = bb.desc;
   const int n = D->n, n0 = D->n0;
   const int64_t kb = D->kbytes, vb = D->vbytes;
   const uint64_t key_base = D->key_base, val_base = D->val_base, vid_base = D->vid_base;
   const int64_t T = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t0 == 0) D->ts[D->n_ts++] = global_ns();
+  if (t0 == 0) D->ctl.ts[D->ctl.n_ts++] = global_ns();
   uint32_t terms = 0, bad = 0, kterms = 0, gap = 0;
   {
     uint64_t *dst = reinterpret_cast<uint64_t *>(const_cast<uint8_t *>(tv.keys) + key_base);
@@ -164,7 +104,6 @@ __global__ void __launch_bounds__(256) k_block_stage(TrieView tv, BlockBufs bb) 
       dst[w] = x;
     }
   }
-  for (int64_t w = t0; w < 2 * (kDepthBins + 1) * 2; w += T) bb.bins[w] = 0;
   for (int64_t i = t0; i < n; i += T) {
     int ks = bb.kidx[2 * i], ke = bb.kidx[2 * i + 1];
     bool badk = ks < 0 || ke < ks || (int64_t)ke >= kb || ke - ks + 1 > kMaxKeyNibbles;
@@ -225,31 +164,22 @@ __device__ __forceinline__ void write_root(const TrieView &tv, uint32_t tr, uint
   if (lane == 0) out[32] = (uint8_t)len;
 }
 
-__global__ void __launch_bounds__(256, 2) k_block(TrieView tv0, DirtyList dl, BlockBufs bb, uint32_t retry_limit) {
-  extern __shared__ __align__(16) uint32_t smem[];  // kStageWords message words per thread; histogram
+__global__ void __launch_bounds__(kGridThreads, 1) k_block(TrieView tv0, DirtyList dl, BlockBufs bb, uint32_t retry_limit) {
+  extern __shared__ __align__(16) uint32_t smem[];  // kStageWords message words per thread, a window per warp
   BlockDesc *D = bb.desc;
   const int n = D->n, n0 = D->n0, n_out = D->n_out;
   const uint64_t vid_base = D->vid_base;
   const int t = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
   TrieView tv = tv0;
-  if (t == 0) D->ts[D->n_ts++] = global_ns();
-  // Spread mapping: warps are numbered CTA-fastest (consecutive warp ids sit
-  // on different SMs) and item j goes to warp j % W, lane j / W, so a level
-  // of a few hundred nodes, or the keys of one storage trie, use one lane in
-  // each of many warps instead of all lanes of a few (divergent Keccak, CAS
-  // retries on one slot serialised inside a warp).
-  const int lane = threadIdx.x & 31;
-  const int W = T >> 5;
-  const int gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  const int t_spread = lane * W + gw;
+  if (t == 0) D->ctl.ts[D->ctl.n_ts++] = global_ns();
+  const GridPlace g;
   // this warp's message buffer for hash_full_warp, after the staging words
   uint8_t *wmsg = reinterpret_cast<uint8_t *>(smem + kStageWords * blockDim.x) + (threadIdx.x >> 5) * kWarpMsgBytes;
   // staging outcome: every CTA reads the same words, so all leave together
   if (D->bad || D->noncontig || D->stream_terms != D->key_terms) {
-    if (t == 0) atomicOr(&D->status, 2u);
+    if (t == 0) atomicOr(&D->ctl.status, 2u);
     return;
   }
-  uint32_t *hist = smem;
   for (int s = 0; s < 2; ++s) {
     const int i0 = s ? n0 : 0, i1 = s ? n : n0;
     tv.gen = D->gen + (uint32_t)s;
@@ -272,113 +202,21 @@ __global__ void __launch_bounds__(256, 2) k_block(TrieView tv0, DirtyList dl, Bl
     const int span = T * kLatchWays;
     for (int base = i0; base < i1; base += span)
       latch_keys(tv, dl, bb.koff + base, bb.klen + base, min(span, i1 - base), vid_base + (uint64_t)base, retry_limit,
-                 bb.tid + base, t_spread, T);
-    if (!grid_barrier(D, tv.ctr)) return;
-    // bucket the dirty nodes: histogram
+                 bb.tid + base, g.t_spread, T);
+    if (!grid_barrier(&D->ctl, tv.ctr)) return;
     const uint32_t nd = __ldcg(&tv.ctr->n_dirty);
-    uint32_t *cnt = bb.bins + (size_t)s * 2 * (kDepthBins + 1);
-    uint32_t *off = cnt + (kDepthBins + 1);
-    for (int b = threadIdx.x; b < kDepthBins; b += blockDim.x) hist[b] = 0;
-    __syncthreads();
-    for (uint32_t i = t; i < nd; i += T) {
-      const uint32_t r = __ldcg(dl.ref + i);
-      atomicAdd(&hist[2u * __ldcg(dl.depth + i) + (ref_kind(r) == KIND_FULL ? 1u : 0u)], 1u);
+    uint32_t waves = 0;
+    if (!hash_grid(tv, dl, nd, bb.ready, tv.cap_full, &D->ctl, D->warp_max, smem + threadIdx.x, wmsg, &waves)) return;
+    if (t == 0) {
+      D->levels[s] = waves;
+      D->dirty[s] = nd;
     }
-    __syncthreads();
-    for (int b = threadIdx.x; b < kDepthBins; b += blockDim.x)
-      if (hist[b]) atomicAdd(&cnt[b], hist[b]);
-    if (!grid_barrier(D, tv.ctr)) return;
-    // offsets (CTA 0): per-thread runs, then a serial scan of the run sums
-    if (blockIdx.x == 0) {
-      constexpr int kPer = (kDepthBins + 255) / 256;
-      uint32_t *sums = hist;  // [blockDim.x]
-      uint32_t *smax = hist + 256;
-      const int b0 = threadIdx.x * kPer;
-      uint32_t v[kPer];
-      uint32_t sum = 0, top = 0;
-#pragma unroll
-      for (int k = 0; k < kPer; ++k) {
-        const int b = b0 + k;
-        v[k] = (b < kDepthBins) ? __ldcg(cnt + b) : 0u;
-        sum += v[k];
-        if (v[k]) top = (uint32_t)b + 1;
-      }
-      if (threadIdx.x == 0) *smax = 0;
-      sums[threadIdx.x] = sum;
-      __syncthreads();
-      if (top) atomicMax(smax, top);
-      if (threadIdx.x == 0) {
-        uint32_t acc = 0;
-        for (int k = 0; k < (int)blockDim.x; ++k) {
-          const uint32_t x = sums[k];
-          sums[k] = acc;
-          acc += x;
-        }
-      }
-      __syncthreads();
-      uint32_t acc = sums[threadIdx.x];
-#pragma unroll
-      for (int k = 0; k < kPer; ++k) {
-        const int b = b0 + k;
-        if (b < kDepthBins) {
-          off[b] = acc;
-          bb.cursor[b] = acc;
-        }
-        acc += v[k];
-      }
-      if (threadIdx.x == blockDim.x - 1) off[kDepthBins] = acc;
-      if (threadIdx.x == 0) {
-        D->maxbin[s] = *smax;
-        D->dirty[s] = nd;
-      }
-    }
-    if (!grid_barrier(D, tv.ctr)) return;
-    // scatter into the buckets (warp-aggregated cursor updates)
-    for (uint32_t i0s = (uint32_t)(t & ~31); i0s < nd; i0s += (uint32_t)T) {
-      const uint32_t i = i0s + (t & 31);
-      const bool ok = i < nd;
-      const uint32_t r = ok ? __ldcg(dl.ref + i) : 0u;
-      const uint32_t b = ok ? 2u * __ldcg(dl.depth + i) + (ref_kind(r) == KIND_FULL ? 1u : 0u) : 0xFFFFFFFFu;
-      const unsigned peers = __match_any_sync(0xffffffffu, b);
-      const int leader = __ffs(peers) - 1;
-      uint32_t pos = 0;
-      if (ok && (int)(threadIdx.x & 31) == leader) pos = atomicAdd(&bb.cursor[b], (uint32_t)__popc(peers));
-      pos = __shfl_sync(0xffffffffu, pos, leader);
-      if (ok) bb.sorted[pos + __popc(peers & ((1u << (threadIdx.x & 31)) - 1u))] = r;
-    }
-    if (!grid_barrier(D, tv.ctr)) return;
-    if (t == 0) atomicExch(&tv.ctr->n_dirty, 0u);  // the list is consumed
-    // hash, deepest level first
-    const CoopLanes coop = coop_lanes(lane);
-    const uint32_t top = __ldcg(&D->maxbin[s]);
-    uint32_t levels = 0;
-    for (int d = (int)(top + 1) / 2 - 1; d >= 0; --d) {
-      const uint32_t a = __ldcg(off + 2 * d), m = __ldcg(off + 2 * d + 1), z = __ldcg(off + 2 * d + 2);
-      if (z == a) continue;
-      ++levels;
-      // short nodes [a, m) from warp 0 up, full nodes [m, z) from warp W-1 down
-      for (uint32_t j = (uint32_t)t_spread; j < m - a; j += (uint32_t)T)
-        hash_node<true, false>(tv, ref_idx(__ldcg(bb.sorted + a + j)), smem + threadIdx.x, blockDim.x);
-      if (z - m <= (uint32_t)(kWarpFullPerWarp * W)) {
-        // few branches: a warp per node (latency)
-        for (uint32_t j = (uint32_t)(W - 1 - gw); j < z - m; j += (uint32_t)W) {
-          hash_full_warp<true>(tv, ref_idx(__ldcg(bb.sorted + m + j)), wmsg, coop);
-          __syncwarp();
-        }
-      } else {
-        const uint32_t t_rev = (uint32_t)(lane * W + (W - 1 - gw));
-        for (uint32_t j = t_rev; j < z - m; j += (uint32_t)T)
-          hash_node<true, true>(tv, ref_idx(__ldcg(bb.sorted + m + j)), smem + threadIdx.x, blockDim.x);
-      }
-      if (!grid_barrier(D, tv.ctr)) return;
-    }
-    if (t == 0) D->levels[s] = levels;
-    if (!grid_barrier(D, tv.ctr)) return;  // the n_dirty reset is seen by every CTA
+    if (!grid_barrier(&D->ctl, tv.ctr)) return;  // the cleared counters are seen by every CTA
   }
   // roots asked for: one warp each
-  for (int w = t >> 5; w < n_out; w += T >> 5) write_root(tv, (uint32_t)bb.out_ids[w], bb.out + 33 * (size_t)w, lane);
+  for (int w = t >> 5; w < n_out; w += T >> 5) write_root(tv, (uint32_t)bb.out_ids[w], bb.out + 33 * (size_t)w, g.lane);
   __syncthreads();
-  if (t == 0 && D->n_ts < kBlockMaxTs) D->ts[D->n_ts++] = global_ns();
+  if (t == 0 && D->ctl.n_ts < kGridMaxTs) D->ctl.ts[D->ctl.n_ts++] = global_ns();
 }
 
 }  // namespace gmpt

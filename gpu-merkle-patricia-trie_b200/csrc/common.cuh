@@ -77,6 +77,8 @@ struct TrieView {
   uint8_t *full_hlen;
   uint8_t *full_dead;     // 1: unlinked by a delete (no longer in any trie)
   uint32_t *full_ext;     // the extension last seen above it (see ext_above), kNoNode before any
+  uint32_t *full_par;     // hash passes: the dirty branch above it,
+  uint32_t *full_pend;    //   and its dirty branch children still to be hashed (grid_hash.cuh)
   // short nodes
   uint64_t *short_key;    // nibble offset into the key arena
   uint32_t *short_klen;

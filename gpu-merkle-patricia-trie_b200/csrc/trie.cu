@@ -19,6 +19,7 @@
 #include "local_sort.cuh"
 #include "block_update.cuh"
 #include "delete_kernels.cuh"
+#include "grid_hash.cuh"
 #include "gen_kernels.cuh"
 
 namespace gmpt {
@@ -34,6 +35,12 @@ constexpr unsigned kWideGrid = 3 * 148;
 constexpr uint32_t kWarpMinClass = 4;
 // up to this many leaves are hashed a warp each
 constexpr uint32_t kWarpLeafMax = 2048;
+// dirty lists of at most this many nodes are hashed by one cooperative launch
+constexpr uint32_t kGridHashMax = 1u << 17;
+constexpr uint64_t kHashBarrierNs = 2000000000ull;  // longest grid-barrier wait of such a launch
+// shared memory of a cooperative launch's CTA: message words per thread, a
+// message window per warp
+constexpr size_t kGridSmem = sizeof(uint32_t) * kStageWords * kGridThreads + (kGridThreads / 32) * kWarpMsgBytes;
 constexpr uint32_t kMaxDepths = kMaxKeyNibbles + 2;  // nibble depths a dirty node can have
 // LockNU batches of at least this many keys drop repeated keys first
 constexpr int kDedupMinKeys = 1 << 16;
@@ -104,7 +111,7 @@ Trie::Trie(int device, int geth_mode, int max_tries, bool unified)
 Trie::~Trie() {
   cudaSetDevice(dev_);
   if (st_) cudaStreamSynchronize(st_);
-  void *ptrs[] = {tv_.full_child, tv_.full_epoch, tv_.full_depth, tv_.full_hash, tv_.full_hlen, tv_.full_dead, tv_.full_ext,
+  void *ptrs[] = {tv_.full_child, tv_.full_epoch, tv_.full_depth, tv_.full_hash, tv_.full_hlen, tv_.full_dead, tv_.full_ext, tv_.full_par, tv_.full_pend,
                   fl_refs_,
                   tv_.short_key, tv_.short_klen, tv_.short_child, tv_.short_epoch, tv_.short_depth,
                   tv_.short_dead, tv_.short_hash, tv_.short_hlen, tv_.short_claim, tv_.short_pseudo,
@@ -137,7 +144,7 @@ Trie::~Trie() {
   sorter_.release();
   scan_ws_.release();
   DevBlock *bblocks[] = {&blk_.keys, &blk_.kidx, &blk_.vals, &blk_.vidx, &blk_.tid, &blk_.ptrie, &blk_.poff,
-                         &blk_.out_ids, &blk_.out, &blk_.koff, &blk_.klen, &blk_.bins, &blk_.sorted};
+                         &blk_.out_ids, &blk_.out, &blk_.koff, &blk_.klen, &blk_.ready};
   for (DevBlock *b : bblocks) b->release();
   for (auto &c : blk_.graphs) {
     if (c.exec) cudaGraphExecDestroy(c.exec);
@@ -151,6 +158,7 @@ Trie::~Trie() {
   }
   if (copy_st_) cudaStreamDestroy(copy_st_);
   if (blk_.d_desc) cudaFree(blk_.d_desc);
+  if (grid_ctl_) cudaFree(grid_ctl_);
   if (blk_.h_desc) cudaFreeHost(blk_.h_desc);
   if (h_ctr_) cudaFreeHost(h_ctr_);
   if (h_small_) cudaFreeHost(h_small_);
@@ -179,6 +187,7 @@ int Trie::apply_counters() {
   n_full_ = h_ctr_->n_full;
   n_short_ = h_ctr_->n_short;
   n_value_ = h_ctr_->n_value;
+  n_dirty_ = h_ctr_->n_dirty;
   uint32_t err = h_ctr_->error;
   if (err) {
     cudaMemsetAsync(&ctr_->error, 0, 4, st_);
@@ -226,6 +235,9 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
     if (e == cudaSuccess) e = grow_array(tv_.full_hlen, o, nc, st_, managed_, dev_);
     if (e == cudaSuccess) e = grow_array(tv_.full_dead, o, nc, st_, managed_, dev_);
     if (e == cudaSuccess) e = grow_array(tv_.full_ext, o, nc, st_, managed_, dev_);
+    if (e == cudaSuccess) e = grow_array(tv_.full_par, 0, nc, st_, managed_, dev_);  // written and read in one pass
+    if (e == cudaSuccess) e = grow_array(tv_.full_pend, 0, nc, st_, managed_, dev_);
+    if (e == cudaSuccess) e = cudaMemsetAsync(tv_.full_par, 0xFF, 4 * (size_t)nc, st_);
     if (e != cudaSuccess) return check_cuda(e, "grow branch pool");
     cap_full_ = (uint32_t)nc;
   }
@@ -296,7 +308,7 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
   tv_.cap_full = cap_full_;
   tv_.cap_short = cap_short_;
   tv_.cap_value = cap_value_;
-  stats_.device_bytes = (uint64_t)cap_full_ * (68 + 4 + 2 + 32 + 1 + 1 + 4) + (uint64_t)cap_short_ * (8 + 4 + 4 + 4 + 2 + 1 + 32 + 1 + 8) +
+  stats_.device_bytes = (uint64_t)cap_full_ * (68 + 4 + 2 + 32 + 1 + 1 + 12) + (uint64_t)cap_short_ * (8 + 4 + 4 + 4 + 2 + 1 + 32 + 1 + 8) +
                         (uint64_t)cap_value_ * 8 + cap_rec_ * 24 + cap_keys_ + cap_vals_ + cap_dirty_ * 6;
   return OK;
 }
@@ -978,14 +990,11 @@ int Trie::bucket_dirty(uint32_t nd, uint32_t **sorted_out, std::vector<uint32_t>
 // PhaseHC over every node marked dirty since the last hash.
 int Trie::bucket_and_hash() {
   cudaError_t e = cudaSuccess;
-  uint32_t nd = 0;
-  if ((e = cudaMemcpyAsync(h_small_, &ctr_->n_dirty, 4, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(st_)) != cudaSuccess)
-    return check_cuda(e, "dirty count");
-  nd = (uint32_t)(h_small_[0] & 0xFFFFFFFFu);
+  const uint32_t nd = n_dirty_;  // every call that marks nodes ends with the counters
   stats_.last_dirty = nd;
   stats_.last_hash_levels = 0;
   if (nd == 0) return OK;
+  if (nd <= kGridHashMax) return hash_by_grid(nd);
   uint32_t *sorted = nullptr;
   std::vector<uint32_t> off;
   int rc = bucket_dirty(nd, &sorted, off);
@@ -1054,6 +1063,70 @@ int Trie::bucket_and_hash() {
     cudaEventDestroy(kz);
   }
   tv_.account = 0;
+  stats_.last_hash_levels = levels;
+  stats_.hash_launches = levels;
+  if ((e = cudaMemsetAsync(&ctr_->n_dirty, 0, 4, st_)) != cudaSuccess) return check_cuda(e, "hash reset");
+  return end_hash(nd);
+}
+
+// PhaseHC of a small or middle dirty list in one cooperative launch
+// (grid_hash.cuh).
+int Trie::hash_by_grid(uint32_t nd) {
+  int rc = grid_limits();
+  if (rc) return rc;
+  cudaError_t e = cudaSuccess;
+  uint32_t *ready = wsp<uint32_t>(ws_.sorted_dirty, nd, e);
+  if (e == cudaSuccess && !grid_ctl_) {
+    GridCtl init{};
+    init.barrier_ns = kHashBarrierNs;
+    e = cudaMalloc(&grid_ctl_, sizeof(GridCtl));
+    if (e == cudaSuccess) e = cudaMemcpyAsync(grid_ctl_, &init, sizeof(init), cudaMemcpyHostToDevice, st_);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+  }
+  GridCtl *ctl = static_cast<GridCtl *>(grid_ctl_);
+  cudaEvent_t ka = nullptr, kz = nullptr;
+  if (e == cudaSuccess && timing_) {
+    cudaEventCreate(&ka);
+    cudaEventCreate(&kz);
+    e = cudaMemsetAsync(&ctr_->hashed, 0, 4, st_);
+    if (e == cudaSuccess) e = cudaMemsetAsync(&ctr_->enc_bytes, 0, 16, st_);
+    cudaEventRecord(ka, st_);
+  }
+  if (e != cudaSuccess) return check_cuda(e, "hash alloc");
+  tv_.account = timing_ ? 1 : 0;
+  // enough warps for one node each, within what fits co-resident
+  const unsigned grid = std::min<unsigned>((unsigned)max_grid_, (nd + kGridThreads / 32 - 1) / (kGridThreads / 32));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kGridThreads);
+  cfg.dynamicSmemBytes = kGridSmem;
+  cfg.stream = st_;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;  // all CTAs co-resident, or the launch fails
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  count_launch();
+  e = cudaLaunchKernelEx(&cfg, k_hash_grid, tv_, DirtyList{dirty_ref_, dirty_depth_}, nd, ready, nd, ctl,
+                         grid_warp_max(grid));
+  tv_.account = 0;
+  if (e != cudaSuccess) return check_cuda(e, "hash launch");
+  if (timing_) {
+    cudaEventRecord(kz, st_);
+    cudaEventSynchronize(kz);
+    cudaEventElapsedTime(&stats_.t_hash_kernels_ms, ka, kz);
+    cudaEventDestroy(ka);
+    cudaEventDestroy(kz);
+  }
+  stats_.last_hash_levels = 1;
+  stats_.hash_launches = 1;
+  return end_hash(nd);
+}
+
+// After a pass (which has emptied the list on the device): the record for
+// flush_dirty and a new generation of dirty marks.
+int Trie::end_hash(uint32_t nd) {
+  cudaError_t e = cudaSuccess;
   if (track_dirty_) {  // keep this pass's nodes for flush_dirty
     if (fl_n_ + nd > fl_cap_) {
       uint64_t nc = std::max<uint64_t>(fl_n_ + nd, fl_cap_ + fl_cap_ / 2 + 1024);
@@ -1066,10 +1139,8 @@ int Trie::bucket_and_hash() {
       return check_cuda(e, "flush record");
     fl_n_ += nd;
   }
-  stats_.last_hash_levels = levels;
-  stats_.hash_launches = levels;
-  if ((e = cudaMemsetAsync(&ctr_->n_dirty, 0, 4, st_)) != cudaSuccess) return check_cuda(e, "hash reset");
   if ((e = cudaGetLastError()) != cudaSuccess) return check_cuda(e, "hash launch");
+  n_dirty_ = 0;
   ++gen_;
   tv_.gen = gen_;
   return OK;
@@ -1084,12 +1155,14 @@ int Trie::hash() {
     cudaEventCreate(&z);
     cudaEventRecord(a, st_);
   }
+  const bool any = n_dirty_ != 0;
   int rc = bucket_and_hash();
   if (rc) return rc;
-  if ((rc = sync_counters())) return rc;
-  stats_.last_hashed = h_ctr_->hashed;
-  stats_.last_enc_bytes = h_ctr_->enc_bytes;
-  stats_.last_keccak_blocks = h_ctr_->keccak_blocks;
+  if (any && (rc = sync_counters())) return rc;  // nothing was launched for an empty list
+  const bool counted = any && timing_;
+  stats_.last_hashed = counted ? h_ctr_->hashed : 0;
+  stats_.last_enc_bytes = counted ? h_ctr_->enc_bytes : 0;
+  stats_.last_keccak_blocks = counted ? h_ctr_->keccak_blocks : 0;
   if (timing_) {
     cudaEventRecord(z, st_);
     cudaEventSynchronize(z);
@@ -1243,10 +1316,12 @@ int Trie::reset() {
   err_.clear();
   cudaSetDevice(dev_);
   cudaError_t e = cudaMemsetAsync(roots_, 0, sizeof(uint32_t) * n_tries_, st_);
+  if (e == cudaSuccess && grid_ctl_)  // a barrier that gave up leaves it half way (barrier_ns, the first word, stays)
+    e = cudaMemsetAsync(static_cast<uint8_t *>(grid_ctl_) + 8, 0, sizeof(GridCtl) - 8, st_);
   if (e == cudaSuccess) e = cudaMemsetAsync(ctr_, 0, sizeof(Counters), st_);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
   if (e != cudaSuccess) return check_cuda(e, "reset");
-  n_full_ = n_short_ = n_value_ = 0;
+  n_full_ = n_short_ = n_value_ = n_dirty_ = 0;
   n_rec_ = key_used_ = val_used_ = 0;
   max_key_nibbles_ = max_value_len_ = depth_bound_ = 0;
   fl_n_ = 0;
@@ -1712,9 +1787,6 @@ namespace gmpt {
 
 namespace {
 
-constexpr int kBlockThreads = 256;
-constexpr size_t kBlockSmem = sizeof(uint32_t) * kStageWords * kBlockThreads + (kBlockThreads / 32) * kWarpMsgBytes;
-
 // everything a captured graph has baked in
 struct BlockSig {
   TrieView tv;
@@ -1727,29 +1799,48 @@ struct BlockSig {
 
 }  // namespace
 
+// CTAs of the cooperative kernels that fit co-resident (asked for once).
+int Trie::grid_limits() {
+  if (max_grid_ > 0) return OK;
+  int occ_b = 0, occ_h = 0;
+  cudaError_t e;
+  if ((e = cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev_)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGridSmem)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_hash_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGridSmem)) !=
+          cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, k_block, kGridThreads, kGridSmem)) != cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k_hash_grid, kGridThreads, kGridSmem)) != cudaSuccess)
+    return check_cuda(e, "cooperative occupancy");
+  if (occ_b < 1 || occ_h < 1) return fail(E_INTERNAL, "persistent kernel does not fit an SM");
+  max_grid_ = std::min(occ_b, occ_h) * sms_;
+  return OK;
+}
+
+int Trie::block_grid() const { return opt_block_grid_ > 0 ? std::min(opt_block_grid_, max_grid_) : max_grid_; }
+
+// hash_grid's warp_max for `grid` CTAs: two nodes per warp, within the
+// warp_full_max option.  A warp's permutations are shuffle-bound (500 cycles
+// each per SM), a thread each takes 35-39 us for any wave of up to 19K
+// branches (three blocks and an extension): the two meet there.
+uint32_t Trie::grid_warp_max(unsigned grid) const {
+  return std::min<uint32_t>((uint32_t)opt_warp_full_max_, 2u * grid * (kGridThreads / 32));
+}
+
 int Trie::block_launch(bool launch) {
   cudaError_t e = cudaSuccess;
-  int sms = 0, occ = 0;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockSmem)) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_block, kBlockThreads, kBlockSmem)) != cudaSuccess)
-    return check_cuda(e, "block occupancy");
-  const int max_grid = occ * sms;
-  if (max_grid < 1) return fail(E_INTERNAL, "persistent kernel does not fit an SM");
-  const int grid = opt_block_grid_ > 0 ? std::min(opt_block_grid_, max_grid) : max_grid;
-  const int stage_grid = sms * 4;
+  if (int rc = grid_limits()) return rc;
+  const int grid = block_grid();
+  const int stage_grid = sms_ * 4;
   BlockSig sig;
   std::memset(&sig, 0, sizeof(sig));
   sig.tv = tv_;
   sig.tv.gen = 0;    // the kernels take the generation from the descriptor
   sig.tv.epoch = 0;  // (LockNU claims no split epochs)
   sig.dl = DirtyList{dirty_ref_, dirty_depth_};
-  uint32_t *bins = blk_.bins.as<uint32_t>();
   sig.bb = BlockBufs{blk_.keys.as<uint8_t>(), blk_.kidx.as<int>(),      blk_.vals.as<uint8_t>(),
                      blk_.vidx.as<int64_t>(), blk_.tid.as<int>(),       blk_.ptrie.as<int>(),
                      blk_.poff.as<int>(),     blk_.out_ids.as<int>(),   blk_.out.as<uint8_t>(),
-                     blk_.koff.as<uint64_t>(), blk_.klen.as<uint32_t>(), bins,
-                     bins + 4 * (kDepthBins + 1), blk_.sorted.as<uint32_t>(),
+                     blk_.koff.as<uint64_t>(), blk_.klen.as<uint32_t>(), blk_.ready.as<uint32_t>(),
                      static_cast<BlockDesc *>(blk_.d_desc)};
   sig.h_desc = blk_.h_desc;
   sig.h_ctr = h_ctr_;
@@ -1758,12 +1849,12 @@ int Trie::block_launch(bool launch) {
   auto issue = [&]() -> cudaError_t {
     cudaError_t x = cudaMemcpyAsync(blk_.d_desc, blk_.h_desc, sizeof(BlockDesc), cudaMemcpyHostToDevice, st_);
     if (x != cudaSuccess) return x;
-    count_launch(), k_block_stage<<<stage_grid, kBlockThreads, 0, st_>>>(sig.tv, sig.bb);
+    count_launch(), k_block_stage<<<stage_grid, kGridThreads, 0, st_>>>(sig.tv, sig.bb);
     if ((x = cudaGetLastError()) != cudaSuccess) return x;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kBlockThreads);
-    cfg.dynamicSmemBytes = kBlockSmem;
+    cfg.blockDim = dim3(kGridThreads);
+    cfg.dynamicSmemBytes = kGridSmem;
     cfg.stream = st_;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;  // all CTAs co-resident, or the launch fails
@@ -1857,7 +1948,7 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   if (kb < 0 || vb < 0 || kb > 0x7FFFFFFFll) return fail(E_ARG, "bad stream lengths");
   int rc = ensure_capacity((uint64_t)n, 3ull * n, (uint64_t)n, (uint64_t)n, (uint64_t)kb + 64, (uint64_t)vb + 80);
   if (rc) return rc;
-  if ((rc = block_buffers(n, kb, vb, b.n_out))) return rc;
+  if ((rc = block_buffers(n, kb, vb, b.n_out)) || (rc = grid_limits())) return rc;
   cudaError_t e = cudaSuccess;
   const cudaMemcpyKind kind = b.device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   if (n > 0) {
@@ -1890,7 +1981,8 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   h->val_base = val_base;
   h->vid_base = n_rec_;
   h->gen = gen_;
-  h->barrier_ns = opt_barrier_ns_;
+  h->warp_max = grid_warp_max((unsigned)block_grid());
+  h->ctl.barrier_ns = opt_barrier_ns_;
   if (timing_) cudaEventRecord(ev[1], st_);
   if ((rc = block_launch())) return rc;
   if (timing_) cudaEventRecord(ev[2], st_);
@@ -1899,8 +1991,9 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   binfo_.levels[1] = h->levels[1];
   binfo_.dirty[0] = h->dirty[0];
   binfo_.dirty[1] = h->dirty[1];
-  binfo_.n_ts = std::min<uint32_t>(h->n_ts, kBlockMaxTs);
-  std::memcpy(binfo_.ts, h->ts, sizeof(uint64_t) * binfo_.n_ts);
+  static_assert(kGridMaxTs == 64, "BlockInfo::ts");
+  binfo_.n_ts = std::min<uint32_t>(h->ctl.n_ts, kGridMaxTs);
+  std::memcpy(binfo_.ts, h->ctl.ts, sizeof(uint64_t) * binfo_.n_ts);
   if (h->bad || h->noncontig || h->stream_terms != h->key_terms) {
     cudaMemsetAsync(&ctr_->error, 0, 4, st_);
     if (h->bad & BLOCK_BAD_TRIE) return fail(E_ARG, "trie id outside [0, max_tries)");
@@ -1922,7 +2015,7 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   stats_.value_bytes = val_used_;
   stats_.n_records = n_rec_;
   if ((rc = apply_counters())) return rc;
-  if (h->status & 1u) return fail(E_INTERNAL, "grid barrier wait gave up");
+  if (h->ctl.status & 1u) return fail(E_INTERNAL, "grid barrier wait gave up");
   stats_.n_full = n_full_;
   stats_.n_short = n_short_;
   stats_.n_value = n_value_;
@@ -1963,8 +2056,7 @@ int Trie::block_buffers(int64_t n, int64_t kb, int64_t vb, int64_t n_out) {
   if (e == cudaSuccess) e = blk_.out.ensure(33 * no);
   if (e == cudaSuccess) e = blk_.koff.ensure(8 * nn);
   if (e == cudaSuccess) e = blk_.klen.ensure(4 * nn);
-  if (e == cudaSuccess) e = blk_.bins.ensure(sizeof(uint32_t) * (5 * (kDepthBins + 1)));
-  if (e == cudaSuccess) e = blk_.sorted.ensure(sizeof(uint32_t) * (cap_dirty_ + 64));
+  if (e == cudaSuccess) e = blk_.ready.ensure(sizeof(uint32_t) * ((size_t)cap_full_ + 64));
   if (e == cudaSuccess && !blk_.d_desc) e = cudaMalloc(&blk_.d_desc, sizeof(BlockDesc));
   if (e == cudaSuccess && !blk_.h_desc) e = cudaMallocHost(&blk_.h_desc, sizeof(BlockDesc));
   return check_cuda(e, "block buffers");

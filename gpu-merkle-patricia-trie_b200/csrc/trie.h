@@ -195,6 +195,9 @@ class Trie {
   uint64_t cap_rec_ = 0;
   uint64_t cap_keys_ = 0, cap_vals_ = 0;
   uint32_t n_full_ = 0, n_short_ = 0, n_value_ = 0;
+  uint32_t n_dirty_ = 0;       // nodes marked since the last hash (as of the last counters)
+  int sms_ = 0, max_grid_ = 0;  // CTAs of the cooperative kernels that fit co-resident
+  void *grid_ctl_ = nullptr;    // GridCtl of the hash launches
   uint64_t n_rec_ = 0, key_used_ = 0, val_used_ = 0;
   // longest key (nibbles) and value (bytes) staged since the last reset:
   // whether the hash pass orders leaves by Keccak block count
@@ -221,7 +224,7 @@ class Trie {
 
   // persistent block launches
   struct BlockRt {
-    DevBlock keys, kidx, vals, vidx, tid, ptrie, poff, out_ids, out, koff, klen, bins, sorted;
+    DevBlock keys, kidx, vals, vidx, tid, ptrie, poff, out_ids, out, koff, klen, ready;
     void *d_desc = nullptr, *h_desc = nullptr;  // BlockDesc (device / pinned)
     struct Captured {
       std::vector<uint8_t> sig;  // launch arguments the graph was captured with
@@ -305,6 +308,11 @@ class Trie {
   // mixed batch: keep only the m kept writes' key bytes in the arena
   int compact_rw_keys(int m, const uint32_t *kept, uint64_t *koff, const uint32_t *klen, uint64_t key_base);
   int bucket_and_hash();
+  int hash_by_grid(uint32_t nd);
+  int end_hash(uint32_t nd);
+  int grid_limits();
+  int block_grid() const;
+  uint32_t grid_warp_max(unsigned grid) const;
   uint64_t read_u64(const void *dptr);
 };
 

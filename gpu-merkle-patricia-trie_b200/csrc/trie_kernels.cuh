@@ -1678,16 +1678,18 @@ __device__ __forceinline__ void window_clear(uint64_t *m64, uint32_t wb, int lan
   __syncwarp();
 }
 
-// Pad the window [lo, lo + 136 wb) of a `total`-byte message of nblk blocks
-// and absorb it into the warp-spread state.
-__device__ __forceinline__ uint64_t window_absorb(uint64_t a, uint8_t *msg, uint32_t lo, uint32_t wb, uint32_t total,
-                                                  uint32_t nblk, const CoopLanes &cl, int lane) {
-  const uint64_t *m64 = reinterpret_cast<const uint64_t *>(msg);
-  if (lane == 0) {  // Keccak padding (pad byte 0x01 ... last byte |= 0x80)
-    if (total >= lo && total < lo + wb * 136) msg[total - lo] ^= 0x01;
-    if (lo + wb * 136 == nblk * 136) msg[wb * 136 - 1] ^= 0x80;
-  }
-  __syncwarp();
+// Keccak padding (0x01 after the message, 0x80 on the last byte) of the bytes
+// in the window [lo, lo + 136 wb) of a `total`-byte message of nblk blocks;
+// nothing else writes these bytes.
+__device__ __forceinline__ void put_padding(uint8_t *msg, uint32_t lo, uint32_t wb, uint32_t total, uint32_t nblk) {
+  const uint32_t end = nblk * 136 - 1;
+  if (total >= lo && total < lo + wb * 136) msg[total - lo] = total == end ? 0x81 : 0x01;
+  if (total != end && end < lo + wb * 136) msg[end - lo] = 0x80;
+}
+
+// Absorb the window's wb blocks into the warp-spread state.
+__device__ __forceinline__ uint64_t window_absorb(uint64_t a, const uint64_t *m64, uint32_t wb, const CoopLanes &cl,
+                                                  int lane) {
   for (uint32_t bb = 0; bb < wb; ++bb) {
     if (lane < 17) a ^= m64[bb * 17 + lane];
     a = keccak_f1600_warp(a, cl);
@@ -1765,35 +1767,76 @@ __device__ __forceinline__ void hash_short_warp(const TrieView &tv, uint32_t idx
                                    : (lane < 24 ? it.body.w[2] : it.body.w[3]);
       if ((uint32_t)lane < it.blen && q >= lo && q < hi) msg[q - lo] = (uint8_t)(w >> (8 * (lane & 7)));
     }
+    if (lane == 28 && !raw) put_padding(msg, lo, wb, total, nblk);
     __syncwarp();
     if (raw) break;  // under 32 bytes: the window holds the whole encoding
-    a = window_absorb(a, msg, lo, wb, total, nblk, cl, lane);
+    a = window_absorb(a, m64, wb, cl, lane);
   }
   store_hash(tv, reinterpret_cast<uint64_t *>(tv.short_hash + (size_t)idx * 32), tv.short_hlen + idx, raw, a, m64,
              total, nblk, lane);
 }
 
+// This lane's child slot word of branch f (lane < 17).
+__device__ __forceinline__ uint32_t child_word(const TrieView &tv, uint32_t f, int lane) {
+  return lane < 17 ? __ldcg(tv.full_child + (size_t)f * 17 + lane) : 0u;
+}
+
 // Warp-cooperative encode + hash of branch node idx and of the extension
 // above it, for levels with few nodes or for branches of many blocks, where
-// one thread's serial chain is the latency.  Lane k < 17 loads child k's
-// item; a scan gives every item its place, and the message is built window
-// by window (kWarpMsgBytes, 8 blocks) in the warp's shared buffer -- every
-// lane its own item's bytes at once, long values by all lanes -- and absorbed
-// with the warp-spread permutation.  All 32 lanes call it with the same idx.
-// Bound by latency: one chain of dependent loads (node, children, hashes),
-// then the serial permutations.  Building item after item (one L2 round trip
-// each) took a 16-child branch 15-17 us per level of a 1M-key trie; this
-// form takes 10-11.
+// one thread's serial chain is the latency.  Lane k < 17 loads the item of
+// child k (slot word r); a scan gives every item its place, and the message
+// is built window by window (kWarpMsgBytes, 8 blocks) in the warp's shared
+// buffer -- every lane its own item's bytes at once, long values by all
+// lanes -- and absorbed with the warp-spread permutation.  All 32 lanes call
+// it with the same idx.  Returns the nibble depth where the hashed nodes
+// start (0: a root).  up: the branch above (or kNoNode); *r_up gets this
+// lane's slot word of it.
+// Bound by latency: the serial permutations (2.2 us each, 4 for 16 children),
+// before them three dependent loads (node, children, the extension's key),
+// each step's loads issued together and none behind a branch.  Building item
+// after item (one L2 round trip each) took a 16-child branch 15-17 us per
+// level of a 1M-key trie; this form takes 10-11.
 template <bool kCoh>
-__device__ __forceinline__ void hash_full_warp(const TrieView &tv, uint32_t idx, uint8_t *msg, const CoopLanes &cl) {
+__device__ __forceinline__ uint32_t hash_full_warp(const TrieView &tv, uint32_t idx, uint32_t r, uint8_t *msg,
+                                                   const CoopLanes &cl, uint32_t up, uint32_t *r_up) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const uint32_t r = lane < 17 ? ldn<kCoh>(tv.full_child + (size_t)idx * 17 + lane) : 0u;
+  const uint32_t kind = ref_kind(r);
+  const bool node = kind == KIND_FULL || kind == KIND_SHORT, full = kind == KIND_FULL;
+  // 1. the node's own words (node 0 stands in where there is none to load)
   const bool dead = ldn<kCoh>(tv.full_dead + idx) != 0;
-  const bool force = tv.geth_mode && ldn<kCoh>(tv.full_depth + idx) == 0;
-  if (dead) return;  // unlinked by a delete: nothing to hash
+  const uint32_t depth = ldn<kCoh>(tv.full_depth + idx);
+  const uint32_t ext = __ldcg(tv.full_ext + idx);
+  // 2. its children's hashes, the extension, the parent's slots
+  const size_t ci = node ? ref_idx(r) : 0;
+  const ulonglong2 *hp = reinterpret_cast<const ulonglong2 *>((full ? tv.full_hash : tv.short_hash) + ci * 32);
+  const ulonglong2 h0 = __ldcg(hp), h1 = __ldcg(hp + 1);
+  const uint32_t hl = __ldcg((full ? tv.full_hlen : tv.short_hlen) + ci);
+  const uint32_t ei = ext != kNoNode ? ext : 0u;
+  const uint64_t eko = __ldcg(tv.short_key + ei);
+  const uint32_t eklen = __ldcg(tv.short_klen + ei), echild = __ldcg(tv.short_child + ei);
+  const uint32_t edepth = __ldcg(tv.short_depth + ei);
+  const bool edead = __ldcg(tv.short_dead + ei) != 0;
+  if (r_up) *r_up = up != kNoNode ? child_word(tv, up, lane) : 0u;
+  if (dead) return depth;  // unlinked by a delete: nothing to hash
+  // 3. the extension's key (full_ext checked as ext_above does): an
+  // extension's key has no terminator; up to 32 packed bytes, one per lane
+  const bool has_ext = ext != kNoNode && !edead && echild == make_ref(KIND_FULL, idx);
+  const uint32_t eodd = eklen & 1u, ebytes = eklen / 2;
+  const bool ext_fits = has_ext && ebytes <= 32;
+  const uint8_t *ek = tv.keys + (ext_fits ? eko : 0);
+  const bool ebyte_on = ext_fits && (uint32_t)lane < ebytes;
+  const uint32_t ek0 = __ldg(ek);
+  const uint32_t ehi = __ldg(ek + (ebyte_on ? eodd + 2 * lane : 0)), elo = __ldg(ek + (ebyte_on ? eodd + 2 * lane + 1 : 0));
   WarpItem it;
-  if (lane < 17) it = warp_child_item<kCoh>(tv, r);
+  if (node) {
+    it.blen = hl;
+    it.body = Bytes32{{h0.x, h0.y, h1.x, h1.y}};
+    node_head(tv, it);
+  } else if (lane < 17) {
+    it = warp_child_item<kCoh>(tv, r);  // an empty slot or a value
+  }
+  const bool force = tv.geth_mode && depth == 0;
   const uint32_t sz = it.pren + it.blen;
   uint32_t incl = sz;
 #pragma unroll
@@ -1811,30 +1854,65 @@ __device__ __forceinline__ void hash_full_warp(const TrieView &tv, uint32_t idx,
   const uint32_t my_off = hn + incl - sz;  // message offset of this lane's item
   const unsigned far = __ballot_sync(kAll, it.far != nullptr);
   uint64_t *m64 = reinterpret_cast<uint64_t *>(msg);
-  uint64_t a = 0;  // this lane's word of the state
-  for (uint32_t b0 = 0; b0 < nblk; b0 += kWarpMsgBytes / 136) {
-    const uint32_t wb = min((uint32_t)(kWarpMsgBytes / 136), nblk - b0);
-    const uint32_t lo = b0 * 136, hi = lo + wb * 136;
+  uint64_t a = 0, hw = 0;  // this lane's word of the state; of the branch's hash
+  bool in_ext = false;     // one absorb site for both messages (instruction fetch)
+  for (uint32_t b0 = 0;;) {
+    const uint32_t wb = in_ext ? 1u : min((uint32_t)(kWarpMsgBytes / 136), nblk - b0);
     window_clear(m64, wb, lane);
-    if (lane == 31) put_prefix(msg, lo, hi, hdr, hn, 0);
-    put_prefix(msg, lo, hi, it.pre, it.pren, my_off);
-    if (!it.far) put_body32(msg, lo, hi, it.body, it.blen, my_off + it.pren);
-    for (unsigned m = far; m; m &= m - 1) {
-      const int k = __ffs(m) - 1;
-      const uint8_t *src = reinterpret_cast<const uint8_t *>(
-          __shfl_sync(kAll, reinterpret_cast<unsigned long long>(it.far), k));
-      const uint32_t n = __shfl_sync(kAll, it.blen, k), p = __shfl_sync(kAll, my_off + it.pren, k);
-      put_far<kCoh>(msg, lo, hi, src, n, p, lane);
+    if (!in_ext) {
+      const uint32_t lo = b0 * 136, hi = lo + wb * 136;
+      if (lane == 31) put_prefix(msg, lo, hi, hdr, hn, 0);
+      if (lane == 30 && !raw) put_padding(msg, lo, wb, total, nblk);
+      put_prefix(msg, lo, hi, it.pre, it.pren, my_off);
+      if (!it.far) put_body32(msg, lo, hi, it.body, it.blen, my_off + it.pren);
+      for (unsigned m = far; m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        const uint8_t *src = reinterpret_cast<const uint8_t *>(
+            __shfl_sync(kAll, reinterpret_cast<unsigned long long>(it.far), k));
+        const uint32_t n = __shfl_sync(kAll, it.blen, k), p = __shfl_sync(kAll, my_off + it.pren, k);
+        put_far<kCoh>(msg, lo, hi, src, n, p, lane);
+      }
+    } else {
+      // [list header][key header + flag][key bytes][0xa0][hash]: 35 to 70
+      // bytes; the compact key is itself when one byte, else a string
+      const uint32_t kpren = ebytes == 0 ? 1u : 2u, ep = kpren + ebytes + 33;
+      const uint32_t en = ep < 56 ? 1u : 2u, kp = en + kpren, bp = kp + ebytes;
+      const uint32_t flag = eodd ? 0x10u | ek0 : 0u;
+      if (lane == 31) {
+        msg[0] = (uint8_t)(ep < 56 ? 0xc0 + ep : 0xf8);
+        if (en == 2) msg[1] = (uint8_t)ep;
+      }
+      if (lane == 30) {
+        if (ebytes) msg[en] = (uint8_t)(0x80 + ebytes + 1);
+        msg[kp - 1] = (uint8_t)flag;
+      }
+      if (lane == 29) put_padding(msg, 0, 1, en + ep, 1);
+      if (lane == 28) msg[bp] = 0xa0;
+      if (ebyte_on) msg[kp + lane] = (uint8_t)((ehi << 4) | elo);
+      if (lane < 4) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) msg[bp + 1 + 8 * lane + j] = (uint8_t)(hw >> (8 * j));
+      }
     }
     __syncwarp();
-    if (raw) break;  // under 32 bytes: the window holds the whole encoding
-    a = window_absorb(a, msg, lo, wb, total, nblk, cl, lane);
-  }
-  const uint64_t hw = store_hash(tv, reinterpret_cast<uint64_t *>(tv.full_hash + (size_t)idx * 32), tv.full_hlen + idx,
-                                 raw, a, m64, total, nblk, lane);
-  if constexpr (!kCoh) {
-    const uint32_t e = ext_above(tv, idx);
-    if (e != kNoNode) hash_short_warp<kCoh>(tv, e, msg, cl, true, hw, raw ? total : 32u);
+    if (in_ext || !raw) a = window_absorb(a, m64, wb, cl, lane);
+    if (in_ext) {
+      const uint32_t ep = (ebytes == 0 ? 1u : 2u) + ebytes + 33;
+      store_hash(tv, reinterpret_cast<uint64_t *>(tv.short_hash + (size_t)ext * 32), tv.short_hlen + ext, false, a, m64,
+                 (ep < 56 ? 1u : 2u) + ep, 1, lane);
+      return edepth;
+    }
+    b0 += wb;
+    if (b0 < nblk) continue;
+    hw = store_hash(tv, reinterpret_cast<uint64_t *>(tv.full_hash + (size_t)idx * 32), tv.full_hlen + idx, raw, a, m64,
+                    total, nblk, lane);
+    if (!has_ext) return depth;
+    if (!ext_fits || raw) {
+      hash_short_warp<kCoh>(tv, ext, msg, cl, true, hw, raw ? total : 32u);
+      return edepth;
+    }
+    in_ext = true;
+    a = 0;
   }
 }
 
@@ -1848,7 +1926,7 @@ __global__ void __launch_bounds__(128) k_hash_warp(TrieView tv, const uint32_t *
   const CoopLanes cl = coop_lanes(threadIdx.x & 31);
   const uint32_t r = refs[j];
   if (ref_kind(r) == KIND_FULL)
-    hash_full_warp<false>(tv, ref_idx(r), msg, cl);
+    hash_full_warp<false>(tv, ref_idx(r), child_word(tv, ref_idx(r), threadIdx.x & 31), msg, cl, kNoNode, nullptr);
   else
     hash_short_warp<false>(tv, ref_idx(r), msg, cl, false, 0, 0);
 }

@@ -59,3 +59,37 @@ def test_extension_and_leaf_key_lengths(gpu_lib, mode, klen):
         keys = [nib(head + bytes([c]) + rng.bytes(tail).tobytes()) for c in range(5)]
         vals = [rng.bytes(1 + 40 * c).tobytes() for c in range(5)]
         check(gpu_lib, keys, vals, mode, 4096)
+
+
+@pytest.mark.parametrize("warp_max", [0, 1, 4096])
+@pytest.mark.parametrize("mode", MODES)
+def test_pass_sizes(gpu_lib, mode, warp_max):
+    """Hash passes of one node to beyond one cooperative launch: new keys,
+    updates and splits above untouched subtrees, deletes, both strategies."""
+    t = gpu_lib.MPT(mode=mode)
+    t.set_option("warp_full_max", warp_max)
+    o = O.OracleTrie(mode)
+    load = W.ycsb_load(60000, value_bytes=24, seed=0x5EED0A01)
+    rand = W.random_keys(70000, 23, 24, seed=0x5EED0A02)  # same key length, other prefixes
+    import numpy as np
+
+    pos = 0
+    for k, n in enumerate((1, 1, 2, 40, 700, 5000, 30000)):
+        for b in (load.subset(np.arange(pos, pos + n)), load.subset(np.arange(max(0, pos - n // 2), pos + 1)),
+                  rand.subset(np.arange(pos, pos + n))):
+            put = t.puts_2phase_with_valuehp if k % 2 else t.puts_latching_with_valuehp_v2
+            put(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)
+            o.puts(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)
+        t.hash_onepass_v2()
+        o.hash()
+        assert t.get_root_hash() == o.root(), (k, n)
+        gone = rand.subset(np.arange(pos, pos + n))
+        t.deletes(gone.keys_hexs, gone.keys_indexs)
+        t.hash_onepass_v2()
+        t.puts_2phase_with_valuehp(gone.keys_hexs, gone.keys_indexs, gone.values, gone.values_indexs)
+        t.hash_onepass_v2()
+        assert t.get_root_hash() == o.root(), (k, n)
+        pos += n
+    t.hash_onepass_v2()  # nothing dirty
+    assert t.get_root_hash() == o.root()
+    t.close()
