@@ -51,12 +51,14 @@ struct Counters {
   uint32_t n_pseudo, retries_max, hashed;
   uint32_t raw_nodes;  // 1: some node's encoding was below 32 bytes since the last reset
   unsigned long long enc_bytes, keccak_blocks;  // last hash pass
-  // staging checks of the last batch
-  unsigned long long stream_terms;  // bytes == 16 in the key stream
+  // staging checks of the last batch, on a line of their own: the insert
+  // reads the verdict while its atomics work on the counters above
+  alignas(128) unsigned long long stream_terms;  // bytes == 16 in the key stream
   uint32_t key_terms;               // keys whose last byte is 16
   uint32_t noncontig;               // key index pairs do not tile the stream
   uint32_t bad_byte;                // a byte > 16 in the stream
-  uint32_t pad3;
+  uint32_t max_klen, max_vlen;      // longest key (nibbles) and value (bytes)
+  uint32_t stage_bad;               // the batch is malformed and must not be applied
 };
 
 // A value record: byte offset into the value arena and length, side by side

@@ -339,6 +339,12 @@ template <int kWays>
 __global__ void __launch_bounds__(256, GMPT_LATCH_CTAS) k_latch_insert(TrieView tv, DirtyList dl, const uint64_t *koff,
                                                       const uint32_t *klen, int n, uint64_t vid_base,
                                                       uint32_t retry_limit, const int *tid, KeySelect ks) {
+  // The staging verdict is looked at here (once per CTA), not by a host round
+  // trip before the launch: a malformed batch is not applied.
+  __shared__ uint32_t s_bad;
+  if (threadIdx.x == 0) s_bad = __ldcg(&tv.ctr->stage_bad);
+  __syncthreads();
+  if (s_bad) return;
   latch_keys<kWays>(tv, dl, koff, klen, n, vid_base, retry_limit, tid, blockIdx.x * blockDim.x + threadIdx.x,
                     gridDim.x * blockDim.x, ks);
 }

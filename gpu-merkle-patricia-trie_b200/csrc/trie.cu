@@ -6,8 +6,10 @@
 #include <cmath>
 #include <mutex>
 #include <cstdio>
+#include <cstddef>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "trie.h"
@@ -35,6 +37,8 @@ constexpr unsigned kWideGrid = 3 * 148;
 constexpr uint32_t kWarpMinClass = 4;
 // up to this many leaves are hashed a warp each
 constexpr uint32_t kWarpLeafMax = 2048;
+// host batches and lookups of at most this many bytes cross in one packed copy
+constexpr size_t kPackBytes = 256 << 10;
 // dirty lists of at most this many nodes are hashed by one cooperative launch
 constexpr uint32_t kGridHashMax = 1u << 17;
 constexpr uint64_t kHashBarrierNs = 2000000000ull;  // longest grid-barrier wait of such a launch
@@ -131,7 +135,7 @@ Trie::~Trie() {
                         &ws_.rw_a, &ws_.rw_b, &ws_.rw_c, &ws_.rw_d, &ws_.rw_e, &ws_.rw_wpos, &ws_.rw_hp,
                         &ws_.rw_len, &ws_.rw_tot, &ws_.rw_kept, &ws_.rw_koff, &ws_.rw_klen, &ws_.rw_tid,
                         &ws_.del_hslot, &ws_.del_hext, &ws_.del_stamp,
-                        &ws_.misc};
+                        &ws_.pack, &ws_.misc};
   for (DevBlock *b : blocks) b->release();
   for (int k = 0; k < 2; ++k) {
     ws_.s_start[k].release();
@@ -160,6 +164,7 @@ Trie::~Trie() {
   if (blk_.d_desc) cudaFree(blk_.d_desc);
   if (grid_ctl_) cudaFree(grid_ctl_);
   if (blk_.h_desc) cudaFreeHost(blk_.h_desc);
+  if (h_pack_) cudaFreeHost(h_pack_);
   if (h_ctr_) cudaFreeHost(h_ctr_);
   if (h_small_) cudaFreeHost(h_small_);
   if (st_) cudaStreamDestroy(st_);
@@ -175,10 +180,14 @@ int Trie::check_cuda(cudaError_t e, const char *what) {
   return fail(E_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-int Trie::sync_counters() {
+int Trie::copy_counters() {
   cudaError_t e = cudaMemcpyAsync(h_ctr_, ctr_, sizeof(Counters), cudaMemcpyDeviceToHost, st_);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
-  if (e != cudaSuccess) return check_cuda(e, "sync counters");
+  return check_cuda(e, "sync counters");
+}
+
+int Trie::sync_counters() {
+  if (int rc = copy_counters()) return rc;
   return apply_counters();
 }
 
@@ -313,18 +322,53 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
   return OK;
 }
 
-// Copy the batch into the arenas and build per-key records.
-int Trie::stage(const BatchIn &b, uint64_t &key_base, uint64_t &vid_base, uint64_t **koff, uint32_t **klen,
-                uint32_t *maxlen, const int **tid_out) {
+// A small host batch copied to the device in one transfer (packed in pinned
+// memory): five pageable copies cost more than the put of a few keys.  b
+// becomes the device batch.
+int Trie::pack_host(BatchIn &b, int64_t kbytes, int64_t vbytes) {
+  const size_t n = (size_t)b.n;
+  const size_t part[6] = {(size_t)kbytes, 8 * n, (size_t)vbytes, 16 * n, b.values_hps ? 8 * n : 0,
+                          b.trie_ids ? 4 * n : 0};
+  const void *src[6] = {b.keys_hexs, b.keys_indexs, b.values, b.values_indexs, b.values_hps, b.trie_ids};
+  size_t off[7] = {0};
+  for (int k = 0; k < 6; ++k) off[k + 1] = off[k] + ((part[k] + 15) & ~(size_t)15);
+  if (off[6] > kPackBytes) return OK;
+  cudaError_t e = cudaSuccess;
+  if (!h_pack_) e = cudaMallocHost(&h_pack_, kPackBytes);
+  uint8_t *d = wsp<uint8_t>(ws_.pack, kPackBytes, e);
+  if (e != cudaSuccess) return check_cuda(e, "pack alloc");
+  for (int k = 0; k < 6; ++k)
+    if (part[k]) std::memcpy(h_pack_ + off[k], src[k], part[k]);
+  if ((e = cudaMemcpyAsync(d, h_pack_, off[6], cudaMemcpyHostToDevice, st_)) != cudaSuccess)
+    return check_cuda(e, "pack copy");
+  b.keys_hexs = d + off[0];
+  b.keys_indexs = reinterpret_cast<const int *>(d + off[1]);
+  b.values = d + off[2];
+  b.values_indexs = reinterpret_cast<const int64_t *>(d + off[3]);
+  if (b.values_hps) b.values_hps = reinterpret_cast<const uint64_t *>(d + off[4]);
+  if (b.trie_ids) b.trie_ids = reinterpret_cast<const int *>(d + off[5]);
+  b.keys_bytes = kbytes;
+  b.values_bytes = vbytes;
+  b.device = true;
+  return OK;
+}
+
+// Copy the batch into the arenas and build per-key records (k_stage), on the
+// stream; stage_done() reads the outcome.
+int Trie::stage(const BatchIn &batch, uint64_t &key_base, uint64_t &vid_base, uint64_t **koff, uint32_t **klen,
+                const int **tid_out) {
+  BatchIn b = batch;
   const int n = b.n;
   cudaError_t e = cudaSuccess;
-  const cudaMemcpyKind kind = b.device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   int64_t kbytes = b.keys_bytes, vbytes = b.values_bytes;
   if (kbytes < 0 || vbytes < 0) {
     if (b.device) return fail(E_ARG, "device batches must give keys_bytes and values_bytes");
     kbytes = (int64_t)b.keys_indexs[2 * n - 1] + 1;
     vbytes = (int64_t)b.values_indexs[2 * n - 1] + 1;
   }
+  if (!b.device && kbytes >= 0 && vbytes >= 0)
+    if (int rc = pack_host(b, kbytes, vbytes)) return rc;
+  const cudaMemcpyKind kind = b.device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   const int64_t raw_bytes = b.raw_keys ? kbytes : 0;
   unsigned long long *raw_pos = nullptr;
   if (b.raw_keys) {
@@ -339,81 +383,105 @@ int Trie::stage(const BatchIn &b, uint64_t &key_base, uint64_t &vid_base, uint64
     if (e != cudaSuccess) return check_cuda(e, "stage raw lengths");
     count_launch(), k_raw_lens<<<blocks_for(n), kThreads, 0, st_>>>(tv_, ki, n, raw_bytes, lens);
     if ((e = exclusive_scan<unsigned long long>(lens, raw_pos, n, d_tot, scan_ws_, st_)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(h_small_, d_tot, 8, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st_)) != cudaSuccess)
+        (e = cudaMemcpyAsync(h_small_, d_tot, 8, cudaMemcpyDeviceToHost, st_)) != cudaSuccess)
       return check_cuda(e, "stage raw scan");
-    kbytes = (int64_t)h_small_[0];
     // malformed pairs are reported (and the error word cleared) before any
     // other early return, so the next call does not inherit them
     if (int rc0 = sync_counters()) return rc0;
+    kbytes = (int64_t)h_small_[0];
     if (kbytes >= (1ll << 31)) return fail(E_ARG, "key stream exceeds the int32 index range");
   }
+  // arenas are filled from aligned offsets (k_stage's words)
+  key_used_ = (key_used_ + 7) & ~7ull;
+  val_used_ = (val_used_ + 15) & ~15ull;
   int rc = ensure_capacity(2ull * n, 4ull * n, (uint64_t)n, (uint64_t)n, (uint64_t)kbytes, (uint64_t)vbytes);
   if (rc) return rc;
   key_base = key_used_;
   vid_base = n_rec_;
-  uint64_t val_base = val_used_;
   uint8_t *karena = const_cast<uint8_t *>(tv_.keys);
   uint8_t *varena = const_cast<uint8_t *>(tv_.vals);
-  int *ki = wsp<int>(ws_.ki, 2 * (size_t)n, e);
-  int64_t *vi = wsp<int64_t>(ws_.vi, 2 * (size_t)n, e);
-  uint64_t *hp = b.values_hps ? wsp<uint64_t>(ws_.hp, (size_t)n, e) : nullptr;
   *koff = wsp<uint64_t>(ws_.koff, (size_t)n, e);
   *klen = wsp<uint32_t>(ws_.klen, (size_t)n, e);
-  uint32_t *d_max = wsp<uint32_t>(ws_.misc, 32, e);  // same block size as the scan totals
-  int *tid = b.trie_ids ? wsp<int>(ws_.tid, (size_t)n, e) : nullptr;
-  if (e != cudaSuccess) return check_cuda(e, "stage alloc");
-  *tid_out = tid;
+  StageIn in{};
+  in.kbytes = kbytes;
+  in.vbytes = vbytes;
+  in.key_base = key_base;
+  in.val_base = val_used_;
+  in.vid_base = vid_base;
+  in.check_stream = b.raw_keys ? 0 : 1;  // expanded raw keys are well formed by construction
+  // device arrays are read where they lie, host arrays (and device arrays
+  // not aligned to their element) are copied
+  auto at = [&](auto *p, DevBlock &w, size_t count) -> decltype(p) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
+    if (!p || e != cudaSuccess || (b.device && reinterpret_cast<uintptr_t>(p) % alignof(T) == 0)) return p;
+    T *d = wsp<T>(w, count, e);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d, p, count * sizeof(T), kind, st_);
+    return d;
+  };
+  in.vi = at(b.values_indexs, ws_.vi, 2 * (size_t)n);
+  in.hp = at(b.values_hps, ws_.hp, (size_t)n);
+  in.tid = at(b.trie_ids, ws_.tid, (size_t)n);
   if (b.raw_keys) {
-    // pass 2: nibbles + terminator written straight into the arena (device
-    // batches are read where they lie; host bytes cross once)
-    const uint8_t *raw = b.device ? b.keys_hexs : wsp<uint8_t>(ws_.raw, (size_t)raw_bytes + 8, e);
-    if (e == cudaSuccess && raw_bytes && !b.device)
-      e = cudaMemcpyAsync(const_cast<uint8_t *>(raw), b.keys_hexs, (size_t)raw_bytes, kind, st_);
+    // pass 2: nibbles + terminator written straight into the arena
+    const uint8_t *raw = raw_bytes ? at(b.keys_hexs, ws_.raw, (size_t)raw_bytes) : b.keys_hexs;
     if (e != cudaSuccess) return check_cuda(e, "stage raw keys");
-    count_launch(), k_raw_expand<<<blocks_for(n), kThreads, 0, st_>>>(raw, ki, raw_pos, n, raw_bytes,
+    count_launch(), k_raw_expand<<<blocks_for(n), kThreads, 0, st_>>>(raw, ws_.ki.as<int>(), raw_pos, n, raw_bytes,
                                                                      karena + key_base);
+    in.ki = ws_.ki.as<int>();
+    in.keys = karena + key_base;
   } else {
-    e = cudaMemcpyAsync(karena + key_base, b.keys_hexs, (size_t)kbytes, kind, st_);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ki, b.keys_indexs, sizeof(int) * 2 * (size_t)n, kind, st_);
+    in.ki = at(b.keys_indexs, ws_.ki, 2 * (size_t)n);
+    in.copy_keys = b.device && (reinterpret_cast<uintptr_t>(b.keys_hexs) & 7) == 0;
+    in.keys = in.copy_keys ? b.keys_hexs : karena + key_base;
+    if (e == cudaSuccess && !in.copy_keys)
+      e = cudaMemcpyAsync(karena + key_base, b.keys_hexs, (size_t)kbytes, kind, st_);
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(varena + val_base, b.values, (size_t)vbytes, kind, st_);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(vi, b.values_indexs, sizeof(int64_t) * 2 * (size_t)n, kind, st_);
-  if (e == cudaSuccess && hp) e = cudaMemcpyAsync(hp, b.values_hps, sizeof(uint64_t) * (size_t)n, kind, st_);
-  if (e == cudaSuccess && tid) e = cudaMemcpyAsync(tid, b.trie_ids, sizeof(int) * (size_t)n, kind, st_);
-  if (e == cudaSuccess) e = cudaMemsetAsync(karena + key_base + kbytes, 0, 64, st_);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_max, 0, 8, st_);
+  in.copy_vals = b.device && (reinterpret_cast<uintptr_t>(b.values) & 15) == 0;
+  in.vals = b.values;
+  if (e == cudaSuccess && !in.copy_vals)
+    e = cudaMemcpyAsync(varena + val_used_, b.values, (size_t)vbytes, kind, st_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(&ctr_->stream_terms, 0, sizeof(Counters) - offsetof(Counters, stream_terms), st_);
   if (e != cudaSuccess) return check_cuda(e, "stage copy");
-  if ((e = cudaMemsetAsync(&ctr_->stream_terms, 0, 24, st_)) != cudaSuccess) return check_cuda(e, "stage reset");
-  count_launch(), k_stage<<<std::min<unsigned>(blocks_for(n), 148 * 8), kThreads, 0, st_>>>(tv_, ki, vi, hp, n, key_base, val_base, vid_base, kbytes, vbytes,
-                                                *koff, *klen, d_max, tid);
-  if (kbytes > 0 && !b.raw_keys)  // expanded raw keys are well formed by construction
-    count_launch(), k_stage_stream<<<std::min<unsigned>(blocks_for(kbytes / 8 + 1), 148 * 8), kThreads, 0, st_>>>(
-        tv_, karena + key_base, kbytes);
-  e = cudaMemcpyAsync(h_small_, d_max, 8, cudaMemcpyDeviceToHost, st_);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h_ctr_, ctr_, sizeof(Counters), cudaMemcpyDeviceToHost, st_);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
-  if (e != cudaSuccess) return check_cuda(e, "stage");
-  *maxlen = (uint32_t)(h_small_[0] & 0xFFFFFFFFu);
-  max_key_nibbles_ = std::max(max_key_nibbles_, *maxlen);
-  depth_bound_ = std::max(depth_bound_, *maxlen);
-  max_value_len_ = std::max(max_value_len_, (uint32_t)(h_small_[0] >> 32));
-  if (b.raw_keys) {
-    // nothing to check beyond k_raw_lens (errors come back with the counters)
-  } else if (h_ctr_->noncontig) {
-    // index pairs do not tile the stream: check every key's interior
-    count_launch(), k_stage_keys<<<blocks_for(n), kThreads, 0, st_>>>(tv_, *koff, *klen, n);
-  } else if (h_ctr_->bad_byte || h_ctr_->stream_terms != h_ctr_->key_terms) {
+  const int64_t work = std::max<int64_t>((int64_t)n, (kbytes + vbytes) / 64);
+  count_launch(), k_stage<<<std::min<unsigned>(blocks_for(work), 148 * 8), kThreads, 0, st_>>>(tv_, in, n, *koff, *klen);
+  if (in.check_stream) count_launch(), k_stage_keys<<<std::min<unsigned>(blocks_for(n), 148 * 8), kThreads, 0, st_>>>(
+        tv_, *koff, *klen, n);
+  if ((e = cudaGetLastError()) != cudaSuccess) return check_cuda(e, "stage launch");
+  *tid_out = in.tid;
+  staged_ = Staged{kbytes, vbytes, n, in.check_stream != 0};
+  return OK;
+}
+
+// The staged batch's outcome, once the counters are in h_ctr_: its bytes and
+// records count as used unless its key stream was malformed.
+int Trie::stage_done() {
+  const Staged &g = staged_;
+  if (g.check_stream && !h_ctr_->noncontig &&
+      (h_ctr_->bad_byte || h_ctr_->stream_terms != h_ctr_->key_terms)) {
+    apply_counters();  // clears the error word
     return fail(E_BAD_KEY, "malformed key: nibble > 16 or a terminator inside a key");
   }
-  // keys are 8-aligned in the arena so chunk loads start aligned more often
-  key_used_ += ((uint64_t)kbytes + 7) & ~7ull;
-  val_used_ += (uint64_t)vbytes;
-  n_rec_ += (uint64_t)n;
+  maxlen_ = h_ctr_->max_klen;
+  max_key_nibbles_ = std::max(max_key_nibbles_, maxlen_);
+  depth_bound_ = std::max(depth_bound_, maxlen_);
+  max_value_len_ = std::max(max_value_len_, h_ctr_->max_vlen);
+  key_used_ += ((uint64_t)g.kbytes + 7) & ~7ull;
+  val_used_ += (uint64_t)g.vbytes;
+  n_rec_ += (uint64_t)g.n;
   stats_.key_bytes = key_used_;
   stats_.value_bytes = val_used_;
   stats_.n_records = n_rec_;
-  return OK;
+  return apply_counters();
+}
+
+// Stage and wait for the outcome.
+int Trie::stage_wait(const BatchIn &b, uint64_t &key_base, uint64_t &vid_base, uint64_t **koff, uint32_t **klen,
+                     uint32_t *maxlen, const int **tid) {
+  if (int rc = stage(b, key_base, vid_base, koff, klen, tid)) return rc;
+  if (int rc = copy_counters()) return rc;
+  const int rc = stage_done();
+  *maxlen = maxlen_;
+  return rc;
 }
 
 // Lexicographic order of keys koff/klen[0..n) (terminator before nibble 0;
@@ -834,9 +902,8 @@ int Trie::put_2phase(const BatchIn &b) {
   uint32_t *klen;
   uint32_t maxlen = 0;
   const int *tid = nullptr;
-  int rc = stage(b, key_base, vid_base, &koff, &klen, &maxlen, &tid);
-  if (rc) return rc;
-  if ((rc = sync_counters())) return rc;  // key validation
+  int rc = stage_wait(b, key_base, vid_base, &koff, &klen, &maxlen, &tid);
+  if (rc) return rc;  // key validation
   if (timing_) cudaEventRecord(ev[1], st_);
   const int n = b.n;
   uint32_t *uord;
@@ -1177,17 +1244,12 @@ int Trie::root(uint8_t out[32], int *len, int trie) {
   err_.clear();
   if (trie < 0 || (uint32_t)trie >= n_tries_) return fail(E_ARG, "trie id outside [0, max_tries)");
   cudaSetDevice(dev_);
-  cudaError_t e = cudaSuccess;
-  uint8_t *d = wsp<uint8_t>(ws_.misc, 256, e) + 128;
-  int *did = reinterpret_cast<int *>(d + 64);
-  if (e != cudaSuccess) return check_cuda(e, "root alloc");
-  if ((e = cudaMemcpyAsync(did, &trie, 4, cudaMemcpyHostToDevice, st_)) != cudaSuccess) return check_cuda(e, "root id");
-  count_launch(), k_roots<<<1, 32, 0, st_>>>(tv_, did, 1, d);
-  uint8_t h[40];
-  if ((e = cudaMemcpyAsync(h_small_, d, 33, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(st_)) != cudaSuccess)
-    return check_cuda(e, "root");
-  std::memcpy(h, h_small_, 33);
+  // the kernel writes the 33 bytes to pinned host memory
+  uint8_t *h = reinterpret_cast<uint8_t *>(h_small_) + 128;
+  count_launch(), k_roots<<<1, 32, 0, st_>>>(tv_, nullptr, trie, 1, h);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+  if (e != cudaSuccess) return check_cuda(e, "root");
   *len = h[32];
   std::memcpy(out, h, 32);
   return OK;
@@ -1206,7 +1268,7 @@ int Trie::roots(const int *ids, int n, uint8_t *out32, int *sizes) {
   uint8_t *d = wsp<uint8_t>(ws_.g_keys, 33 * (size_t)n, e);
   if (e == cudaSuccess && ids) e = cudaMemcpyAsync(did, ids, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, st_);
   if (e != cudaSuccess) return check_cuda(e, "roots alloc");
-  count_launch(), k_roots<<<blocks_for(32 * (int64_t)n), kThreads, 0, st_>>>(tv_, did, n, d);
+  count_launch(), k_roots<<<blocks_for(32 * (int64_t)n), kThreads, 0, st_>>>(tv_, did, 0, n, d);
   std::vector<uint8_t> h(33 * (size_t)n);
   if ((e = cudaMemcpyAsync(h.data(), d, h.size(), cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
       (e = cudaStreamSynchronize(st_)) != cudaSuccess)
@@ -1227,6 +1289,32 @@ int Trie::gets(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool dev
   if (keys_bytes < 0) {
     if (device_inputs) return fail(E_ARG, "device lookups need keys_bytes");
     keys_bytes = (int64_t)keys_indexs[2 * n - 1] + 1;
+  }
+  const size_t nn = (size_t)n;
+  if (!device_inputs && !device_outputs && keys_bytes >= 0 && (size_t)keys_bytes + 24 * nn + 256 <= kPackBytes) {
+    // a few host keys: one copy in (packed), one out (results side by side)
+    const size_t o_idx = ((size_t)keys_bytes + 64 + 15) & ~(size_t)15, o_tid = (o_idx + 8 * nn + 15) & ~(size_t)15;
+    const size_t in_bytes = o_tid + (trie_ids ? 4 * nn : 0);
+    if (!h_pack_) e = cudaMallocHost(&h_pack_, kPackBytes);
+    uint8_t *d = wsp<uint8_t>(ws_.pack, kPackBytes, e);
+    uint8_t *r = wsp<uint8_t>(ws_.g_hp, 12 * nn, e);
+    if (e != cudaSuccess) return check_cuda(e, "gets alloc");
+    std::memcpy(h_pack_, keys_hexs, (size_t)keys_bytes);
+    std::memset(h_pack_ + keys_bytes, 0, o_idx - (size_t)keys_bytes);  // 8-byte loads read past a key's last byte
+    std::memcpy(h_pack_ + o_idx, keys_indexs, 8 * nn);
+    if (trie_ids) std::memcpy(h_pack_ + o_tid, trie_ids, 4 * nn);
+    if ((e = cudaMemcpyAsync(d, h_pack_, in_bytes, cudaMemcpyHostToDevice, st_)) != cudaSuccess)
+      return check_cuda(e, "gets copy");
+    count_launch(), k_gets<<<blocks_for(n), kThreads, 0, st_>>>(
+                        tv_, d, reinterpret_cast<const int *>(d + o_idx), n, keys_bytes, reinterpret_cast<uint64_t *>(r),
+                        reinterpret_cast<int *>(r + 8 * nn), nullptr,
+                        trie_ids ? reinterpret_cast<const int *>(d + o_tid) : nullptr);
+    if ((e = cudaMemcpyAsync(h_pack_, r, 12 * nn, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st_)) != cudaSuccess)
+      return check_cuda(e, "gets");
+    std::memcpy(out_hp, h_pack_, 8 * nn);
+    std::memcpy(out_len, h_pack_ + 8 * nn, 4 * nn);
+    return OK;
   }
   cudaMemcpyKind kind = device_inputs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   uint8_t *dk = wsp<uint8_t>(ws_.g_keys, (size_t)keys_bytes + 64, e);
@@ -1355,9 +1443,11 @@ int Trie::put_latching(const BatchIn &b) {
   uint32_t *klen;
   uint32_t maxlen = 0;
   const int *tid = nullptr;
-  int rc = stage(b, key_base, vid_base, &koff, &klen, &maxlen, &tid);
+  // a mixed batch answers its reads first and waits for the staging outcome;
+  // otherwise the insert kernel looks at it and one wait ends the put
+  int rc = rw_ ? stage_wait(b, key_base, vid_base, &koff, &klen, &maxlen, &tid)
+               : stage(b, key_base, vid_base, &koff, &klen, &tid);
   if (rc) return rc;
-  if ((rc = sync_counters())) return rc;
   if (timing_) cudaEventRecord(ev[1], st_);
   DirtyList dl{dirty_ref_, dirty_depth_};
   KeySelect ks;
@@ -1412,8 +1502,9 @@ int Trie::put_latching(const BatchIn &b) {
   count_launch(), kern<<<blocks_for((b.n + ways - 1) / ways), kThreads, 0, st_>>>(tv_, dl, koff, klen, b.n, vid_base,
                                                                                  opt_retry_limit_, tid, ks);
   if ((rc = check_cuda(cudaGetLastError(), "latch launch"))) return rc;
-  empty_ = false;  // keys may be in even when the batch stops on an error
-  if ((rc = sync_counters())) return rc;
+  if ((rc = copy_counters())) return rc;
+  if (h_ctr_->n_value > 0) empty_ = false;  // keys may be in even when the batch stops on an error
+  if ((rc = rw_ ? apply_counters() : stage_done())) return rc;
   if (timing_) {
     cudaEventRecord(ev[2], st_);
     cudaEventSynchronize(ev[2]);
@@ -1426,7 +1517,6 @@ int Trie::put_latching(const BatchIn &b) {
   stats_.n_short = n_short_;
   stats_.n_value = n_value_;
   stats_.last_unique = (uint64_t)b.n;
-  empty_ = false;
   return OK;
 }
 
@@ -1946,7 +2036,7 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
     vb = n ? (int64_t)b.values_indexs[2 * n - 1] + 1 : 0;
   }
   if (kb < 0 || vb < 0 || kb > 0x7FFFFFFFll) return fail(E_ARG, "bad stream lengths");
-  int rc = ensure_capacity((uint64_t)n, 3ull * n, (uint64_t)n, (uint64_t)n, (uint64_t)kb + 64, (uint64_t)vb + 80);
+  int rc = ensure_capacity((uint64_t)n, 3ull * n, (uint64_t)n, (uint64_t)n, (uint64_t)kb + 72, (uint64_t)vb + 80);
   if (rc) return rc;
   if ((rc = block_buffers(n, kb, vb, b.n_out)) || (rc = grid_limits())) return rc;
   cudaError_t e = cudaSuccess;
@@ -1971,13 +2061,13 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   if (e != cudaSuccess) return check_cuda(e, "block inputs");
   BlockDesc *h = static_cast<BlockDesc *>(blk_.h_desc);
   std::memset(h, 0, sizeof(BlockDesc));
-  const uint64_t val_base = (val_used_ + 7) & ~7ull;
+  const uint64_t key_base = (key_used_ + 7) & ~7ull, val_base = (val_used_ + 7) & ~7ull;
   h->n = n;
   h->n0 = b.n0;
   h->n_out = b.n_out;
   h->kbytes = kb;
   h->vbytes = vb;
-  h->key_base = key_used_;
+  h->key_base = key_base;
   h->val_base = val_base;
   h->vid_base = n_rec_;
   h->gen = gen_;
@@ -2004,7 +2094,7 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
     return fail(E_BAD_KEY, "malformed key: nibble > 16, terminator not last, or too long");
   }
   // the launch got past staging: the arena bytes and records are in use
-  key_used_ += ((uint64_t)kb + 7) & ~7ull;
+  key_used_ = key_base + (uint64_t)kb;
   val_used_ = val_base + (uint64_t)vb;
   n_rec_ += (uint64_t)n;
   gen_ += 2;

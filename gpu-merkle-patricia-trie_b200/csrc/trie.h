@@ -267,11 +267,19 @@ class Trie {
     DevBlock rw_flags, rw_a, rw_b, rw_c, rw_d, rw_e, rw_wpos;   // mixed read/write resolution
     DevBlock rw_hp, rw_len, rw_tot, rw_kept, rw_koff, rw_klen, rw_tid;
     DevBlock del_hslot, del_hext, del_stamp;                    // deletes: how each path branch is linked
+    DevBlock pack;                                              // a small host batch, or lookups
     DevBlock misc;
   } ws_;
   RadixSorter sorter_;
   DevBlock scan_ws_;
   uint64_t *h_small_ = nullptr;  // pinned scratch for small readbacks
+  uint8_t *h_pack_ = nullptr;    // pinned: small host batches and lookups
+  struct Staged {                // the batch of the last stage()
+    int64_t kbytes = 0, vbytes = 0;
+    int n = 0;
+    bool check_stream = false;
+  } staged_;
+  uint32_t maxlen_ = 0;          // its longest key
   // set by put_rw for the duration of one put: sort_unique then resolves the
   // reads and keeps the last write of every key
   struct RwState {
@@ -291,8 +299,13 @@ class Trie {
   // exact: grow to exactly what is asked (reservations) instead of by 1.5x steps
   int ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_value, uint64_t add_rec,
                       uint64_t add_key_bytes, uint64_t add_val_bytes, bool exact = false);
+  int copy_counters();
+  int pack_host(BatchIn &b, int64_t kbytes, int64_t vbytes);
   int stage(const BatchIn &b, uint64_t &key_base, uint64_t &vid_base, uint64_t **koff, uint32_t **klen,
-            uint32_t *maxlen, const int **tid);
+            const int **tid);
+  int stage_done();
+  int stage_wait(const BatchIn &b, uint64_t &key_base, uint64_t &vid_base, uint64_t **koff, uint32_t **klen,
+                 uint32_t *maxlen, const int **tid);
   int bucket_dirty(uint32_t nd, uint32_t **sorted_out, std::vector<uint32_t> &off);
   int sort_unique_dedup(int n, const uint64_t *koff, const uint32_t *klen, uint32_t maxlen, const int *tid,
                         uint32_t **uord_out, int *m_out, bool *done);

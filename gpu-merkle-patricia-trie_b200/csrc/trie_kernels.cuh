@@ -101,80 +101,180 @@ __device__ __forceinline__ uint32_t new_short(const TrieView &tv, DirtyList d, u
 // ---------------------------------------------------------------------------
 // staging
 
-// Per-key records of a staged batch.  Grid-stride, with the stream counters
-// (terminated keys, index-pair gaps; maxlen[0] = longest key, maxlen[1] =
-// longest value) reduced per CTA: one atomic per CTA and counter instead of
-// one per warp, which serialised on the counter addresses at 16M keys.
-__global__ void __launch_bounds__(256) k_stage(TrieView tv, const int *ki, const int64_t *vi, const uint64_t *hp,
-                                               int n, uint64_t key_base, uint64_t val_base, uint64_t vid_base,
-                                               int64_t kbytes, int64_t vbytes, uint64_t *koff, uint32_t *klen,
-                                               uint32_t *maxlen, const int *tid) {
-  uint32_t terms = 0, gaps = 0, lmax = 0, vmax = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    if (tid && (uint32_t)tid[i] >= tv.n_tries) set_error(tv.ctr, ERR_BAD_TRIE);
-    int ks = ki[2 * i], ke = ki[2 * i + 1];
-    bool bad = ks < 0 || ke < ks || (int64_t)ke >= kbytes;  // index pair outside the key stream
+// A batch where it lies (caller's device arrays, or copies made for a host
+// batch), and where its bytes go.
+struct StageIn {
+  const uint8_t *keys;   // key stream; the arena's own copy when copy_keys is off
+  const uint8_t *vals;
+  const int *ki;
+  const int64_t *vi;
+  const uint64_t *hp;    // or null
+  const int *tid;        // or null
+  int64_t kbytes, vbytes;
+  uint64_t key_base, val_base, vid_base;  // key_base is 8-byte aligned, val_base 16
+  int copy_keys, copy_vals;  // copy the stream into the arena (its source is aligned alike)
+  int check_stream;          // the key stream is checked whole (hex keys)
+};
+
+__device__ __forceinline__ void stage_error(Counters *c, uint32_t bits) {
+  set_error(c, bits);
+  c->stage_bad = 1;
+}
+
+// Eight nibble bytes: any of 17 or more, and how many 16s.
+__device__ __forceinline__ void check_nibbles8(uint64_t x, uint32_t &bad, uint32_t &terms) {
+  const uint64_t hi = x & 0x1010101010101010ull;  // bit 4 set: 16..31
+  bad |= (x & 0xE0E0E0E0E0E0E0E0ull) != 0 || (x & ((hi >> 4) * 0x0Full)) != 0;
+  terms += __popcll(hi);
+}
+
+// Stage a batch in one pass: copy the key and value streams into the arenas
+// (64 bytes in flight per thread), check the key stream as it
+// goes by -- no byte > 16, and exactly as many 16s as keys that end in one (so
+// none is interior, given that the index pairs tile the stream; k_stage_keys
+// looks at batches that do not) -- and build the per-key and value records.
+// Grid-stride, counters reduced per CTA.
+// Bound by HBM.  Separate copies, record and check launches read the key
+// stream twice and cost a 16K-key put eight operations before its insert;
+// 16M YCSB keys: 1.36 ms, now 1.11 (5.9 GB: 5.3 TB/s).
+__global__ void __launch_bounds__(256) k_stage(TrieView tv, StageIn in, int n, uint64_t *koff, uint32_t *klen) {
+  uint32_t terms = 0, gaps = 0, lmax = 0, vmax = 0, sterms = 0, sbad = 0;
+  const int64_t T = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  // streams: whole words, then the tail bytes and 64 zero bytes
+  // behind them (8-byte loads may read past a key's or a value's last byte)
+  if (in.copy_keys || in.check_stream) {
+    const int64_t nv = in.kbytes / 8;
+    const uint64_t *src = reinterpret_cast<const uint64_t *>(in.keys);
+    uint64_t *dst = reinterpret_cast<uint64_t *>(const_cast<uint8_t *>(tv.keys) + in.key_base);
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {  // the usual source: 16 bytes a load
+      const int64_t np = nv / 2;
+      const ulonglong2 *s2 = reinterpret_cast<const ulonglong2 *>(src);
+      const bool even = (in.key_base & 15) == 0;
+      for (int64_t w = t0; w < np; w += 4 * T) {
+        ulonglong2 x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (w + k * T < np) x[k] = s2[w + k * T];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (w + k * T >= np) continue;
+          uint64_t *d = dst + 2 * (w + k * T);
+          if (in.copy_keys && even) {
+            *reinterpret_cast<ulonglong2 *>(d) = x[k];
+          } else if (in.copy_keys) {
+            d[0] = x[k].x;
+            d[1] = x[k].y;
+          }
+          check_nibbles8(x[k].x, sbad, sterms);
+          check_nibbles8(x[k].y, sbad, sterms);
+        }
+      }
+      if (t0 == 0 && (nv & 1)) {
+        const uint64_t x = src[nv - 1];
+        if (in.copy_keys) dst[nv - 1] = x;
+        check_nibbles8(x, sbad, sterms);
+      }
+    } else {
+      for (int64_t w = t0; w < nv; w += T) {
+        const uint64_t x = src[w];
+        if (in.copy_keys) dst[w] = x;
+        check_nibbles8(x, sbad, sterms);
+      }
+    }
+    if (t0 < (in.kbytes & 7)) {
+      const uint8_t b = in.keys[8 * nv + t0];
+      if (in.copy_keys) reinterpret_cast<uint8_t *>(dst)[8 * nv + t0] = b;
+      sbad |= b > 16;
+      sterms += b == 16;
+    }
+  }
+  if (in.copy_vals) {
+    const int64_t nv = in.vbytes / 16;
+    const uint4 *src = reinterpret_cast<const uint4 *>(in.vals);
+    uint4 *dst = reinterpret_cast<uint4 *>(const_cast<uint8_t *>(tv.vals) + in.val_base);
+    for (int64_t w = t0; w < nv; w += 4 * T) {
+      uint4 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (w + k * T < nv) x[k] = __ldcs(src + w + k * T);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (w + k * T < nv) dst[w + k * T] = x[k];
+    }
+    if (t0 < (in.vbytes & 15)) reinterpret_cast<uint8_t *>(dst)[16 * nv + t0] = in.vals[16 * nv + t0];
+  }
+  if (t0 < 64) const_cast<uint8_t *>(tv.keys)[in.key_base + in.kbytes + t0] = 0;
+  // records
+  for (int64_t i = t0; i < n; i += T) {
+    if (in.tid && (uint32_t)in.tid[i] >= tv.n_tries) stage_error(tv.ctr, ERR_BAD_TRIE);
+    int ks = in.ki[2 * i], ke = in.ki[2 * i + 1];
+    bool bad = ks < 0 || ke < ks || (int64_t)ke >= in.kbytes;  // index pair outside the key stream
     if (bad) ks = ke = 0;
     int len = ke - ks + 1;
-    uint64_t off = key_base + (uint64_t)ks;
     if (len > kMaxKeyNibbles) {
-      set_error(tv.ctr, ERR_KEY_TOO_LONG);
+      stage_error(tv.ctr, ERR_KEY_TOO_LONG);
       bad = true;
     }
-    // Interior nibbles are checked by k_stage_stream over the whole stream
-    // when the index pairs tile it (the usual layout), else by k_stage_keys.
     bool term = false;
     if (!bad) {
-      uint8_t last = tv.keys[off + len - 1];
+      const uint8_t last = in.keys[ke];
       if (last > 16) bad = true;
       term = last == 16;
     }
-    const bool gap = (i == 0) ? (ks != 0) : (ks != ki[2 * i - 1] + 1);
+    const bool gap = (i == 0) ? (ks != 0) : (ks != in.ki[2 * i - 1] + 1);
     terms += (term && !bad) ? 1u : 0u;
     gaps |= gap ? 1u : 0u;
     if (bad) {
-      set_error(tv.ctr, ERR_BAD_KEY);
+      stage_error(tv.ctr, ERR_BAD_KEY);
       len = 1;  // keep later stages in bounds
     }
-    koff[i] = off;
+    koff[i] = in.key_base + (uint64_t)ks;
     klen[i] = (uint32_t)len;
     lmax = max(lmax, (uint32_t)len);
-    int64_t vs = vi[2 * i], ve = vi[2 * i + 1];
-    if (vs < 0 || ve < vs - 1 || ve >= vbytes || ve - vs + 1 > 0x7FFFFFFF) {  // empty values allowed
-      set_error(tv.ctr, ERR_BAD_KEY);
+    int64_t vs = in.vi[2 * i], ve = in.vi[2 * i + 1];
+    if (vs < 0 || ve < vs - 1 || ve >= in.vbytes || ve - vs + 1 > 0x7FFFFFFF) {  // empty values allowed
+      stage_error(tv.ctr, ERR_BAD_KEY);
       vs = 0;
       ve = -1;
     }
-    uint64_t vid = vid_base + (uint64_t)i;
+    const uint64_t vid = in.vid_base + (uint64_t)i;
     vmax = max(vmax, (uint32_t)(ve - vs + 1));
-    tv.rec[vid] = ValueRec{val_base + (uint64_t)vs, (uint32_t)(ve - vs + 1), 0u};
-    tv.rec_hp[vid] = hp ? hp[i] : 0ull;
+    tv.rec[vid] = ValueRec{in.val_base + (uint64_t)vs, (uint32_t)(ve - vs + 1), 0u};
+    tv.rec_hp[vid] = in.hp ? in.hp[i] : 0ull;
   }
-  __shared__ uint32_t red[4][8];
+  __shared__ uint32_t red[6][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   terms = __reduce_add_sync(0xffffffffu, terms);
   gaps = __reduce_or_sync(0xffffffffu, gaps);
   lmax = __reduce_max_sync(0xffffffffu, lmax);
   vmax = __reduce_max_sync(0xffffffffu, vmax);
+  sterms = __reduce_add_sync(0xffffffffu, sterms);
+  sbad = __reduce_or_sync(0xffffffffu, sbad);
   if (lane == 0) {
     red[0][warp] = terms;
     red[1][warp] = gaps;
     red[2][warp] = lmax;
     red[3][warp] = vmax;
+    red[4][warp] = sterms;
+    red[5][warp] = sbad;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t t = 0, g = 0, m = 0, v = 0;
+    uint32_t t = 0, g = 0, m = 0, v = 0, st = 0, sb = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
       t += red[0][w];
       g |= red[1][w];
       m = max(m, red[2][w]);
       v = max(v, red[3][w]);
+      st += red[4][w];
+      sb |= red[5][w];
     }
     if (t) atomicAdd(&tv.ctr->key_terms, t);
     if (g) atomicOr(&tv.ctr->noncontig, 1u);
-    if (m) atomicMax(maxlen, m);
-    if (v) atomicMax(maxlen + 1, v);  // longest value of the batch
+    if (m) atomicMax(&tv.ctr->max_klen, m);
+    if (v) atomicMax(&tv.ctr->max_vlen, v);
+    if (st) atomicAdd(&tv.ctr->stream_terms, (unsigned long long)st);
+    if (sb) atomicOr(&tv.ctr->bad_byte, 1u);
   }
 }
 
@@ -197,63 +297,52 @@ __global__ void k_raw_lens(TrieView tv, const int *ki, int n, int64_t raw_bytes,
   flags[i] = 2ull * (uint64_t)max(len, 0) + 1ull;
 }
 
-// Expand key i to nibbles (high, low per byte) + terminator 16 at hex offset
-// pos[i] of `out`, and rewrite its index pair (in place) to the hex range.
-__global__ void k_raw_expand(const uint8_t *raw, int *ki, const unsigned long long *pos, int n, int64_t raw_bytes,
-                             uint8_t *out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int len = max(raw_key_len(ki, i, raw_bytes), 0);
-  const int s = ki[2 * i];
-  const uint64_t p = pos[i];
-  uint8_t *o = out + p;
-  for (int b = 0; b < len; ++b) {
-    const uint8_t x = raw[s + b];
-    o[2 * b] = x >> 4;
-    o[2 * b + 1] = x & 15;
+// Expand every key to nibbles (high, low per byte) + terminator 16 at hex
+// offset pos[i] of `out`, and rewrite its index pair (in place) to the hex
+// range.  A warp takes 32 keys and walks them with a byte per lane, so loads
+// and stores are coalesced (a key per thread, byte after byte, took 76 us for
+// 300K 20-byte keys; this takes 23).
+__global__ void __launch_bounds__(256) k_raw_expand(const uint8_t *raw, int *ki, const unsigned long long *pos, int n,
+                                                    int64_t raw_bytes, uint8_t *out) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31, i = i0 + lane;
+  const int len = i < n ? max(raw_key_len(ki, i, raw_bytes), 0) : 0;
+  const int s = i < n ? ki[2 * i] : 0;
+  const unsigned long long p = i < n ? pos[i] : 0ull;
+  for (int k = 0; k < 32 && i0 + k < n; ++k) {
+    const int kl = __shfl_sync(kAll, len, k), ks = __shfl_sync(kAll, s, k);
+    uint8_t *o = out + __shfl_sync(kAll, p, k);
+    for (int b = lane; b < kl; b += 32) {
+      const uint8_t x = raw[ks + b];
+      o[2 * b] = x >> 4;
+      o[2 * b + 1] = x & 15;
+    }
+    if (lane == 0) o[2 * kl] = 16;
   }
-  o[2 * len] = 16;
-  ki[2 * i] = (int)p;
-  ki[2 * i + 1] = (int)(p + 2 * (uint64_t)len);
-}
-
-// Coalesced check of a key stream that the index pairs tile: no byte > 16,
-// and exactly as many 16s as keys that end in one (so none is interior).
-__global__ void k_stage_stream(TrieView tv, const uint8_t *stream, int64_t nbytes) {
-  unsigned long long terms = 0;
-  uint32_t bad = 0;
-  const int64_t nvec = nbytes / 8;
-  const uint64_t *v = reinterpret_cast<const uint64_t *>(stream);  // 8-aligned arena base
-  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nvec; q += (int64_t)gridDim.x * blockDim.x) {
-    uint64_t x = __ldg(v + q);
-    bad |= (x & 0xE0E0E0E0E0E0E0E0ull) != 0;                    // >= 32
-    uint64_t hi = x & 0x1010101010101010ull;                      // bit 4 set: 16..31
-    bad |= (x & ((hi >> 4) * 0x0Full)) ? 1u : 0u;                 // 17..31: low nibble != 0
-    terms += __popcll(hi);
-  }
-  if (blockIdx.x == 0 && threadIdx.x < (nbytes & 7)) {
-    uint8_t b = stream[nvec * 8 + threadIdx.x];
-    bad |= b > 16;
-    terms += b == 16;
-  }
-  unsigned am = __activemask();
-  terms = __reduce_add_sync(am, (uint32_t)terms);
-  bad = __reduce_or_sync(am, bad);
-  if ((int)(threadIdx.x & 31) == __ffs(am) - 1) {
-    if (terms) atomicAdd(&tv.ctr->stream_terms, terms);
-    if (bad) atomicOr(&tv.ctr->bad_byte, 1u);
+  if (i < n) {
+    ki[2 * i] = (int)p;
+    ki[2 * i + 1] = (int)(p + 2 * (uint64_t)len);
   }
 }
 
-// Per-key interior check for streams the index pairs do not tile.
+// Verdict on a staged hex-key batch: one whose index pairs tile the stream is
+// checked whole (k_stage), the others key by key here.  (The host reports
+// the reason when it reads the counters.)
 __global__ void k_stage_keys(TrieView tv, const uint64_t *koff, const uint32_t *klen, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint8_t *k = tv.keys + koff[i];
-  int len = (int)klen[i];
-  uint64_t acc = 0;
-  for (int j = 0; j < len - 1; j += 8) acc |= load_u64_unaligned(k + j) & low_mask64(min(8, len - 1 - j));
-  if (acc & 0xF0F0F0F0F0F0F0F0ull) set_error(tv.ctr, ERR_BAD_KEY);
+  if (!__ldcg(&tv.ctr->noncontig)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 &&
+        (__ldcg(&tv.ctr->bad_byte) || __ldcg(&tv.ctr->stream_terms) != __ldcg(&tv.ctr->key_terms)))
+      tv.ctr->stage_bad = 1;
+    return;
+  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint8_t *k = tv.keys + koff[i];
+    int len = (int)klen[i];
+    uint64_t acc = 0;
+    for (int j = 0; j < len - 1; j += 8) acc |= load_u64_unaligned(k + j) & low_mask64(min(8, len - 1 - j));
+    if (acc & 0xF0F0F0F0F0F0F0F0ull) stage_error(tv.ctr, ERR_BAD_KEY);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2013,13 +2102,13 @@ __global__ void k_gets(TrieView tv, const uint8_t *keys, const int *idx, int n, 
   }
 }
 
-// Root bytes of trie ids[i] (or trie i when ids is null) into out[33 i ..]:
+// Root bytes of trie ids[i] (or trie first + i when ids is null) into out[33 i ..]:
 // 32 bytes (zero-padded) and the length (0 = empty trie).  Warp per trie.
-__global__ void k_roots(TrieView tv, const int *ids, int n, uint8_t *out) {
+__global__ void k_roots(TrieView tv, const int *ids, int first, int n, uint8_t *out) {
   const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (i >= n) return;
   const int t = threadIdx.x & 31;
-  const uint32_t tr = ids ? (uint32_t)ids[i] : (uint32_t)i;
+  const uint32_t tr = ids ? (uint32_t)ids[i] : (uint32_t)(first + i);
   out += 33 * (size_t)i;
   uint32_t r = tr < tv.n_tries ? tv.roots[tr] : 0u;
   uint32_t kind = ref_kind(r), idx = ref_idx(r);

@@ -1,0 +1,87 @@
+"""Staging of a batch in one pass: device streams at any byte offset, pairs
+that do not tile the stream, host batches on both sides of the packed copy,
+and malformed batches, which must leave the trie as it was."""
+import numpy as np
+import pytest
+
+import oracle as O
+from gmpt import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def oracle_root(*batches):
+    o = O.OracleTrie()
+    for b in batches:
+        o.puts(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)
+    o.hash()
+    return o.root()
+
+
+def at_offset(a, off):
+    """A device copy of array a starting `off` bytes into an allocation."""
+    import torch
+
+    raw = np.ascontiguousarray(a).view(np.uint8)
+    t = torch.zeros(len(raw) + 64, dtype=torch.uint8, device="cuda:0")
+    t[off: off + len(raw)] = torch.from_numpy(raw.copy()).cuda()
+    return t, t.data_ptr() + off
+
+
+@pytest.mark.parametrize("two_phase", [False, True])
+@pytest.mark.parametrize("off", [0, 1, 4, 8, 15])
+def test_device_streams_at_any_offset(gpu_lib, two_phase, off):
+    import torch
+
+    for n, vb in ((1, 1), (3, 7), (1000, 33), (20001, 5)):
+        b = W.random_keys(n, 11, vb, seed=0x5EED0B00 + n)
+        keep = [at_offset(a, off) for a in (b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)]
+        torch.cuda.synchronize()
+        t = gpu_lib.MPT()
+        for _ in range(2):  # the second batch starts at another arena offset
+            t.puts_device(two_phase, *[p for _, p in keep], n, len(b.keys_hexs), len(b.values))
+        t.hash_onepass_v2()
+        assert t.get_root_hash() == oracle_root(b), (n, vb)
+        t.close()
+
+
+@pytest.mark.parametrize("two_phase", [False, True])
+@pytest.mark.parametrize("n", [1, 900, 1100, 40000])  # 256 KiB of host arrays lie in between
+def test_host_batches_and_lookups(gpu_lib, two_phase, n):
+    b = W.random_keys(n, 32, 100, seed=0x5EED0B10 + n)
+    hps = np.arange(1, n + 1, dtype=np.uint64)
+    t = gpu_lib.MPT()
+    put = t.puts_2phase_with_valuehp if two_phase else t.puts_latching_with_valuehp_v2
+    put(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs, hps)
+    t.hash_onepass_v2()
+    assert t.get_root_hash() == oracle_root(b)
+    hp, size = t.gets_parallel(b.keys_hexs, b.keys_indexs)
+    assert np.array_equal(hp, hps) and np.all(size == 100)
+    t.close()
+
+
+@pytest.mark.parametrize("two_phase", [False, True])
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("bad", [17, 200, 16])
+def test_malformed_batches_are_not_applied(gpu_lib, two_phase, tiled, bad):
+    first = W.random_keys(500, 8, 20, seed=0x5EED0B20)
+    b = W.random_keys(3000, 8, 20, seed=0x5EED0B21)
+    kh, ki = b.keys_hexs.copy(), b.keys_indexs.copy()
+    if not tiled:  # a hole in front of every key
+        kh = np.concatenate([np.zeros((b.n, 1), np.uint8), kh.reshape(b.n, -1)], axis=1).reshape(-1)
+        ki = ki + np.repeat(np.arange(1, b.n + 1, dtype=np.int32), 2)
+    t = gpu_lib.MPT()
+    put = t.puts_2phase_with_valuehp if two_phase else t.puts_latching_with_valuehp_v2
+    put(first.keys_hexs, first.keys_indexs, first.values, first.values_indexs)
+    t.hash_onepass_v2()
+    good = kh.copy()
+    kh[ki[2 * 1234] + 3] = bad  # an interior nibble
+    with pytest.raises(gpu_lib.GmptError) as ei:
+        put(kh, ki, b.values, b.values_indexs)
+    assert ei.value.code == 2
+    t.hash_onepass_v2()
+    assert t.get_root_hash() == oracle_root(first)
+    put(good, ki, b.values, b.values_indexs)
+    t.hash_onepass_v2()
+    assert t.get_root_hash() == oracle_root(first, b)
+    t.close()
