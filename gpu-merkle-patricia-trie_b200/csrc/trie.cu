@@ -46,6 +46,8 @@ constexpr uint64_t kHashBarrierNs = 2000000000ull;  // longest grid-barrier wait
 // message window per warp
 constexpr size_t kGridSmem = sizeof(uint32_t) * kStageWords * kGridThreads + (kGridThreads / 32) * kWarpMsgBytes;
 constexpr uint32_t kMaxDepths = kMaxKeyNibbles + 2;  // nibble depths a dirty node can have
+// LockNU: up to this many keys are inserted one, two per thread
+constexpr int kLatchOneWay = 1 << 17, kLatchTwoWays = 1 << 23;
 // LockNU batches of at least this many keys drop repeated keys first
 constexpr int kDedupMinKeys = 1 << 16;
 
@@ -1465,6 +1467,7 @@ int Trie::put_latching(const BatchIn &b) {
         for (auto &x : ev) cudaEventDestroy(x);
       return OK;
     }
+    rw_kept_ = m;
     ks.sel = uord;
     ks.count = ws_.rw_tot.as<unsigned long long>() + 3;
     ks.collision = reinterpret_cast<const uint32_t *>(ws_.rw_tot.as<unsigned long long>() + 4);  // zeroed
@@ -1497,9 +1500,15 @@ int Trie::put_latching(const BatchIn &b) {
     ks.count = d_tot;
     ks.collision = collision;
   }
-  const int ways = opt_latch_ways_;
+  // Keys per thread: a few keys are a chain of loads each, and four chains
+  // in one thread advance in step (16K-key update 107 us with four, 46 with
+  // one); from more keys than threads fit the GPU on, two (300K keys 304,
+  // 266, 305 us with four, two, one; 4M keys 2.07, 1.88, 1.90 ms); four for
+  // the largest (16M zipf updates 3.48, 3.61, 3.82 ms).
+  const int n_ins = rw_ ? rw_kept_ : b.n;
+  const int ways = std::min(opt_latch_ways_, n_ins <= kLatchOneWay ? 1 : (n_ins <= kLatchTwoWays ? 2 : 4));
   auto kern = ways == 1 ? k_latch_insert<1> : (ways == 2 ? k_latch_insert<2> : k_latch_insert<4>);
-  count_launch(), kern<<<blocks_for((b.n + ways - 1) / ways), kThreads, 0, st_>>>(tv_, dl, koff, klen, b.n, vid_base,
+  count_launch(), kern<<<blocks_for((n_ins + ways - 1) / ways), kThreads, 0, st_>>>(tv_, dl, koff, klen, b.n, vid_base,
                                                                                  opt_retry_limit_, tid, ks);
   if ((rc = check_cuda(cudaGetLastError(), "latch launch"))) return rc;
   if ((rc = copy_counters())) return rc;
@@ -1910,7 +1919,7 @@ int Trie::block_grid() const { return opt_block_grid_ > 0 ? std::min(opt_block_g
 
 // hash_grid's warp_max for `grid` CTAs: two nodes per warp, within the
 // warp_full_max option.  A warp's permutations are shuffle-bound (500 cycles
-// each per SM), a thread each takes 35-39 us for any wave of up to 19K
+// each per SM), a pair of lanes each takes 30-32 us for any wave of up to 9K
 // branches (three blocks and an extension): the two meet there.
 uint32_t Trie::grid_warp_max(unsigned grid) const {
   return std::min<uint32_t>((uint32_t)opt_warp_full_max_, 2u * grid * (kGridThreads / 32));

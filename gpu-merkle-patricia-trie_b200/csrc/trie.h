@@ -280,6 +280,7 @@ class Trie {
     bool check_stream = false;
   } staged_;
   uint32_t maxlen_ = 0;          // its longest key
+  int rw_kept_ = 0;              // writes a mixed batch's insert is left with
   // set by put_rw for the duration of one put: sort_unique then resolves the
   // reads and keeps the last write of every key
   struct RwState {
