@@ -175,6 +175,48 @@ __device__ __forceinline__ uint64_t keccak_f1600_warp(uint64_t a, const CoopLane
   return a;
 }
 
+// Keccak-f[1600] over a pair of lanes (2k, 2k + 1): the even lane holds the low
+// halves of the 25 words, the odd lane the high ones.  XOR, AND-NOT and NOT
+// stay in a lane; a rotation takes the partner's half by shuffle and is the
+// same funnel shift in both lanes.  Half the instructions per lane of the
+// one-thread form at the same total (91 integer ops and 29 shuffles a round
+// against 190 ops), so a warp of 16 states has about half the latency: the
+// form for a few thousand nodes, too many for a warp each and too few to fill
+// the schedulers with a thread each.  All 32 lanes call it together; odd:
+// this lane holds the high halves.
+__device__ __forceinline__ void keccak_f1600_pair(uint32_t (&a)[25], bool odd) {
+  constexpr unsigned kAll = 0xffffffffu;
+  // rho offsets r[x][y] (FIPS 202), indexed x + 5y
+  constexpr int kRho[25] = {0,  1,  62, 28, 27, 36, 44, 6,  55, 20, 3,  10, 43,
+                            25, 39, 41, 45, 15, 21, 8,  18, 2,  61, 56, 14};
+#pragma unroll 2
+  for (int r = 0; r < 24; ++r) {
+    uint32_t c[5], d[5], b[25];
+#pragma unroll
+    for (int x = 0; x < 5; ++x) c[x] = a[x] ^ a[x + 5] ^ a[x + 10] ^ a[x + 15] ^ a[x + 20];
+#pragma unroll
+    for (int x = 0; x < 5; ++x) d[x] = __funnelshift_l(__shfl_xor_sync(kAll, c[x], 1), c[x], 1);
+#pragma unroll
+    for (int i = 0; i < 25; ++i) {
+      const int x = i % 5, y = i / 5;
+      const uint32_t own = a[i] ^ c[(x + 4) % 5] ^ d[(x + 1) % 5];
+      const int to = y + 5 * ((2 * x + 3 * y) % 5);  // pi
+      const int n = kRho[i] & 31;
+      if (kRho[i] == 0) {
+        b[to] = own;
+      } else {
+        const uint32_t other = __shfl_xor_sync(kAll, own, 1);
+        b[to] = kRho[i] < 32 ? __funnelshift_l(other, own, n) : __funnelshift_l(own, other, n);
+      }
+    }
+#pragma unroll
+    for (int y = 0; y < 5; ++y)
+#pragma unroll
+      for (int x = 0; x < 5; ++x) a[x + 5 * y] = b[x + 5 * y] ^ (~b[(x + 1) % 5 + 5 * y] & b[(x + 2) % 5 + 5 * y]);
+    a[0] ^= odd ? (uint32_t)(kKeccakRC[r] >> 32) : (uint32_t)kKeccakRC[r];
+  }
+}
+
 // Streaming sponge.  Message bytes are pushed in little-endian runs of <= 8
 // bytes; whole 64-bit words go to this thread's 17-word staging block in
 // shared memory (a column of 32-bit halves: half h at stage[h * stride]),

@@ -1413,6 +1413,59 @@ __device__ __forceinline__ void write_nibbles(WordWriter &o, const uint8_t *src,
 // bytes, tag and hash) can run past its end.
 constexpr uint32_t kStageWords = 34 + 14;
 
+// Message of a regular branch, block by block: 0x80 per empty slot, 0xa0 + 32
+// hash bytes per child, then the Keccak padding (rlp.cuh:132-155,
+// node.cuh:46-112).  A child at a time: its hash in two 16-byte loads, eight
+// funnel-shifted words out; what the last child writes past a block moves to
+// the front of the next.
+template <bool kCoh>
+struct BranchWriter {
+  WordWriter o;
+  uint32_t left;
+  int prev = -1;
+  bool done = false;
+  __device__ __forceinline__ BranchWriter(uint32_t *st, uint32_t stride, uint64_t hdr, uint32_t hn, uint32_t present)
+      : o(st, stride), left(present) {
+    o.bytes((uint32_t)hdr, hn);
+  }
+  // stage the next block; true: it is the last one
+  __device__ __forceinline__ bool fill(const TrieView &tv, const uint32_t *chp) {
+    while (o.w < 34 && !done) {
+      const int k = left ? __ffs(left) - 1 : 17;  // next child, or the end
+      left &= left - 1;
+      uint32_t gap = (uint32_t)(k - prev - 1);
+      prev = k;
+      if (k < 17) {
+        const uint32_t r = ldn<kCoh>(chp + k);
+        const uint4 *h = reinterpret_cast<const uint4 *>(
+            (ref_kind(r) == KIND_FULL ? tv.full_hash : tv.short_hash) + (size_t)ref_idx(r) * 32);
+        const uint4 x = ldn<kCoh>(h), y = ldn<kCoh>(h + 1);
+        for (; gap >= 4; gap -= 4) o.word(0x80808080u);
+        // gap (0..3) empty slots, then the child's tag
+        o.bytes((0x80808080u & ((1u << (8 * gap)) - 1u)) | (0xa0u << (8 * gap)), gap + 1);
+        o.word(x.x), o.word(x.y), o.word(x.z), o.word(x.w);
+        o.word(y.x), o.word(y.y), o.word(y.z), o.word(y.w);
+      } else {
+        for (; gap >= 4; gap -= 4) o.word(0x80808080u);
+        o.bytes((0x80808080u & ((1u << (8 * gap)) - 1u)) | (0x01u << (8 * gap)), gap + 1);
+        o.bytes(0u, o.pb ? 4 - o.pb : 0u);  // whole words from here on
+        done = true;
+      }
+    }
+    const bool last = done && o.w <= 34;
+    if (last) {
+      for (uint32_t w = o.w; w < 34; ++w) o.st[w * o.stride] = 0;
+      o.st[33 * o.stride] |= 0x80000000u;
+    }
+    return last;
+  }
+  // after a block that was not the last
+  __device__ __forceinline__ void next() {
+    for (uint32_t w = 34; w < o.w; ++w) o.st[(w - 34) * o.stride] = o.st[w * o.stride];
+    o.w -= 34;
+  }
+};
+
 // Encode + hash one dirty node; `stage` is this thread's column of the
 // message block in shared memory (kStageWords 32-bit words, word w at
 // stage[w * stride]).
@@ -1525,47 +1578,12 @@ __device__ __forceinline__ void hash_node(const TrieView &tv, uint32_t idx, uint
       sp.absorb();
     }
   } else if (regular) {
-    // 0x80 per empty slot, 0xa0 + 32 hash bytes per child, then the Keccak
-    // padding (rlp.cuh:132-155, node.cuh:46-112).  A child at a time: its
-    // hash in two 16-byte loads, eight funnel-shifted words out.  A block is
-    // permuted when full; what the last child wrote past it moves to the front.
-    WordWriter o(stage, stride);
-    o.bytes((uint32_t)hdr, hn);
-    uint32_t left = present;
-    int prev = -1;
-    bool done = false;
+    BranchWriter<kCoh> bw(stage, stride, hdr, hn, present);
     while (true) {
-      while (o.w < 34 && !done) {
-        const int k = left ? __ffs(left) - 1 : 17;  // next child, or the end
-        left &= left - 1;
-        uint32_t gap = (uint32_t)(k - prev - 1);
-        prev = k;
-        if (k < 17) {
-          const uint32_t r = ldn<kCoh>(chp + k);
-          const uint4 *h = reinterpret_cast<const uint4 *>(
-              (ref_kind(r) == KIND_FULL ? tv.full_hash : tv.short_hash) + (size_t)ref_idx(r) * 32);
-          const uint4 x = ldn<kCoh>(h), y = ldn<kCoh>(h + 1);
-          for (; gap >= 4; gap -= 4) o.word(0x80808080u);
-          // gap (0..3) empty slots, then the child's tag
-          o.bytes((0x80808080u & ((1u << (8 * gap)) - 1u)) | (0xa0u << (8 * gap)), gap + 1);
-          o.word(x.x), o.word(x.y), o.word(x.z), o.word(x.w);
-          o.word(y.x), o.word(y.y), o.word(y.z), o.word(y.w);
-        } else {
-          for (; gap >= 4; gap -= 4) o.word(0x80808080u);
-          o.bytes((0x80808080u & ((1u << (8 * gap)) - 1u)) | (0x01u << (8 * gap)), gap + 1);
-          o.bytes(0u, o.pb ? 4 - o.pb : 0u);  // whole words from here on
-          done = true;
-        }
-      }
-      const bool last = done && o.w <= 34;
-      if (last) {
-        for (uint32_t w = o.w; w < 34; ++w) stage[w * stride] = 0;
-        stage[33 * stride] |= 0x80000000u;
-      }
+      const bool last = bw.fill(tv, chp);
       sp.absorb();
       if (last) break;
-      for (uint32_t w = 34; w < o.w; ++w) stage[(w - 34) * stride] = stage[w * stride];
-      o.w -= 34;
+      bw.next();
     }
   } else {
   // pass 2: stream
