@@ -161,10 +161,13 @@ __device__ __forceinline__ void child_done(const TrieView &tv, uint32_t par, uin
 
 // A wave of n ready branches, a pair of lanes each: the even lane writes the
 // message into its column, both permute (keccak_f1600_pair), then the same for
-// the extension above.  Branches that are not regular (values, children below
-// 32 bytes) and extensions of more than one block are left to the whole warp.
+// the extension above.  Branches of more than kPairBlocks blocks (a long value:
+// its serial blocks are shorter a warp each) or below 32 bytes are left to the
+// whole warp, an extension of more than one block to the even lane.
 // A thread each, a wave of 2^13 branches of 10 children with their extensions
 // took 38 us; a pair each, 31 (2.9 us a permutation against 4.9).
+constexpr uint32_t kPairBlocks = 12;
+
 __device__ inline void wave_by_pairs(const TrieView &tv, const GridPlace &g, const uint32_t *list, uint32_t n,
                                      uint32_t at0, uint32_t *next, uint32_t *ready, uint32_t cap, uint32_t *stage,
                                      uint8_t *wmsg, const CoopLanes &cl) {
@@ -197,21 +200,32 @@ __device__ inline void wave_by_pairs(const TrieView &tv, const GridPlace &g, con
       }
       regular = regular && present < (1u << 16) && present != 0;
     }
-    regular = __shfl_sync(kAll, regular, even);
-    const unsigned other = __ballot_sync(kAll, on && !regular && !odd);
-    // the branch
+    uint32_t body = 17u + 32u * __popc(present);
+    if (on && !odd && !regular) {
+      body = 0;
+#pragma unroll 1
+      for (int k = 0; k < 17; ++k) {
+        const EncItem it = child_item<true>(tv, __ldcg(chp + k));
+        body += it.pren + it.blen;
+      }
+    }
     uint64_t hdr;
     uint32_t hn;
-    rlp_head(17u + 32u * __popc(present), 0xc0, 0xf7, hdr, hn);
+    rlp_head(body, 0xc0, 0xf7, hdr, hn);
+    const uint32_t total = body + hn;
+    const bool pair = __shfl_sync(kAll, on && total >= 32 && total < kPairBlocks * 136, even);
+    const unsigned other = __ballot_sync(kAll, on && !pair && !odd);
+    // the branch
     BranchWriter<true> bw(st, S, hdr, hn, present);
+    ItemWriter<true> iw(st, S, hdr, hn);
     uint32_t a[25], h[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int i = 0; i < 25; ++i) a[i] = 0;
-    bool going = regular;
+    bool going = pair;
     uint32_t blocks = 0;
     while (__any_sync(kAll, going)) {
       bool last = false;
-      if (going && !odd) last = bw.fill(tv, chp);
+      if (going && !odd) last = regular ? bw.fill(tv, chp) : iw.fill(tv, chp);
       __syncwarp();
       last = __shfl_sync(kAll, last, even);
       if (going) {
@@ -225,11 +239,11 @@ __device__ inline void wave_by_pairs(const TrieView &tv, const GridPlace &g, con
 #pragma unroll
         for (int i = 0; i < 4; ++i) h[i] = a[i];
       }
-      if (going && !last && !odd) bw.next();
+      if (going && !last && !odd) regular ? bw.next() : iw.next();
       going = going && !last;
     }
     uint32_t e = kNoNode, top = 0;
-    if (regular) {
+    if (pair) {
       uint32_t *o = reinterpret_cast<uint32_t *>(tv.full_hash + (size_t)f * 32);
 #pragma unroll
       for (int i = 0; i < 4; ++i) o[2 * i + (odd ? 1 : 0)] = h[i];
@@ -280,14 +294,14 @@ __device__ inline void wave_by_pairs(const TrieView &tv, const GridPlace &g, con
       }
     }
     if (e != kNoNode && !one) hash_node<true, false>(tv, e, stage, S);
-    if (tv.account && regular && !odd) {
-      atomicAdd(&tv.ctr->enc_bytes, 20ull + 32u * __popc(present) + (e != kNoNode ? payload + hn : 0u));
+    if (tv.account && pair && !odd) {
+      atomicAdd(&tv.ctr->enc_bytes, (unsigned long long)total + (one ? payload + hn : 0u));
       atomicAdd(&tv.ctr->keccak_blocks, (unsigned long long)blocks + (one ? 1u : 0u));
       atomicAdd(&tv.ctr->hashed, one ? 2u : 1u);
     }
     __threadfence();  // both lanes' halves before the parent's count
     __syncwarp();
-    if (regular && !odd) child_done(tv, __ldcg(tv.full_par + f), top, at0, next, ready, cap);
+    if (pair && !odd) child_done(tv, __ldcg(tv.full_par + f), top, at0, next, ready, cap);
     for (unsigned m = other; m; m &= m - 1) {
       const uint32_t fi = __shfl_sync(kAll, f, __ffs(m) - 1);
       const uint32_t t = hash_full_warp<true>(tv, fi, child_word(tv, fi, g.lane), wmsg, cl, kNoNode, nullptr);

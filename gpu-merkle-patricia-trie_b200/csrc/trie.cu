@@ -41,6 +41,9 @@ constexpr uint32_t kWarpLeafMax = 2048;
 constexpr size_t kPackBytes = 256 << 10;
 // dirty lists of at most this many nodes are hashed by one cooperative launch
 constexpr uint32_t kGridHashMax = 1u << 17;
+// larger lists whose branches are spread over at least this many nibble
+// depths have their branches hashed by one, after the leaves
+constexpr int kGridLevels = 24;
 constexpr uint64_t kHashBarrierNs = 2000000000ull;  // longest grid-barrier wait of such a launch
 // shared memory of a cooperative launch's CTA: message words per thread, a
 // message window per warp
@@ -137,7 +140,7 @@ Trie::~Trie() {
                         &ws_.rw_a, &ws_.rw_b, &ws_.rw_c, &ws_.rw_d, &ws_.rw_e, &ws_.rw_wpos, &ws_.rw_hp,
                         &ws_.rw_len, &ws_.rw_tot, &ws_.rw_kept, &ws_.rw_koff, &ws_.rw_klen, &ws_.rw_tid,
                         &ws_.del_hslot, &ws_.del_hext, &ws_.del_stamp,
-                        &ws_.pack, &ws_.misc};
+                        &ws_.pack, &ws_.ready, &ws_.misc};
   for (DevBlock *b : blocks) b->release();
   for (int k = 0; k < 2; ++k) {
     ws_.s_start[k].release();
@@ -1063,24 +1066,21 @@ int Trie::bucket_and_hash() {
   stats_.last_dirty = nd;
   stats_.last_hash_levels = 0;
   if (nd == 0) return OK;
-  if (nd <= kGridHashMax) return hash_by_grid(nd);
+  if (nd <= kGridHashMax) {
+    int rc = begin_hash_timing();
+    if (!rc) rc = launch_hash_grid(dirty_ref_, nd);
+    if (rc || (rc = end_hash_timing())) return rc;
+    stats_.last_hash_levels = stats_.hash_launches = 1;
+    return end_hash(nd);
+  }
   uint32_t *sorted = nullptr;
   std::vector<uint32_t> off;
   int rc = bucket_dirty(nd, &sorted, off);
   if (rc) return rc;
   size_t smem = sizeof(uint32_t) * kStageWords * kHashThreads;
   int levels = 0;
-  if ((e = cudaMemsetAsync(&ctr_->hashed, 0, 4, st_)) != cudaSuccess ||
-      (e = cudaMemsetAsync(&ctr_->enc_bytes, 0, 16, st_)) != cudaSuccess)
-    return check_cuda(e, "hash counters");
-  cudaEvent_t ka = nullptr, kz = nullptr;
-  if (timing_) {
-    cudaEventCreate(&ka);
-    cudaEventCreate(&kz);
-    cudaEventRecord(ka, st_);
-  }
+  if ((rc = begin_hash_timing())) return rc;
   const size_t smem_warp = 4 * kWarpMsgBytes;
-  tv_.account = timing_ ? 1 : 0;  // per-node accounting atomics only when measuring
   // a launch of at most kWideGrid CTAs cannot fill the SMs at the
   // throughput form's occupancy: it runs the wide form (more registers per
   // thread, no spills, shorter serial chains)
@@ -1101,7 +1101,18 @@ int Trie::bucket_and_hash() {
     else
       level(false, sorted, off[kLeafClasses]);
   }
-  for (int d = (int)dirty_depths() - 1; d >= 0; --d) {
+  int branch_levels = 0;
+  for (uint32_t d = 0; d < dirty_depths(); ++d) branch_levels += off[level_bin(d) + kHashClasses] > off[level_bin(d)];
+  const bool deep = branch_levels >= kGridLevels;
+  if (deep) {
+    // many levels, each as long as its slowest branch: one cooperative launch
+    // over all branches (the first wave holds the lowest branch of every path,
+    // whatever its depth)
+    ++levels;
+    const uint32_t a = off[level_bin(0)];
+    if ((rc = launch_hash_grid(sorted + a, nd - a))) return rc;
+  }
+  for (int d = deep ? -1 : (int)dirty_depths() - 1; d >= 0; --d) {
     // branches [a, m), the extensions above them [m, z)
     const uint32_t a = off[level_bin(d)], m = off[level_bin(d) + kHashClasses], z = off[level_bin(d + 1)];
     if (m == a) continue;  // (an extension is listed with its branch's level)
@@ -1124,27 +1135,47 @@ int Trie::bucket_and_hash() {
     }
     if (z > m) level(false, sorted + m, z - m);
   }
-  if (timing_) {
-    cudaEventRecord(kz, st_);
-    cudaEventSynchronize(kz);
-    cudaEventElapsedTime(&stats_.t_hash_kernels_ms, ka, kz);
-    cudaEventDestroy(ka);
-    cudaEventDestroy(kz);
-  }
-  tv_.account = 0;
+  if ((rc = end_hash_timing())) return rc;
   stats_.last_hash_levels = levels;
   stats_.hash_launches = levels;
   if ((e = cudaMemsetAsync(&ctr_->n_dirty, 0, 4, st_)) != cudaSuccess) return check_cuda(e, "hash reset");
   return end_hash(nd);
 }
 
-// PhaseHC of a small or middle dirty list in one cooperative launch
-// (grid_hash.cuh).
-int Trie::hash_by_grid(uint32_t nd) {
+// Timing mode: events around a pass's kernels, and per-node accounting (its
+// atomics only when measuring).
+int Trie::begin_hash_timing() {
+  tv_.account = 0;
+  if (!timing_) return OK;
+  cudaError_t e = cudaMemsetAsync(&ctr_->hashed, 0, 4, st_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(&ctr_->enc_bytes, 0, 16, st_);
+  if (e == cudaSuccess) e = cudaEventCreate(&hash_ev_[0]);
+  if (e == cudaSuccess) e = cudaEventCreate(&hash_ev_[1]);
+  if (e == cudaSuccess) e = cudaEventRecord(hash_ev_[0], st_);
+  tv_.account = 1;
+  return check_cuda(e, "hash timing");
+}
+
+int Trie::end_hash_timing() {
+  tv_.account = 0;
+  if (!timing_) return OK;
+  cudaError_t e = cudaEventRecord(hash_ev_[1], st_);
+  if (e == cudaSuccess) e = cudaEventSynchronize(hash_ev_[1]);
+  if (e == cudaSuccess) e = cudaEventElapsedTime(&stats_.t_hash_kernels_ms, hash_ev_[0], hash_ev_[1]);
+  for (auto &x : hash_ev_) {
+    if (x) cudaEventDestroy(x);
+    x = nullptr;
+  }
+  return check_cuda(e, "hash timing");
+}
+
+// Hash a list of dirty nodes in one cooperative launch (grid_hash.cuh); it
+// empties the dirty list.
+int Trie::launch_hash_grid(const uint32_t *refs, uint32_t nd) {
   int rc = grid_limits();
   if (rc) return rc;
   cudaError_t e = cudaSuccess;
-  uint32_t *ready = wsp<uint32_t>(ws_.sorted_dirty, nd, e);
+  uint32_t *ready = wsp<uint32_t>(ws_.ready, nd, e);
   if (e == cudaSuccess && !grid_ctl_) {
     GridCtl init{};
     init.barrier_ns = kHashBarrierNs;
@@ -1152,17 +1183,7 @@ int Trie::hash_by_grid(uint32_t nd) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(grid_ctl_, &init, sizeof(init), cudaMemcpyHostToDevice, st_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
   }
-  GridCtl *ctl = static_cast<GridCtl *>(grid_ctl_);
-  cudaEvent_t ka = nullptr, kz = nullptr;
-  if (e == cudaSuccess && timing_) {
-    cudaEventCreate(&ka);
-    cudaEventCreate(&kz);
-    e = cudaMemsetAsync(&ctr_->hashed, 0, 4, st_);
-    if (e == cudaSuccess) e = cudaMemsetAsync(&ctr_->enc_bytes, 0, 16, st_);
-    cudaEventRecord(ka, st_);
-  }
   if (e != cudaSuccess) return check_cuda(e, "hash alloc");
-  tv_.account = timing_ ? 1 : 0;
   // enough warps for one node each, within what fits co-resident
   const unsigned grid = std::min<unsigned>((unsigned)max_grid_, (nd + kGridThreads / 32 - 1) / (kGridThreads / 32));
   cudaLaunchConfig_t cfg = {};
@@ -1176,20 +1197,9 @@ int Trie::hash_by_grid(uint32_t nd) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   count_launch();
-  e = cudaLaunchKernelEx(&cfg, k_hash_grid, tv_, DirtyList{dirty_ref_, dirty_depth_}, nd, ready, nd, ctl,
-                         grid_warp_max(grid));
-  tv_.account = 0;
-  if (e != cudaSuccess) return check_cuda(e, "hash launch");
-  if (timing_) {
-    cudaEventRecord(kz, st_);
-    cudaEventSynchronize(kz);
-    cudaEventElapsedTime(&stats_.t_hash_kernels_ms, ka, kz);
-    cudaEventDestroy(ka);
-    cudaEventDestroy(kz);
-  }
-  stats_.last_hash_levels = 1;
-  stats_.hash_launches = 1;
-  return end_hash(nd);
+  e = cudaLaunchKernelEx(&cfg, k_hash_grid, tv_, DirtyList{const_cast<uint32_t *>(refs), nullptr}, nd, ready, nd,
+                         static_cast<GridCtl *>(grid_ctl_), grid_warp_max(grid));
+  return check_cuda(e, "hash launch");
 }
 
 // After a pass (which has emptied the list on the device): the record for

@@ -198,6 +198,7 @@ class Trie {
   uint32_t n_dirty_ = 0;       // nodes marked since the last hash (as of the last counters)
   int sms_ = 0, max_grid_ = 0;  // CTAs of the cooperative kernels that fit co-resident
   void *grid_ctl_ = nullptr;    // GridCtl of the hash launches
+  cudaEvent_t hash_ev_[2] = {nullptr, nullptr};  // timing mode, during a hash pass
   uint64_t n_rec_ = 0, key_used_ = 0, val_used_ = 0;
   // longest key (nibbles) and value (bytes) staged since the last reset:
   // whether the hash pass orders leaves by Keccak block count
@@ -267,6 +268,7 @@ class Trie {
     DevBlock rw_flags, rw_a, rw_b, rw_c, rw_d, rw_e, rw_wpos;   // mixed read/write resolution
     DevBlock rw_hp, rw_len, rw_tot, rw_kept, rw_koff, rw_klen, rw_tid;
     DevBlock del_hslot, del_hext, del_stamp;                    // deletes: how each path branch is linked
+    DevBlock ready;                                             // branches ready to be hashed
     DevBlock pack;                                              // a small host batch, or lookups
     DevBlock misc;
   } ws_;
@@ -322,7 +324,9 @@ class Trie {
   // mixed batch: keep only the m kept writes' key bytes in the arena
   int compact_rw_keys(int m, const uint32_t *kept, uint64_t *koff, const uint32_t *klen, uint64_t key_base);
   int bucket_and_hash();
-  int hash_by_grid(uint32_t nd);
+  int begin_hash_timing();
+  int end_hash_timing();
+  int launch_hash_grid(const uint32_t *refs, uint32_t nd);
   int end_hash(uint32_t nd);
   int grid_limits();
   int block_grid() const;

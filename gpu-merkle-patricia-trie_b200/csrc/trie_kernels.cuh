@@ -1466,6 +1466,48 @@ struct BranchWriter {
   }
 };
 
+// Message of any branch, block by block: its items one after another (values
+// of up to kilobytes, children below 32 bytes).
+template <bool kCoh>
+struct ItemWriter {
+  WordWriter o;
+  EncItem cur;
+  uint32_t item = 0, off = 0;  // item 0: the list header, then the 17 slots
+  bool pre = true, done = false;
+  __device__ __forceinline__ ItemWriter(uint32_t *st, uint32_t stride, uint64_t hdr, uint32_t hn)
+      : o(st, stride), cur{hdr, hn, 0, nullptr, 0} {}
+  __device__ __forceinline__ bool fill(const TrieView &tv, const uint32_t *chp) {
+    while (o.w < 34 && !done) {
+      if (pre) {
+        pre = false;
+        o.bytes8(cur.pre, cur.pren);
+      } else if (off < cur.blen) {
+        const uint32_t n = min(cur.blen - off, 32u);
+        write_body<kCoh>(o, cur.body + off, n);
+        off += n;
+      } else if (++item <= 17) {
+        cur = child_item<kCoh>(tv, ldn<kCoh>(chp + item - 1));
+        off = 0;
+        pre = true;
+      } else {
+        o.bytes(0x01u, 1);
+        o.bytes(0u, o.pb ? 4 - o.pb : 0u);
+        done = true;
+      }
+    }
+    const bool last = done && o.w <= 34;
+    if (last) {
+      for (uint32_t w = o.w; w < 34; ++w) o.st[w * o.stride] = 0;
+      o.st[33 * o.stride] |= 0x80000000u;
+    }
+    return last;
+  }
+  __device__ __forceinline__ void next() {
+    for (uint32_t w = 34; w < o.w; ++w) o.st[(w - 34) * o.stride] = o.st[w * o.stride];
+    o.w -= 34;
+  }
+};
+
 // Encode + hash one dirty node; `stage` is this thread's column of the
 // message block in shared memory (kStageWords 32-bit words, word w at
 // stage[w * stride]).
