@@ -14,45 +14,56 @@
 namespace gmpt {
 
 constexpr int kLocalCap = 2048;     // items per segment
-constexpr int kLocalThreads = 256;  // items [tid*8, tid*8+8) per thread
-constexpr int kLocalIpt = kLocalCap / kLocalThreads;
-constexpr int kLocalSegs = kLocalCap / 2;  // a segment has >= 2 items
+constexpr int kLocalThreads = 256;
+// Segments of at most kLocalSmallCap items (the usual end of a build of
+// random keys: 2^20 keys leave 4096 segments of 256) run in CTAs of two warps,
+// whose barriers are cheap and of which many fit an SM.
+constexpr int kLocalSmallCap = 512, kLocalSmallThreads = 64;
+constexpr int kLocalIptMax = 8;
+static_assert(kLocalCap == kLocalIptMax * kLocalThreads && kLocalSmallCap == kLocalIptMax * kLocalSmallThreads, "");
 // resident CTAs per SM the register allocation is bounded for
 #ifndef GMPT_LOCAL_BUILD_CTAS
 #define GMPT_LOCAL_BUILD_CTAS 4
 #endif
 
+template <int kCap>
 struct LocalSegs {
-  uint64_t slot[kLocalSegs];  // where the segment's top node is linked
-  uint32_t D[kLocalSegs];     // branch depth (min interior LCP)
-  uint32_t branch[kLocalSegs];
-  uint16_t start[kLocalSegs];
-  uint16_t end[kLocalSegs];
-  uint16_t depth[kLocalSegs];
+  uint64_t slot[kCap / 2];  // where the segment's top node is linked (a segment has >= 2 items)
+  uint32_t D[kCap / 2];     // branch depth (min interior LCP)
+  uint32_t branch[kCap / 2];
+  uint16_t start[kCap / 2];
+  uint16_t end[kCap / 2];
+  uint16_t depth[kCap / 2];
 };
 
+template <int kCap, int kThreads>
 struct LocalSmem {
-  LocalSegs s[2];
-  uint16_t lcp[kLocalCap + 1];
-  uint16_t seg[kLocalCap];  // segment of each item at this level, 0xFFFF = done
-  uint32_t warp_sums[kLocalThreads / 32 + 1];
+  LocalSegs<kCap> s[2];
+  uint16_t lcp[kCap + 1];
+  uint16_t seg[kCap];  // segment of each item at this level, 0xFFFF = done
+  uint32_t warp_sums[kThreads / 32 + 1];
   uint32_t nseg;
   uint32_t leaf_base, dirty_base, leaf_ok;  // this level's leaf short nodes
 };
 
-__global__ void __launch_bounds__(kLocalThreads, GMPT_LOCAL_BUILD_CTAS) k_local_build(TrieView tv, DirtyList dl, SortedItems si,
-                                                               SegArrays gs, uint32_t gen) {
+// Thread t holds the items [t * ipt, t * ipt + ipt), ipt = the fewest that
+// cover the segment, so a short segment still uses every thread.
+template <int kCap, int kThreads>
+__global__ void __launch_bounds__(kThreads, GMPT_LOCAL_BUILD_CTAS * kLocalThreads / kThreads)
+k_local_build(TrieView tv, DirtyList dl, SortedItems si, SegArrays gs, uint32_t gen) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  LocalSmem &L = *reinterpret_cast<LocalSmem *>(smem_raw);
+  using Smem = LocalSmem<kCap, kThreads>;
+  Smem &L = *reinterpret_cast<Smem *>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const uint32_t gseg = blockIdx.x;
   const uint32_t base = gs.start[gseg];
   const int m = (int)(gs.end[gseg] - base);
-  if (m > kLocalCap || m < 2) {  // the host launches only 2 <= m <= cap
+  if (m > kCap || m < 2) {  // the host launches only 2 <= m <= cap
     if (tid == 0) set_error(tv.ctr, ERR_INTERNAL);
     return;
   }
-  for (int k = tid; k < m; k += kLocalThreads) {
+  const int ipt = (m + kThreads - 1) / kThreads;
+  for (int k = tid; k < m; k += kThreads) {
     L.lcp[k] = k == 0 ? kLcpInf : si.lcp[base + k];
     L.seg[k] = 0;
   }
@@ -69,18 +80,18 @@ __global__ void __launch_bounds__(kLocalThreads, GMPT_LOCAL_BUILD_CTAS) k_local_
   for (int level = 0; level < kMaxKeyNibbles + 2; ++level) {
     const uint32_t nseg = L.nseg;
     if (nseg == 0) break;
-    LocalSegs &S = L.s[cur];
-    LocalSegs &N = L.s[cur ^ 1];
-    for (uint32_t q = tid; q < nseg; q += kLocalThreads) S.D[q] = 0xFFFFFFFFu;
+    LocalSegs<kCap> &S = L.s[cur];
+    LocalSegs<kCap> &N = L.s[cur ^ 1];
+    for (uint32_t q = tid; q < nseg; q += kThreads) S.D[q] = 0xFFFFFFFFu;
     __syncthreads();
     // 1. D = min LCP over each segment's interior boundaries
-    for (int k = tid; k < m; k += kLocalThreads) {
+    for (int k = tid; k < m; k += kThreads) {
       uint16_t q = L.seg[k];
       if (q != 0xFFFF && k != S.start[q]) atomicMin(&S.D[q], (uint32_t)L.lcp[k]);
     }
     __syncthreads();
     // 2. one branch (+ extension above it) per segment
-    for (uint32_t q = tid; q < nseg; q += kLocalThreads) {
+    for (uint32_t q = tid; q < nseg; q += kThreads) {
       uint32_t D = S.D[q], d = S.depth[q];
       uint32_t i0 = base + S.start[q];
       uint32_t f = 0xFFFFFFFFu;
@@ -103,17 +114,17 @@ __global__ void __launch_bounds__(kLocalThreads, GMPT_LOCAL_BUILD_CTAS) k_local_
     // 3b, their short nodes allocated once for the whole CTA: one global
     // atomic per level instead of one per warp); count next-level segment
     // starts and leaves
-    uint8_t fl[kLocalIpt];
-    uint8_t nb[kLocalIpt];
-    uint16_t lq[kLocalIpt];
+    uint8_t fl[kLocalIptMax];
+    uint8_t nb[kLocalIptMax];
+    uint16_t lq[kLocalIptMax];
     uint32_t leafbits = 0, my_starts = 0, my_leaves = 0;
 #pragma unroll
-    for (int r = 0; r < kLocalIpt; ++r) {
-      const int k = tid * kLocalIpt + r;
+    for (int r = 0; r < kLocalIptMax; ++r) {
+      const int k = tid * ipt + r;
       fl[r] = 0;
       nb[r] = 0;
       lq[r] = 0;
-      if (k >= m) continue;
+      if (r >= ipt || k >= m) continue;
       const uint16_t q = L.seg[k];
       if (q == 0xFFFF) continue;
       const uint32_t D = S.D[q], f = S.branch[q];
@@ -147,12 +158,12 @@ __global__ void __launch_bounds__(kLocalThreads, GMPT_LOCAL_BUILD_CTAS) k_local_
     __syncthreads();
     if (tid == 0) {
       uint32_t run = 0;
-      for (int w = 0; w < kLocalThreads / 32; ++w) {
+      for (int w = 0; w < kThreads / 32; ++w) {
         uint32_t c = L.warp_sums[w];
         L.warp_sums[w] = run;
         run += c;
       }
-      L.warp_sums[kLocalThreads / 32] = run & 0xFFFFu;
+      L.warp_sums[kThreads / 32] = run & 0xFFFFu;
       const uint32_t tl = run >> 16;
       L.leaf_ok = 1;
       if (tl) {
@@ -172,9 +183,9 @@ __global__ void __launch_bounds__(kLocalThreads, GMPT_LOCAL_BUILD_CTAS) k_local_
     uint32_t run = before & 0xFFFFu;  // starts before this thread
     uint32_t lb = before >> 16;       // leaf short nodes before this thread
 #pragma unroll
-    for (int r = 0; r < kLocalIpt; ++r) {
+    for (int r = 0; r < kLocalIptMax; ++r) {
       if (!((leafbits >> r) & 1u)) continue;
-      const uint32_t q = lq[r], i = base + tid * kLocalIpt + r;
+      const uint32_t q = lq[r], i = base + tid * ipt + r;
       const uint32_t x = S.D[q] + 1, len = si.len[i];
       const uint64_t slot = ((uint64_t)S.branch[q] << 5) | nb[r];
       if (x >= len) {
@@ -198,8 +209,8 @@ __global__ void __launch_bounds__(kLocalThreads, GMPT_LOCAL_BUILD_CTAS) k_local_
       write_slot(tv, slot, ref);
     }
 #pragma unroll
-    for (int r = 0; r < kLocalIpt; ++r) {
-      const int k = tid * kLocalIpt + r;
+    for (int r = 0; r < kLocalIptMax; ++r) {
+      const int k = tid * ipt + r;
       if (!(fl[r] & 1)) continue;
       const uint16_t q = L.seg[k];
       if (fl[r] & 2) {
@@ -214,7 +225,7 @@ __global__ void __launch_bounds__(kLocalThreads, GMPT_LOCAL_BUILD_CTAS) k_local_
       L.seg[k] = (uint16_t)id;
     }
     __syncthreads();
-    if (tid == 0) L.nseg = L.warp_sums[kLocalThreads / 32];
+    if (tid == 0) L.nseg = L.warp_sums[kThreads / 32];
     __syncthreads();
     cur ^= 1;
   }

@@ -856,11 +856,13 @@ int Trie::build_levels(int T) {
     const uint32_t lcap = opt_local_build_cap_ > 0 ? (uint32_t)opt_local_build_cap_ : (uint32_t)kLocalCap;
     if (opt_local_build_ && maxseg <= lcap) {
       // every remaining segment fits one CTA: finish all subtries there
-      const size_t smem = sizeof(LocalSmem);
-      if ((e = cudaFuncSetAttribute(k_local_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-          cudaSuccess)
+      const bool small = maxseg <= (uint32_t)kLocalSmallCap;
+      const size_t smem = small ? sizeof(LocalSmem<kLocalSmallCap, kLocalSmallThreads>)
+                                : sizeof(LocalSmem<kLocalCap, kLocalThreads>);
+      auto kern = small ? k_local_build<kLocalSmallCap, kLocalSmallThreads> : k_local_build<kLocalCap, kLocalThreads>;
+      if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
         return check_cuda(e, "local build attr");
-      count_launch(), k_local_build<<<S, kLocalThreads, smem, st_>>>(tv_, dl, si, sg[cur], gen_);
+      count_launch(), kern<<<S, small ? kLocalSmallThreads : kLocalThreads, smem, st_>>>(tv_, dl, si, sg[cur], gen_);
       if ((e = cudaGetLastError()) != cudaSuccess) return check_cuda(e, "local build");
       break;
     }
