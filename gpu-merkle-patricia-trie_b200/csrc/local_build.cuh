@@ -48,7 +48,7 @@ struct LocalSmem {
 
 // Thread t holds the items [t * ipt, t * ipt + ipt), ipt = the fewest that
 // cover the segment, so a short segment still uses every thread.
-template <int kCap, int kThreads>
+template <int kMin, int kCap, int kThreads>
 __global__ void __launch_bounds__(kThreads, GMPT_LOCAL_BUILD_CTAS * kLocalThreads / kThreads)
 k_local_build(TrieView tv, DirtyList dl, SortedItems si, SegArrays gs, uint32_t gen) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -58,10 +58,7 @@ k_local_build(TrieView tv, DirtyList dl, SortedItems si, SegArrays gs, uint32_t 
   const uint32_t gseg = blockIdx.x;
   const uint32_t base = gs.start[gseg];
   const int m = (int)(gs.end[gseg] - base);
-  if (m > kCap || m < 2) {  // the host launches only 2 <= m <= cap
-    if (tid == 0) set_error(tv.ctr, ERR_INTERNAL);
-    return;
-  }
+  if (m > kCap || m <= kMin) return;  // another launch's
   const int ipt = (m + kThreads - 1) / kThreads;
   for (int k = tid; k < m; k += kThreads) {
     L.lcp[k] = k == 0 ? kLcpInf : si.lcp[base + k];

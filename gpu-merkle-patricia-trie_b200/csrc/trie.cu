@@ -547,11 +547,20 @@ int Trie::sort_batch(int n, const uint64_t *koff, const uint32_t *klen, uint32_t
       uint32_t maxrun = (uint32_t)(h_small_[0] & 0xFFFFFFFFu);
       const uint32_t cap = opt_local_sort_cap_ > 0 ? (uint32_t)opt_local_sort_cap_ : (uint32_t)kSortLocalCap;
       if (maxrun <= cap) {
-        const size_t smem = sizeof(LocalSortSmem);
-        if ((e = cudaFuncSetAttribute(k_local_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-            cudaSuccess)
-          return check_cuda(e, "local sort attr");
-        count_launch(), k_local_sort<<<S, kSortLocalThreads, smem, st_>>>(tv_, rs, re, c, order, eqprev, koff, klen);
+        count_launch(), k_local_sort_warp<<<blocks_for(32 * (int64_t)S), kThreads, 0, st_>>>(tv_, rs, re, S, c, order,
+                                                                                             eqprev, koff, klen);
+        if (maxrun > (uint32_t)kSortWarpCap) {
+          auto kern = k_local_sort<kSortWarpCap, kSortSmallCap, kSortSmallThreads>;
+          const size_t smem = sizeof(LocalSortSmem<kSortSmallCap, kSortSmallThreads>);
+          count_launch(), kern<<<S, kSortSmallThreads, smem, st_>>>(tv_, rs, re, c, order, eqprev, koff, klen);
+        }
+        if (maxrun > (uint32_t)kSortSmallCap) {
+          auto kern = k_local_sort<kSortSmallCap, kSortLocalCap, kSortLocalThreads>;
+          const size_t smem = sizeof(LocalSortSmem<kSortLocalCap, kSortLocalThreads>);
+          if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+            return check_cuda(e, "local sort attr");
+          count_launch(), kern<<<S, kSortLocalThreads, smem, st_>>>(tv_, rs, re, c, order, eqprev, koff, klen);
+        }
         if ((e = cudaGetLastError()) != cudaSuccess) return check_cuda(e, "local sort");
         break;
       }
@@ -856,13 +865,17 @@ int Trie::build_levels(int T) {
     const uint32_t lcap = opt_local_build_cap_ > 0 ? (uint32_t)opt_local_build_cap_ : (uint32_t)kLocalCap;
     if (opt_local_build_ && maxseg <= lcap) {
       // every remaining segment fits one CTA: finish all subtries there
-      const bool small = maxseg <= (uint32_t)kLocalSmallCap;
-      const size_t smem = small ? sizeof(LocalSmem<kLocalSmallCap, kLocalSmallThreads>)
-                                : sizeof(LocalSmem<kLocalCap, kLocalThreads>);
-      auto kern = small ? k_local_build<kLocalSmallCap, kLocalSmallThreads> : k_local_build<kLocalCap, kLocalThreads>;
-      if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-        return check_cuda(e, "local build attr");
-      count_launch(), kern<<<S, small ? kLocalSmallThreads : kLocalThreads, smem, st_>>>(tv_, dl, si, sg[cur], gen_);
+      // (segments of the other launch's sizes leave at once)
+      auto small = k_local_build<1, kLocalSmallCap, kLocalSmallThreads>;
+      count_launch(), small<<<S, kLocalSmallThreads, sizeof(LocalSmem<kLocalSmallCap, kLocalSmallThreads>), st_>>>(
+                          tv_, dl, si, sg[cur], gen_);
+      if (maxseg > (uint32_t)kLocalSmallCap) {
+        auto kern = k_local_build<kLocalSmallCap, kLocalCap, kLocalThreads>;
+        const size_t smem = sizeof(LocalSmem<kLocalCap, kLocalThreads>);
+        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+          return check_cuda(e, "local build attr");
+        count_launch(), kern<<<S, kLocalThreads, smem, st_>>>(tv_, dl, si, sg[cur], gen_);
+      }
       if ((e = cudaGetLastError()) != cudaSuccess) return check_cuda(e, "local build");
       break;
     }
