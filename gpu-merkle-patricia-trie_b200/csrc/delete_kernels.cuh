@@ -86,31 +86,20 @@ __global__ void k_del_walk(TrieView tv, DirtyList dl, const uint8_t *keys, const
   }
 }
 
-// Key bytes the collapses of one level will append (same rule as below).
-__global__ void k_del_need(TrieView tv, const uint32_t *refs, int count, const uint32_t *hext, const uint8_t *stamp,
-                           unsigned long long *need) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t total = 0;
-  if (j < count && ref_kind(refs[j]) == KIND_FULL && stamp[ref_idx(refs[j])]) {
-    const uint32_t id = ref_idx(refs[j]);
-    const uint32_t *ch = tv.full_child + (size_t)id * 17;
-    uint32_t cnt = 0, c1 = 0, r1 = 0;
-    for (uint32_t k = 0; k < 17; ++k) {
-      const uint32_t v = ch[k];
-      if (v) {
-        ++cnt;
-        c1 = k;
-        r1 = v;
-      }
-    }
-    if (cnt == 1) {
-      const uint32_t e = hext[id];
-      total = 1u + (e != kNoExt ? tv.short_klen[e] : 0u) +
-              ((c1 < 16 && ref_kind(r1) == KIND_SHORT) ? tv.short_klen[ref_idx(r1)] : 0u);
-    }
+// Eight key bytes from byte j of a merged key: [extension key e, le nibbles]
+// [c1][child's key k, ls nibbles]; bytes past the end are zero.
+__device__ __forceinline__ uint64_t merged_key8(const uint8_t *e, uint32_t le, uint32_t c1, const uint8_t *k,
+                                                uint32_t ls, uint32_t j) {
+  uint64_t v = 0;
+  if (j < le) v = load_u64_unaligned(e + j) & low_mask64((int)min(8u, le - j));
+  if (le >= j && le - j < 8) v |= (uint64_t)c1 << (8 * (le - j));
+  const uint32_t at = le + 1;  // first nibble of the child's key
+  if (j >= at) {
+    if (j - at < ls) v = load_u64_unaligned(k + (j - at)) & low_mask64((int)min(8u, ls - (j - at)));
+  } else if (at - j < 8 && ls > 0) {
+    v |= (load_u64_unaligned(k) & low_mask64((int)min(8u - (at - j), ls))) << (8 * (at - j));
   }
-  const unsigned long long w = __reduce_add_sync(0xffffffffu, total);
-  if ((threadIdx.x & 31) == 0 && w) atomicAdd(need, w);
+  return v;
 }
 
 __global__ void k_del_collapse(TrieView tv, DirtyList dl, const uint32_t *refs, int count, const uint64_t *hslot,
@@ -155,16 +144,18 @@ __global__ void k_del_collapse(TrieView tv, DirtyList dl, const uint32_t *refs, 
     child = tv.short_child[s];
     tv.short_dead[s] = 1;
   }
-  const uint32_t total = le + 1u + ls;
-  const unsigned long long off = atomicAdd(key_cursor, (unsigned long long)total);
-  if (off + total > key_cap) {
+  // the merged key goes to a whole number of aligned words (the host has made
+  // room for the longest key per collapse); the keys read lie below the
+  // cursor or were written by an earlier launch
+  const uint32_t total = le + 1u + ls, room = (total + 7u) & ~7u;
+  const unsigned long long off = atomicAdd(key_cursor, (unsigned long long)room);
+  if (off + room > key_cap) {
     set_error(tv.ctr, ERR_CAPACITY);
     return;
   }
-  uint8_t *dst = const_cast<uint8_t *>(tv.keys) + off;
-  for (uint32_t k = 0; k < le; ++k) dst[k] = tv.keys[oe + k];
-  dst[le] = (uint8_t)c1;
-  for (uint32_t k = 0; k < ls; ++k) dst[le + 1 + k] = tv.keys[os + k];
+  uint64_t *dst = reinterpret_cast<uint64_t *>(const_cast<uint8_t *>(tv.keys) + off);
+  for (uint32_t w = 0; 8 * w < total; ++w)
+    dst[w] = merged_key8(tv.keys + oe, le, c1, tv.keys + os, ls, 8 * w);
   if (e != kNoExt) {  // the extension above takes the merged key (it is dirty: on the path)
     tv.short_key[e] = off;
     tv.short_klen[e] = total;
@@ -174,6 +165,12 @@ __global__ void k_del_collapse(TrieView tv, DirtyList dl, const uint32_t *refs, 
     if (ns == 0xFFFFFFFFu) return;
     write_slot(tv, hs, make_ref(KIND_SHORT, ns));
   }
+}
+
+// The cursor once every level is collapsed, and 64 zero bytes behind it.
+__global__ void k_del_tail(uint8_t *keys, const unsigned long long *key_cursor, uint64_t key_cap) {
+  const unsigned long long at = *key_cursor + threadIdx.x;
+  if (at < key_cap) keys[at] = 0;
 }
 
 }  // namespace gmpt

@@ -132,7 +132,7 @@ Trie::~Trie() {
                         &ws_.flags, &ws_.pos, &ws_.act, &ws_.skey, &ws_.sval, &ws_.uord, &ws_.w_status,
                         &ws_.w_code, &ws_.w_d0, &ws_.w_slot, &ws_.w_short, &ws_.w_after, &ws_.p_short,
                         &ws_.p_d0, &ws_.p_slot, &ws_.p_amin, &ws_.p_max, &ws_.it_key, &ws_.it_id,
-                        &ws_.it_base, &ws_.it_len, &ws_.it_ref, &ws_.it_d0, &ws_.it_slot, &ws_.sb_base,
+                        &ws_.it_base, &ws_.it_len, &ws_.it_ref, &ws_.it_d0, &ws_.it_slot, &ws_.it_code, &ws_.sb_base,
                         &ws_.sb_len, &ws_.sb_ref, &ws_.sb_d0, &ws_.sb_slot, &ws_.sb_code, &ws_.lcp,
                         &ws_.act2, &ws_.aseg, &ws_.aseg2, &ws_.kflags, &ws_.knib, &ws_.bins, &ws_.cursor,
                         &ws_.sorted_dirty, &ws_.g_keys, &ws_.g_idx, &ws_.g_hp, &ws_.g_len, &ws_.g_tid,
@@ -975,50 +975,68 @@ int Trie::put_2phase(const BatchIn &b) {
   wo.p_max = wsp<uint32_t>(ws_.p_max, (size_t)m, e);
   unsigned long long *flags = wsp<unsigned long long>(ws_.flags, (size_t)m, e);
   unsigned long long *pos = wsp<unsigned long long>(ws_.pos, (size_t)m, e);
-  unsigned long long *d_tot = wsp<unsigned long long>(ws_.misc, 16, e) + 2;
+  unsigned long long *d_tot = wsp<unsigned long long>(ws_.misc, 16, e) + 2;  // [0] items, [1] runs of split groups
+  uint32_t *before = wsp<uint32_t>(ws_.act, (size_t)m, e), *after = wsp<uint32_t>(ws_.act2, (size_t)m, e);
+  // every key may bring a pseudo item
+  auto items = [&](DevBlock &base, DevBlock &len, DevBlock &ref, DevBlock &d0, DevBlock &slot, DevBlock &code, size_t c) {
+    ItemArrays it;
+    it.base = wsp<uint64_t>(base, c, e);
+    it.len = wsp<uint32_t>(len, c, e);
+    it.ref = wsp<uint32_t>(ref, c, e);
+    it.d0 = wsp<uint32_t>(d0, c, e);
+    it.slot = wsp<uint64_t>(slot, c, e);
+    it.code = wsp<uint64_t>(code, c, e);
+    return it;
+  };
+  ItemArrays sb = items(ws_.sb_base, ws_.sb_len, ws_.sb_ref, ws_.sb_d0, ws_.sb_slot, ws_.sb_code, 2 * (size_t)m);
+  if (e == cudaSuccess) e = scan_ws_.ensure(scan_ws_bytes<unsigned long long>(m));
   if (e == cudaSuccess) e = cudaMemsetAsync(&ctr_->n_pseudo, 0, 4, st_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(before, 0, 4 * (size_t)m, st_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(after, 0, 4 * (size_t)m, st_);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_tot, 0, 16, st_);
   if (e != cudaSuccess) return check_cuda(e, "walk alloc");
   DirtyList dl{dirty_ref_, dirty_depth_};
   count_launch(), k_walk<<<blocks_for((m + kWalkWays - 1) / kWalkWays), kThreads, 0, st_>>>(tv_, dl, uord, m, koff,
                                                                                              klen, vid_base, wo, tid);
   count_launch(), k_pseudo_ranks<<<blocks_for(m), kThreads, 0, st_>>>(tv_, wo, m);
-  count_launch(), k_new_flags<<<blocks_for(m), kThreads, 0, st_>>>(wo.status, m, flags);
+  count_launch(), k_pseudo_place<<<blocks_for(m), kThreads, 0, st_>>>(tv_, wo, m, before, after);
+  count_launch(), k_item_counts<<<blocks_for(m), kThreads, 0, st_>>>(wo.status, before, after, m, flags);
   e = exclusive_scan<unsigned long long>(flags, pos, m, d_tot, scan_ws_, st_);
   if (e != cudaSuccess) return check_cuda(e, "walk scan");
+  count_launch(), k_items_place<<<blocks_for(m), kThreads, 0, st_>>>(tv_, wo, before, after, pos, m, uord, koff, klen,
+                                                                     vid_base, sb);
+  count_launch(), k_item_runs<<<std::min<unsigned>(blocks_for(m), 148 * 4), kThreads, 0, st_>>>(sb.code, d_tot, d_tot + 1);
+  if ((e = cudaMemcpyAsync(h_small_, d_tot, 16, cudaMemcpyDeviceToHost, st_)) != cudaSuccess)
+    return check_cuda(e, "walk items");
   if ((rc = sync_counters())) return rc;
-  uint32_t n_pseudo = h_ctr_->n_pseudo;
-  int n_new = (int)(read_u64(d_tot) & 0xFFFFFFFFu);
-  stats_.last_new = (uint64_t)n_new;
+  const uint32_t n_pseudo = h_ctr_->n_pseudo;
+  const int T = (int)h_small_[0];
+  const bool grouped = h_small_[1] == n_pseudo;
+  stats_.last_new = (uint64_t)T - n_pseudo;
   stats_.last_pseudo = n_pseudo;
   if (timing_) cudaEventRecord(ev[3], st_);
-  int T = n_new + (int)n_pseudo;
   if (T > 0) {
-    Items it;
-    it.key = wsp<uint64_t>(ws_.it_key, (size_t)T, e);
-    it.id = wsp<uint32_t>(ws_.it_id, (size_t)T, e);
-    it.base = wsp<uint64_t>(ws_.it_base, (size_t)T, e);
-    it.len = wsp<uint32_t>(ws_.it_len, (size_t)T, e);
-    it.ref = wsp<uint32_t>(ws_.it_ref, (size_t)T, e);
-    it.d0 = wsp<uint32_t>(ws_.it_d0, (size_t)T, e);
-    it.slot = wsp<uint64_t>(ws_.it_slot, (size_t)T, e);
-    uint64_t *sb_base = wsp<uint64_t>(ws_.sb_base, (size_t)T, e);
-    uint32_t *sb_len = wsp<uint32_t>(ws_.sb_len, (size_t)T, e);
-    uint32_t *sb_ref = wsp<uint32_t>(ws_.sb_ref, (size_t)T, e);
-    uint32_t *sb_d0 = wsp<uint32_t>(ws_.sb_d0, (size_t)T, e);
-    uint64_t *sb_slot = wsp<uint64_t>(ws_.sb_slot, (size_t)T, e);
-    uint64_t *sb_code = wsp<uint64_t>(ws_.sb_code, (size_t)T, e);
+    if (!grouped) {
+      uint64_t *key = wsp<uint64_t>(ws_.it_key, (size_t)T, e);
+      uint32_t *id = wsp<uint32_t>(ws_.it_id, (size_t)T, e);
+      ItemArrays it = items(ws_.it_base, ws_.it_len, ws_.it_ref, ws_.it_d0, ws_.it_slot, ws_.it_code, (size_t)T);
+      if (e != cudaSuccess) return check_cuda(e, "items alloc");
+      count_launch(), k_item_keys<<<blocks_for(T), kThreads, 0, st_>>>(sb.code, T, key, id);
+      int passes = 0;
+      if ((e = sorter_.sort(key, id, T, st_, &passes)) != cudaSuccess) return check_cuda(e, "group sort");
+      count_launch(), k_items_gather<<<blocks_for(T), kThreads, 0, st_>>>(sb, id, T, it);
+      // the build reads the items from the sb_* blocks
+      std::swap(ws_.sb_base, ws_.it_base);
+      std::swap(ws_.sb_len, ws_.it_len);
+      std::swap(ws_.sb_ref, ws_.it_ref);
+      std::swap(ws_.sb_d0, ws_.it_d0);
+      std::swap(ws_.sb_slot, ws_.it_slot);
+      std::swap(ws_.sb_code, ws_.it_code);
+      sb = it;
+    }
     uint16_t *lcp = wsp<uint16_t>(ws_.lcp, (size_t)T + 1, e);
     if (e != cudaSuccess) return check_cuda(e, "items alloc");
-    if (n_new > 0)
-      count_launch(), k_items_new<<<blocks_for(m), kThreads, 0, st_>>>(tv_, wo, pos, m, uord, koff, klen, vid_base, it);
-    if (n_pseudo > 0) {
-      count_launch(), k_items_pseudo<<<blocks_for(n_pseudo), kThreads, 0, st_>>>(tv_, wo, (int)n_pseudo, n_new, it);
-      int passes = 0;
-      if ((e = sorter_.sort(it.key, it.id, T, st_, &passes)) != cudaSuccess) return check_cuda(e, "group sort");
-    }
-    count_launch(), k_items_gather<<<blocks_for(T), kThreads, 0, st_>>>(it, n_pseudo > 0 ? it.id : nullptr, T, sb_base, sb_len,
-                                                        sb_ref, sb_d0, sb_slot, sb_code);
-    count_launch(), k_items_lcp<<<blocks_for(T), kThreads, 0, st_>>>(tv_, sb_base, sb_len, sb_d0, sb_code, T, lcp);
+    count_launch(), k_items_lcp<<<blocks_for(T), kThreads, 0, st_>>>(tv_, sb.base, sb.len, sb.d0, sb.code, T, lcp);
     if ((rc = build_levels(T))) return rc;
   }
   }
@@ -2390,64 +2408,62 @@ int Trie::del(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool devi
     keys_bytes = (int64_t)keys_indexs[2 * n - 1] + 1;
   }
   if (keys_bytes < 0) return fail(E_ARG, "bad index pairs");
-  int rc = sync_counters();
-  if (rc) return rc;
+  int rc = OK;  // the node counts are as of the last call
   const cudaMemcpyKind kind = device_inputs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   uint8_t *dk = wsp<uint8_t>(ws_.g_keys, (size_t)keys_bytes + 64, e);
-  int *di = wsp<int>(ws_.g_idx, 2 * (size_t)n, e);
-  int *dtid = trie_ids ? wsp<int>(ws_.g_tid, (size_t)n, e) : nullptr;
+  // index pairs and trie ids of device batches are read where they lie
+  const bool di_here = device_inputs && reinterpret_cast<uintptr_t>(keys_indexs) % alignof(int) == 0;
+  const bool tid_here = device_inputs && reinterpret_cast<uintptr_t>(trie_ids) % alignof(int) == 0;
+  int *di = di_here ? nullptr : wsp<int>(ws_.g_idx, 2 * (size_t)n, e);
+  int *dtid = trie_ids && !tid_here ? wsp<int>(ws_.g_tid, (size_t)n, e) : nullptr;
   const size_t nf = (size_t)n_full_ + 1;
   uint64_t *hslot = wsp<uint64_t>(ws_.del_hslot, nf, e);
   uint32_t *hext = wsp<uint32_t>(ws_.del_hext, nf, e);
   uint8_t *stamp = wsp<uint8_t>(ws_.del_stamp, nf, e);
-  unsigned long long *dcnt = wsp<unsigned long long>(ws_.rw_tot, 8, e);  // [0] need, [1] key cursor
+  unsigned long long *dcnt = wsp<unsigned long long>(ws_.rw_tot, 8, e);  // key cursor
   if (e == cudaSuccess) e = cudaMemcpyAsync(dk, keys_hexs, (size_t)keys_bytes, kind, st_);
   if (e == cudaSuccess) e = cudaMemsetAsync(dk + keys_bytes, 0, 64, st_);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(di, keys_indexs, sizeof(int) * 2 * (size_t)n, kind, st_);
+  if (e == cudaSuccess && di) e = cudaMemcpyAsync(di, keys_indexs, sizeof(int) * 2 * (size_t)n, kind, st_);
   if (e == cudaSuccess && dtid) e = cudaMemcpyAsync(dtid, trie_ids, sizeof(int) * (size_t)n, kind, st_);
   if (e == cudaSuccess) e = cudaMemsetAsync(stamp, 0, nf, st_);
   if (e != cudaSuccess) return check_cuda(e, "delete copy");
   DirtyList dl{dirty_ref_, dirty_depth_};
-  count_launch(), k_del_walk<<<blocks_for(n), kThreads, 0, st_>>>(tv_, dl, dk, di, n, keys_bytes, dtid, hslot, hext,
-                                                                  stamp);
+  count_launch(), k_del_walk<<<blocks_for(n), kThreads, 0, st_>>>(tv_, dl, dk, di ? di : keys_indexs, n, keys_bytes,
+                                                                  dtid ? dtid : trie_ids, hslot, hext, stamp);
   if ((rc = sync_counters())) return rc;
   const uint32_t nd = h_ctr_->n_dirty;
   if (nd == 0) return OK;
   uint32_t *sorted = nullptr;
   std::vector<uint32_t> off;
   if ((rc = bucket_dirty(nd, &sorted, off))) return rc;
+  // Room for every level at once, so no level waits for the host: a branch
+  // collapses after at least one delete below it, into a key no longer than
+  // the longest, and makes at most one short node.
+  uint64_t branches = 0;
+  for (uint32_t d = 0; d < dirty_depths(); ++d) branches += off[level_bin(d) + kHashClasses] - off[level_bin(d)];
+  const uint64_t collapses = std::min<uint64_t>(branches, (uint64_t)n);
+  key_used_ = (key_used_ + 7) & ~7ull;
+  if ((rc = ensure_capacity(0, collapses, 0, 0, collapses * ((depth_bound_ + 8ull) & ~7ull) + 64, 0))) return rc;
+  dl = DirtyList{dirty_ref_, dirty_depth_};  // the list may have grown with the short pool
+  h_small_[0] = key_used_;
+  if ((e = cudaMemcpyAsync(dcnt, h_small_, 8, cudaMemcpyHostToDevice, st_)) != cudaSuccess)
+    return check_cuda(e, "delete cursor");
   for (int d = (int)dirty_depths() - 1; d >= 0; --d) {
     const uint32_t a = off[level_bin(d)], z = off[level_bin(d) + kHashClasses];  // branches at depth d
     if (z == a) continue;
-    const int cnt = (int)(z - a);
-    // room for this level's new keys and short nodes, then collapse
-    if ((e = cudaMemsetAsync(dcnt, 0, 8, st_)) != cudaSuccess) return check_cuda(e, "delete need");
-    count_launch(), k_del_need<<<blocks_for(cnt), kThreads, 0, st_>>>(tv_, sorted + a, cnt, hext, stamp, dcnt);
-    if ((e = cudaMemcpyAsync(h_small_, dcnt, 8, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st_)) != cudaSuccess)
-      return check_cuda(e, "delete need");
-    const uint64_t need = h_small_[0];
-    if ((rc = sync_counters())) return rc;
-    if ((rc = ensure_capacity(0, (uint64_t)cnt, 0, 0, need + 64, 0))) return rc;
-    dl = DirtyList{dirty_ref_, dirty_depth_};  // the list may have grown with the short pool
-    h_small_[1] = key_used_;
-    if ((e = cudaMemcpyAsync(dcnt + 1, h_small_ + 1, 8, cudaMemcpyHostToDevice, st_)) != cudaSuccess)
-      return check_cuda(e, "delete cursor");
-    count_launch(), k_del_collapse<<<blocks_for(cnt), kThreads, 0, st_>>>(tv_, dl, sorted + a, cnt, hslot, hext, stamp,
-                                                                          dcnt + 1, cap_keys_);
-    if ((e = cudaMemcpyAsync(h_small_, dcnt + 1, 8, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st_)) != cudaSuccess)
-      return check_cuda(e, "delete collapse");
-    const uint64_t cursor = h_small_[0];
-    // k_del_collapse advances the cursor even when a level's key bytes did
-    // not fit (it then raises ERR_CAPACITY): check before the arena is touched
-    if ((rc = sync_counters())) return rc;
-    if (cursor + 64 > cap_keys_) return fail(E_CAPACITY, "key arena capacity exceeded by a delete collapse");
-    key_used_ = (cursor + 7) & ~7ull;
-    if ((e = cudaMemsetAsync(const_cast<uint8_t *>(tv_.keys) + cursor, 0, 64, st_)) != cudaSuccess)
-      return check_cuda(e, "delete tail");
+    count_launch(), k_del_collapse<<<blocks_for(z - a), kThreads, 0, st_>>>(tv_, dl, sorted + a, (int)(z - a), hslot,
+                                                                          hext, stamp, dcnt, cap_keys_);
   }
-  if ((rc = sync_counters())) return rc;
+  count_launch(), k_del_tail<<<1, 64, 0, st_>>>(const_cast<uint8_t *>(tv_.keys), dcnt, cap_keys_);
+  if ((e = cudaMemcpyAsync(h_small_, dcnt, 8, cudaMemcpyDeviceToHost, st_)) != cudaSuccess)
+    return check_cuda(e, "delete collapse");
+  if ((rc = copy_counters())) return rc;
+  const uint64_t cursor = h_small_[0];
+  // k_del_collapse advances the cursor even when its key bytes did not fit
+  // (it then raises ERR_CAPACITY): check before the arena is taken as used
+  if ((rc = apply_counters())) return rc;
+  if (cursor + 64 > cap_keys_) return fail(E_CAPACITY, "key arena capacity exceeded by a delete collapse");
+  key_used_ = cursor;
   stats_.key_bytes = key_used_;
   stats_.n_full = n_full_;
   stats_.n_short = n_short_;

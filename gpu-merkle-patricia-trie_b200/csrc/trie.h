@@ -255,7 +255,7 @@ class Trie {
     DevBlock order, eqprev, flags, pos, act, skey, sval, uord;  // sort / dedup
     DevBlock w_status, w_code, w_d0, w_slot, w_short, w_after;  // walk
     DevBlock p_short, p_d0, p_slot, p_amin, p_max;              // pseudo items
-    DevBlock it_key, it_id, it_base, it_len, it_ref, it_d0, it_slot;  // items
+    DevBlock it_key, it_id, it_base, it_len, it_ref, it_d0, it_slot, it_code;  // items
     DevBlock sb_base, sb_len, sb_ref, sb_d0, sb_slot, sb_code, lcp;   // sorted items
     DevBlock act2, aseg, aseg2, kflags, knib;                   // builder levels
     DevBlock s_start[2], s_end[2], s_depth[2], s_slot[2], s_D[2], s_branch[2];

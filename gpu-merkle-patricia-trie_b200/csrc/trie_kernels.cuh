@@ -9,7 +9,8 @@
 //                  the path dirty, overwrites values of keys that exist,
 //                  and finds where new keys attach (anchor)
 //   k_items_*      new keys + one "pseudo" item per short node that must be
-//                  split, grouped by anchor
+//                  split, in key order, which groups them by anchor (or
+//                  nearly: k_item_runs)
 //   k_level_*      level-synchronous construction of the compressed
 //                  subtries of every group (branch / extension / leaf)
 //   k_hash_level   fused RLP encode + Keccak-256 of every dirty node of one
@@ -682,13 +683,6 @@ __global__ void __launch_bounds__(256, 2) k_walk(TrieView tv, DirtyList dl, cons
   }
 }
 
-__global__ void k_new_flags(const uint8_t *status, int m, unsigned long long *flags) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= m) return;
-  uint8_t st = status[j];
-  flags[j] = (st == W_NEW || st == W_SPLIT) ? 1ull : 0ull;
-}
-
 __global__ void k_pseudo_ranks(TrieView tv, const WalkOut wo, int m) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= m) return;
@@ -698,60 +692,93 @@ __global__ void k_pseudo_ranks(TrieView tv, const WalkOut wo, int m) {
   atomicMax(&wo.p_max[p], (uint32_t)j);
 }
 
-struct Items {
-  uint64_t *key;
-  uint32_t *id;
-  uint64_t *base;
-  uint32_t *len;
-  uint32_t *ref;
-  uint32_t *d0;
-  uint64_t *slot;
-};
-
-// new keys (status NEW / SPLIT) -> items [0, n_new)
-__global__ void k_items_new(TrieView tv, const WalkOut wo, const unsigned long long *pos, int m,
-                            const uint32_t *uord, const uint64_t *koff, const uint32_t *klen, uint64_t vid_base,
-                            Items it) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= m) return;
-  uint8_t st = wo.status[j];
-  if (st != W_NEW && st != W_SPLIT) return;
-  uint32_t i = (uint32_t)pos[j];
-  uint32_t item = uord[j];
-  uint32_t v = warp_alloc(&tv.ctr->n_value, 1);
-  if (v >= tv.cap_value) {
-    set_error(tv.ctr, ERR_CAPACITY);
-    v = 0;
-  }
-  tv.value_vid[v] = vid_base + item;
-  it.key[i] = (wo.code[j] << 27) | (2ull * (uint64_t)j + 1ull);
-  it.id[i] = i;
-  it.base[i] = koff[item];
-  it.len[i] = klen[item];
-  it.ref[i] = make_ref(KIND_VALUE, v);
-  it.d0[i] = wo.d0[j];
-  it.slot[i] = wo.slot[j];
+// Where a pseudo item (a short node re-inserted as a key ending in its old
+// child) goes in key order: just before the first key that sorts after the
+// short node's key, else after the last diverger.  Both are divergers of that
+// short node alone, so a key has at most one pseudo item on either side.
+__global__ void k_pseudo_place(TrieView tv, const WalkOut wo, int m, uint32_t *before, uint32_t *after) {
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= min(tv.ctr->n_pseudo, (uint32_t)m)) return;
+  if (wo.p_amin[p] != 0xFFFFFFFFu)
+    before[wo.p_amin[p]] = p + 1;
+  else
+    after[wo.p_max[p]] = p + 1;
 }
 
-// pseudo items [n_new, n_new + n_pseudo): the existing short node re-inserted
-// as a key ending in its old child
-__global__ void k_items_pseudo(TrieView tv, const WalkOut wo, int n_pseudo, int n_new, Items it) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n_pseudo) return;
-  uint32_t s = wo.p_short[p];
-  uint32_t d0 = wo.p_d0[p];
-  uint32_t amin = wo.p_amin[p];
-  // real keys rank 2j+1; the pseudo item sits just before the first key
-  // that sorts after the short node's key, else after the last diverger
-  uint64_t rank = (amin != 0xFFFFFFFFu) ? (2ull * amin) : (2ull * wo.p_max[p] + 2ull);
-  uint32_t i = (uint32_t)n_new + (uint32_t)p;
-  it.key[i] = (code_short(s) << 27) | rank;
-  it.id[i] = i;
+// items at and around key j
+__global__ void k_item_counts(const uint8_t *status, const uint32_t *before, const uint32_t *after, int m,
+                              unsigned long long *flags) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= m) return;
+  const uint8_t st = status[j];
+  flags[j] = (st == W_NEW || st == W_SPLIT ? 1ull : 0ull) + (before[j] ? 1ull : 0ull) + (after[j] ? 1ull : 0ull);
+}
+
+// the items of a build: key ending in `ref`, anchored at `code` / `slot` from nibble d0 on
+struct ItemArrays {
+  uint64_t *base;
+  uint32_t *len, *ref, *d0;
+  uint64_t *slot, *code;
+};
+
+__device__ __forceinline__ void put_pseudo(const TrieView &tv, const WalkOut &wo, const ItemArrays &it, uint64_t i,
+                                           uint32_t p) {
+  const uint32_t s = wo.p_short[p], d0 = wo.p_d0[p];
   it.base[i] = tv.short_key[s] - d0;
   it.len[i] = d0 + tv.short_klen[s];
   it.ref[i] = tv.short_child[s];
   it.d0[i] = d0;
   it.slot[i] = wo.p_slot[p];
+  it.code[i] = code_short(s);
+}
+
+// new keys (status NEW / SPLIT) and pseudo items, in key order
+__global__ void k_items_place(TrieView tv, const WalkOut wo, const uint32_t *before, const uint32_t *after,
+                              const unsigned long long *pos, int m, const uint32_t *uord, const uint64_t *koff,
+                              const uint32_t *klen, uint64_t vid_base, ItemArrays it) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= m) return;
+  const uint8_t st = wo.status[j];
+  uint64_t i = pos[j];
+  if (before[j]) put_pseudo(tv, wo, it, i++, before[j] - 1);
+  if (st == W_NEW || st == W_SPLIT) {
+    const uint32_t item = uord[j];
+    uint32_t v = warp_alloc(&tv.ctr->n_value, 1);
+    if (v >= tv.cap_value) {
+      set_error(tv.ctr, ERR_CAPACITY);
+      v = 0;
+    }
+    tv.value_vid[v] = vid_base + item;
+    it.base[i] = koff[item];
+    it.len[i] = klen[item];
+    it.ref[i] = make_ref(KIND_VALUE, v);
+    it.d0[i] = wo.d0[j];
+    it.slot[i] = wo.slot[j];
+    it.code[i] = wo.code[j];
+    ++i;
+  }
+  if (after[j]) put_pseudo(tv, wo, it, i, after[j] - 1);
+}
+
+// Runs of split groups among the *total items in key order: as many as split
+// nodes when every group is in one piece.  A group comes in pieces when keys
+// anchored deeper, below the split extension's branch, sort between its own;
+// the groups are then sorted by anchor.
+__global__ void k_item_runs(const uint64_t *code, const unsigned long long *total, unsigned long long *runs) {
+  const uint64_t T = *total;
+  uint32_t c = 0;
+  for (uint64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < T; i += (uint64_t)gridDim.x * blockDim.x)
+    c += (code[i] >> 35) == 2ull && (i == 0 || code[i - 1] != code[i]) ? 1u : 0u;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(runs, (unsigned long long)c);
+}
+
+// sort keys (anchor, position) of the items
+__global__ void k_item_keys(const uint64_t *code, int T, uint64_t *key, uint32_t *id) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= T) return;
+  key[i] = (code[i] << 27) | (uint64_t)i;
+  id[i] = (uint32_t)i;
 }
 
 // Empty trie: every unique key is a new item of the single root group, already
@@ -775,20 +802,20 @@ __global__ void k_items_bulk(TrieView tv, const uint32_t *uord, int m, const uin
   sb_code[j] = code_root(tr);
 }
 
-// gather items into sorted order, group starts, and adjacent LCPs
-__global__ void k_items_gather(const Items it, const uint32_t *order, int T, uint64_t *sb_base, uint32_t *sb_len,
-                               uint32_t *sb_ref, uint32_t *sb_d0, uint64_t *sb_slot, uint64_t *sb_code) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// items in anchor order
+__global__ void k_items_gather(const ItemArrays it, const uint32_t *order, int T, ItemArrays out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T) return;
-  uint32_t s = order ? order[i] : (uint32_t)i;
-  sb_base[i] = it.base[s];
-  sb_len[i] = it.len[s];
-  sb_ref[i] = it.ref[s];
-  sb_d0[i] = it.d0[s];
-  sb_slot[i] = it.slot[s];
-  sb_code[i] = it.key[order ? i : s] >> 27;
+  const uint32_t s = order[i];
+  out.base[i] = it.base[s];
+  out.len[i] = it.len[s];
+  out.ref[i] = it.ref[s];
+  out.d0[i] = it.d0[s];
+  out.slot[i] = it.slot[s];
+  out.code[i] = it.code[s];
 }
 
+// group starts and adjacent LCPs
 __global__ void k_items_lcp(TrieView tv, const uint64_t *sb_base, const uint32_t *sb_len, const uint32_t *sb_d0,
                             const uint64_t *sb_code, int T, uint16_t *lcp) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;

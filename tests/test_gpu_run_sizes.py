@@ -62,3 +62,32 @@ def test_scan_tiles(gpu_lib, n):
         t.hash_onepass_v2()
         assert t.get_root_hash() == o.root()
         t.close()
+
+
+@pytest.mark.parametrize("mode", [O.MODE_REF, O.MODE_GETH])
+@pytest.mark.parametrize("width", [1, 2, 40])
+def test_split_groups_in_pieces(gpu_lib, mode, width):
+    """PhaseNU onto extensions that split while keys anchored below their
+    branch sort between the splitting ones (and extensions that split on one
+    side only, or next to each other)."""
+    rng = W.Xoshiro256ss(width, lanes=64)
+    first, second = [], []
+    for g in range(width):
+        p = [g >> 4, g & 15]
+        first += [p + [5, 5, 5, c, 7, 7, 16] for c in range(4)]  # extension 5 5 5 above a branch of 4
+        second += [p + [5, 5, 1, 0, 0, 0, 16], p + [5, 5, 5, 9, 0, 0, 16], p + [5, 5, 5, 1, 3, 0, 16],
+                   p + [5, 5, 9, 0, 0, 0, 16], p + [5, 6, 0, 0, 0, 0, 16]][: 5 - g % 4]
+        second += [p + [5, 5, 5, c, 7, 7, 16] for c in range(0, 4, 2)]  # updates in between
+    batches = []
+    for keys in (first, second):
+        keys = [keys[i] for i in np.argsort(rng.words(len(keys)), kind="stable")]
+        batches.append(make_batch(keys, [rng.bytes(1 + i % 50).tobytes() for i in range(len(keys))]))
+    o = O.OracleTrie(mode)
+    t = gpu_lib.MPT(mode=mode)
+    for b in batches:
+        o.puts(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)
+        o.hash()
+        t.puts_2phase_with_valuehp(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)
+        t.hash_onepass_v2()
+        assert t.get_root_hash() == o.root()
+    t.close()
