@@ -84,6 +84,41 @@ cudaError_t grow_array(T *&p, size_t old_n, size_t new_n, cudaStream_t st, bool 
   return cudaSuccess;
 }
 
+// One array of a node pool: its pointer, element size, and whether its old
+// elements are kept.
+struct PoolArray {
+  void **p;
+  size_t elem;
+  bool keep;
+};
+template <typename T>
+PoolArray pool_array(T *&p, size_t per_node = 1, bool keep = true) {
+  return PoolArray{reinterpret_cast<void **>(&p), per_node * sizeof(T), keep};
+}
+
+// Grow a pool of parallel arrays to new_n nodes, all in one allocation (base):
+// a pool of ten arrays paid ten cudaMalloc / cudaFree pairs at every growth.
+template <size_t N>
+cudaError_t grow_pool(uint8_t *&base, const PoolArray (&arrays)[N], size_t old_n, size_t new_n, cudaStream_t st,
+                      bool managed, int dev) {
+  size_t off[N + 1] = {0};
+  for (size_t k = 0; k < N; ++k) off[k + 1] = off[k] + ((new_n * arrays[k].elem + 64 + 255) & ~(size_t)255);
+  uint8_t *q = nullptr;
+  cudaError_t e = grow_array(q, 0, off[N], st, managed, dev);
+  for (size_t k = 0; k < N && e == cudaSuccess; ++k)
+    if (base && old_n && arrays[k].keep)
+      e = cudaMemcpyAsync(q + off[k], *arrays[k].p, old_n * arrays[k].elem, cudaMemcpyDeviceToDevice, st);
+  if (e == cudaSuccess && base) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    if (q) cudaFree(q);
+    return e;
+  }
+  if (base) cudaFree(base);
+  base = q;
+  for (size_t k = 0; k < N; ++k) *arrays[k].p = q + off[k];
+  return cudaSuccess;
+}
+
 template <typename T>
 T *wsp(DevBlock &b, size_t n, cudaError_t &e) {
   if (e != cudaSuccess) return nullptr;
@@ -120,12 +155,8 @@ Trie::Trie(int device, int geth_mode, int max_tries, bool unified)
 Trie::~Trie() {
   cudaSetDevice(dev_);
   if (st_) cudaStreamSynchronize(st_);
-  void *ptrs[] = {tv_.full_child, tv_.full_epoch, tv_.full_depth, tv_.full_hash, tv_.full_hlen, tv_.full_dead, tv_.full_ext, tv_.full_par, tv_.full_pend,
-                  fl_refs_,
-                  tv_.short_key, tv_.short_klen, tv_.short_child, tv_.short_epoch, tv_.short_depth,
-                  tv_.short_dead, tv_.short_hash, tv_.short_hlen, tv_.short_claim, tv_.short_pseudo,
-                  tv_.value_vid, tv_.rec, tv_.rec_hp, (void *)tv_.keys, (void *)tv_.vals,
-                  roots_, ctr_, dirty_ref_, dirty_depth_};
+  void *ptrs[] = {full_base_,         short_base_,        rec_base_, dirty_base_, tv_.value_vid, (void *)tv_.keys,
+                  (void *)tv_.vals, fl_refs_, roots_,    ctr_};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   DevBlock *blocks[] = {&ws_.koff, &ws_.klen, &ws_.ki, &ws_.vi, &ws_.hp, &ws_.kin, &ws_.order, &ws_.eqprev,
@@ -241,16 +272,12 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
   if (need_full > cap_full_) {
     uint64_t nc = std::min<uint64_t>(grow_to(need_full, cap_full_), kMaxNodes);
     if (opt_max_full_) nc = std::min<uint64_t>(nc, std::max<uint64_t>(opt_max_full_, need_full));
-    size_t o = n_full_;
-    if (e == cudaSuccess) e = grow_array(tv_.full_child, o * 17, nc * 17, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.full_epoch, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.full_depth, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.full_hash, o * 32, nc * 32, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.full_hlen, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.full_dead, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.full_ext, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.full_par, 0, nc, st_, managed_, dev_);  // written and read in one pass
-    if (e == cudaSuccess) e = grow_array(tv_.full_pend, 0, nc, st_, managed_, dev_);
+    const PoolArray arrays[] = {pool_array(tv_.full_child, 17), pool_array(tv_.full_epoch),
+                                pool_array(tv_.full_depth),     pool_array(tv_.full_hash, 32),
+                                pool_array(tv_.full_hlen),      pool_array(tv_.full_dead),
+                                pool_array(tv_.full_ext),       pool_array(tv_.full_par, 1, false),
+                                pool_array(tv_.full_pend, 1, false)};  // the last two: written and read in one pass
+    e = grow_pool(full_base_, arrays, n_full_, nc, st_, managed_, dev_);
     if (e == cudaSuccess) e = cudaMemsetAsync(tv_.full_par, 0xFF, 4 * (size_t)nc, st_);
     if (e != cudaSuccess) return check_cuda(e, "grow branch pool");
     cap_full_ = (uint32_t)nc;
@@ -259,17 +286,12 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
   if (need_short > kMaxNodes) return fail(E_CAPACITY, "short node count exceeds 2^30");
   if (need_short > cap_short_) {
     uint64_t nc = std::min<uint64_t>(grow_to(need_short, cap_short_), kMaxNodes);
-    size_t o = n_short_;
-    if (e == cudaSuccess) e = grow_array(tv_.short_key, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.short_klen, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.short_child, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.short_epoch, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.short_depth, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.short_dead, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.short_hash, o * 32, nc * 32, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.short_hlen, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.short_claim, o, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.short_pseudo, o, nc, st_, managed_, dev_);
+    const PoolArray arrays[] = {pool_array(tv_.short_key),      pool_array(tv_.short_klen),
+                                pool_array(tv_.short_child),    pool_array(tv_.short_epoch),
+                                pool_array(tv_.short_depth),    pool_array(tv_.short_dead),
+                                pool_array(tv_.short_hash, 32), pool_array(tv_.short_hlen),
+                                pool_array(tv_.short_claim),    pool_array(tv_.short_pseudo)};
+    e = grow_pool(short_base_, arrays, n_short_, nc, st_, managed_, dev_);
     if (e != cudaSuccess) return check_cuda(e, "grow short pool");
     cap_short_ = (uint32_t)nc;
   }
@@ -283,8 +305,8 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
   uint64_t need_rec = n_rec_ + add_rec;
   if (need_rec > cap_rec_) {
     uint64_t nc = grow_to(need_rec, cap_rec_);
-    if (e == cudaSuccess) e = grow_array(tv_.rec, n_rec_, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(tv_.rec_hp, n_rec_, nc, st_, managed_, dev_);
+    const PoolArray arrays[] = {pool_array(tv_.rec), pool_array(tv_.rec_hp)};
+    e = grow_pool(rec_base_, arrays, n_rec_, nc, st_, managed_, dev_);
     if (e != cudaSuccess) return check_cuda(e, "grow value records");
     cap_rec_ = nc;
   }
@@ -314,8 +336,8 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
       cudaStreamSynchronize(st_);
       nd = (uint32_t)(h_small_[0] & 0xFFFFFFFFu);
     }
-    if (e == cudaSuccess) e = grow_array(dirty_ref_, nd, nc, st_, managed_, dev_);
-    if (e == cudaSuccess) e = grow_array(dirty_depth_, nd, nc, st_, managed_, dev_);
+    const PoolArray arrays[] = {pool_array(dirty_ref_), pool_array(dirty_depth_)};
+    e = grow_pool(dirty_base_, arrays, nd, nc, st_, managed_, dev_);
     if (e != cudaSuccess) return check_cuda(e, "grow dirty list");
     cap_dirty_ = nc;
   }
