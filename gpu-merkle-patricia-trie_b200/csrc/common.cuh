@@ -191,4 +191,30 @@ __device__ __forceinline__ int match_nibbles(const uint8_t *a, const uint8_t *b,
   return m;
 }
 
+// Whether nibbles a[0..n) and b[0..n) are equal, reading no byte past either
+// end: four 8-byte pairs in flight at a time, the last word overlapping the
+// one before it.
+__device__ __forceinline__ bool equal_nibbles(const uint8_t *a, const uint8_t *b, uint32_t n) {
+  uint32_t o = 0;
+  for (; o + 32 <= n; o += 32) {
+    uint64_t d = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) d |= load_u64_unaligned(a + o + 8 * k) ^ load_u64_unaligned(b + o + 8 * k);
+    if (d) return false;
+  }
+  const uint32_t r = n - o;
+  if (r == 0) return true;
+  if (n < 8) {
+    bool same = true;
+    for (uint32_t k = 0; k < n; ++k) same = same && a[k] == b[k];
+    return same;
+  }
+  // up to three whole words, then the last 8 nibbles
+  uint64_t d = load_u64_unaligned(a + n - 8) ^ load_u64_unaligned(b + n - 8);
+#pragma unroll
+  for (uint32_t k = 0; k < 3; ++k)
+    if (o + 8 * (k + 1) <= n) d |= load_u64_unaligned(a + o + 8 * k) ^ load_u64_unaligned(b + o + 8 * k);
+  return d == 0;
+}
+
 }  // namespace gmpt

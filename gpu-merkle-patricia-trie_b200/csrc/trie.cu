@@ -1384,16 +1384,19 @@ int Trie::gets(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool dev
     return OK;
   }
   cudaMemcpyKind kind = device_inputs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  uint8_t *dk = wsp<uint8_t>(ws_.g_keys, (size_t)keys_bytes + 64, e);
-  int *di = wsp<int>(ws_.g_idx, 2 * (size_t)n, e);
   uint64_t *dhp = wsp<uint64_t>(ws_.g_hp, (size_t)n, e);
   int *dlen = wsp<int>(ws_.g_len, (size_t)n, e);
-  int *dtid = trie_ids ? wsp<int>(ws_.g_tid, (size_t)n, e) : nullptr;
-  // the keys are copied next to a zeroed 64-byte tail (the 8-byte key loads
-  // may read past a key's last byte); index pairs and trie ids of device
-  // batches are read where they are
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dk, keys_hexs, (size_t)keys_bytes, kind, st_);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dk + keys_bytes, 0, 64, st_);
+  // keys, index pairs and trie ids of device batches are read where they lie
+  // (a lookup reads no byte outside its key)
+  const uint8_t *dk = keys_hexs;
+  int *di = nullptr, *dtid = nullptr;
+  if (!device_inputs) {
+    uint8_t *k = wsp<uint8_t>(ws_.g_keys, (size_t)keys_bytes + 64, e);
+    di = wsp<int>(ws_.g_idx, 2 * (size_t)n, e);
+    dtid = trie_ids ? wsp<int>(ws_.g_tid, (size_t)n, e) : nullptr;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(k, keys_hexs, (size_t)keys_bytes, kind, st_);
+    dk = k;
+  }
   const int *ki = device_inputs ? keys_indexs : di;
   const int *ti = device_inputs ? trie_ids : dtid;
   if (e == cudaSuccess && !device_inputs)
@@ -2432,8 +2435,10 @@ int Trie::del(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool devi
   if (keys_bytes < 0) return fail(E_ARG, "bad index pairs");
   int rc = OK;  // the node counts are as of the last call
   const cudaMemcpyKind kind = device_inputs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  uint8_t *dk = wsp<uint8_t>(ws_.g_keys, (size_t)keys_bytes + 64, e);
-  // index pairs and trie ids of device batches are read where they lie
+  // keys, index pairs and trie ids of device batches are read where they lie
+  // (the walk reads no byte outside its key)
+  uint8_t *dk_copy = device_inputs ? nullptr : wsp<uint8_t>(ws_.g_keys, (size_t)keys_bytes + 64, e);
+  const uint8_t *dk = device_inputs ? keys_hexs : dk_copy;
   const bool di_here = device_inputs && reinterpret_cast<uintptr_t>(keys_indexs) % alignof(int) == 0;
   const bool tid_here = device_inputs && reinterpret_cast<uintptr_t>(trie_ids) % alignof(int) == 0;
   int *di = di_here ? nullptr : wsp<int>(ws_.g_idx, 2 * (size_t)n, e);
@@ -2443,8 +2448,7 @@ int Trie::del(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool devi
   uint32_t *hext = wsp<uint32_t>(ws_.del_hext, nf, e);
   uint8_t *stamp = wsp<uint8_t>(ws_.del_stamp, nf, e);
   unsigned long long *dcnt = wsp<unsigned long long>(ws_.rw_tot, 8, e);  // key cursor
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dk, keys_hexs, (size_t)keys_bytes, kind, st_);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dk + keys_bytes, 0, 64, st_);
+  if (e == cudaSuccess && dk_copy) e = cudaMemcpyAsync(dk_copy, keys_hexs, (size_t)keys_bytes, kind, st_);
   if (e == cudaSuccess && di) e = cudaMemcpyAsync(di, keys_indexs, sizeof(int) * 2 * (size_t)n, kind, st_);
   if (e == cudaSuccess && dtid) e = cudaMemcpyAsync(dtid, trie_ids, sizeof(int) * (size_t)n, kind, st_);
   if (e == cudaSuccess) e = cudaMemsetAsync(stamp, 0, nf, st_);

@@ -2146,6 +2146,9 @@ __global__ void __launch_bounds__(kHashLevelThreads, 1) k_hash_level_wide(TrieVi
 // ---------------------------------------------------------------------------
 // gets (gpu_mpt_kernels.cuh:2267-2340)
 
+// Record id of key kb[0..len), or -1.  A chain of dependent loads (a slot per
+// level, then the leaf's fields, its key and its record); a leaf's fields are
+// loaded together and its key compared 32 nibbles at a time.
 __device__ __forceinline__ int64_t lookup(const TrieView &tv, uint32_t root, const uint8_t *kb, uint32_t len) {
   uint32_t ref = root;
   uint32_t x = 0;
@@ -2161,11 +2164,12 @@ __device__ __forceinline__ int64_t lookup(const TrieView &tv, uint32_t root, con
       ++x;
       continue;
     }
-    uint32_t sl = tv.short_klen[idx];
+    const uint32_t sl = tv.short_klen[idx], child = tv.short_child[idx];
+    const uint8_t *sk = tv.keys + tv.short_key[idx];
     if (len - x < sl) return -1;
-    if ((uint32_t)match_nibbles(tv.keys + tv.short_key[idx], kb + x, (int)sl) != sl) return -1;
+    if (!equal_nibbles(sk, kb + x, sl)) return -1;
     x += sl;
-    ref = tv.short_child[idx];
+    ref = child;
   }
   return -1;
 }

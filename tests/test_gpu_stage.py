@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import oracle as O
+from conftest import make_batch, nib
 from gmpt import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -84,4 +85,43 @@ def test_malformed_batches_are_not_applied(gpu_lib, two_phase, tiled, bad):
     put(good, ki, b.values, b.values_indexs)
     t.hash_onepass_v2()
     assert t.get_root_hash() == oracle_root(first, b)
+    t.close()
+
+
+@pytest.mark.parametrize("off", [0, 1, 7])
+def test_lookups_of_every_key_length(gpu_lib, off):
+    """Stored keys, and keys that differ in the first, a middle or the last
+    nibble, of 1 to 70 bytes (leaf keys of 1 to 140 nibbles), read from device
+    memory at any byte offset, the last key ending its allocation's view."""
+    import torch
+
+    rng = W.Xoshiro256ss(5 + off, lanes=256)
+    keys, vals = [], []
+    for size in range(1, 71):
+        for c in (1, 2):
+            keys.append(nib(bytes([size, c]) + rng.bytes(size).tobytes()))
+            vals.append(bytes(size))
+    b = make_batch(keys, vals)
+    hps = np.arange(1, len(keys) + 1, dtype=np.uint64)
+    t = gpu_lib.MPT()
+    t.puts_2phase_with_valuehp(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs, hps)
+    asked, want = [], []
+    for i, k in enumerate(keys):
+        asked.append(k)
+        want.append(i + 1)
+        for at in (4, 4 + (len(k) - 5) // 2, len(k) - 2):  # behind the two bytes every key has its own
+            asked.append(k[:at] + [k[at] ^ 5] + k[at + 1:])
+            want.append(0)
+    q = make_batch(asked, [b"x"] * len(asked))
+    n = len(asked)
+    dk = at_offset(q.keys_hexs, off)
+    di = torch.from_numpy(q.keys_indexs.copy()).cuda()
+    hp = torch.zeros(n, dtype=torch.int64, device="cuda:0")
+    ln = torch.zeros(n, dtype=torch.int32, device="cuda:0")
+    torch.cuda.synchronize()
+    t.gets_device(dk[1], di.data_ptr(), n, len(q.keys_hexs), hp.data_ptr(), ln.data_ptr())
+    assert hp.cpu().tolist() == want
+    assert ln.cpu().tolist() == [len(vals[w - 1]) if w else 0 for w in want]
+    host_hp, _ = t.gets_parallel(q.keys_hexs, q.keys_indexs)
+    assert host_hp.tolist() == want
     t.close()
