@@ -229,10 +229,13 @@ k_local_build(TrieView tv, DirtyList dl, SortedItems si, SegArrays gs, uint32_t 
 }
 
 // largest segment of the current global level (decides the switch to local)
-__global__ void k_seg_max(const SegArrays sg, int S, uint32_t *out) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t v = s < S ? sg.end[s] - sg.start[s] : 0u;
-  uint32_t w = __reduce_max_sync(0xffffffffu, v);
+// (counted in the high half of *total, so it needs no host round trip first)
+__global__ void k_seg_max(const SegArrays sg, const unsigned long long *total, uint32_t *out) {
+  const uint32_t S = (uint32_t)(*total >> 32);
+  uint32_t v = 0;
+  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x)
+    v = max(v, sg.end[s] - sg.start[s]);
+  const uint32_t w = __reduce_max_sync(0xffffffffu, v);
   if ((threadIdx.x & 31) == 0 && w) atomicMax(out, w);
 }
 

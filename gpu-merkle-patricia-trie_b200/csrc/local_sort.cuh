@@ -347,10 +347,13 @@ __global__ void k_sort_runs(const unsigned long long *flags, const unsigned long
   if (!eqprev[p + 1]) seg_end[seg] = (uint32_t)p + 1;
 }
 
-__global__ void k_run_max(const uint32_t *start, const uint32_t *end, int S, uint32_t *out) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t v = s < S ? end[s] - start[s] : 0u;
-  uint32_t w = __reduce_max_sync(0xffffffffu, v);
+// longest run; the runs are counted in the high half of *total
+__global__ void k_run_max(const uint32_t *start, const uint32_t *end, const unsigned long long *total, uint32_t *out) {
+  const uint32_t S = (uint32_t)(*total >> 32);
+  uint32_t v = 0;
+  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x)
+    v = max(v, end[s] - start[s]);
+  const uint32_t w = __reduce_max_sync(0xffffffffu, v);
   if ((threadIdx.x & 31) == 0 && w) atomicMax(out, w);
 }
 

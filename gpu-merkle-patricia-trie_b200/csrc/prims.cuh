@@ -52,6 +52,7 @@ struct DevBlock {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int64_t kScanFront = 1024;  // tiles whose sums a CTA adds up itself
 
 template <typename T>
 __device__ __forceinline__ T block_excl_scan(T v, T *smem_warp, T &total) {
@@ -98,14 +99,25 @@ __global__ void k_scan_reduce(const T *in, T *tile_sums, int64_t n) {
   if (threadIdx.x == 0) tile_sums[blockIdx.x] = tot;
 }
 
-// exclusive scan of one tile per CTA, adding tile_offsets[blockIdx.x].  A
+// Exclusive scan of one tile per CTA, offset by what is in front of it: with
+// kSums, `front` holds the sums of all tiles and the CTA adds up those before
+// its own (at most kScanFront, a few loads a thread, in place of a launch that
+// scans them: 2-4 us of a scan's 8 at 1M elements); else the offset itself.  A
 // thread scans 16 neighbouring elements, which cross shared memory (one
 // padding element per 16) so that global loads and stores are coalesced: 16M
 // 8-byte elements 135 us with 128-byte strides between lanes, 45 so (268 MB).
-template <typename T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const T *in, T *out, const T *tile_offsets, int64_t n,
+template <typename T, bool kSums>
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const T *in, T *out, const T *front, int64_t n,
                                                             T *total_out) {
   __shared__ T sw[33];
+  T off = 0;
+  if (kSums) {
+    T mine = 0;
+    for (unsigned t = threadIdx.x; t < blockIdx.x; t += kScanThreads) mine += front[t];
+    block_excl_scan<T>(mine, sw, off);
+  } else if (front) {
+    off = front[blockIdx.x];
+  }
   __shared__ T tile[kScanTile + kScanTile / kScanItems];
   const int64_t base = (int64_t)blockIdx.x * kScanTile;
   auto at = [&](int j) -> T & { return tile[j + j / kScanItems]; };
@@ -124,7 +136,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const T *in, T *out
   }
   T tot;
   T run = block_excl_scan<T>(s, sw, tot);
-  const T off = tile_offsets ? tile_offsets[blockIdx.x] : T(0);
   run += off;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
@@ -151,7 +162,7 @@ cudaError_t exclusive_scan(const T *in, T *out, int64_t n, T *total_out, DevBloc
   }
   int64_t tiles = (n + kScanTile - 1) / kScanTile;
   if (tiles == 1) {
-    count_launch(), k_scan_tiles<T><<<1, kScanThreads, 0, st>>>(in, out, nullptr, n, total_out);
+    count_launch(), k_scan_tiles<T, false><<<1, kScanThreads, 0, st>>>(in, out, nullptr, n, total_out);
     return cudaGetLastError();
   }
   size_t need = ws_off + (size_t)(2 * tiles + 64) * sizeof(T);
@@ -159,10 +170,14 @@ cudaError_t exclusive_scan(const T *in, T *out, int64_t n, T *total_out, DevBloc
   T *sums = reinterpret_cast<T *>(static_cast<char *>(ws.p) + ws_off);
   T *offs = sums + tiles;
   count_launch(), k_scan_reduce<T><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, sums, n);
+  if (tiles <= kScanFront) {
+    count_launch(), k_scan_tiles<T, true><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, sums, n, total_out);
+    return cudaGetLastError();
+  }
   cudaError_t e = exclusive_scan<T>(sums, offs, tiles, (T *)nullptr, ws, st,
                                     ws_off + (size_t)(2 * tiles + 32) * sizeof(T));
   if (e != cudaSuccess) return e;
-  count_launch(), k_scan_tiles<T><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, offs, n, total_out);
+  count_launch(), k_scan_tiles<T, false><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, offs, n, total_out);
   return cudaGetLastError();
 }
 
@@ -191,6 +206,7 @@ static __global__ void k_or_diff(const uint64_t *keys, int64_t n, unsigned long 
   if (threadIdx.x == 0) s = 0;
   __syncthreads();
   uint64_t k0 = keys[0];
+  if (blockIdx.x == 0 && threadIdx.x == 0) mask[1] = k0;  // its nibbles are every key's common ones
   uint64_t acc = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
@@ -327,9 +343,8 @@ struct RadixSorter {
     int grid = (int)((n + 1023) / 1024);
     if (grid > 2048) grid = 2048;
     count_launch(), k_or_diff<<<grid, 256, 0, st>>>(keys, n, mask.as<unsigned long long>());
-    // the varying bits and the first key (its nibbles are every key's common ones)
-    if ((e = cudaMemcpyAsync(h_mask, mask.p, 8, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(h_mask + 1, keys, 8, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+    // the varying bits and the first key
+    if ((e = cudaMemcpyAsync(h_mask, mask.p, 16, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
     uint64_t m = h_mask[0];
     const uint64_t k0 = h_mask[1];

@@ -548,25 +548,26 @@ int Trie::sort_batch(int n, const uint64_t *koff, const uint32_t *klen, uint32_t
     int cc = (c == nchunks) ? -1 : (c < 0 ? -2 : c);  // final pass: key length
     count_launch(), k_sort_flags<<<blocks_for(n), kThreads, 0, st_>>>(eqprev, n, flags);
     e = exclusive_scan<unsigned long long>(flags, pos, n, d_tot, scan_ws_, st_);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_small_, d_tot, 8, cudaMemcpyDeviceToHost, st_);
+    // still-tied runs and the longest, read back with the counts: if it fits
+    // one CTA, every run is finished there
+    const bool local = opt_local_sort_ && c >= 0;
+    uint32_t *rs = local ? wsp<uint32_t>(ws_.it_id, (size_t)n / 2 + 1, e) : nullptr;
+    uint32_t *re = local ? wsp<uint32_t>(ws_.it_len, (size_t)n / 2 + 1, e) : nullptr;
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_tot + 1, 0, 8, st_);
+    if (e != cudaSuccess) return check_cuda(e, "sort flags");
+    if (local) {
+      count_launch(), k_sort_runs<<<blocks_for(n), kThreads, 0, st_>>>(flags, pos, eqprev, n, rs, re);
+      count_launch(), k_run_max<<<std::min<unsigned>(blocks_for(n / 2 + 1), 148 * 4), kThreads, 0, st_>>>(
+                          rs, re, d_tot, reinterpret_cast<uint32_t *>(d_tot + 1));
+    }
+    e = cudaMemcpyAsync(h_small_, d_tot, 16, cudaMemcpyDeviceToHost, st_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
     if (e != cudaSuccess) return check_cuda(e, "sort flags");
     int K = (int)(h_small_[0] & 0xFFFFFFFFu);
     int S = (int)(h_small_[0] >> 32);
     if (K == 0) break;
-    if (opt_local_sort_ && c >= 0) {
-      // still-tied runs; if the largest fits one CTA, finish every run there
-      uint32_t *rs = wsp<uint32_t>(ws_.it_id, (size_t)S, e);
-      uint32_t *re = wsp<uint32_t>(ws_.it_len, (size_t)S, e);
-      uint32_t *d_max = reinterpret_cast<uint32_t *>(d_tot + 1);
-      if (e == cudaSuccess) e = cudaMemsetAsync(d_max, 0, 4, st_);
-      if (e != cudaSuccess) return check_cuda(e, "sort runs alloc");
-      count_launch(), k_sort_runs<<<blocks_for(n), kThreads, 0, st_>>>(flags, pos, eqprev, n, rs, re);
-      count_launch(), k_run_max<<<blocks_for(S), kThreads, 0, st_>>>(rs, re, S, d_max);
-      if ((e = cudaMemcpyAsync(h_small_, d_max, 4, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-          (e = cudaStreamSynchronize(st_)) != cudaSuccess)
-        return check_cuda(e, "sort runs");
-      uint32_t maxrun = (uint32_t)(h_small_[0] & 0xFFFFFFFFu);
+    if (local) {
+      const uint32_t maxrun = (uint32_t)(h_small_[1] & 0xFFFFFFFFu);
       const uint32_t cap = opt_local_sort_cap_ > 0 ? (uint32_t)opt_local_sort_cap_ : (uint32_t)kSortLocalCap;
       if (maxrun <= cap) {
         count_launch(), k_local_sort_warp<<<blocks_for(32 * (int64_t)S), kThreads, 0, st_>>>(tv_, rs, re, S, c, order,
@@ -864,21 +865,20 @@ int Trie::build_levels(int T) {
   e = exclusive_scan<unsigned long long>(flags, pos, T, d_tot, scan_ws_, st_);
   if (e != cudaSuccess) return check_cuda(e, "groups scan");
   count_launch(), k_groups_scatter<<<blocks_for(T), kThreads, 0, st_>>>(si, kflags, pos, T, act[0], aseg[0], sg[0]);
-  uint32_t *d_max = reinterpret_cast<uint32_t *>(d_tot + 1);
-  auto read_level = [&](int S_now, int cur_now) -> cudaError_t {
-    cudaError_t x = cudaMemsetAsync(d_max, 0, 4, st_);
-    if (x == cudaSuccess && S_now > 0 && opt_local_build_)
-      count_launch(), k_seg_max<<<blocks_for(S_now), kThreads, 0, st_>>>(sg[cur_now], S_now, d_max);
+  // items and segments of the level just scattered into sg[cur_now], and the
+  // largest segment, in one read
+  auto read_level = [&](int cur_now, int items) -> cudaError_t {
+    cudaError_t x = cudaMemsetAsync(d_tot + 1, 0, 8, st_);
+    if (x == cudaSuccess && opt_local_build_)
+      count_launch(), k_seg_max<<<std::min<unsigned>(blocks_for(items / 2 + 1), 148 * 4), kThreads, 0, st_>>>(
+                          sg[cur_now], d_tot, reinterpret_cast<uint32_t *>(d_tot + 1));
     if (x == cudaSuccess) x = cudaMemcpyAsync(h_small_, d_tot, 16, cudaMemcpyDeviceToHost, st_);
     if (x == cudaSuccess) x = cudaStreamSynchronize(st_);
     return x;
   };
-  if ((e = cudaMemcpyAsync(h_small_, d_tot, 8, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(st_)) != cudaSuccess)
-    return check_cuda(e, "groups");
+  if ((e = read_level(0, T)) != cudaSuccess) return check_cuda(e, "groups");
   int K = (int)(h_small_[0] & 0xFFFFFFFFu);
   int S = (int)(h_small_[0] >> 32);
-  if ((e = read_level(S, 0)) != cudaSuccess) return check_cuda(e, "groups max");
   uint32_t maxseg = (uint32_t)(h_small_[1] & 0xFFFFFFFFu);
   int cur = 0, levels = 0;
   while (K > 0) {
@@ -909,18 +909,11 @@ int Trie::build_levels(int T) {
     if (e != cudaSuccess) return check_cuda(e, "level scan");
     count_launch(), k_level_scatter<<<blocks_for(K), kThreads, 0, st_>>>(act[cur], aseg[cur], kflags, knib, pos, K, sg[cur],
                                                          act[cur ^ 1], aseg[cur ^ 1], sg[cur ^ 1]);
-    K = 0;
     cur ^= 1;
-    // K, S of the next level are in d_tot; the largest segment comes with them
-    if ((e = cudaMemcpyAsync(h_small_, d_tot, 8, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st_)) != cudaSuccess)
-      return check_cuda(e, "level");
+    if ((e = read_level(cur, K)) != cudaSuccess) return check_cuda(e, "level");
     K = (int)(h_small_[0] & 0xFFFFFFFFu);
     S = (int)(h_small_[0] >> 32);
-    if (K > 0 && opt_local_build_) {
-      if ((e = read_level(S, cur)) != cudaSuccess) return check_cuda(e, "level max");
-      maxseg = (uint32_t)(h_small_[1] & 0xFFFFFFFFu);
-    }
+    maxseg = (uint32_t)(h_small_[1] & 0xFFFFFFFFu);
   }
   stats_.build_levels = levels;
   return OK;
