@@ -36,6 +36,17 @@ struct BlockDesc {
   uint64_t key_base, val_base, vid_base;
   uint32_t gen, pad1;              // dirty generation of stage 0 (stage 1: gen + 1)
   uint32_t warp_max, pad2;         // hash_grid's warp_max
+  // the block where it lies (the caller's device arrays, or copies of host
+  // arrays); the streams are 8-byte aligned
+  const uint8_t *keys;             // key stream (nibble bytes)
+  const uint8_t *vals;             // value stream
+  const int *kidx;                 // [2n] inclusive pairs; must tile the stream
+  const int64_t *vidx;             // [2n]
+  const int *tid;                  // [n] trie of each key (null: trie 0)
+  const int *patch_trie;           // [n] -1 = no patch (null: none)
+  const int *patch_off;            // [n] byte offset of the 32-byte root in the value
+  const int *out_ids;              // [n_out] tries whose roots are reported (pinned host memory)
+  uint8_t *out;                    // [n_out * 33] root bytes + length (pinned host memory)
   GridCtl ctl;                     // barrier_ns set, the rest zero
   // filled by k_block_stage
   uint32_t stream_terms, key_terms, noncontig, bad;  // bad: BLOCK_BAD_* bits
@@ -46,15 +57,6 @@ struct BlockDesc {
 enum : uint32_t { BLOCK_BAD_KEY = 1, BLOCK_BAD_TRIE = 2, BLOCK_BAD_PATCH = 4, BLOCK_BAD_VALUE = 8 };
 
 struct BlockBufs {
-  const uint8_t *keys;     // key stream (nibble bytes)
-  const int *kidx;         // [2n] inclusive pairs; must tile the stream
-  const uint8_t *vals;     // value stream
-  const int64_t *vidx;     // [2n]
-  const int *tid;          // [n] trie of each key
-  const int *patch_trie;   // [n] -1 = no patch
-  const int *patch_off;    // [n] byte offset of the 32-byte root in the value
-  const int *out_ids;      // [n_out] tries whose roots are reported
-  uint8_t *out;            // [n_out * 33] root bytes + length
   uint64_t *koff;          // [n] staged key offsets
   uint32_t *klen;          // [n]
   uint32_t *ready;         // branches whose dirty children are hashed
@@ -70,11 +72,14 @@ __global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, Block
   const int64_t kb = D->kbytes, vb = D->vbytes;
   const uint64_t key_base = D->key_base, val_base = D->val_base, vid_base = D->vid_base;
   const int64_t T = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int *kidx = D->kidx, *tid = D->tid, *patch_trie = D->patch_trie, *patch_off = D->patch_off;
+  const int64_t *vidx = D->vidx;
+  const uint8_t *keys = D->keys;
   if (t0 == 0) D->ctl.ts[D->ctl.n_ts++] = global_ns();
   uint32_t terms = 0, bad = 0, kterms = 0, gap = 0;
   {
     uint64_t *dst = reinterpret_cast<uint64_t *>(const_cast<uint8_t *>(tv.keys) + key_base);
-    const uint64_t *src = reinterpret_cast<const uint64_t *>(bb.keys);
+    const uint64_t *src = reinterpret_cast<const uint64_t *>(D->keys);
     const int64_t words = (kb + 7) / 8 + 8;
     for (int64_t w = t0; w < words; w += T) {
       uint64_t x = 0;
@@ -92,7 +97,7 @@ __global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, Block
   }
   {
     uint64_t *dst = reinterpret_cast<uint64_t *>(const_cast<uint8_t *>(tv.vals) + val_base);
-    const uint64_t *src = reinterpret_cast<const uint64_t *>(bb.vals);
+    const uint64_t *src = reinterpret_cast<const uint64_t *>(D->vals);
     const int64_t words = (vb + 7) / 8 + 8;
     for (int64_t w = t0; w < words; w += T) {
       uint64_t x = 0;
@@ -105,14 +110,14 @@ __global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, Block
     }
   }
   for (int64_t i = t0; i < n; i += T) {
-    int ks = bb.kidx[2 * i], ke = bb.kidx[2 * i + 1];
+    int ks = kidx[2 * i], ke = kidx[2 * i + 1];
     bool badk = ks < 0 || ke < ks || (int64_t)ke >= kb || ke - ks + 1 > kMaxKeyNibbles;
     if (!badk) {
-      const uint8_t last = bb.keys[ke];
+      const uint8_t last = keys[ke];
       if (last > 16) badk = true;
       kterms += last == 16 ? 1u : 0u;
     }
-    if (i == 0 ? ks != 0 : ks != bb.kidx[2 * i - 1] + 1) gap = 1;
+    if (i == 0 ? ks != 0 : ks != kidx[2 * i - 1] + 1) gap = 1;
     if (i + 1 == n && (int64_t)ke + 1 != kb) gap = 1;
     if (badk) {
       bad |= BLOCK_BAD_KEY;
@@ -120,16 +125,16 @@ __global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, Block
     }
     bb.koff[i] = key_base + (uint64_t)ks;
     bb.klen[i] = (uint32_t)(ke - ks + 1);
-    if ((uint32_t)bb.tid[i] >= tv.n_tries) bad |= BLOCK_BAD_TRIE;
-    int64_t vs = bb.vidx[2 * i], ve = bb.vidx[2 * i + 1];
+    if (tid && (uint32_t)tid[i] >= tv.n_tries) bad |= BLOCK_BAD_TRIE;
+    int64_t vs = vidx[2 * i], ve = vidx[2 * i + 1];
     if (vs < 0 || ve < vs - 1 || ve >= vb) {
       bad |= BLOCK_BAD_VALUE;
       vs = 0;
       ve = -1;
     }
-    const int pt = bb.patch_trie[i];
-    if (pt >= 0 && ((uint32_t)pt >= tv.n_tries || i < n0 || bb.patch_off[i] < 0 ||
-                    (int64_t)bb.patch_off[i] + 32 > ve - vs + 1))
+    const int pt = patch_trie ? patch_trie[i] : -1;
+    if (pt >= 0 && ((uint32_t)pt >= tv.n_tries || i < n0 || patch_off[i] < 0 ||
+                    (int64_t)patch_off[i] + 32 > ve - vs + 1))
       bad |= BLOCK_BAD_PATCH;
     const uint64_t vid = vid_base + (uint64_t)i;
     tv.rec[vid] = ValueRec{val_base + (uint64_t)vs, (uint32_t)(ve - vs + 1), 0u};
@@ -185,10 +190,10 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_block(TrieView tv0, DirtyLi
     tv.gen = D->gen + (uint32_t)s;
     if (s == 1) {
       // stage-1 values take the roots their stage-0 tries just got
-      for (int i = n0 + t; i < n; i += T) {
-        const int pt = bb.patch_trie[i];
+      for (int i = n0 + t; i < n && D->patch_trie; i += T) {
+        const int pt = D->patch_trie[i];
         if (pt < 0) continue;
-        uint8_t *dst = const_cast<uint8_t *>(tv.vals) + tv.rec[vid_base + (uint64_t)i].off + bb.patch_off[i];
+        uint8_t *dst = const_cast<uint8_t *>(tv.vals) + tv.rec[vid_base + (uint64_t)i].off + D->patch_off[i];
         const uint32_t r = __ldcg(tv.roots + pt);
         const uint32_t kind = ref_kind(r), idx = ref_idx(r);
         const uint8_t *h = kind == KIND_FULL ? tv.full_hash + (size_t)idx * 32
@@ -202,7 +207,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_block(TrieView tv0, DirtyLi
     const int span = T * kLatchWays;
     for (int base = i0; base < i1; base += span)
       latch_keys(tv, dl, bb.koff + base, bb.klen + base, min(span, i1 - base), vid_base + (uint64_t)base, retry_limit,
-                 bb.tid + base, g.t_spread, T);
+                 D->tid ? D->tid + base : nullptr, g.t_spread, T);
     if (!grid_barrier(&D->ctl, tv.ctr)) return;
     const uint32_t nd = __ldcg(&tv.ctr->n_dirty);
     uint32_t waves = 0;
@@ -214,7 +219,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_block(TrieView tv0, DirtyLi
     if (!grid_barrier(&D->ctl, tv.ctr)) return;  // the cleared counters are seen by every CTA
   }
   // roots asked for: one warp each
-  for (int w = t >> 5; w < n_out; w += T >> 5) write_root(tv, (uint32_t)bb.out_ids[w], bb.out + 33 * (size_t)w, g.lane);
+  for (int w = t >> 5; w < n_out; w += T >> 5) write_root(tv, (uint32_t)D->out_ids[w], D->out + 33 * (size_t)w, g.lane);
   __syncthreads();
   if (t == 0 && D->ctl.n_ts < kGridMaxTs) D->ctl.ts[D->ctl.n_ts++] = global_ns();
 }

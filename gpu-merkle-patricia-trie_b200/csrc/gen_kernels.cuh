@@ -151,8 +151,7 @@ __global__ void __launch_bounds__(64) k_sample_features(const uint8_t *keys, con
       const int lb = s_len[k];
       const int m = la < lb ? la : lb;
       const uint8_t *b = keys + s_off[k];
-      int l = 0;
-      while (l < m && a[l] == b[l]) ++l;
+      const int l = match_nibbles(a, b, m);
       if (l == m && la == lb && k < j) earlier = true;
       best = l > best ? l : best;
     }

@@ -184,7 +184,7 @@ Trie::~Trie() {
   sorter_.release();
   scan_ws_.release();
   DevBlock *bblocks[] = {&blk_.keys, &blk_.kidx, &blk_.vals, &blk_.vidx, &blk_.tid, &blk_.ptrie, &blk_.poff,
-                         &blk_.out_ids, &blk_.out, &blk_.koff, &blk_.klen, &blk_.ready};
+                         &blk_.koff, &blk_.klen, &blk_.ready};
   for (DevBlock *b : bblocks) b->release();
   for (auto &c : blk_.graphs) {
     if (c.exec) cudaGraphExecDestroy(c.exec);
@@ -200,6 +200,8 @@ Trie::~Trie() {
   if (blk_.d_desc) cudaFree(blk_.d_desc);
   if (grid_ctl_) cudaFree(grid_ctl_);
   if (blk_.h_desc) cudaFreeHost(blk_.h_desc);
+  if (blk_.h_out_ids) cudaFreeHost(blk_.h_out_ids);
+  if (blk_.h_out) cudaFreeHost(blk_.h_out);
   if (h_pack_) cudaFreeHost(h_pack_);
   if (h_ctr_) cudaFreeHost(h_ctr_);
   if (h_small_) cudaFreeHost(h_small_);
@@ -1324,6 +1326,22 @@ int Trie::roots(const int *ids, int n, uint8_t *out32, int *sizes) {
   if (!ids && (uint32_t)n > n_tries_) return fail(E_ARG, "more roots than tries");
   cudaSetDevice(dev_);
   cudaError_t e = cudaSuccess;
+  if (37 * (size_t)n + 64 <= kPackBytes) {
+    // a few roots: the kernel reads the ids from pinned host memory and
+    // writes the roots there
+    if (!h_pack_ && (e = cudaMallocHost(&h_pack_, kPackBytes)) != cudaSuccess) return check_cuda(e, "roots alloc");
+    int *pid = reinterpret_cast<int *>(h_pack_);
+    uint8_t *po = h_pack_ + ((4 * (size_t)n + 63) & ~(size_t)63);
+    if (ids) std::memcpy(pid, ids, 4 * (size_t)n);
+    count_launch(), k_roots<<<blocks_for(32 * (int64_t)n), kThreads, 0, st_>>>(tv_, ids ? pid : nullptr, 0, n, po);
+    if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(st_)) != cudaSuccess)
+      return check_cuda(e, "roots");
+    for (int i = 0; i < n; ++i) {
+      std::memcpy(out32 + 32 * (size_t)i, po + 33 * (size_t)i, 32);
+      sizes[i] = po[33 * (size_t)i + 32];
+    }
+    return OK;
+  }
   int *did = ids ? wsp<int>(ws_.g_tid, (size_t)n, e) : nullptr;
   uint8_t *d = wsp<uint8_t>(ws_.g_keys, 33 * (size_t)n, e);
   if (e == cudaSuccess && ids) e = cudaMemcpyAsync(did, ids, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, st_);
@@ -1997,10 +2015,7 @@ int Trie::block_launch(bool launch) {
   sig.tv.gen = 0;    // the kernels take the generation from the descriptor
   sig.tv.epoch = 0;  // (LockNU claims no split epochs)
   sig.dl = DirtyList{dirty_ref_, dirty_depth_};
-  sig.bb = BlockBufs{blk_.keys.as<uint8_t>(), blk_.kidx.as<int>(),      blk_.vals.as<uint8_t>(),
-                     blk_.vidx.as<int64_t>(), blk_.tid.as<int>(),       blk_.ptrie.as<int>(),
-                     blk_.poff.as<int>(),     blk_.out_ids.as<int>(),   blk_.out.as<uint8_t>(),
-                     blk_.koff.as<uint64_t>(), blk_.klen.as<uint32_t>(), blk_.ready.as<uint32_t>(),
+  sig.bb = BlockBufs{blk_.koff.as<uint64_t>(), blk_.klen.as<uint32_t>(), blk_.ready.as<uint32_t>(),
                      static_cast<BlockDesc *>(blk_.d_desc)};
   sig.h_desc = blk_.h_desc;
   sig.h_ctr = h_ctr_;
@@ -2110,27 +2125,31 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   if (rc) return rc;
   if ((rc = block_buffers(n, kb, vb, b.n_out)) || (rc = grid_limits())) return rc;
   cudaError_t e = cudaSuccess;
-  const cudaMemcpyKind kind = b.device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  if (n > 0) {
-    e = cudaMemcpyAsync(blk_.keys.p, b.keys_hexs, (size_t)kb, kind, st_);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(blk_.kidx.p, b.keys_indexs, 8 * (size_t)n, kind, st_);
-    if (e == cudaSuccess && vb) e = cudaMemcpyAsync(blk_.vals.p, b.values, (size_t)vb, kind, st_);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(blk_.vidx.p, b.values_indexs, 16 * (size_t)n, kind, st_);
-    if (e == cudaSuccess)
-      e = b.trie_ids ? cudaMemcpyAsync(blk_.tid.p, b.trie_ids, 4 * (size_t)n, kind, st_)
-                     : cudaMemsetAsync(blk_.tid.p, 0, 4 * (size_t)n, st_);
-    if (b.patch_trie) {
-      if (e == cudaSuccess) e = cudaMemcpyAsync(blk_.ptrie.p, b.patch_trie, 4 * (size_t)n, kind, st_);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(blk_.poff.p, b.patch_off, 4 * (size_t)n, kind, st_);
-    } else if (e == cudaSuccess) {
-      e = cudaMemsetAsync(blk_.ptrie.p, 0xFF, 4 * (size_t)n, st_);  // -1: no patch
-    }
-  }
-  if (e == cudaSuccess && b.n_out > 0)
-    e = cudaMemcpyAsync(blk_.out_ids.p, b.out_ids, 4 * (size_t)b.n_out, cudaMemcpyHostToDevice, st_);
-  if (e != cudaSuccess) return check_cuda(e, "block inputs");
   BlockDesc *h = static_cast<BlockDesc *>(blk_.h_desc);
   std::memset(h, 0, sizeof(BlockDesc));
+  // device arrays are read where they lie, host arrays (and device arrays
+  // without the alignment the kernels read with) are copied
+  const cudaMemcpyKind kind = b.device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+  auto at = [&](auto *p, DevBlock &w, size_t bytes, size_t align) -> decltype(p) {
+    if (!p || e != cudaSuccess || (b.device && reinterpret_cast<uintptr_t>(p) % align == 0)) return p;
+    if (bytes) e = cudaMemcpyAsync(w.p, p, bytes, kind, st_);
+    return static_cast<decltype(p)>(w.p);
+  };
+  if (n > 0) {
+    h->keys = at(b.keys_hexs, blk_.keys, (size_t)kb, 8);
+    h->kidx = at(b.keys_indexs, blk_.kidx, 8 * (size_t)n, alignof(int));
+    h->vals = at(b.values, blk_.vals, (size_t)vb, 8);
+    h->vidx = at(b.values_indexs, blk_.vidx, 16 * (size_t)n, alignof(int64_t));
+    h->tid = at(b.trie_ids, blk_.tid, 4 * (size_t)n, alignof(int));
+    h->patch_trie = at(b.patch_trie, blk_.ptrie, 4 * (size_t)n, alignof(int));
+    h->patch_off = at(b.patch_off, blk_.poff, 4 * (size_t)n, alignof(int));
+  }
+  if (e != cudaSuccess) return check_cuda(e, "block inputs");
+  // the kernel reads the tries asked for from pinned host memory and writes
+  // their roots there
+  if (b.n_out > 0) std::memcpy(blk_.h_out_ids, b.out_ids, 4 * (size_t)b.n_out);
+  h->out_ids = blk_.h_out_ids;
+  h->out = blk_.h_out;
   const uint64_t key_base = (key_used_ + 7) & ~7ull, val_base = (val_used_ + 7) & ~7ull;
   h->n = n;
   h->n0 = b.n0;
@@ -2181,15 +2200,9 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   stats_.n_value = n_value_;
   stats_.last_dirty = (uint64_t)h->dirty[0] + h->dirty[1];
   stats_.last_hash_levels = (uint64_t)h->levels[0] + h->levels[1];
-  if (b.n_out > 0) {
-    std::vector<uint8_t> o(33 * (size_t)b.n_out);
-    if ((e = cudaMemcpyAsync(o.data(), blk_.out.p, o.size(), cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st_)) != cudaSuccess)
-      return check_cuda(e, "block roots");
-    for (int i = 0; i < b.n_out; ++i) {
-      std::memcpy(out32 + 32 * (size_t)i, o.data() + 33 * (size_t)i, 32);
-      sizes[i] = o[33 * (size_t)i + 32];
-    }
+  for (int i = 0; i < b.n_out; ++i) {
+    std::memcpy(out32 + 32 * (size_t)i, blk_.h_out + 33 * (size_t)i, 32);
+    sizes[i] = blk_.h_out[33 * (size_t)i + 32];
   }
   if (timing_) {
     cudaEventRecord(ev[3], st_);
@@ -2212,8 +2225,17 @@ int Trie::block_buffers(int64_t n, int64_t kb, int64_t vb, int64_t n_out) {
   if (e == cudaSuccess) e = blk_.tid.ensure(4 * nn);
   if (e == cudaSuccess) e = blk_.ptrie.ensure(4 * nn);
   if (e == cudaSuccess) e = blk_.poff.ensure(4 * nn);
-  if (e == cudaSuccess) e = blk_.out_ids.ensure(4 * no);
-  if (e == cudaSuccess) e = blk_.out.ensure(33 * no);
+  if (e == cudaSuccess && no > blk_.h_out_cap) {
+    if (blk_.h_out_ids) cudaFreeHost(blk_.h_out_ids);
+    if (blk_.h_out) cudaFreeHost(blk_.h_out);
+    blk_.h_out_ids = nullptr;
+    blk_.h_out = nullptr;
+    blk_.h_out_cap = 0;
+    const size_t c = no + no / 4 + 64;
+    e = cudaMallocHost(&blk_.h_out_ids, 4 * c);
+    if (e == cudaSuccess) e = cudaMallocHost(&blk_.h_out, 33 * c);
+    if (e == cudaSuccess) blk_.h_out_cap = c;
+  }
   if (e == cudaSuccess) e = blk_.koff.ensure(8 * nn);
   if (e == cudaSuccess) e = blk_.klen.ensure(4 * nn);
   if (e == cudaSuccess) e = blk_.ready.ensure(sizeof(uint32_t) * ((size_t)cap_full_ + 64));

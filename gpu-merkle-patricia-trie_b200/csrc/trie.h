@@ -226,7 +226,10 @@ class Trie {
 
   // persistent block launches
   struct BlockRt {
-    DevBlock keys, kidx, vals, vidx, tid, ptrie, poff, out_ids, out, koff, klen, ready;
+    DevBlock keys, kidx, vals, vidx, tid, ptrie, poff, koff, klen, ready;
+    int *h_out_ids = nullptr;  // pinned: tries whose roots are reported, and their roots
+    uint8_t *h_out = nullptr;
+    size_t h_out_cap = 0;
     void *d_desc = nullptr, *h_desc = nullptr;  // BlockDesc (device / pinned)
     struct Captured {
       std::vector<uint8_t> sig;  // launch arguments the graph was captured with

@@ -125,3 +125,29 @@ def test_lookups_of_every_key_length(gpu_lib, off):
     host_hp, _ = t.gets_parallel(q.keys_hexs, q.keys_indexs)
     assert host_hp.tolist() == want
     t.close()
+
+
+@pytest.mark.parametrize("off", [0, 1, 4, 8])
+def test_block_arrays_at_any_offset(gpu_lib, off):
+    """A block update from device arrays read where they lie (or copied, where
+    their alignment asks for it) equals the same block from host arrays."""
+    import torch
+
+    rng = W.Xoshiro256ss(31 + off, lanes=64)
+    n0, n = 700, 741
+    b = W.random_keys(n, 16, 48, seed=0x5EED0B30)
+    tid = np.concatenate([1 + (rng.words(n0) % np.uint64(40)).astype(np.int32), np.zeros(n - n0, np.int32)])
+    pt = np.concatenate([np.full(n0, -1, np.int32), np.arange(n - n0, dtype=np.int32)])
+    po = np.full(n, 5, np.int32)
+    out_ids = np.arange(41, dtype=np.int32)
+    host = gpu_lib.MPT(max_tries=41)
+    keep = [at_offset(a, off) for a in (b.keys_hexs, b.keys_indexs, b.values, b.values_indexs, tid, pt, po)]
+    torch.cuda.synchronize()
+    t = gpu_lib.MPT(max_tries=41)
+    for _ in range(2):  # the second one replays the captured launch (and patches another root of trie 0 in)
+        want = host.block_update(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs, tid, n0, out_ids, pt, po)
+        got = t.block_update_device(*[p for _, p in keep], n, n0, len(b.keys_hexs), len(b.values), out_ids)
+        assert got == want
+    assert t.get_roots(out_ids) == want
+    host.close()
+    t.close()
