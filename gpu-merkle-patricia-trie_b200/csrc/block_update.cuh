@@ -35,7 +35,8 @@ struct BlockDesc {
   int64_t kbytes, vbytes;          // stream lengths
   uint64_t key_base, val_base, vid_base;
   uint32_t gen, pad1;              // dirty generation of stage 0 (stage 1: gen + 1)
-  uint32_t warp_max, pad2;         // hash_grid's warp_max
+  uint32_t warp_max;               // hash_grid's warp_max
+  uint32_t max_klen;               // filled by k_block_stage: the longest key
   // the block where it lies (the caller's device arrays, or copies of host
   // arrays); the streams are 8-byte aligned
   const uint8_t *keys;             // key stream (nibble bytes)
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, Block
   const int64_t *vidx = D->vidx;
   const uint8_t *keys = D->keys;
   if (t0 == 0) D->ctl.ts[D->ctl.n_ts++] = global_ns();
-  uint32_t terms = 0, bad = 0, kterms = 0, gap = 0;
+  uint32_t terms = 0, bad = 0, kterms = 0, gap = 0, lmax = 0;
   {
     uint64_t *dst = reinterpret_cast<uint64_t *>(const_cast<uint8_t *>(tv.keys) + key_base);
     const uint64_t *src = reinterpret_cast<const uint64_t *>(D->keys);
@@ -125,6 +126,7 @@ __global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, Block
     }
     bb.koff[i] = key_base + (uint64_t)ks;
     bb.klen[i] = (uint32_t)(ke - ks + 1);
+    lmax = max(lmax, (uint32_t)(ke - ks + 1));
     if (tid && (uint32_t)tid[i] >= tv.n_tries) bad |= BLOCK_BAD_TRIE;
     int64_t vs = vidx[2 * i], ve = vidx[2 * i + 1];
     if (vs < 0 || ve < vs - 1 || ve >= vb) {
@@ -144,11 +146,13 @@ __global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, Block
   kterms = __reduce_add_sync(0xffffffffu, kterms);
   bad = __reduce_or_sync(0xffffffffu, bad);
   gap = __reduce_or_sync(0xffffffffu, gap);
+  lmax = __reduce_max_sync(0xffffffffu, lmax);
   if ((threadIdx.x & 31) == 0) {
     if (terms) atomicAdd(&D->stream_terms, terms);
     if (kterms) atomicAdd(&D->key_terms, kterms);
     if (bad) atomicOr(&D->bad, bad);
     if (gap) atomicOr(&D->noncontig, 1u);
+    if (lmax) atomicMax(&D->max_klen, lmax);
   }
 }
 

@@ -235,6 +235,7 @@ int Trie::apply_counters() {
   n_short_ = h_ctr_->n_short;
   n_value_ = h_ctr_->n_value;
   n_dirty_ = h_ctr_->n_dirty;
+  ctr_stale_ = false;
   uint32_t err = h_ctr_->error;
   if (err) {
     cudaMemsetAsync(&ctr_->error, 0, 4, st_);
@@ -388,6 +389,7 @@ int Trie::stage(const BatchIn &batch, uint64_t &key_base, uint64_t &vid_base, ui
                 const int **tid_out) {
   BatchIn b = batch;
   const int n = b.n;
+  ctr_stale_ = true;  // until the counters are read
   cudaError_t e = cudaSuccess;
   int64_t kbytes = b.keys_bytes, vbytes = b.values_bytes;
   if (kbytes < 0 || vbytes < 0) {
@@ -1284,9 +1286,11 @@ int Trie::hash() {
     cudaEventCreate(&z);
     cudaEventRecord(a, st_);
   }
+  int rc = OK;
+  // a call that stopped half way left marks the counters at hand do not have
+  if (ctr_stale_ && (rc = sync_counters())) return rc;
   const bool any = n_dirty_ != 0;
-  int rc = bucket_and_hash();
-  if (rc) return rc;
+  if ((rc = bucket_and_hash())) return rc;
   if (any && (rc = sync_counters())) return rc;  // nothing was launched for an empty list
   const bool counted = any && timing_;
   stats_.last_hashed = counted ? h_ctr_->hashed : 0;
@@ -2163,6 +2167,7 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   h->warp_max = grid_warp_max((unsigned)block_grid());
   h->ctl.barrier_ns = opt_barrier_ns_;
   if (timing_) cudaEventRecord(ev[1], st_);
+  ctr_stale_ = true;  // until the counters are read
   if ((rc = block_launch())) return rc;
   if (timing_) cudaEventRecord(ev[2], st_);
   if ((e = cudaStreamSynchronize(st_)) != cudaSuccess) return check_cuda(e, "block");
@@ -2189,7 +2194,7 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   gen_ += 2;
   tv_.gen = gen_;
   if (n > 0) empty_ = false;
-  if (n > 0) depth_bound_ = kMaxKeyNibbles;  // the launch does not report its longest key
+  depth_bound_ = std::max(depth_bound_, h->max_klen);
   stats_.key_bytes = key_used_;
   stats_.value_bytes = val_used_;
   stats_.n_records = n_rec_;
@@ -2469,6 +2474,7 @@ int Trie::del(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool devi
   if (e == cudaSuccess) e = cudaMemsetAsync(stamp, 0, nf, st_);
   if (e != cudaSuccess) return check_cuda(e, "delete copy");
   DirtyList dl{dirty_ref_, dirty_depth_};
+  ctr_stale_ = true;  // until the counters are read
   count_launch(), k_del_walk<<<blocks_for(n), kThreads, 0, st_>>>(tv_, dl, dk, di ? di : keys_indexs, n, keys_bytes,
                                                                   dtid ? dtid : trie_ids, hslot, hext, stamp);
   if ((rc = sync_counters())) return rc;

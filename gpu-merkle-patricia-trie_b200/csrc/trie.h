@@ -196,6 +196,7 @@ class Trie {
   uint64_t cap_keys_ = 0, cap_vals_ = 0;
   uint32_t n_full_ = 0, n_short_ = 0, n_value_ = 0;
   uint32_t n_dirty_ = 0;       // nodes marked since the last hash (as of the last counters)
+  bool ctr_stale_ = false;     // a call launched work whose counters have not been read
   int sms_ = 0, max_grid_ = 0;  // CTAs of the cooperative kernels that fit co-resident
   void *grid_ctl_ = nullptr;    // GridCtl of the hash launches
   cudaEvent_t hash_ev_[2] = {nullptr, nullptr};  // timing mode, during a hash pass
