@@ -1206,7 +1206,7 @@ def run_ours(args, world, rank, local):
                      "avg_launch_us": round(avg_launch_s * 1e6, 2),
                      # the hash kernels are integer-pipe bound: Keccak-f permutations per second
                      # over the measured rate of the same permutation in a register-only loop
-                     "int_pipe": {"kernel": "k_hash_level + k_hash_full_warp",
+                     "int_pipe": {"kernel": "k_hash_level + k_hash_warp",
                                   "permutations_per_step": int(sum(perms) / len(stats_all)),
                                   "achieved_perm_per_s": round(sum(perms) / (sum(hk_ms) / 1e3), 1),
                                   "peak_perm_per_s": round(kpeak, 1),

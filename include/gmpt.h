@@ -356,8 +356,9 @@ int gmpt_flush_dirty(gmpt_trie *t, const uint8_t **hashs, const uint8_t **encs,
  *   "local_sort"  1/0: same for the still-tied runs of the batch sort;
  *   "local_build_cap", "local_sort_cap" N (<= 2048; 0 = 2048): the largest
  *                      segment / run finished inside one CTA;
- *   "latch_ways"  1/2/4: keys each LockNU thread walks together (default 4:
- *                      more loads in flight; 1: more threads for small batches);
+ *   "latch_ways"  1/2/4: most keys a LockNU thread walks together (default 4:
+ *                      more loads in flight); batches of up to 2^17 keys take
+ *                      1 and of up to 2^23 at most 2, for more threads;
  *   "latch_dedup" 0/1/2: LockNU drops repeated keys of a batch before the
  *                      walk: never / batches of >= 64K keys (default) / always;
  *   "sort_dedup"  0/1/2: PhaseNU drops repeated keys of a batch (keeping the
