@@ -699,6 +699,28 @@ int gmpt_set_timing(gmpt_trie *t, int on) {
 
 uint64_t gmpt_launch_count(void) { return gmpt::launch_count(); }
 
+// n messages of host memory in `bytes` bytes of data: index pairs, or rows of
+// `width` bytes when there are none.  One device allocation per call.
+static int keccak_host(const uint8_t *data, int64_t bytes, const int64_t *indexs, int64_t width, int n,
+                       uint8_t *out32) {
+  const size_t idx_bytes = indexs ? sizeof(int64_t) * 2 * (size_t)n : 0, out_bytes = 32 * (size_t)n;
+  uint8_t *d_out = nullptr;  // digests, index pairs, messages and the over-read of their last word
+  cudaStream_t st = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMalloc(&d_out, out_bytes + idx_bytes + (size_t)bytes + 64);
+  uint8_t *d_data = d_out + out_bytes + idx_bytes;
+  int64_t *d_idx = indexs ? reinterpret_cast<int64_t *>(d_out + out_bytes) : nullptr;
+  if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(d_data, data, (size_t)bytes, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && indexs) e = cudaMemcpyAsync(d_idx, indexs, idx_bytes, cudaMemcpyHostToDevice, st);
+  int rc = e == cudaSuccess ? gmpt::keccak256_batch_device(d_data, d_idx, n, d_out, st, width) : GMPT_E_CUDA;
+  if (rc == 0) e = cudaMemcpyAsync(out32, d_out, out_bytes, cudaMemcpyDeviceToHost, st);
+  if (rc == 0 && e == cudaSuccess) e = cudaStreamSynchronize(st);
+  cudaFree(d_out);
+  if (st) cudaStreamDestroy(st);
+  if (rc == 0 && e != cudaSuccess) rc = GMPT_E_CUDA;
+  return record(rc, rc ? std::string("keccak batch: ") + cudaGetErrorString(e) : std::string());
+}
+
 int gmpt_keccak256_batch(const uint8_t *data, const int64_t *indexs, int n, uint8_t *out32) {
   if (n < 0 || (n > 0 && (!data || !indexs || !out32))) return record(GMPT_E_ARG, "null argument");
   if (n == 0) return record(0, "");
@@ -709,24 +731,14 @@ int gmpt_keccak256_batch(const uint8_t *data, const int64_t *indexs, int n, uint
       return record(GMPT_E_ARG, "bad index pair");
     bytes = std::max<int64_t>(bytes, indexs[2 * i + 1] + 1);
   }
-  uint8_t *d_data = nullptr, *d_out = nullptr;
-  int64_t *d_idx = nullptr;
-  cudaStream_t st = nullptr;
-  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&d_data, (size_t)bytes + 64);
-  if (e == cudaSuccess) e = cudaMalloc(&d_idx, sizeof(int64_t) * 2 * (size_t)n);
-  if (e == cudaSuccess) e = cudaMalloc(&d_out, 32 * (size_t)n);
-  if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(d_data, data, (size_t)bytes, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_idx, indexs, sizeof(int64_t) * 2 * (size_t)n, cudaMemcpyHostToDevice, st);
-  int rc = e == cudaSuccess ? gmpt::keccak256_batch_device(d_data, d_idx, n, d_out, st) : GMPT_E_CUDA;
-  if (rc == 0) e = cudaMemcpyAsync(out32, d_out, 32 * (size_t)n, cudaMemcpyDeviceToHost, st);
-  if (rc == 0 && e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(d_data);
-  cudaFree(d_idx);
-  cudaFree(d_out);
-  if (st) cudaStreamDestroy(st);
-  if (rc == 0 && e != cudaSuccess) rc = GMPT_E_CUDA;
-  return record(rc, rc ? std::string("keccak batch: ") + cudaGetErrorString(e) : std::string());
+  return keccak_host(data, bytes, indexs, 0, n, out32);
+}
+
+int gmpt_keccak256_rows(const uint8_t *data, int64_t width, int n, uint8_t *out32) {
+  if (n < 0 || (n > 0 && (!data || !out32))) return record(GMPT_E_ARG, "null argument");
+  if (n == 0) return record(0, "");
+  if (width < 0 || width > (INT64_MAX >> 8) / n) return record(GMPT_E_ARG, "bad row width");
+  return keccak_host(data, width * n, nullptr, width, n, out32);
 }
 
 int gmpt_keccak256_batch_device(const uint8_t *d_data, const int64_t *d_indexs, int n, uint8_t *d_out32,

@@ -10,12 +10,13 @@
 
 namespace gmpt {
 
-__global__ void __launch_bounds__(128) k_keccak256_batch(const uint8_t *data, const int64_t *offs, int n,
-                                                         uint8_t *out) {
+__global__ void __launch_bounds__(128) k_keccak256_batch(const uint8_t *data, const int64_t *offs,
+                                                         int64_t width, int n, uint8_t *out) {
   extern __shared__ uint32_t stage_all[];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int64_t s = offs[2 * i], e = offs[2 * i + 1];
+  // no index pairs: rows of `width` bytes, one after the other
+  int64_t s = offs ? offs[2 * i] : i * width, e = offs ? offs[2 * i + 1] : s + width - 1;
   uint64_t len = (e >= s - 1 && s >= 0) ? (uint64_t)(e - s + 1) : 0;
   const uint8_t *p = data + s;
   Sponge sp;

@@ -1741,11 +1741,12 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 uint64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 // Keccak-256 of n messages (inclusive [start, end] int64 index pairs into
-// data); device pointers, synchronous.
-int keccak256_batch_device(const uint8_t *d_data, const int64_t *d_idx, int n, uint8_t *d_out, cudaStream_t st) {
+// data, or rows of `width` bytes without pairs); device pointers, synchronous.
+int keccak256_batch_device(const uint8_t *d_data, const int64_t *d_idx, int n, uint8_t *d_out, cudaStream_t st,
+                           int64_t width) {
   if (n <= 0) return OK;
   size_t smem = sizeof(uint64_t) * 17 * kHashThreads;
-  count_launch(), k_keccak256_batch<<<blocks_for(n, kHashThreads), kHashThreads, smem, st>>>(d_data, d_idx, n, d_out);
+  count_launch(), k_keccak256_batch<<<blocks_for(n, kHashThreads), kHashThreads, smem, st>>>(d_data, d_idx, width, n, d_out);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return e == cudaSuccess ? OK : E_CUDA;
@@ -1867,7 +1868,7 @@ int keccak256_batch_noalloc(const uint8_t *data, const int64_t *indexs, int n, u
   if (e == cudaSuccess) {
     size_t smem = sizeof(uint64_t) * 17 * kHashThreads;
     count_launch(),
-        k_keccak256_batch<<<blocks_for(n, kHashThreads), kHashThreads, smem, st>>>(d_data, d_idx, n, d_out);
+        k_keccak256_batch<<<blocks_for(n, kHashThreads), kHashThreads, smem, st>>>(d_data, d_idx, 0, n, d_out);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(out32, d_out, 32 * (size_t)n, cudaMemcpyDeviceToHost, st);

@@ -31,7 +31,8 @@ EXPORTS = [
     "gmpt_puts_2phase_device", "gmpt_puts_latching_device", "gmpt_hash_onepass", "gmpt_pending_targets",
     "gmpt_get_root_hash", "gmpt_gets_parallel", "gmpt_get_values", "gmpt_get_stats", "gmpt_set_timing",
     "gmpt_last_error", "gmpt_last_error_message", "gmpt_free_buffer", "gmpt_stream",
-    "gmpt_keccak256_batch", "gmpt_keccak256_batch_device", "gmpt_keccak_peak", "gmpt_launch_count",
+    "gmpt_keccak256_batch", "gmpt_keccak256_rows", "gmpt_keccak256_batch_device", "gmpt_keccak_peak",
+    "gmpt_launch_count",
     "gmpt_keccak256_batch_noalloc", "gmpt_set_option",
     "gmpt_create_forest", "gmpt_max_tries", "gmpt_puts_2phase_forest", "gmpt_puts_latching_forest",
     "gmpt_get_roots", "gmpt_gets_forest", "gmpt_block_update", "gmpt_block_update_device", "gmpt_block_info",
@@ -164,6 +165,7 @@ def lib():
     L.gmpt_stream.argtypes = [vp]
     L.gmpt_free_buffer.argtypes = [vp]
     L.gmpt_keccak256_batch.argtypes = [vp, vp, i32, vp]
+    L.gmpt_keccak256_rows.argtypes = [vp, C.c_int64, i32, vp]
     L.gmpt_keccak256_batch_device.argtypes = [vp, vp, i32, vp, vp]
     L.gmpt_keccak256_batch_noalloc.argtypes = [vp, vp, i32, vp]
     L.gmpt_keccak256_batch_noalloc.restype = i32
@@ -238,16 +240,8 @@ def keccak256_rows(msgs: np.ndarray, chunk: int = 1 << 22) -> np.ndarray:
     rows, width = msgs.shape
     out = np.empty((rows, 32), dtype=np.uint8)
     for a in range(0, rows, chunk):
-        m = msgs[a: a + chunk]
-        k = len(m)
-        idx = np.empty(2 * k, dtype=np.int64)
-        starts = np.arange(k, dtype=np.int64) * width
-        idx[0::2] = starts
-        idx[1::2] = starts + width - 1
-        data = np.concatenate([m.reshape(-1), np.zeros(8, np.uint8)])
-        o = np.empty(32 * k, dtype=np.uint8)
-        _check(lib().gmpt_keccak256_batch(_p(data), _p(idx), k, _p(o)))
-        out[a: a + k] = o.reshape(k, 32)
+        m, o = msgs[a: a + chunk], out[a: a + chunk]  # read and written in place
+        _check(lib().gmpt_keccak256_rows(_p(m), width, len(m), _p(o)))
     return out
 
 

@@ -466,7 +466,9 @@ void *gmpt_stream(gmpt_trie *t);
  * standalone batch kernel is keccak_kernel_batch
  * (hash/batch_mode_hash.cuh:89-115). */
 int gmpt_keccak256_batch(const uint8_t *data, const int64_t *indexs, int n, uint8_t *out32);
-/* Same with device arrays, on `stream` (a cudaStream_t, or NULL). */
+/* Same for n messages of `width` bytes that lie one after the other. */
+int gmpt_keccak256_rows(const uint8_t *data, int64_t width, int n, uint8_t *out32);
+/* gmpt_keccak256_batch with device arrays, on `stream` (a cudaStream_t, or NULL). */
 int gmpt_keccak256_batch_device(const uint8_t *d_data, const int64_t *d_indexs, int n, uint8_t *d_out32,
                                 void *stream);
 /* gmpt_keccak256_batch without any device allocation.  No counterpart in the
