@@ -41,9 +41,10 @@ constexpr uint32_t kWarpLeafMax = 2048;
 constexpr size_t kPackBytes = 256 << 10;
 // dirty lists of at most this many nodes are hashed by one cooperative launch
 constexpr uint32_t kGridHashMax = 1u << 17;
-// larger lists whose branches are spread over at least this many nibble
-// depths have their branches hashed by one, after the leaves
+// larger lists whose branches (at most kGridDeepMax) are spread over at least
+// this many nibble depths have their branches hashed by one, after the leaves
 constexpr int kGridLevels = 24;
+constexpr uint32_t kGridDeepMax = 1u << 20;
 constexpr uint64_t kHashBarrierNs = 2000000000ull;  // longest grid-barrier wait of such a launch
 // shared memory of a cooperative launch's CTA: message words per thread, a
 // message window per warp
@@ -1155,13 +1156,15 @@ int Trie::bucket_and_hash() {
   }
   int branch_levels = 0;
   for (uint32_t d = 0; d < dirty_depths(); ++d) branch_levels += off[level_bin(d) + kHashClasses] > off[level_bin(d)];
-  const bool deep = branch_levels >= kGridLevels;
+  // many levels, each as long as its slowest branch: one cooperative launch
+  // over all branches (the first wave holds the lowest branch of every path,
+  // whatever its depth).  With more branches the levels fill the GPU and the
+  // level kernels' six CTAs an SM win: 8M word keys of 8-96 bytes take 32 ms
+  // of hashing this way, 25 ms by levels; 512K take 6.8 and 7.4 ms a pass.
+  const uint32_t a = off[level_bin(0)];
+  const bool deep = branch_levels >= kGridLevels && nd - a <= kGridDeepMax;
   if (deep) {
-    // many levels, each as long as its slowest branch: one cooperative launch
-    // over all branches (the first wave holds the lowest branch of every path,
-    // whatever its depth)
     ++levels;
-    const uint32_t a = off[level_bin(0)];
     if ((rc = launch_hash_grid(sorted + a, nd - a))) return rc;
   }
   for (int d = deep ? -1 : (int)dirty_depths() - 1; d >= 0; --d) {
