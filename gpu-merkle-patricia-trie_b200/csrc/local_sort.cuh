@@ -144,7 +144,9 @@ __global__ void __launch_bounds__(256) k_local_sort_warp(TrieView tv, const uint
   uint64_t ko = on ? koff[it] : 0ull;
   uint32_t group = on ? 0u : 1u;  // first position of the lane's tied group (lanes past m: one of their own)
   const int nchunks = (int)((maxlen + 7) / 8);
-  for (int c = c0; c <= nchunks; ++c) {  // the last pass: the key length
+  // the last pass is the key length; a run whose keys all end before chunk c0
+  // (longer keys elsewhere kept the batch sort going) still takes it
+  for (int c = min(c0, nchunks); c <= nchunks; ++c) {
     const uint32_t ch = !on ? 0u : (c < nchunks ? key_chunk(tv.keys, ko, len, c) : len);
     // place inside the group: members with a smaller chunk, or an equal one and before this lane
     uint32_t less = 0, eq = 0;
@@ -195,10 +197,12 @@ __global__ void __launch_bounds__(kThreads) k_local_sort(TrieView tv, const uint
   }
   __syncthreads();
   const int nchunks = (int)((L.maxlen + 7) / 8);
+  // keys that all end before chunk c0 are still parted by their length
+  const int first = min(c0, nchunks);
   int src = 0;
   // tied[k] == 1: item k equals item k-1 on everything compared so far
-  // (all items start tied: they share the chunks before c0)
-  for (int c = c0; c <= nchunks; ++c) {
+  // (all items start tied: they share the chunks before `first`)
+  for (int c = first; c <= nchunks; ++c) {
     // group rank of each item = number of group starts before it
     // (thread t owns items [t * ipt, t * ipt + ipt))
     uint32_t starts = 0;
@@ -208,7 +212,7 @@ __global__ void __launch_bounds__(kThreads) k_local_sort(TrieView tv, const uint
       if (r > ipt) break;
       int k = threadIdx.x * ipt + r;  // r == ipt: the next thread's first item
       bool tied_prev;
-      if (c == c0)
+      if (c == first)
         tied_prev = k > 0 && k < m;
       else
         tied_prev = k > 0 && k < m && L.key[src][k] == L.key[src][k - 1];
@@ -252,12 +256,12 @@ __global__ void __launch_bounds__(kThreads) k_local_sort(TrieView tv, const uint
       if (r >= ipt || k >= m) continue;
       rank += st[r];
       gid[r] = (uint16_t)(rank - 1);
-      if (c > c0 && st[r]) L.gbeg[rank - 1] = (uint16_t)k;
+      if (c > first && st[r]) L.gbeg[rank - 1] = (uint16_t)k;
       L.key[src][k] = ((uint64_t)(rank - 1) << 32) | ch[r];
     }
-    if (c > c0 && threadIdx.x == 0) L.gbeg[ngroups] = (uint16_t)m;  // ngroups < m <= kSortLocalCap
+    if (c > first && threadIdx.x == 0) L.gbeg[ngroups] = (uint16_t)m;  // ngroups < m <= kSortLocalCap
     __syncthreads();
-    if (c > c0) {
+    if (c > first) {
       // Largest tied group: when every group is small (the usual tail, a
       // few pairs among singletons), each item finds its place in its group
       // by counting the members that order before it -- one pass instead
