@@ -46,7 +46,8 @@ __device__ __forceinline__ uint64_t global_ns() {
 // A barrier wait longer than GridCtl::barrier_ns (2 s unless the trie's
 // "block_barrier_ns" option says otherwise) gives up: the CTA raises
 // ERR_BARRIER and leaves the kernel, and so does every CTA at its next
-// barrier.
+// barrier.  A hash call then hashes its list again level by level, a block
+// update ends with an error.
 
 // Grid-wide barrier of a cooperative launch (all CTAs co-resident).
 // Returns false when this CTA must stop.

@@ -45,7 +45,10 @@ constexpr uint32_t kGridHashMax = 1u << 17;
 // this many nibble depths have their branches hashed by one, after the leaves
 constexpr int kGridLevels = 24;
 constexpr uint32_t kGridDeepMax = 1u << 20;
-constexpr uint64_t kHashBarrierNs = 2000000000ull;  // longest grid-barrier wait of such a launch
+// while the trie holds no value longer than this: a value is one serial chain
+// (2.2 us a 136-byte block in a warp, 4.9 in a thread: 0.3 and 0.6 s here),
+// which the others of such a launch would wait for at its grid barrier
+constexpr uint32_t kGridValueMax = 16u << 20;
 // shared memory of a cooperative launch's CTA: message words per thread, a
 // message window per warp
 constexpr size_t kGridSmem = sizeof(uint32_t) * kStageWords * kGridThreads + (kGridThreads / 32) * kWarpMsgBytes;
@@ -1112,27 +1115,55 @@ int Trie::bucket_dirty(uint32_t nd, uint32_t **sorted_out, std::vector<uint32_t>
   return OK;
 }
 
-// PhaseHC over every node marked dirty since the last hash.
+// PhaseHC over every node marked dirty since the last hash, and the counters.
 int Trie::bucket_and_hash() {
-  cudaError_t e = cudaSuccess;
   const uint32_t nd = n_dirty_;  // every call that marks nodes ends with the counters
   stats_.last_dirty = nd;
   stats_.last_hash_levels = 0;
   if (nd == 0) return OK;
-  if (nd <= kGridHashMax) {
-    int rc = begin_hash_timing();
-    if (!rc) rc = launch_hash_grid(dirty_ref_, nd);
-    if (rc || (rc = end_hash_timing())) return rc;
-    stats_.last_hash_levels = stats_.hash_launches = 1;
-    return end_hash(nd);
+  bool coop = max_value_len_ <= kGridValueMax;
+  int rc = hash_pass(nd, coop);
+  if (rc || (rc = copy_counters())) return rc;
+  if (coop && (h_ctr_->error & ERR_BARRIER)) {
+    // A grid barrier of the cooperative launch gave up (block_barrier_ns) and
+    // some nodes have no hash yet.  Every CTA has left, and neither the list
+    // nor its marks have changed: hash it all again level by level, where no
+    // CTA waits for another.
+    const uint32_t others = h_ctr_->error & ~ERR_BARRIER;
+    cudaError_t e = cudaMemsetAsync(&ctr_->error, 0, 4, st_);
+    if (e == cudaSuccess) e = clear_grid_ctl();
+    if (e != cudaSuccess) return check_cuda(e, "hash again");
+    coop = false;
+    if ((rc = hash_pass(nd, coop)) || (rc = copy_counters())) return rc;
+    h_ctr_->error |= others;
   }
+  if ((rc = end_hash(nd))) return rc;
+  return apply_counters();
+}
+
+// One pass over the nd nodes of the dirty list, which it empties.  coop: it
+// may use cooperative launches; set to whether it did.
+int Trie::hash_pass(uint32_t nd, bool &coop) {
+  const bool whole = coop && nd <= kGridHashMax;
   uint32_t *sorted = nullptr;
   std::vector<uint32_t> off;
-  int rc = bucket_dirty(nd, &sorted, off);
+  int rc = whole ? OK : bucket_dirty(nd, &sorted, off);
   if (rc) return rc;
+  rc = begin_hash_timing();
+  if (!rc && whole) {
+    stats_.last_hash_levels = stats_.hash_launches = 1;
+    rc = launch_hash_grid(dirty_ref_, nd);
+  } else if (!rc) {
+    rc = hash_levels(sorted, off, nd, coop);
+  }
+  const int rc_t = end_hash_timing();  // after an error too
+  return rc ? rc : rc_t;
+}
+
+// The pass over a list that bucket_dirty has ordered.
+int Trie::hash_levels(const uint32_t *sorted, const std::vector<uint32_t> &off, uint32_t nd, bool &coop) {
   size_t smem = sizeof(uint32_t) * kStageWords * kHashThreads;
   int levels = 0;
-  if ((rc = begin_hash_timing())) return rc;
   const size_t smem_warp = 4 * kWarpMsgBytes;
   // a launch of at most kWideGrid CTAs cannot fill the SMs at the
   // throughput form's occupancy: it runs the wide form (more registers per
@@ -1162,10 +1193,11 @@ int Trie::bucket_and_hash() {
   // level kernels' six CTAs an SM win: 8M word keys of 8-96 bytes take 32 ms
   // of hashing this way, 25 ms by levels; 512K take 6.8 and 7.4 ms a pass.
   const uint32_t a = off[level_bin(0)];
-  const bool deep = branch_levels >= kGridLevels && nd - a <= kGridDeepMax;
+  const bool deep = coop && branch_levels >= kGridLevels && nd - a <= kGridDeepMax;
+  coop = deep;
   if (deep) {
     ++levels;
-    if ((rc = launch_hash_grid(sorted + a, nd - a))) return rc;
+    if (int rc = launch_hash_grid(sorted + a, nd - a)) return rc;
   }
   for (int d = deep ? -1 : (int)dirty_depths() - 1; d >= 0; --d) {
     // branches [a, m), the extensions above them [m, z)
@@ -1190,11 +1222,9 @@ int Trie::bucket_and_hash() {
     }
     if (z > m) level(false, sorted + m, z - m);
   }
-  if ((rc = end_hash_timing())) return rc;
   stats_.last_hash_levels = levels;
   stats_.hash_launches = levels;
-  if ((e = cudaMemsetAsync(&ctr_->n_dirty, 0, 4, st_)) != cudaSuccess) return check_cuda(e, "hash reset");
-  return end_hash(nd);
+  return check_cuda(cudaMemsetAsync(&ctr_->n_dirty, 0, 4, st_), "hash reset");
 }
 
 // Timing mode: events around a pass's kernels, and per-node accounting (its
@@ -1207,16 +1237,16 @@ int Trie::begin_hash_timing() {
   if (e == cudaSuccess) e = cudaEventCreate(&hash_ev_[0]);
   if (e == cudaSuccess) e = cudaEventCreate(&hash_ev_[1]);
   if (e == cudaSuccess) e = cudaEventRecord(hash_ev_[0], st_);
-  tv_.account = 1;
+  tv_.account = e == cudaSuccess ? 1 : 0;
   return check_cuda(e, "hash timing");
 }
 
 int Trie::end_hash_timing() {
   tv_.account = 0;
   if (!timing_) return OK;
-  cudaError_t e = cudaEventRecord(hash_ev_[1], st_);
-  if (e == cudaSuccess) e = cudaEventSynchronize(hash_ev_[1]);
-  if (e == cudaSuccess) e = cudaEventElapsedTime(&stats_.t_hash_kernels_ms, hash_ev_[0], hash_ev_[1]);
+  cudaError_t e = hash_ev_[1] ? cudaEventRecord(hash_ev_[1], st_) : cudaSuccess;
+  if (e == cudaSuccess && hash_ev_[1]) e = cudaEventSynchronize(hash_ev_[1]);
+  if (e == cudaSuccess && hash_ev_[1]) e = cudaEventElapsedTime(&stats_.t_hash_kernels_ms, hash_ev_[0], hash_ev_[1]);
   for (auto &x : hash_ev_) {
     if (x) cudaEventDestroy(x);
     x = nullptr;
@@ -1232,11 +1262,13 @@ int Trie::launch_hash_grid(const uint32_t *refs, uint32_t nd) {
   cudaError_t e = cudaSuccess;
   uint32_t *ready = wsp<uint32_t>(ws_.ready, nd, e);
   if (e == cudaSuccess && !grid_ctl_) {
-    GridCtl init{};
-    init.barrier_ns = kHashBarrierNs;
     e = cudaMalloc(&grid_ctl_, sizeof(GridCtl));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(grid_ctl_, &init, sizeof(init), cudaMemcpyHostToDevice, st_);
+    if (e == cudaSuccess) e = clear_grid_ctl();
+  }
+  if (e == cudaSuccess && grid_ns_ != opt_barrier_ns_) {  // 0 before the first launch
+    e = cudaMemcpyAsync(grid_ctl_, &opt_barrier_ns_, 8, cudaMemcpyHostToDevice, st_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+    if (e == cudaSuccess) grid_ns_ = opt_barrier_ns_;
   }
   if (e != cudaSuccess) return check_cuda(e, "hash alloc");
   // enough warps for one node each, within what fits co-resident
@@ -1255,6 +1287,13 @@ int Trie::launch_hash_grid(const uint32_t *refs, uint32_t nd) {
   e = cudaLaunchKernelEx(&cfg, k_hash_grid, tv_, DirtyList{const_cast<uint32_t *>(refs), nullptr}, nd, ready, nd,
                          static_cast<GridCtl *>(grid_ctl_), grid_warp_max(grid));
   return check_cuda(e, "hash launch");
+}
+
+// The control block as a launch expects it (a barrier that gave up leaves it
+// half way); barrier_ns, its first word, stays.
+cudaError_t Trie::clear_grid_ctl() {
+  static_assert(offsetof(GridCtl, barrier_ns) == 0 && sizeof(GridCtl::barrier_ns) == 8, "");
+  return cudaMemsetAsync(static_cast<uint8_t *>(grid_ctl_) + 8, 0, sizeof(GridCtl) - 8, st_);
 }
 
 // After a pass (which has emptied the list on the device): the record for
@@ -1294,7 +1333,6 @@ int Trie::hash() {
   if (ctr_stale_ && (rc = sync_counters())) return rc;
   const bool any = n_dirty_ != 0;
   if ((rc = bucket_and_hash())) return rc;
-  if (any && (rc = sync_counters())) return rc;  // nothing was launched for an empty list
   const bool counted = any && timing_;
   stats_.last_hashed = counted ? h_ctr_->hashed : 0;
   stats_.last_enc_bytes = counted ? h_ctr_->enc_bytes : 0;
@@ -1492,8 +1530,7 @@ int Trie::reset() {
   err_.clear();
   cudaSetDevice(dev_);
   cudaError_t e = cudaMemsetAsync(roots_, 0, sizeof(uint32_t) * n_tries_, st_);
-  if (e == cudaSuccess && grid_ctl_)  // a barrier that gave up leaves it half way (barrier_ns, the first word, stays)
-    e = cudaMemsetAsync(static_cast<uint8_t *>(grid_ctl_) + 8, 0, sizeof(GridCtl) - 8, st_);
+  if (e == cudaSuccess && grid_ctl_) e = clear_grid_ctl();
   if (e == cudaSuccess) e = cudaMemsetAsync(ctr_, 0, sizeof(Counters), st_);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
   if (e != cudaSuccess) return check_cuda(e, "reset");

@@ -186,7 +186,7 @@ class Trie {
   int opt_local_build_cap_ = 0;  // largest segment finished in one CTA (0 = the kernel's capacity)
   int opt_local_sort_cap_ = 0;   // largest tied run finished in one CTA (0 = the kernel's capacity)
   uint32_t opt_retry_limit_ = 1u << 20;  // failed CASes per LockNU key before GMPT_E_RETRY_LIMIT
-  uint64_t opt_barrier_ns_ = 2000000000ull;  // persistent kernel: longest grid-barrier wait
+  uint64_t opt_barrier_ns_ = 2000000000ull;  // cooperative kernels: longest grid-barrier wait
   uint32_t opt_max_full_ = 0;    // branch pool cap (0 = none)
 
   // node pools (capacities in elements)
@@ -199,6 +199,7 @@ class Trie {
   bool ctr_stale_ = false;     // a call launched work whose counters have not been read
   int sms_ = 0, max_grid_ = 0;  // CTAs of the cooperative kernels that fit co-resident
   void *grid_ctl_ = nullptr;    // GridCtl of the hash launches
+  uint64_t grid_ns_ = 0;        // barrier_ns in it
   cudaEvent_t hash_ev_[2] = {nullptr, nullptr};  // timing mode, during a hash pass
   uint64_t n_rec_ = 0, key_used_ = 0, val_used_ = 0;
   // longest key (nibbles) and value (bytes) staged since the last reset:
@@ -329,6 +330,9 @@ class Trie {
   // mixed batch: keep only the m kept writes' key bytes in the arena
   int compact_rw_keys(int m, const uint32_t *kept, uint64_t *koff, const uint32_t *klen, uint64_t key_base);
   int bucket_and_hash();
+  int hash_pass(uint32_t nd, bool &coop);
+  int hash_levels(const uint32_t *sorted, const std::vector<uint32_t> &off, uint32_t nd, bool &coop);
+  cudaError_t clear_grid_ctl();
   int begin_hash_timing();
   int end_hash_timing();
   int launch_hash_grid(const uint32_t *refs, uint32_t nd);

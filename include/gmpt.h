@@ -379,11 +379,12 @@ int gmpt_flush_dirty(gmpt_trie *t, const uint8_t **hashs, const uint8_t **encs,
  *                      reports GMPT_E_RETRY_LIMIT (default 2^20).  Keys that
  *                      hit it are left out and every other key is in; putting
  *                      the batch again completes it;
- *   "block_barrier_ns" N: longest grid-barrier wait of the persistent block
- *                      kernel (default 2e9); a wait that runs out ends the
- *                      launch with GMPT_E_INTERNAL ("grid barrier wait gave
- *                      up") with the block partly applied: gmpt_reset and
- *                      reload the trie;
+ *   "block_barrier_ns" N: longest grid-barrier wait of the cooperative
+ *                      kernels (default 2e9).  A wait that runs out ends a
+ *                      block update with GMPT_E_INTERNAL ("grid barrier wait
+ *                      gave up") with the block partly applied: gmpt_reset
+ *                      and reload the trie.  gmpt_hash_onepass hashes the
+ *                      same nodes again level by level, without such waits;
  *   "max_branch_nodes" N: the branch pool stops growing at N nodes (0 = no
  *                      cap); a batch that needs more fails with
  *                      GMPT_E_CAPACITY from the kernel that ran out, partly
