@@ -254,6 +254,7 @@ __device__ inline void wave_by_pairs(const TrieView &tv, const GridPlace &g, con
         top = e != kNoNode ? __ldcg(tv.short_depth + e) : __ldcg(tv.full_depth + f);
       }
     }
+    __syncwarp();  // an extension of more blocks than one reads both lanes' halves back (hash_node below)
     // the extension above: [header][key][0xa0][hash], one block
     EncItem key{0, 0, 0, nullptr, 0};
     if (e != kNoNode) key = compact_item(tv, __ldcg(tv.short_key + e), __ldcg(tv.short_klen + e));
