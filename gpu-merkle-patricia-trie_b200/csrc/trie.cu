@@ -219,6 +219,7 @@ int Trie::fail(int code, const std::string &msg) {
 
 int Trie::check_cuda(cudaError_t e, const char *what) {
   if (e == cudaSuccess) return OK;
+  cudaGetLastError();  // reported here, not again by the next call's launch check
   return fail(E_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
@@ -393,6 +394,8 @@ int Trie::stage(const BatchIn &batch, uint64_t &key_base, uint64_t &vid_base, ui
                 const int **tid_out) {
   BatchIn b = batch;
   const int n = b.n;
+  if (ctr_stale_)  // the pools are sized from the node counts
+    if (int rc = sync_counters()) return rc;
   ctr_stale_ = true;  // until the counters are read
   cudaError_t e = cudaSuccess;
   int64_t kbytes = b.keys_bytes, vbytes = b.values_bytes;
@@ -851,6 +854,7 @@ int Trie::build_levels(int T) {
                  ws_.sb_d0.as<uint32_t>(),   ws_.sb_slot.as<uint64_t>(), ws_.sb_code.as<uint64_t>(),
                  ws_.lcp.as<uint16_t>()};
   DirtyList dl{dirty_ref_, dirty_depth_};
+  ctr_stale_ = true;  // until the counters are read
   uint8_t *kflags = wsp<uint8_t>(ws_.kflags, (size_t)T, e);
   uint8_t *knib = wsp<uint8_t>(ws_.knib, (size_t)T, e);
   unsigned long long *flags = wsp<unsigned long long>(ws_.flags, (size_t)T, e);
@@ -1019,6 +1023,7 @@ int Trie::put_2phase(const BatchIn &b) {
   if (e == cudaSuccess) e = cudaMemsetAsync(d_tot, 0, 16, st_);
   if (e != cudaSuccess) return check_cuda(e, "walk alloc");
   DirtyList dl{dirty_ref_, dirty_depth_};
+  ctr_stale_ = true;  // until the counters are read
   count_launch(), k_walk<<<blocks_for((m + kWalkWays - 1) / kWalkWays), kThreads, 0, st_>>>(tv_, dl, uord, m, koff,
                                                                                              klen, vid_base, wo, tid);
   count_launch(), k_pseudo_ranks<<<blocks_for(m), kThreads, 0, st_>>>(tv_, wo, m);
@@ -1630,6 +1635,7 @@ int Trie::put_latching(const BatchIn &b) {
   // the largest (16M zipf updates 3.48, 3.61, 3.82 ms).
   const int n_ins = rw_ ? rw_kept_ : b.n;
   const int ways = std::min(opt_latch_ways_, n_ins <= kLatchOneWay ? 1 : (n_ins <= kLatchTwoWays ? 2 : 4));
+  ctr_stale_ = true;  // until the counters are read
   auto kern = ways == 1 ? k_latch_insert<1> : (ways == 2 ? k_latch_insert<2> : k_latch_insert<4>);
   count_launch(), kern<<<blocks_for((n_ins + ways - 1) / ways), kThreads, 0, st_>>>(tv_, dl, koff, klen, b.n, vid_base,
                                                                                  opt_retry_limit_, tid, ks);
@@ -2166,7 +2172,8 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
     vb = n ? (int64_t)b.values_indexs[2 * n - 1] + 1 : 0;
   }
   if (kb < 0 || vb < 0 || kb > 0x7FFFFFFFll) return fail(E_ARG, "bad stream lengths");
-  int rc = ensure_capacity((uint64_t)n, 3ull * n, (uint64_t)n, (uint64_t)n, (uint64_t)kb + 72, (uint64_t)vb + 80);
+  int rc = ctr_stale_ ? sync_counters() : OK;  // the pools are sized from the node counts
+  if (!rc) rc = ensure_capacity((uint64_t)n, 3ull * n, (uint64_t)n, (uint64_t)n, (uint64_t)kb + 72, (uint64_t)vb + 80);
   if (rc) return rc;
   if ((rc = block_buffers(n, kb, vb, b.n_out)) || (rc = grid_limits())) return rc;
   cudaError_t e = cudaSuccess;
@@ -2494,7 +2501,10 @@ int Trie::del(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool devi
     keys_bytes = (int64_t)keys_indexs[2 * n - 1] + 1;
   }
   if (keys_bytes < 0) return fail(E_ARG, "bad index pairs");
-  int rc = OK;  // the node counts are as of the last call
+  // the node counts are as of the last call, unless it stopped half way; the
+  // walk's arrays are sized from them
+  int rc = ctr_stale_ ? sync_counters() : OK;
+  if (rc) return rc;
   const cudaMemcpyKind kind = device_inputs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   // keys, index pairs and trie ids of device batches are read where they lie
   // (the walk reads no byte outside its key)
