@@ -1,4 +1,5 @@
 // trie.cu -- host orchestration of the B200 MPT update path.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -121,6 +122,37 @@ cudaError_t grow_pool(uint8_t *&base, const PoolArray (&arrays)[N], size_t old_n
   base = q;
   for (size_t k = 0; k < N; ++k) *arrays[k].p = q + off[k];
   return cudaSuccess;
+}
+
+// Whether kernels on device dev can read [p, p + bytes) of a caller's array
+// where it lies: aligned, and whole inside one allocation of that device (or
+// of pinned host memory).  An array on another device, one that runs past its
+// allocation or one the driver does not know is copied instead, and the copy
+// decides, as a kernel's read of it would fault.  Asked anew on every call;
+// the driver answers from its table of allocations.
+bool in_place(const void *p, size_t bytes, size_t align, int dev) {
+  using Attrs = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+  static const Attrs attrs = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<Attrs>(f);
+  }();
+  if (!attrs || reinterpret_cast<uintptr_t>(p) % align != 0) return false;
+  if (bytes == 0) return true;
+  unsigned type = 0;
+  int ordinal = -1;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void *out[] = {&type, &ordinal, &start, &size};
+  const CUdeviceptr a = reinterpret_cast<CUdeviceptr>(p);
+  if (attrs(4, which, out, a) != CUDA_SUCCESS) return false;
+  if (type != CU_MEMORYTYPE_HOST && (type != CU_MEMORYTYPE_DEVICE || ordinal != dev)) return false;
+  return a >= start && bytes <= size && a - start <= size - bytes;
 }
 
 template <typename T>
@@ -447,11 +479,11 @@ int Trie::stage(const BatchIn &batch, uint64_t &key_base, uint64_t &vid_base, ui
   in.val_base = val_used_;
   in.vid_base = vid_base;
   in.check_stream = b.raw_keys ? 0 : 1;  // expanded raw keys are well formed by construction
-  // device arrays are read where they lie, host arrays (and device arrays
-  // not aligned to their element) are copied
+  // device arrays are read where they lie if they can be (in_place), others
+  // and host arrays are copied
   auto at = [&](auto *p, DevBlock &w, size_t count) -> decltype(p) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
-    if (!p || e != cudaSuccess || (b.device && reinterpret_cast<uintptr_t>(p) % alignof(T) == 0)) return p;
+    if (!p || e != cudaSuccess || (b.device && in_place(p, count * sizeof(T), alignof(T), dev_))) return p;
     T *d = wsp<T>(w, count, e);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d, p, count * sizeof(T), kind, st_);
     return d;
@@ -469,12 +501,12 @@ int Trie::stage(const BatchIn &batch, uint64_t &key_base, uint64_t &vid_base, ui
     in.keys = karena + key_base;
   } else {
     in.ki = at(b.keys_indexs, ws_.ki, 2 * (size_t)n);
-    in.copy_keys = b.device && (reinterpret_cast<uintptr_t>(b.keys_hexs) & 7) == 0;
+    in.copy_keys = b.device && in_place(b.keys_hexs, (size_t)kbytes, 8, dev_);
     in.keys = in.copy_keys ? b.keys_hexs : karena + key_base;
     if (e == cudaSuccess && !in.copy_keys)
       e = cudaMemcpyAsync(karena + key_base, b.keys_hexs, (size_t)kbytes, kind, st_);
   }
-  in.copy_vals = b.device && (reinterpret_cast<uintptr_t>(b.values) & 15) == 0;
+  in.copy_vals = b.device && in_place(b.values, (size_t)vbytes, 16, dev_);
   in.vals = b.values;
   if (e == cudaSuccess && !in.copy_vals)
     e = cudaMemcpyAsync(varena + val_used_, b.values, (size_t)vbytes, kind, st_);
@@ -1448,22 +1480,17 @@ int Trie::gets(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool dev
   uint64_t *dhp = wsp<uint64_t>(ws_.g_hp, (size_t)n, e);
   int *dlen = wsp<int>(ws_.g_len, (size_t)n, e);
   // keys, index pairs and trie ids of device batches are read where they lie
-  // (a lookup reads no byte outside its key)
-  const uint8_t *dk = keys_hexs;
-  int *di = nullptr, *dtid = nullptr;
-  if (!device_inputs) {
-    uint8_t *k = wsp<uint8_t>(ws_.g_keys, (size_t)keys_bytes + 64, e);
-    di = wsp<int>(ws_.g_idx, 2 * (size_t)n, e);
-    dtid = trie_ids ? wsp<int>(ws_.g_tid, (size_t)n, e) : nullptr;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(k, keys_hexs, (size_t)keys_bytes, kind, st_);
-    dk = k;
-  }
-  const int *ki = device_inputs ? keys_indexs : di;
-  const int *ti = device_inputs ? trie_ids : dtid;
-  if (e == cudaSuccess && !device_inputs)
-    e = cudaMemcpyAsync(di, keys_indexs, sizeof(int) * 2 * (size_t)n, kind, st_);
-  if (e == cudaSuccess && dtid && !device_inputs)
-    e = cudaMemcpyAsync(dtid, trie_ids, sizeof(int) * (size_t)n, kind, st_);
+  // if they can be (in_place)
+  auto at = [&](auto *p, DevBlock &w, size_t count, size_t room) -> decltype(p) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
+    if (!p || e != cudaSuccess || (device_inputs && in_place(p, count * sizeof(T), alignof(T), dev_))) return p;
+    T *d = wsp<T>(w, room, e);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d, p, count * sizeof(T), kind, st_);
+    return d;
+  };
+  const uint8_t *dk = at(keys_hexs, ws_.g_keys, (size_t)keys_bytes, (size_t)keys_bytes + 64);
+  const int *ki = at(keys_indexs, ws_.g_idx, 2 * nn, 2 * nn);
+  const int *ti = at(trie_ids, ws_.g_tid, nn, nn);
   if (e != cudaSuccess) return check_cuda(e, "gets copy");
   if (device_outputs) {
     count_launch(), k_gets<<<blocks_for(n), kThreads, 0, st_>>>(tv_, dk, ki, n, keys_bytes, out_hp, out_len, nullptr,
@@ -2179,11 +2206,11 @@ int Trie::block_update(const BlockIn &b, uint8_t *out32, int *sizes) {
   cudaError_t e = cudaSuccess;
   BlockDesc *h = static_cast<BlockDesc *>(blk_.h_desc);
   std::memset(h, 0, sizeof(BlockDesc));
-  // device arrays are read where they lie, host arrays (and device arrays
-  // without the alignment the kernels read with) are copied
+  // device arrays are read where they lie if they can be (in_place, with the
+  // alignment the kernels read with), others and host arrays are copied
   const cudaMemcpyKind kind = b.device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   auto at = [&](auto *p, DevBlock &w, size_t bytes, size_t align) -> decltype(p) {
-    if (!p || e != cudaSuccess || (b.device && reinterpret_cast<uintptr_t>(p) % align == 0)) return p;
+    if (!p || e != cudaSuccess || (b.device && in_place(p, bytes, align, dev_))) return p;
     if (bytes) e = cudaMemcpyAsync(w.p, p, bytes, kind, st_);
     return static_cast<decltype(p)>(w.p);
   };
@@ -2507,11 +2534,13 @@ int Trie::del(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool devi
   if (rc) return rc;
   const cudaMemcpyKind kind = device_inputs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   // keys, index pairs and trie ids of device batches are read where they lie
-  // (the walk reads no byte outside its key)
-  uint8_t *dk_copy = device_inputs ? nullptr : wsp<uint8_t>(ws_.g_keys, (size_t)keys_bytes + 64, e);
-  const uint8_t *dk = device_inputs ? keys_hexs : dk_copy;
-  const bool di_here = device_inputs && reinterpret_cast<uintptr_t>(keys_indexs) % alignof(int) == 0;
-  const bool tid_here = device_inputs && reinterpret_cast<uintptr_t>(trie_ids) % alignof(int) == 0;
+  // if they can be (in_place)
+  const size_t nn = (size_t)n;
+  const bool dk_here = device_inputs && in_place(keys_hexs, (size_t)keys_bytes, 1, dev_);
+  uint8_t *dk_copy = dk_here ? nullptr : wsp<uint8_t>(ws_.g_keys, (size_t)keys_bytes + 64, e);
+  const uint8_t *dk = dk_here ? keys_hexs : dk_copy;
+  const bool di_here = device_inputs && in_place(keys_indexs, 8 * nn, alignof(int), dev_);
+  const bool tid_here = device_inputs && trie_ids && in_place(trie_ids, 4 * nn, alignof(int), dev_);
   int *di = di_here ? nullptr : wsp<int>(ws_.g_idx, 2 * (size_t)n, e);
   int *dtid = trie_ids && !tid_here ? wsp<int>(ws_.g_tid, (size_t)n, e) : nullptr;
   const size_t nf = (size_t)n_full_ + 1;
