@@ -102,6 +102,58 @@ __device__ __forceinline__ uint64_t merged_key8(const uint8_t *e, uint32_t le, u
   return v;
 }
 
+// What becomes of a stamped branch: still a branch (0), nothing left of it
+// (kFateGone), or a short node, by its key's length.
+constexpr uint32_t kFateGone = 0xFFFFFFFFu;
+
+// The collapses of one level, reckoned without being made (deeper levels
+// first): every branch's fate, and in need[0] the key bytes and in need[1] the
+// short nodes that k_del_collapse will take for the level.
+__global__ void k_del_need(TrieView tv, const uint32_t *refs, int count, const uint32_t *hext, const uint8_t *stamp,
+                           uint32_t *fate, unsigned long long *need) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t bytes = 0, shorts = 0;
+  if (j < count && ref_kind(refs[j]) == KIND_FULL && stamp[ref_idx(refs[j])]) {
+    const uint32_t id = ref_idx(refs[j]);
+    const uint32_t *ch = tv.full_child + (size_t)id * 17;
+    uint32_t cnt = 0, c1 = 0, ls = 0;  // children left; the last one's slot, and its key's length if it will be short
+    for (uint32_t k = 0; k < 17; ++k) {
+      const uint32_t v = ch[k];
+      if (!v) continue;
+      uint32_t kl = 0, f = kNoNode;  // f: the branch below, straight or under its extension
+      if (ref_kind(v) == KIND_SHORT) {
+        kl = tv.short_klen[ref_idx(v)];
+        const uint32_t below = tv.short_child[ref_idx(v)];
+        if (ref_kind(below) == KIND_FULL) f = ref_idx(below);
+      } else if (ref_kind(v) == KIND_FULL) {
+        f = ref_idx(v);
+      }
+      if (f != kNoNode && stamp[f] && fate[f] != 0) {
+        if (fate[f] == kFateGone) continue;
+        kl = fate[f];
+      }
+      ++cnt;
+      c1 = k;
+      ls = kl;
+    }
+    if (cnt == 0) {
+      fate[id] = kFateGone;
+    } else if (cnt == 1) {
+      const uint32_t e = hext[id];
+      const uint32_t total = (e != kNoExt ? tv.short_klen[e] : 0u) + 1u + (c1 < 16 ? ls : 0u);
+      fate[id] = total;
+      bytes = (total + 7u) & ~7u;
+      shorts = e == kNoExt ? 1u : 0u;
+    }
+  }
+  bytes = __reduce_add_sync(0xffffffffu, bytes);
+  shorts = __reduce_add_sync(0xffffffffu, shorts);
+  if ((threadIdx.x & 31) == 0 && bytes) {
+    atomicAdd(need, (unsigned long long)bytes);
+    atomicAdd(need + 1, (unsigned long long)shorts);
+  }
+}
+
 __global__ void k_del_collapse(TrieView tv, DirtyList dl, const uint32_t *refs, int count, const uint64_t *hslot,
                                const uint32_t *hext, const uint8_t *stamp, unsigned long long *key_cursor,
                                uint64_t key_cap) {
@@ -145,7 +197,8 @@ __global__ void k_del_collapse(TrieView tv, DirtyList dl, const uint32_t *refs, 
     tv.short_dead[s] = 1;
   }
   // the merged key goes to a whole number of aligned words (the host has made
-  // room for the longest key per collapse); the keys read lie below the
+  // room for the longest key per collapse, or for what k_del_need added up);
+  // the keys read lie below the
   // cursor or were written by an earlier launch
   const uint32_t total = le + 1u + ls, room = (total + 7u) & ~7u;
   const unsigned long long off = atomicAdd(key_cursor, (unsigned long long)room);

@@ -206,7 +206,7 @@ Trie::~Trie() {
                         &ws_.tid, &ws_.dd_hash, &ws_.dd_pos, &ws_.dd_sel, &ws_.dd_slot, &ws_.raw, &ws_.dirty_bin, &ws_.rw_flags,
                         &ws_.rw_a, &ws_.rw_b, &ws_.rw_c, &ws_.rw_d, &ws_.rw_e, &ws_.rw_wpos, &ws_.rw_hp,
                         &ws_.rw_len, &ws_.rw_tot, &ws_.rw_kept, &ws_.rw_koff, &ws_.rw_klen, &ws_.rw_tid,
-                        &ws_.del_hslot, &ws_.del_hext, &ws_.del_stamp,
+                        &ws_.del_hslot, &ws_.del_hext, &ws_.del_stamp, &ws_.del_fate,
                         &ws_.pack, &ws_.ready, &ws_.misc};
   for (DevBlock *b : blocks) b->release();
   for (int k = 0; k < 2; ++k) {
@@ -2547,7 +2547,7 @@ int Trie::del(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool devi
   uint64_t *hslot = wsp<uint64_t>(ws_.del_hslot, nf, e);
   uint32_t *hext = wsp<uint32_t>(ws_.del_hext, nf, e);
   uint8_t *stamp = wsp<uint8_t>(ws_.del_stamp, nf, e);
-  unsigned long long *dcnt = wsp<unsigned long long>(ws_.rw_tot, 8, e);  // key cursor
+  unsigned long long *dcnt = wsp<unsigned long long>(ws_.rw_tot, 8, e);  // key cursor; key bytes and short nodes needed
   if (e == cudaSuccess && dk_copy) e = cudaMemcpyAsync(dk_copy, keys_hexs, (size_t)keys_bytes, kind, st_);
   if (e == cudaSuccess && di) e = cudaMemcpyAsync(di, keys_indexs, sizeof(int) * 2 * (size_t)n, kind, st_);
   if (e == cudaSuccess && dtid) e = cudaMemcpyAsync(dtid, trie_ids, sizeof(int) * (size_t)n, kind, st_);
@@ -2568,10 +2568,31 @@ int Trie::del(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool devi
   // the longest, and makes at most one short node.
   uint64_t branches = 0;
   for (uint32_t d = 0; d < dirty_depths(); ++d) branches += off[level_bin(d) + kHashClasses] - off[level_bin(d)];
-  const uint64_t collapses = std::min<uint64_t>(branches, (uint64_t)n);
+  uint64_t collapses = std::min<uint64_t>(branches, (uint64_t)n);
+  uint64_t key_room = collapses * ((depth_bound_ + 8ull) & ~7ull);
   key_used_ = (key_used_ + 7) & ~7ull;
-  if ((rc = ensure_capacity(0, collapses, 0, 0, collapses * ((depth_bound_ + 8ull) & ~7ull) + 64, 0))) return rc;
-  dl = DirtyList{dirty_ref_, dirty_depth_};  // the list may have grown with the short pool
+  if (key_used_ + key_room + 128 > cap_keys_ || n_short_ + collapses > cap_short_) {
+    // That is more than there is: one long key in the trie makes the bound
+    // many times what the collapses append, so add up their real keys first
+    // (launches of a level each, one wait) and grow by those.
+    uint32_t *fate = wsp<uint32_t>(ws_.del_fate, nf, e);
+    if (e == cudaSuccess) e = cudaMemsetAsync(fate, 0, 4 * nf, st_);
+    if (e == cudaSuccess) e = cudaMemsetAsync(dcnt + 1, 0, 16, st_);
+    if (e != cudaSuccess) return check_cuda(e, "delete need");
+    for (int d = (int)dirty_depths() - 1; d >= 0; --d) {
+      const uint32_t a = off[level_bin(d)], z = off[level_bin(d) + kHashClasses];
+      if (z > a)
+        count_launch(), k_del_need<<<blocks_for(z - a), kThreads, 0, st_>>>(tv_, sorted + a, (int)(z - a), hext, stamp,
+                                                                          fate, dcnt + 1);
+    }
+    if ((e = cudaMemcpyAsync(h_small_, dcnt + 1, 16, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st_)) != cudaSuccess)
+      return check_cuda(e, "delete need");
+    key_room = h_small_[0];
+    collapses = h_small_[1];
+    if ((rc = ensure_capacity(0, collapses, 0, 0, key_room + 64, 0))) return rc;
+    dl = DirtyList{dirty_ref_, dirty_depth_};  // the list may have grown with the short pool
+  }
   h_small_[0] = key_used_;
   if ((e = cudaMemcpyAsync(dcnt, h_small_, 8, cudaMemcpyHostToDevice, st_)) != cudaSuccess)
     return check_cuda(e, "delete cursor");

@@ -273,7 +273,7 @@ class Trie {
     DevBlock dirty_bin;                                         // hash bin of each dirty node
     DevBlock rw_flags, rw_a, rw_b, rw_c, rw_d, rw_e, rw_wpos;   // mixed read/write resolution
     DevBlock rw_hp, rw_len, rw_tot, rw_kept, rw_koff, rw_klen, rw_tid;
-    DevBlock del_hslot, del_hext, del_stamp;                    // deletes: how each path branch is linked
+    DevBlock del_hslot, del_hext, del_stamp, del_fate;          // deletes: how each path branch is linked, what becomes of it
     DevBlock ready;                                             // branches ready to be hashed
     DevBlock pack;                                              // a small host batch, or lookups
     DevBlock misc;
