@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <mutex>
@@ -101,28 +102,95 @@ PoolArray pool_array(T *&p, size_t per_node = 1, bool keep = true) {
   return PoolArray{reinterpret_cast<void **>(&p), per_node * sizeof(T), keep};
 }
 
-// Grow a pool of parallel arrays to new_n nodes, all in one allocation (base):
-// a pool of ten arrays paid ten cudaMalloc / cudaFree pairs at every growth.
+// A pool of up to this many bytes is one allocation (if there is one that
+// large); a larger one has an allocation per array.
+constexpr size_t kPoolBlockMax = 4ull << 30;
+
+// Grow a pool of parallel arrays to new_n nodes.  Small pools lie in one
+// allocation (base): ten arrays would take ten cudaMalloc / cudaFree pairs at
+// every growth (a trie of 16M nodes of each kind reserved in 4 ms, against 10).
+// That holds the old pool and the new one at once, which beyond kPoolBlockMax
+// could be most of the device: there every array has its own allocation (base
+// null), and as the pool grows array by array, only one of them is held twice.
+// (If that fails part way, the arrays already moved are longer than the pool's
+// capacity, which is harmless.)
 template <size_t N>
-cudaError_t grow_pool(uint8_t *&base, const PoolArray (&arrays)[N], size_t old_n, size_t new_n, cudaStream_t st,
+cudaError_t grow_pool(uint8_t *&base, const std::array<PoolArray, N> &arrays, size_t old_n, size_t new_n, cudaStream_t st,
                       bool managed, int dev) {
   size_t off[N + 1] = {0};
   for (size_t k = 0; k < N; ++k) off[k + 1] = off[k] + ((new_n * arrays[k].elem + 64 + 255) & ~(size_t)255);
-  uint8_t *q = nullptr;
-  cudaError_t e = grow_array(q, 0, off[N], st, managed, dev);
-  for (size_t k = 0; k < N && e == cudaSuccess; ++k)
-    if (base && old_n && arrays[k].keep)
-      e = cudaMemcpyAsync(q + off[k], *arrays[k].p, old_n * arrays[k].elem, cudaMemcpyDeviceToDevice, st);
-  if (e == cudaSuccess && base) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) {
-    if (q) cudaFree(q);
-    return e;
+  const bool own = !base && *arrays[0].p;  // the old arrays have their own allocations
+  auto fill = [&](size_t k, uint8_t *q) {  // the kept elements of array k into its new place
+    return *arrays[k].p && old_n && arrays[k].keep
+               ? cudaMemcpyAsync(q, *arrays[k].p, old_n * arrays[k].elem, cudaMemcpyDeviceToDevice, st)
+               : cudaSuccess;
+  };
+  auto free_old = [&] {
+    for (size_t k = 0; k < N && own; ++k) cudaFree(*arrays[k].p);
+    if (base) cudaFree(base);
+    base = nullptr;
+  };
+  cudaError_t e = cudaSuccess;
+  uint8_t *block = nullptr;
+  if (off[N] <= kPoolBlockMax && grow_array(block, 0, off[N], st, managed, dev) == cudaSuccess) {
+    for (size_t k = 0; k < N && e == cudaSuccess; ++k) e = fill(k, block + off[k]);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+      cudaFree(block);
+      return e;
+    }
+    free_old();
+    base = block;
+    for (size_t k = 0; k < N; ++k) *arrays[k].p = block + off[k];
+    return cudaSuccess;
   }
-  if (base) cudaFree(base);
-  base = q;
-  for (size_t k = 0; k < N; ++k) *arrays[k].p = q + off[k];
-  return cudaSuccess;
+  cudaGetLastError();  // no such block: smaller pieces may fit
+  uint8_t *fresh[N] = {nullptr};
+  for (size_t k = 0; k < N && e == cudaSuccess; ++k) {
+    e = grow_array(fresh[k], 0, off[k + 1] - off[k], st, managed, dev);
+    if (e == cudaSuccess) e = fill(k, fresh[k]);
+    if (e == cudaSuccess && own && (e = cudaStreamSynchronize(st)) == cudaSuccess) {
+      cudaFree(*arrays[k].p);
+      *arrays[k].p = fresh[k];
+      fresh[k] = nullptr;
+    }
+  }
+  if (e == cudaSuccess && !own && (e = cudaStreamSynchronize(st)) == cudaSuccess) {
+    free_old();
+    for (size_t k = 0; k < N; ++k) {
+      *arrays[k].p = fresh[k];
+      fresh[k] = nullptr;
+    }
+  }
+  for (uint8_t *q : fresh)
+    if (q) cudaFree(q);
+  return e;
 }
+
+// Free a pool in either form.
+template <size_t N>
+void free_pool(uint8_t *&base, const std::array<PoolArray, N> &arrays) {
+  if (base) cudaFree(base);
+  for (const PoolArray &a : arrays) {
+    if (!base && *a.p) cudaFree(*a.p);
+    *a.p = nullptr;
+  }
+  base = nullptr;
+}
+
+// The arrays of the two node pools (of the branch pool, the last two are
+// written and read in one pass).
+std::array<PoolArray, 9> full_arrays(TrieView &tv) {
+  return {pool_array(tv.full_child, 17), pool_array(tv.full_epoch), pool_array(tv.full_depth),
+          pool_array(tv.full_hash, 32),  pool_array(tv.full_hlen),  pool_array(tv.full_dead),
+          pool_array(tv.full_ext),       pool_array(tv.full_par, 1, false), pool_array(tv.full_pend, 1, false)};
+}
+std::array<PoolArray, 10> short_arrays(TrieView &tv) {
+  return {pool_array(tv.short_key),   pool_array(tv.short_klen), pool_array(tv.short_child),    pool_array(tv.short_epoch),
+          pool_array(tv.short_depth), pool_array(tv.short_dead), pool_array(tv.short_hash, 32), pool_array(tv.short_hlen),
+          pool_array(tv.short_claim), pool_array(tv.short_pseudo)};
+}
+using PoolPair = std::array<PoolArray, 2>;
 
 // Whether kernels on device dev can read [p, p + bytes) of a caller's array
 // where it lies: aligned, and whole inside one allocation of that device (or
@@ -191,8 +259,11 @@ Trie::Trie(int device, int geth_mode, int max_tries, bool unified)
 Trie::~Trie() {
   cudaSetDevice(dev_);
   if (st_) cudaStreamSynchronize(st_);
-  void *ptrs[] = {full_base_,         short_base_,        rec_base_, dirty_base_, tv_.value_vid, (void *)tv_.keys,
-                  (void *)tv_.vals, fl_refs_, roots_,    ctr_};
+  free_pool(full_base_, full_arrays(tv_));
+  free_pool(short_base_, short_arrays(tv_));
+  free_pool(rec_base_, PoolPair{pool_array(tv_.rec), pool_array(tv_.rec_hp)});
+  free_pool(dirty_base_, PoolPair{pool_array(dirty_ref_), pool_array(dirty_depth_)});
+  void *ptrs[] = {tv_.value_vid, (void *)tv_.keys, (void *)tv_.vals, fl_refs_, roots_, ctr_};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   DevBlock *blocks[] = {&ws_.koff, &ws_.klen, &ws_.ki, &ws_.vi, &ws_.hp, &ws_.kin, &ws_.order, &ws_.eqprev,
@@ -312,12 +383,7 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
   if (need_full > cap_full_) {
     uint64_t nc = std::min<uint64_t>(grow_to(need_full, cap_full_), kMaxNodes);
     if (opt_max_full_) nc = std::min<uint64_t>(nc, std::max<uint64_t>(opt_max_full_, need_full));
-    const PoolArray arrays[] = {pool_array(tv_.full_child, 17), pool_array(tv_.full_epoch),
-                                pool_array(tv_.full_depth),     pool_array(tv_.full_hash, 32),
-                                pool_array(tv_.full_hlen),      pool_array(tv_.full_dead),
-                                pool_array(tv_.full_ext),       pool_array(tv_.full_par, 1, false),
-                                pool_array(tv_.full_pend, 1, false)};  // the last two: written and read in one pass
-    e = grow_pool(full_base_, arrays, n_full_, nc, st_, managed_, dev_);
+    e = grow_pool(full_base_, full_arrays(tv_), n_full_, nc, st_, managed_, dev_);
     if (e == cudaSuccess) e = cudaMemsetAsync(tv_.full_par, 0xFF, 4 * (size_t)nc, st_);
     if (e != cudaSuccess) return check_cuda(e, "grow branch pool");
     cap_full_ = (uint32_t)nc;
@@ -326,12 +392,7 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
   if (need_short > kMaxNodes) return fail(E_CAPACITY, "short node count exceeds 2^30");
   if (need_short > cap_short_) {
     uint64_t nc = std::min<uint64_t>(grow_to(need_short, cap_short_), kMaxNodes);
-    const PoolArray arrays[] = {pool_array(tv_.short_key),      pool_array(tv_.short_klen),
-                                pool_array(tv_.short_child),    pool_array(tv_.short_epoch),
-                                pool_array(tv_.short_depth),    pool_array(tv_.short_dead),
-                                pool_array(tv_.short_hash, 32), pool_array(tv_.short_hlen),
-                                pool_array(tv_.short_claim),    pool_array(tv_.short_pseudo)};
-    e = grow_pool(short_base_, arrays, n_short_, nc, st_, managed_, dev_);
+    e = grow_pool(short_base_, short_arrays(tv_), n_short_, nc, st_, managed_, dev_);
     if (e != cudaSuccess) return check_cuda(e, "grow short pool");
     cap_short_ = (uint32_t)nc;
   }
@@ -345,8 +406,7 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
   uint64_t need_rec = n_rec_ + add_rec;
   if (need_rec > cap_rec_) {
     uint64_t nc = grow_to(need_rec, cap_rec_);
-    const PoolArray arrays[] = {pool_array(tv_.rec), pool_array(tv_.rec_hp)};
-    e = grow_pool(rec_base_, arrays, n_rec_, nc, st_, managed_, dev_);
+    e = grow_pool(rec_base_, PoolPair{pool_array(tv_.rec), pool_array(tv_.rec_hp)}, n_rec_, nc, st_, managed_, dev_);
     if (e != cudaSuccess) return check_cuda(e, "grow value records");
     cap_rec_ = nc;
   }
@@ -376,8 +436,7 @@ int Trie::ensure_capacity(uint64_t add_full, uint64_t add_short, uint64_t add_va
       cudaStreamSynchronize(st_);
       nd = (uint32_t)(h_small_[0] & 0xFFFFFFFFu);
     }
-    const PoolArray arrays[] = {pool_array(dirty_ref_), pool_array(dirty_depth_)};
-    e = grow_pool(dirty_base_, arrays, nd, nc, st_, managed_, dev_);
+    e = grow_pool(dirty_base_, PoolPair{pool_array(dirty_ref_), pool_array(dirty_depth_)}, nd, nc, st_, managed_, dev_);
     if (e != cudaSuccess) return check_cuda(e, "grow dirty list");
     cap_dirty_ = nc;
   }

@@ -207,7 +207,7 @@ class Trie {
   uint32_t max_key_nibbles_ = 0, max_value_len_ = 0;
   uint32_t depth_bound_ = 0;   // no node is deeper: the longest key of any put since the last reset
   uint32_t dirty_depths() const;
-  uint8_t *full_base_ = nullptr, *short_base_ = nullptr, *rec_base_ = nullptr, *dirty_base_ = nullptr;  // allocations
+  uint8_t *full_base_ = nullptr, *short_base_ = nullptr, *rec_base_ = nullptr, *dirty_base_ = nullptr;  // pools of one allocation (null: one per array)
   uint32_t *roots_ = nullptr;  // [n_tries_] root words
   uint32_t n_tries_ = 1;
   Counters *ctr_ = nullptr;
