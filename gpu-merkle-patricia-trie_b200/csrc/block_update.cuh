@@ -64,9 +64,19 @@ struct BlockBufs {
   BlockDesc *desc;
 };
 
-// Copy the streams into the arenas (8-byte words; the last partial word is
-// masked and 64 zero bytes follow each stream), validate keys and pairs, and
-// build the value records.  Grid-stride; every thread runs to the end.
+// Word w of a stream of n bytes, zero past its end.  A last partial word is
+// taken byte by byte: the stream may be the caller's array, of which no byte
+// past the end is read.
+__device__ __forceinline__ uint64_t stream_word(const uint8_t *src, int64_t n, int64_t w) {
+  if (8 * w + 8 <= n) return reinterpret_cast<const uint64_t *>(src)[w];
+  uint64_t x = 0;
+  for (int64_t b = 8 * w; b < n; ++b) x |= (uint64_t)src[b] << (8 * (b - 8 * w));
+  return x;
+}
+
+// Copy the streams into the arenas (8-byte words; 64 zero bytes follow each
+// stream), validate keys and pairs, and build the value records.  Grid-stride;
+// every thread runs to the end.
 __global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, BlockBufs bb) {
   BlockDesc *D = bb.desc;
   const int n = D->n, n0 = D->n0;
@@ -80,35 +90,21 @@ __global__ void __launch_bounds__(kGridThreads) k_block_stage(TrieView tv, Block
   uint32_t terms = 0, bad = 0, kterms = 0, gap = 0, lmax = 0;
   {
     uint64_t *dst = reinterpret_cast<uint64_t *>(const_cast<uint8_t *>(tv.keys) + key_base);
-    const uint64_t *src = reinterpret_cast<const uint64_t *>(D->keys);
     const int64_t words = (kb + 7) / 8 + 8;
     for (int64_t w = t0; w < words; w += T) {
-      uint64_t x = 0;
-      if (8 * w < kb) {
-        x = src[w];
-        const int64_t rem = kb - 8 * w;
-        if (rem < 8) x &= (1ull << (8 * rem)) - 1;
-        if (x & 0xE0E0E0E0E0E0E0E0ull) bad |= BLOCK_BAD_KEY;  // >= 32
-        const uint64_t hi = x & 0x1010101010101010ull;        // 16..31
-        if (x & ((hi >> 4) * 0x0Full)) bad |= BLOCK_BAD_KEY;  // 17..31
-        terms += __popcll(hi);
-      }
+      const uint64_t x = stream_word(keys, kb, w);
+      if (x & 0xE0E0E0E0E0E0E0E0ull) bad |= BLOCK_BAD_KEY;  // >= 32
+      const uint64_t hi = x & 0x1010101010101010ull;        // 16..31
+      if (x & ((hi >> 4) * 0x0Full)) bad |= BLOCK_BAD_KEY;  // 17..31
+      terms += __popcll(hi);
       dst[w] = x;
     }
   }
   {
     uint64_t *dst = reinterpret_cast<uint64_t *>(const_cast<uint8_t *>(tv.vals) + val_base);
-    const uint64_t *src = reinterpret_cast<const uint64_t *>(D->vals);
+    const uint8_t *vals = D->vals;
     const int64_t words = (vb + 7) / 8 + 8;
-    for (int64_t w = t0; w < words; w += T) {
-      uint64_t x = 0;
-      if (8 * w < vb) {
-        x = src[w];
-        const int64_t rem = vb - 8 * w;
-        if (rem < 8) x &= (1ull << (8 * rem)) - 1;
-      }
-      dst[w] = x;
-    }
+    for (int64_t w = t0; w < words; w += T) dst[w] = stream_word(vals, vb, w);
   }
   for (int64_t i = t0; i < n; i += T) {
     int ks = kidx[2 * i], ke = kidx[2 * i + 1];

@@ -140,7 +140,9 @@ __device__ __forceinline__ ValueRec load_rec(const TrieView &tv, uint64_t vid) {
   return ValueRec{v.x, (uint32_t)v.y, 0u};
 }
 
-// Unaligned 8-byte little-endian load from a byte array padded by >= 8 bytes.
+// Unaligned 8-byte little-endian load: the one or two aligned words that hold
+// a byte of [p, p + 8) (and so up to 7 bytes on either side of it, in the same
+// words).
 __device__ __forceinline__ uint64_t load_u64_unaligned(const uint8_t *p) {
   uintptr_t a = reinterpret_cast<uintptr_t>(p);
   const uint64_t *q = reinterpret_cast<const uint64_t *>(a & ~uintptr_t(7));
@@ -191,9 +193,9 @@ __device__ __forceinline__ int match_nibbles(const uint8_t *a, const uint8_t *b,
   return m;
 }
 
-// Whether nibbles a[0..n) and b[0..n) are equal, reading no byte past either
-// end: four 8-byte pairs in flight at a time, the last word overlapping the
-// one before it.
+// Whether nibbles a[0..n) and b[0..n) are equal: four 8-byte pairs in flight
+// at a time, the last one overlapping the one before it, so that only the
+// aligned words that hold a byte of either range are read.
 __device__ __forceinline__ bool equal_nibbles(const uint8_t *a, const uint8_t *b, uint32_t n) {
   uint32_t o = 0;
   for (; o + 32 <= n; o += 32) {

@@ -1519,7 +1519,7 @@ int Trie::gets(const uint8_t *keys_hexs, const int *keys_indexs, int n, bool dev
     uint8_t *r = wsp<uint8_t>(ws_.g_hp, 12 * nn, e);
     if (e != cudaSuccess) return check_cuda(e, "gets alloc");
     std::memcpy(h_pack_, keys_hexs, (size_t)keys_bytes);
-    std::memset(h_pack_ + keys_bytes, 0, o_idx - (size_t)keys_bytes);  // 8-byte loads read past a key's last byte
+    std::memset(h_pack_ + keys_bytes, 0, o_idx - (size_t)keys_bytes);  // 8-byte loads: words around a key's last byte
     std::memcpy(h_pack_ + o_idx, keys_indexs, 8 * nn);
     if (trie_ids) std::memcpy(h_pack_ + o_tid, trie_ids, 4 * nn);
     if ((e = cudaMemcpyAsync(d, h_pack_, in_bytes, cudaMemcpyHostToDevice, st_)) != cudaSuccess)
