@@ -187,29 +187,23 @@ def run_reference(args, world, rank):
     sys.path.insert(0, str(REPO / "oracle"))
     import oracle as O
 
+    if O.ref_lib(big=True) is None:  # nothing of this repository stands in for it
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's CPU MPT is not built (oracle/_ref is "
+                          "compiled from the reference's sources, which are not at hand)"}), flush=True)
+        return
     threads = os.cpu_count() or 1
     n = min(args.cpu_sample, args.n)
     batches = make_workload(args.n)
     sample = [b.subset(np.arange(n)) for b in batches]
-    kind = "reference" if O.ref_lib(big=True) is not None else "port"
     times = []
     for it in range(args.warmup + args.steps):
-        if kind == "reference":
-            t = O.RefTrie(big=True, threads=threads)
-            t0 = time.perf_counter()
-            for b in sample:
-                t.puts_lock_and_hash(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)
-            root = t.root(parallel=True)
-            dt = time.perf_counter() - t0
-            t.close()
-        else:
-            t = O.OracleTrie()
-            t0 = time.perf_counter()
-            for b in sample:
-                t.puts(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)
-                t.hash()
-            root = t.root()
-            dt = time.perf_counter() - t0
+        t = O.RefTrie(big=True, threads=threads)
+        t0 = time.perf_counter()
+        for b in sample:
+            t.puts_lock_and_hash(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)
+        root = t.root(parallel=True)
+        dt = time.perf_counter() - t0
+        t.close()
         if it >= args.warmup:
             times.append(dt)
     keys = 2 * n
@@ -221,8 +215,7 @@ def run_reference(args, world, rank):
         "vs_baseline": None, "dtype": "u8", "data": "synthetic",
         "config": {"workload": f"ycsb load {args.n} + zipf0.99 updates {args.n}, 23 B keys / 100 B values",
                    "sample_keys_per_batch": n},
-        "cpu_baseline": {"value": round(v, 4), "unit": "Mkeys/s", "cores": threads if kind == "reference" else 1,
-                         "kind": kind,
+        "cpu_baseline": {"value": round(v, 4), "unit": "Mkeys/s", "cores": threads, "kind": "reference",
                          "sample": f"first {n} keys of each batch (load, update); reference CpuMPT "
                                    "puts_lock + hashs_onepass on std::thread parallel_for"},
         "e2e": {"value": round(v, 4), "unit": "Mkeys/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
