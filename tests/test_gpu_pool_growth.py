@@ -1,4 +1,4 @@
-"""Growth of large node pools: past 4 GiB a pool has an allocation per array
+"""Growth of large node pools: past 8 GiB a pool has an allocation per array
 and grows array by array, so a branch pool of 84 GB can still grow to 120 on a
 device that could not hold both; tries keep their nodes through every form of
 a pool."""
@@ -24,7 +24,7 @@ def test_nodes_survive_every_form_of_the_pools(gpu_lib):
     bs = [W.random_keys(4000, 20, 30, seed=0x5EED1100 + k) for k in range(4)]
     t = gpu_lib.MPT()
     # branch pool: 120 bytes a node, short pool 64, records 24: one block, then arrays, then larger arrays
-    for b, nodes in zip(bs, (0, 4 << 20, 80 << 20, 120 << 20)):
+    for b, nodes in zip(bs, (0, 4 << 20, 80 << 20, 140 << 20)):
         if nodes:
             t.reserve_nodes(nodes, nodes, nodes, nodes, 1 << 20, 1 << 20)
         t.puts_latching_with_valuehp_v2(b.keys_hexs, b.keys_indexs, b.values, b.values_indexs)
