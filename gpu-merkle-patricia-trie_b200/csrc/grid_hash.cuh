@@ -15,9 +15,10 @@
 // No warp waits for another inside a phase; phases end at a grid barrier with
 // a bounded wait.
 //
-// Put + root of 16K zipf keys on a 1M-key trie 548 -> 491 us, 31 keys through
-// the host API 321 -> 278 us, an Ethereum block of 275 accounts (19K keys)
-// 626 -> 429 us, against launches (or grid barriers) per nibble depth.
+// A hash call of 7.7K dirty nodes of a 1M-key trie takes 141 us so, 178 as a
+// launch per nibble depth; of 3.8K nodes of random keys 109 and 180 (larger
+// lists at kGridHashMax); an Ethereum block of 275 accounts (19K keys), with a
+// grid barrier per depth instead, took 626 us, 429 so.
 #pragma once
 #include "trie_kernels.cuh"
 

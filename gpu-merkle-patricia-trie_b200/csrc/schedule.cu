@@ -25,8 +25,11 @@ const Schedule kSchedules[] = {
     {"locknu-4", false, false, 1, 1, 4, 1, 0, 4096},
     {"locknu-2", false, false, 1, 1, 2, 1, 0, 4096},
     {"locknu-1", false, false, 1, 1, 1, 1, 0, 4096},
+    // (the LockNU ways are an upper bound: up to 2^17 keys the three are one
+    // schedule, up to 2^23 the first two)
     // LockNU insert + PhaseHC + root read in one graph-replayed persistent
-    // launch, with all co-resident CTAs or one CTA per SM
+    // launch.  The kernel fits one CTA per SM, so the two grids are the same
+    // on a GPU of 148 SMs; both names stay for saved selectors.
     {"persistent-2cta", false, true, 1, 1, 4, 1, 0, 4096},
     {"persistent-1cta", false, true, 1, 1, 4, 1, 148, 4096},
     {"locknu-4-nodedup", false, false, 1, 1, 4, 0, 0, 4096},

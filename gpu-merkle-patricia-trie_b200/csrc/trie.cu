@@ -37,14 +37,33 @@ constexpr int kHashThreads = kHashLevelThreads;
 constexpr unsigned kWideGrid = 3 * 148;
 // branch hash class (blocks - 1) from which a branch is hashed by a warp
 constexpr uint32_t kWarpMinClass = 4;
-// up to this many leaves are hashed a warp each
+// Up to this many leaves are hashed a warp each in a pass by levels.  In a pass
+// of 200K nodes with values of 1000 bytes the warps save 20-30 of 1200 us up to
+// 2048 leaves, nothing at 4096, and cost 65 at 8192 and 180 at 16384; with
+// values of 60 bytes neither form shows below 8192 (490 us), then warps cost 18.
 constexpr uint32_t kWarpLeafMax = 2048;
 // host batches and lookups of at most this many bytes cross in one packed copy
 constexpr size_t kPackBytes = 256 << 10;
-// dirty lists of at most this many nodes are hashed by one cooperative launch
+// Dirty lists of at most this many nodes are hashed by one cooperative launch.
+// us of a hash call, so and by levels, updates of k keys on a 1M-key trie:
+//   YCSB keys    k = 1000 (7.7K nodes) 141, 178; 4000 (26K) 214, 243;
+//                16000 (85K) 263, 264; 24000 (118K) 288, 287;
+//                32000 (150K) 313, 296; 64000 (262K) 434, 342
+//   random keys  k = 1000 (3.8K) 109, 180; 4000 (14K) 178, 239; 24000 (65K)
+//                261, 270; 32000 (84K) 289, 283; 48000 (119K) 335, 310;
+//                64000 (151K) 384, 331
+// The two meet between 65K nodes (random) and 120K (YCSB).
 constexpr uint32_t kGridHashMax = 1u << 17;
-// larger lists whose branches (at most kGridDeepMax) are spread over at least
-// this many nibble depths have their branches hashed by one, after the leaves
+// Larger lists whose branches and extensions (at most kGridDeepMax) are spread
+// over at least this many nibble depths have them hashed by one, after the
+// leaves.  us of a hash call, so and by levels:
+//   24 depths (binary words)    199K listed 461, 506; 496K 684, 686; 985K
+//                               1019, 946; 1.9M 1682, 1415
+//   20 depths (ternary words)   147K 355, 421; 369K 559, 560; 738K 835, 814
+//   16 depths (quaternary)      124K 360, 414; 311K 573, 529
+//   vocabulary (8-96 bytes, values to 4 KB) 512K keys 6800, 7400 (put and
+//                               hash); 8M keys 32000, 25000
+// So the deeper the trie, the larger the list up to which it pays.
 constexpr int kGridLevels = 24;
 constexpr uint32_t kGridDeepMax = 1u << 20;
 // while the trie holds no value longer than this: a value is one serial chain
@@ -1287,8 +1306,7 @@ int Trie::hash_levels(const uint32_t *sorted, const std::vector<uint32_t> &off, 
   // many levels, each as long as its slowest branch: one cooperative launch
   // over all branches (the first wave holds the lowest branch of every path,
   // whatever its depth).  With more branches the levels fill the GPU and the
-  // level kernels' six CTAs an SM win: 8M word keys of 8-96 bytes take 32 ms
-  // of hashing this way, 25 ms by levels; 512K take 6.8 and 7.4 ms a pass.
+  // level kernels' six CTAs an SM win (figures at kGridLevels).
   const uint32_t a = off[level_bin(0)];
   const bool deep = coop && branch_levels >= kGridLevels && nd - a <= kGridDeepMax;
   coop = deep;

@@ -1751,8 +1751,8 @@ struct Bytes32 {
   uint64_t w[4];
 };
 
-// One lane's item of a message: at most 9 prefix bytes (pre, the header of a
-// string or a list; kept as 8 + the length) and a body that is in registers
+// One lane's item of a message: at most 8 prefix bytes in pre (a string's or a
+// list's header: 5 for a length of 32 bits), and a body that is in registers
 // when it has at most 32 bytes (a node's hash, a short value), else in memory.
 struct WarpItem {
   uint64_t pre = 0;

@@ -33,9 +33,12 @@ CONFIGS = [
     {"name": "locknu-4", "two_phase": False, "latch_ways": 4},
     {"name": "locknu-2", "two_phase": False, "latch_ways": 2},
     {"name": "locknu-1", "two_phase": False, "latch_ways": 1},
+    # (latch_ways is an upper bound: up to 2^17 keys the three LockNU entries
+    # are one schedule, up to 2^23 the first two)
     # LockNU insert + PhaseHC + root read in one graph-replayed persistent
-    # launch (gmpt_block_update with every key in stage 0), with two or one
-    # co-resident CTAs per SM (block_grid 0 = the device's maximum)
+    # launch (gmpt_block_update with every key in stage 0).  The kernel fits
+    # one CTA per SM, so block_grid 0 (all that fit) and 148 are the same on a
+    # B200; both names stay for saved selectors.
     {"name": "persistent-2cta", "two_phase": False, "persistent": True, "block_grid": 0},
     {"name": "persistent-1cta", "two_phase": False, "persistent": True, "block_grid": 148},
     # LockNU without the repeated-key drop (latch_dedup 0)
