@@ -36,8 +36,8 @@ from gmpt import workloads as W  # noqa: E402
 PEAKS_FILE = REPO / "MEASURED_PEAKS.json"
 # DRAM bytes per hashed node of k_hash_level: ncu dram__bytes_read.sum +
 # dram__bytes_write.sum over every k_hash_level launch of one 1M-key YCSB
-# load + update step (786.9 MB) over the 2,519,879 nodes it hashed
-HASH_TRAFFIC_B_PER_NODE = 312.3
+# load + update step (786.0 MB) over the 2,519,879 nodes it hashed
+HASH_TRAFFIC_B_PER_NODE = 311.9
 FALLBACK_HBM_GBS = 6650.0
 
 
@@ -494,7 +494,7 @@ def run_gets(t, d, n, dev, stream, hbm_peak):
     gbs = alg / (m / 1e3) / 1e9
     return {"keys": n, "found": found, "ms": round(m, 3), "mkeys_s": round(n / (m / 1e3) / 1e6, 2),
             "alg_bytes": int(alg), "achieved_gbs": round(gbs, 1), "frac": round(gbs / hbm_peak, 4),
-            "path": "gmpt_gets_device (keys copied next to a zero tail, k_gets, device results)"}
+            "path": "gmpt_gets_device (keys read where they lie, k_gets, device results)"}
 
 
 def run_vocab(args, local, dev, hbm_peak, perm_peak):
